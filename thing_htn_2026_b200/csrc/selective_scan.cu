@@ -56,6 +56,82 @@ __global__ void causal_conv_kernel(T* __restrict__ out, const T* __restrict__ pr
     out[e] = from_f32<T>(silu_of<T>(acc));
 }
 
+// The same for bfloat16 rows of 8-byte pieces and four taps: a thread takes four neighbouring channels of
+// kConvRows rows, with the raw inputs ahead of a row in registers, so that an input is loaded once for
+// its four uses.  2,048 rows of 4,096 channels on B200: 22 us against 78 with a thread per entry (2-byte
+// accesses, two divisions an entry); the inputs once and the outputs once take 5.  (Eight channels a
+// thread need 114 registers and leave too few warps to cover the loads: 29 us.)
+constexpr int kConvTaps = 4;
+constexpr int kConvRows = 8;
+
+__global__ void __launch_bounds__(128) causal_conv_vec_kernel(
+    __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ proj, int proj_width, int offset,
+    const float* __restrict__ weight, const float* __restrict__ bias, const __nv_bfloat16* __restrict__ ring,
+    const int* __restrict__ row_slot, const int* __restrict__ row_pos, const int* __restrict__ seq_lens, int n_rows,
+    int channels) {
+    pdl_launch_dependents();
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    const int first = blockIdx.y * kConvRows, n_here = min(kConvRows, n_rows - first);
+    if (c >= channels) return;
+    float w[4][kConvTaps], b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float4 v = *reinterpret_cast<const float4*>(weight + (size_t)(c + i) * kConvTaps);
+        w[i][0] = v.x; w[i][1] = v.y; w[i][2] = v.z; w[i][3] = v.w;
+        b[i] = bias ? bias[c + i] : 0.f;
+    }
+    pdl_wait();
+    const __nv_bfloat16* src = proj + (size_t)first * proj_width + offset + c;
+    // raw[j]: the row j - 3 rows after `first`
+    uint2 raw[kConvRows + kConvTaps - 1];
+#pragma unroll
+    for (int j = 0; j < kConvRows + kConvTaps - 1; ++j) {
+        const int back = kConvTaps - 1 - j;
+        raw[j] = back <= first && -back < n_here ? *reinterpret_cast<const uint2*>(src - (long long)back * proj_width)
+                                                 : make_uint2(0, 0);
+    }
+    int slot[kConvRows], pos[kConvRows], local[kConvRows];
+#pragma unroll
+    for (int t = 0; t < kConvRows; ++t) {
+        const int row = first + min(t, n_here - 1);
+        slot[t] = row_slot[row];
+        pos[t] = row_pos[row];
+    }
+#pragma unroll
+    for (int t = 0; t < kConvRows; ++t) local[t] = pos[t] - seq_lens[slot[t]];   // its index among its sequence's rows of this step
+    __nv_bfloat16* dst = out + (size_t)first * channels + c;
+#pragma unroll
+    for (int t = 0; t < kConvRows; ++t) {
+        if (t >= n_here) break;
+        uint2 in[kConvTaps];
+#pragma unroll
+        for (int j = 0; j < kConvTaps; ++j) in[j] = raw[t + j];
+        if (local[t] < kConvTaps - 1) {
+#pragma unroll
+            for (int back = 1; back < kConvTaps; ++back) {
+                if (back <= local[t]) continue;
+                in[kConvTaps - 1 - back] = back > pos[t] ? make_uint2(0, 0)          // before the sequence's start
+                    : *reinterpret_cast<const uint2*>(ring + ((size_t)slot[t] * kConvTaps + (pos[t] - back) % kConvTaps) * channels + c);
+            }
+        }
+        float acc[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) acc[i] = b[i];
+#pragma unroll
+        for (int j = 0; j < kConvTaps; ++j) {
+            if (kConvTaps - 1 - j > pos[t]) continue;
+            acc[0] += w[0][j] * __uint_as_float(in[j].x << 16);
+            acc[1] += w[1][j] * __uint_as_float(in[j].x & 0xffff0000u);
+            acc[2] += w[2][j] * __uint_as_float(in[j].y << 16);
+            acc[3] += w[3][j] * __uint_as_float(in[j].y & 0xffff0000u);
+        }
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(silu_of<__nv_bfloat16>(acc[0]), silu_of<__nv_bfloat16>(acc[1]));
+        const __nv_bfloat162 hi = __floats2bfloat162_rn(silu_of<__nv_bfloat16>(acc[2]), silu_of<__nv_bfloat16>(acc[3]));
+        *reinterpret_cast<uint2*>(dst + (size_t)t * channels) =
+            make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+    }
+}
+
 template <typename T>
 __global__ void conv_ring_update_kernel(T* __restrict__ ring, const T* __restrict__ proj, int proj_width, int offset,
                                         const int* __restrict__ cu_seqlens, const int* __restrict__ slots,
@@ -242,6 +318,222 @@ __global__ void __launch_bounds__(kScanThreads) selective_scan_kernel(
     }
 }
 
+// ---------------------------------------------------------------- several tokens, bfloat16, states up to 32
+//
+// What a token costs a channel beside its state (loads, the softplus of the step size, the silu of the gate,
+// the write) is more work than the state itself, and none of it waits for the token before.  So four warps
+// of a block walk the state and nothing else, and four others run ahead of and behind them: they load a
+// stage of tokens, leave (step size, step size * input) and B, C in shared memory a stage ahead, and add up,
+// gate and write the read-outs of the stage before.  LANES lanes hold a channel's state, PER neighbouring
+// entries each, in pairs for the two-wide multiply-add; a lane leaves its share of a token's sum in shared
+// memory for the other warps to add.  One barrier per stage, two buffers of everything.
+// What bounds it is instruction issue (58 million warp instructions for 2,048 tokens of 4,096 channels, 16
+// entries; half of them the loads, softplus and silu) with few warps to cover latencies.  B200, against the
+// kernel above, us: one prompt of 2,048 tokens, 4,096 channels 140 / 763, 8,192 channels 201 / 770; 8 x 512
+// tokens of 4,096 162 / 447; 100 tokens 14 / 46.  (One set of warps for everything took 211 for the first; cutting
+// the tokens into segments that run side by side, twice, 134, but 230 for 8 x 512: it doubles the exponentials.)
+constexpr int kWalkThreads = 128;          // threads of each of the two halves of a block
+constexpr int kWalkStage = 16;
+
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long v;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long v;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+    return v;
+}
+// the hardware's base-2 exponential (as Decay above; what would be below 2^-126 is zero)
+__device__ __forceinline__ float decay_exp2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+
+template <int LANES, int PER>
+__global__ void __launch_bounds__(2 * kWalkThreads) selective_scan_walk_kernel(
+    __nv_bfloat16* __restrict__ y, float* __restrict__ state, const __nv_bfloat16* __restrict__ x,
+    const float* __restrict__ dt_pre, const float* __restrict__ dt_bias, const __nv_bfloat16* __restrict__ bc, int bc_width,
+    const float* __restrict__ A, const float* __restrict__ D, const __nv_bfloat16* __restrict__ z, int z_stride,
+    const int* __restrict__ cu_seqlens, const int* __restrict__ slots, int channels, int n_state) {
+    pdl_launch_dependents();
+    pdl_wait();
+    using T = __nv_bfloat16;
+    constexpr int N = LANES * PER, ST = kWalkStage, PAIRS = PER / 2, CH = kWalkThreads / LANES;
+    using ull = unsigned long long;
+    // a staged token: per lane its entries of B, then of C; per channel the step size twice, then its product with the input twice
+    __shared__ __align__(16) float bc_mem[2][ST][2 * N];
+    __shared__ __align__(16) float4 step_mem[2][ST][CH];
+    __shared__ __align__(16) float share_mem[2][ST][CH * LANES];
+    const int seq = blockIdx.y;
+    const int row0 = cu_seqlens[seq], n_tokens = cu_seqlens[seq + 1] - row0;
+    if (n_tokens <= 0) return;
+    const int n_stages = (n_tokens + ST - 1) / ST;
+    const int c0 = blockIdx.x * CH;
+
+    if (threadIdx.x < kWalkThreads) {
+        const int lane = threadIdx.x % LANES, group = threadIdx.x / LANES;
+        const bool live = c0 + group < channels;
+        const int c = live ? c0 + group : channels - 1;
+        float* S = state + ((size_t)slots[seq] * channels + c) * n_state;
+        ull s[PAIRS], a[PAIRS];
+#pragma unroll
+        for (int i = 0; i < PAIRS; ++i) {
+            const int n = lane * PER + 2 * i;
+            s[i] = pack2(n < n_state ? S[n] : 0.f, n + 1 < n_state ? S[n + 1] : 0.f);
+            a[i] = pack2(n < n_state ? A[(size_t)c * n_state + n] * 1.4426950408889634f : 0.f,
+                         n + 1 < n_state ? A[(size_t)c * n_state + n + 1] * 1.4426950408889634f : 0.f);
+        }
+        __syncthreads();                       // the first stage is in place
+        for (int stage = 0; stage < n_stages; ++stage) {
+            const int buf = stage & 1;
+            // (tokens beyond the step's have a step size of zero and leave the state as it is)
+#pragma unroll
+            for (int t = 0; t < ST; ++t) {
+                const ulonglong2 step = *reinterpret_cast<const ulonglong2*>(&step_mem[buf][t][group]);
+                const ull* b = reinterpret_cast<const ull*>(bc_mem[buf][t] + lane * 2 * PER);
+                ull sum = 0;
+#pragma unroll
+                for (int i = 0; i < PAIRS; ++i) {
+                    float e0, e1;
+                    unpack2(mul2(step.x, a[i]), e0, e1);
+                    s[i] = fma2(pack2(decay_exp2(e0), decay_exp2(e1)), s[i], mul2(step.y, b[i]));
+                    sum = i == 0 ? mul2(s[i], b[PAIRS + i]) : fma2(s[i], b[PAIRS + i], sum);
+                }
+                float s0, s1;
+                unpack2(sum, s0, s1);
+                share_mem[buf][t][threadIdx.x] = s0 + s1;
+            }
+            __syncthreads();
+        }
+        if (!live) return;
+#pragma unroll
+        for (int i = 0; i < PAIRS; ++i) {
+            const int n = lane * PER + 2 * i;
+            float s0, s1;
+            unpack2(s[i], s0, s1);
+            if (n < n_state) S[n] = s0;
+            if (n + 1 < n_state) S[n + 1] = s1;
+        }
+        return;
+    }
+
+    // the other half: a thread serves one channel and every (kWalkThreads / CH)-th token of a stage
+    const int tid = threadIdx.x - kWalkThreads;
+    constexpr int STRIDE = kWalkThreads / CH, OWN = ST / STRIDE;
+    const int group = tid % CH, t0 = tid / CH;
+    const bool live = c0 + group < channels;
+    const int c = live ? c0 + group : channels - 1;
+    const float skip = D[c], bias = dt_bias[c];
+    constexpr int kShare = ST * 2 * N / kWalkThreads, kShareStep = kWalkThreads / (2 * N);
+    static_assert(ST * 2 * N % kWalkThreads == 0 && kWalkThreads % (2 * N) == 0 && ST % STRIDE == 0, "whole shares");
+    // this thread's column of the staged B and C: lane, B or C, entry
+    const int share_col = tid % (2 * N), share_t = tid / (2 * N);
+    const int share_n = share_col / (2 * PER) * PER + share_col % PER, share_which = share_col % (2 * PER) / PER;
+    const bool share_in = share_n < n_state;
+    const T* bc_src = bc + (size_t)(row0 + share_t) * bc_width + share_which * n_state + (share_in ? share_n : 0);
+    const size_t first_row = row0 + t0, own_step = (size_t)STRIDE * channels, z_step = (size_t)STRIDE * z_stride;
+    const float* dt_src = dt_pre + first_row * channels + c;
+    const T* x_src = x + first_row * channels + c;
+    const T* z_src = z + first_row * z_stride + c;
+    T* y_dst = y + first_row * channels + c;
+    uint32_t bc_raw[kShare] = {}, x_raw[OWN] = {}, z_raw[OWN] = {};
+    float dt_raw[OWN] = {};
+    float skipped[2][OWN], gate[2][OWN];
+    auto fetch = [&](int stage) {
+        const int left = n_tokens - stage * ST;
+#pragma unroll
+        for (int j = 0; j < kShare; ++j)
+            if (share_in && share_t + j * kShareStep < left) bc_raw[j] = raw_load<T>(bc_src + (size_t)(j * kShareStep) * bc_width);
+        bc_src += (size_t)ST * bc_width;
+#pragma unroll
+        for (int j = 0; j < OWN; ++j)
+            if (t0 + j * STRIDE < left) {
+                dt_raw[j] = dt_src[j * own_step];
+                x_raw[j] = raw_load<T>(x_src + j * own_step);
+                z_raw[j] = raw_load<T>(z_src + j * z_step);
+            }
+        dt_src += OWN * own_step;
+        x_src += OWN * own_step;
+        z_src += OWN * z_step;
+    };
+    auto transform = [&](int stage, int buf, float (&skipped_)[OWN], float (&gate_)[OWN]) {
+        const int left = n_tokens - stage * ST;
+#pragma unroll
+        for (int j = 0; j < kShare; ++j) (&bc_mem[buf][0][0])[tid + j * kWalkThreads] = from_raw<T>(bc_raw[j]);
+#pragma unroll
+        for (int j = 0; j < OWN; ++j) {
+            const float d = t0 + j * STRIDE < left ? softplus_of<T>(dt_raw[j] + bias) : 0.f;
+            const float in = from_raw<T>(x_raw[j]), din = d * in;
+            step_mem[buf][t0 + j * STRIDE][group] = make_float4(d, d, din, din);
+            skipped_[j] = skip * in;
+            gate_[j] = silu_of<T>(from_raw<T>(z_raw[j]));
+        }
+    };
+    auto finish = [&](int stage, int buf, const float (&skipped_)[OWN], const float (&gate_)[OWN]) {
+        const int left = n_tokens - stage * ST;
+#pragma unroll
+        for (int j = 0; j < OWN; ++j) {
+            const float4* share = reinterpret_cast<const float4*>(&share_mem[buf][t0 + j * STRIDE][group * LANES]);
+            float sum = 0.f;
+#pragma unroll
+            for (int l = 0; l < LANES / 4; ++l) {
+                const float4 v = share[l];
+                sum += (v.x + v.y) + (v.z + v.w);
+            }
+            if (live && t0 + j * STRIDE < left) y_dst[j * own_step] = from_f32<T>((sum + skipped_[j]) * gate_[j]);
+        }
+        y_dst += OWN * own_step;
+    };
+    // (two stages a turn, so that the buffers' numbers are constants)
+    fetch(0);
+    transform(0, 0, skipped[0], gate[0]);
+    if (1 < n_stages) fetch(1);
+    __syncthreads();
+    for (int stage = 0; stage < n_stages; stage += 2) {
+        // the walk is at `stage`: read out the one before, prepare the one after
+        if (stage > 0) finish(stage - 1, 1, skipped[1], gate[1]);
+        if (stage + 1 < n_stages) transform(stage + 1, 1, skipped[1], gate[1]);
+        if (stage + 2 < n_stages) fetch(stage + 2);
+        __syncthreads();
+        if (stage + 1 >= n_stages) break;
+        finish(stage, 0, skipped[0], gate[0]);
+        if (stage + 2 < n_stages) transform(stage + 2, 0, skipped[0], gate[0]);
+        if (stage + 3 < n_stages) fetch(stage + 3);
+        __syncthreads();
+    }
+    if (n_stages & 1) finish(n_stages - 1, 0, skipped[0], gate[0]);
+    else finish(n_stages - 1, 1, skipped[1], gate[1]);
+}
+
+int launch_walk(void* y, float* state, const void* x, const float* dt_pre, const float* dt_bias, const void* bc, int bc_width,
+                const float* A, const float* D, const void* z, int z_stride, const int* cu_seqlens, const int* slots, int n_seqs,
+                int channels, int n_state, cudaStream_t stream) {
+    using T = __nv_bfloat16;
+#define THN_WALK_LAUNCH(L, P)                                                                                               \
+    thn_launch_ordered(selective_scan_walk_kernel<L, P>, dim3((channels + kWalkThreads / L - 1) / (kWalkThreads / L), n_seqs), \
+                       2 * kWalkThreads, 0, stream, (T*)y, state, (const T*)x, dt_pre, dt_bias, (const T*)bc, bc_width, A, D, \
+                       (const T*)z, z_stride, cu_seqlens, slots, channels, n_state)
+    // Eight lanes a channel put twice as many warps on the chip and issue more for the same sums: they win while the
+    // blocks of four lanes (32 channels) do not fill it once.  us with 8 / 4 lanes: one prompt of 2,048 tokens, 4,096
+    // channels 140 / 181, 8,192 channels 284 / 201; 2 x 700 tokens of 4,096 channels 104 / 76; 8 x 512 200 / 162.
+    const bool few = (long long)channels * n_seqs <= 148ll * 32;
+    if (n_state <= 8) THN_WALK_LAUNCH(4, 2);
+    else if (n_state <= 16 && few) THN_WALK_LAUNCH(8, 2);
+    else if (n_state <= 16) THN_WALK_LAUNCH(4, 4);
+    else THN_WALK_LAUNCH(8, 4);
+#undef THN_WALK_LAUNCH
+    return thn_launch_status("selective_scan");
+}
+
 template <typename T>
 int launch_scan(void* y, float* state, const void* x, const float* dt_pre, const float* dt_bias, const void* bc,
                 int bc_width, const float* A, const float* D, const void* z, int z_stride, const int* cu_seqlens,
@@ -275,7 +567,13 @@ THN_API int thn_causal_conv(void* out, const void* proj, int proj_width, int off
     const long long n = (long long)n_rows * channels;
     if (n == 0) return THN_OK;
     const unsigned blocks = (unsigned)((n + 255) / 256);
-    if (dtype == THN_F32)
+    const bool pieces = channels % 4 == 0 && offset % 4 == 0 && proj_width % 4 == 0 &&
+                        (((uintptr_t)out | (uintptr_t)proj | (uintptr_t)ring) & 7) == 0 && ((uintptr_t)weight & 15) == 0;
+    if (dtype == THN_BF16 && taps == kConvTaps && pieces && (n_rows + kConvRows - 1) / kConvRows <= 65535)
+        thn_launch(causal_conv_vec_kernel, dim3((unsigned)((channels / 4 + 127) / 128), (unsigned)((n_rows + kConvRows - 1) / kConvRows)),
+                   128, 0, stream, (__nv_bfloat16*)out, (const __nv_bfloat16*)proj, proj_width, offset, weight, bias,
+                   (const __nv_bfloat16*)ring, row_slot, row_pos, seq_lens, n_rows, channels);
+    else if (dtype == THN_F32)
         thn_launch(causal_conv_kernel<float>, blocks, 256, 0, stream, (float*)out, (const float*)proj, proj_width, offset,
                    weight, bias, (const float*)ring, row_slot, row_pos, seq_lens, n, channels, taps);
     else if (dtype == THN_BF16)
@@ -313,7 +611,7 @@ THN_API int thn_conv_ring_update(void* ring, const void* proj, int proj_width, i
 // (negative); D float32 [channels]; z of the activation type, rows z_stride apart.
 THN_API int thn_selective_scan(void* y, float* state, const void* x, const float* dt_pre, const float* dt_bias,
                                const void* bc, int bc_width, const float* A, const float* D, const void* z, int z_stride,
-                               const int* cu_seqlens, const int* slots, int n_seqs, int channels, int n_state, int dtype,
+                               const int* cu_seqlens, const int* slots, int n_rows, int n_seqs, int channels, int n_state, int dtype,
                                cudaStream_t stream) {
     THN_CHECK_ARG(n_seqs >= 0 && channels > 0 && n_state > 0 && bc_width >= 2 * n_state && z_stride >= channels,
                   "selective_scan: bad sizes");
@@ -323,6 +621,10 @@ THN_API int thn_selective_scan(void* y, float* state, const void* x, const float
     if (dtype == THN_F32)
         return launch_scan<float>(y, state, x, dt_pre, dt_bias, bc, bc_width, A, D, z, z_stride, cu_seqlens, slots, n_seqs,
                                   channels, n_state, stream);
+    // (steps of one token per sequence move a state and nothing else: the kernel above reads it without a stage)
+    if (dtype == THN_BF16 && n_state <= 32 && n_rows > n_seqs)
+        return launch_walk(y, state, x, dt_pre, dt_bias, bc, bc_width, A, D, z, z_stride, cu_seqlens, slots, n_seqs, channels,
+                           n_state, stream);
     if (dtype == THN_BF16)
         return launch_scan<__nv_bfloat16>(y, state, x, dt_pre, dt_bias, bc, bc_width, A, D, z, z_stride, cu_seqlens, slots,
                                           n_seqs, channels, n_state, stream);
