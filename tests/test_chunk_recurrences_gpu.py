@@ -1,0 +1,72 @@
+"""Recurrences that are walked in chunks of 32 tokens on the tensor cores, against the same token by token
+in 64 bits: lengths at the edges of chunks, a prompt that goes on from a state, values at the edges of a
+block's columns."""
+
+import pytest
+import torch
+
+from thing_htn_2026_b200 import ops
+
+pytestmark = pytest.mark.gpu
+BF16 = torch.bfloat16
+
+
+def step(lens, held=0):
+    dev = torch.device("cuda", 0)
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    seq_lens = torch.full((len(lens) + 1,), held, dtype=torch.int32, device=dev)
+    slots = torch.arange(len(lens), 0, -1, dtype=torch.int32, device=dev)      # sequence i in slot len - i
+    rows = ops.step_rows(torch.tensor(cu, dtype=torch.int32, device=dev), slots, seq_lens, cu[-1], max(lens))
+    return rows, seq_lens, cu, slots.cpu().tolist()
+
+
+def close(got, want, tokens):
+    """float32 sums of a few dozen products per token and a state that is rounded once per token or chunk:
+    2^-20 of the result's size, and a token's roundings add up at most linearly."""
+    scale = want.abs().amax()
+    assert torch.isfinite(got).all()
+    assert (got.double() - want).abs().max() <= (8 + tokens / 8) * 2 ** -23 * scale
+
+
+@pytest.mark.parametrize("lens,held,n_heads,n_kv,vdim", [
+    ([16], 0, 2, 1, 128), ([31, 1, 33], 0, 4, 2, 16), ([32, 64, 65, 2], 0, 2, 2, 48), ([100], 7, 4, 1, 128),
+    ([40, 17], 1, 2, 1, 256), ([70] * 8, 0, 16, 4, 64), ([35] * 5, 2, 16, 4, 96), ([20, 97], 64, 2, 2, 160)])
+def test_delta_matches_64_bits(lens, held, n_heads, n_kv, vdim):
+    g = torch.Generator().manual_seed(sum(lens) + vdim)
+    rows, seq_lens, cu, slots = step(lens, held)
+    dev, key, taps, eps = rows.slots.device, 128, 4, 1e-6
+    shape = ops.DeltaShape(n_heads, n_kv, key, vdim, taps)
+    draw = lambda *s: torch.randn(*s, generator=g)
+    proj, w = draw(cu[-1], shape.proj_width).to(BF16), draw(shape.conv_channels, taps) * 0.5
+    a_log, dt_bias = torch.rand(n_heads, generator=g) * 4 - 2, draw(n_heads)
+    state, ring = draw(len(lens) + 1, n_heads, vdim, key) * 0.2, draw(len(lens) + 1, taps, shape.conv_channels).to(BF16)
+    got_state, got_ring = state.to(dev), ring.to(dev)
+    assert ops._delta_in_chunks(proj.to(dev), w.to(dev), got_state, got_ring, rows, shape)
+    got = ops.delta_rule(proj.to(dev), w.to(dev), a_log.to(dev), dt_bias.to(dev), got_state, got_ring, rows, seq_lens, shape, eps)
+    want, want_state = torch.zeros(cu[-1], n_heads, vdim, dtype=torch.float64), state.double()
+    qk, gate_end = n_kv * key, shape.gate_offset + n_heads * vdim
+    for i, slot in enumerate(slots):
+        S = want_state[slot]
+        for r in range(cu[i], cu[i + 1]):
+            pos, acc = held + r - cu[i], torch.zeros(shape.conv_channels, dtype=torch.float64)
+            for back in range(min(taps - 1, pos) + 1):
+                raw = proj[r - back, :shape.conv_channels] if back <= r - cu[i] else ring[slot, (pos - back) % taps]
+                acc += w[:, taps - 1 - back].double() * raw.double()
+            y = torch.nn.functional.silu(acc)
+            q, k = y[:qk].view(n_kv, key), y[qk:2 * qk].view(n_kv, key)
+            q = (q / torch.sqrt((q * q).sum(-1, keepdim=True) + eps) * key ** -0.5).repeat_interleave(n_heads // n_kv, 0)
+            k = (k / torch.sqrt((k * k).sum(-1, keepdim=True) + eps)).repeat_interleave(n_heads // n_kv, 0)
+            b = torch.sigmoid(proj[r, gate_end:gate_end + n_heads].double())
+            step_size = torch.nn.functional.softplus(proj[r, gate_end + n_heads:gate_end + 2 * n_heads].double() + dt_bias.double())
+            S = torch.exp(-torch.exp(a_log.double()) * step_size)[:, None, None] * S
+            u = b[:, None] * (y[2 * qk:].view(n_heads, vdim) - torch.einsum("hek,hk->he", S, k))
+            S = S + u[:, :, None] * k[:, None, :]
+            want[r] = torch.einsum("hek,hk->he", S, q)
+        want_state[slot] = S
+    close(got.cpu(), want, max(lens))
+    close(got_state.cpu(), want_state, max(lens))
+    for i, slot in enumerate(slots):
+        for r in range(max(cu[i], cu[i + 1] - (taps - 1)), cu[i + 1]):
+            assert torch.equal(got_ring[slot, (held + r - cu[i]) % taps].cpu(), proj[r, :shape.conv_channels])

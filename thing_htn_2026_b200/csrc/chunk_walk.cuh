@@ -1,0 +1,587 @@
+// Recurrences over a matrix state S [128 keys, values] whose decay is one number per head and token,
+// walked a chunk of 32 tokens at a time, for prompts with bfloat16 activations.  Token by token such a
+// kernel is a chain of thousands of dependent steps.  Inside a chunk the sums can be taken in any order:
+//
+//     o_i  = alpha_i S0^T q_i + beta_i sum_{j <= i} G_ij v_j
+//     S    = alpha_last S0 + beta_last sum_j w_j k_j v_j^T
+//
+// with S0 the state ahead of the chunk.  A kernel of the mixer works out, for all chunks at once, G (the
+// products q_i . k_j with the decays between the two tokens, zero for j > i) and the numbers per token;
+// what is left to walk is three products per chunk.  The delta rule's values are v = u - W S0 with rows u
+// and W that its kernel has worked out too.  The gated matrix memory keeps the logarithms' running maximum
+// m, a number that only the walk knows: alpha and beta come from it, and a vector n beside S.
+//
+// The products run on the tensor cores in bfloat16 with operands split into three parts, x = h + m + l exactly (24
+// bits), and the six products of parts that reach 2^-24: h h; and, in an accumulator of their own, h m, m h, m m,
+// h l, l h (operands that come in bfloat16 are exact in one part, and the products fewer).  The tensor core's
+// accumulation rounds towards zero, so every step of 16 along the sum's axis has a fresh accumulator and
+// the steps meet in float32 additions.  (tf32 in two parts costs the same and is off by 2.4e-7 where the
+// token-by-token delta rule is off by 1.3e-7 and this by 1.4e-7.)  The mixer's kernels leave their operands split, as
+// planes of bfloat16 in rows that ldmatrix reads without bank conflicts: split in the walk they were half
+// of its instructions (177 us for 2,048 tokens of 16 heads of the delta rule, 157 with planes).
+//
+// A block walks one sequence, head and 16 CG columns of values.  S^T lives in the accumulator registers of
+// its warps: warp (cg, ks) holds 16 columns and 128 / KS keys; the accumulator layout of two groups of eight
+// keys is the A operand's layout, so S never moves.  With KS > 1 the warps' shares of W S0 and S0^T q meet in
+// shared memory, each warp then finishes some of the tokens.  The next chunk's operands travel by
+// asynchronous copies into the other of STAGES buffers (with one buffer, other blocks of the
+// multiprocessor cover the wait); rows beyond the sequence's are filled with zeros.
+#pragma once
+
+#include "common.cuh"
+
+namespace chunk {
+
+constexpr int kTokens = 32;           // tokens per chunk
+constexpr int kKeys = 128;
+// rows of the planes, in bfloat16: eight rows of 16 bytes lie on distinct banks
+constexpr int kKeyRow = kKeys + 8, kScoreRow = kTokens + 8;
+
+struct WalkArgs {
+    float* o;                  // [rows, heads, value_dim]
+    float* state;              // [slots, heads, value_dim, kKeys], read and updated
+    // planes of bfloat16 (three, or one where q, k and v are bfloat16): plane p, unit u, row m from
+    // q + p * key_plane + u * key_unit + m * key_row (elements); k likewise
+    const __nv_bfloat16* q;
+    const __nv_bfloat16* k;
+    long long key_plane, key_unit, key_row;
+    const void* v;             // float32 or bfloat16; row m, head h: v + m * v_row + h * v_head
+    long long v_row, v_head;
+    const __nv_bfloat16* w;    // delta: [heads][3][rows][kKeyRow]
+    const __nv_bfloat16* scores;   // G: [heads][3][rows][kScoreRow]
+    const float4* scalars;     // [heads][rows]: (alpha, -, w, -); gated: (sum of log f, maximum, w, sum of the row of G)
+    const int* cu_seqlens;
+    const int* slots;
+    int n_rows, n_heads, heads_per_unit, value_dim;
+    float scale;               // on every read-out
+    // the gated matrix memory
+    float* normaliser;         // [slots, heads, value_dim / 16, kKeys + 1]: copies of n, then m
+    const float* key_sums;     // [sequences, chunks, heads, kKeys]: sum_j w_j k_j of every chunk
+    int max_chunks;
+    float floor_;
+};
+
+__device__ __forceinline__ void copy16(void* smem, const void* gmem, bool there) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem),
+                 "r"(there ? 16 : 0));
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void copy_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+
+// kTokens rows of ROW elements that lie one behind the other, to shared memory as they are; zeros beyond
+// `there` rows (the addresses of those are not read).
+template <int ROW, int THREADS>
+__device__ __forceinline__ void copy_rows(__nv_bfloat16* smem, const __nv_bfloat16* gmem, int there) {
+    static_assert(ROW % 8 == 0, "whole pieces");
+    constexpr int kPieces = kTokens * ROW / 8;
+    const int end = there * (ROW / 8);
+#pragma unroll
+    for (int e = 0; e < kPieces; e += THREADS) {
+        const int i = e + (int)threadIdx.x;
+        if (kPieces % THREADS == 0 || i < kPieces) copy16(smem + i * 8, gmem + (i < end ? i * 8 : 0), i < end);
+    }
+}
+
+__device__ __forceinline__ uint32_t pack_bf16(float x, float y) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ float low_half(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float high_half(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+// two floats in three parts each: part[0] + part[1] + part[2], exactly
+struct Split {
+    uint32_t part[3];
+};
+__device__ __forceinline__ Split split(float x, float y) {
+    Split s;
+    s.part[0] = pack_bf16(x, y);
+    x -= low_half(s.part[0]);
+    y -= high_half(s.part[0]);
+    s.part[1] = pack_bf16(x, y);
+    x -= low_half(s.part[1]);
+    y -= high_half(s.part[1]);
+    s.part[2] = pack_bf16(x, y);
+    return s;
+}
+__device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// four 8 x 8 matrices of bfloat16; lane l gives the address of row l % 8 of matrix l / 8
+__device__ __forceinline__ void load_matrices(uint32_t (&r)[4], const __nv_bfloat16* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+}
+__device__ __forceinline__ void load_matrices_transposed(uint32_t (&r)[4], const __nv_bfloat16* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+}
+// Where a lane's address lies inside a 16 x 16 tile of rows of `row` elements:
+// an A operand [m][k], or B operands of two neighbouring groups of n stored [k][n] (loaded transposed)
+__device__ __forceinline__ int a_tile(int lane, int row) { return ((lane & 7) + (lane >> 3 & 1) * 8) * row + (lane >> 4) * 8; }
+// B operands of two neighbouring groups of n stored [n][k], or an A operand stored [k][m] (loaded transposed)
+__device__ __forceinline__ int b_tile(int lane, int row) { return ((lane & 7) + (lane >> 4) * 8) * row + (lane >> 3 & 1) * 8; }
+
+// The A operand of a step of 16 along the sum's axis, in parts.
+struct Parts {
+    uint32_t part[3][4];
+};
+// from rows g and g + 8 at k = 2t, 2t + 1 and at k = 2t + 8, 2t + 9
+__device__ __forceinline__ Parts parts_of(float2 g_lo, float2 g8_lo, float2 g_hi, float2 g8_hi) {
+    Parts p;
+    const Split s[4] = {split(g_lo.x, g_lo.y), split(g8_lo.x, g8_lo.y), split(g_hi.x, g_hi.y), split(g8_hi.x, g8_hi.y)};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) p.part[j][i] = s[i].part[j];
+    return p;
+}
+// The B operands of two neighbouring groups of eight columns, in parts: part[p][2 n + half of k]
+template <int PARTS>
+struct Columns {
+    uint32_t part[PARTS][4];
+};
+template <int PARTS>
+__device__ __forceinline__ Columns<PARTS> columns_of(const __nv_bfloat16* p, int plane) {
+    Columns<PARTS> c;
+#pragma unroll
+    for (int i = 0; i < PARTS; ++i) load_matrices(c.part[i], p + i * plane);
+    return c;
+}
+template <int PARTS>
+__device__ __forceinline__ Columns<PARTS> columns_transposed(const __nv_bfloat16* p, int plane) {
+    Columns<PARTS> c;
+#pragma unroll
+    for (int i = 0; i < PARTS; ++i) load_matrices_transposed(c.part[i], p + i * plane);
+    return c;
+}
+// large += h h, small += the other products, over PAIRS pairs of groups of columns: product by product, so that
+// neighbouring instructions have accumulators of their own.  A_PARTS 1: A is exact in one part.
+template <int A_PARTS = 3, int PARTS, int PAIRS>
+__device__ __forceinline__ void multiply(float (&large)[2 * PAIRS][4], float (&small)[2 * PAIRS][4], const Parts& a,
+                                         const Columns<PARTS> (&b)[PAIRS]) {
+    auto all = [&](float (&d)[2 * PAIRS][4], int x, int y) {
+#pragma unroll
+        for (int n = 0; n < 2 * PAIRS; ++n) mma(d[n], a.part[x], b[n / 2].part[y % PARTS][2 * (n & 1)], b[n / 2].part[y % PARTS][2 * (n & 1) + 1]);
+    };
+    if (A_PARTS == 3) all(small, 2, 0);
+    if (PARTS == 3) all(small, 0, 2);
+    if (A_PARTS == 3 && PARTS == 3) all(small, 1, 1);
+    all(large, 0, 0);
+    if (A_PARTS == 3) all(small, 1, 0);
+    if (PARTS == 3) all(small, 0, 1);
+}
+// One step's sum.  The accumulation rounds towards zero; kLean of the result is put back in the finer units of
+// the small products (the factor of least error: 0 and 4.3e-8 are both worse by a tenth).
+constexpr float kLean = 2.2e-8f;
+__device__ __forceinline__ float joined(float large, float small) { return large + fmaf(large, kLean, small); }
+template <int N>
+__device__ __forceinline__ void clear(float (&d)[N][4]) {
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) d[n][i] = 0.f;
+}
+__device__ __forceinline__ float2 pair_of(const float* p) { return *reinterpret_cast<const float2*>(p); }
+__device__ __forceinline__ float2 pair_of(const __nv_bfloat16* p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); }
+
+template <typename T, int CG, int KS, bool DELTA, int STAGES>
+struct Layout {
+    static constexpr int kParts = sizeof(T) == 2 ? 1 : 3;
+    static constexpr int kThreads = 32 * CG * KS, kColumns = 16 * CG;
+    static constexpr int kValueRow = kColumns + (sizeof(T) == 2 ? 8 : 4);
+    static constexpr int kKeyPlane = kTokens * kKeyRow, kScorePlane = kTokens * kScoreRow;      // elements
+    static constexpr int kQ = 0;
+    static constexpr int kK = kQ + kParts * kKeyPlane * 2;
+    static constexpr int kW = kK + kParts * kKeyPlane * 2;
+    static constexpr int kG = kW + (DELTA ? 3 * kKeyPlane * 2 : 0);
+    static constexpr int kV = kG + 3 * kScorePlane * 2;
+    static constexpr int kScalars = kV + kTokens * kValueRow * (int)sizeof(T);
+    static constexpr int kStage = kScalars + kTokens * 16;
+    static constexpr int kShares = KS > 1 ? KS * CG * (DELTA ? 2 : 1) * 4 * 32 * 16 : 0;    // [ks][cg][which][8 tokens][lane] float4
+    static constexpr int kBytes = STAGES * kStage + kShares + (kTokens * 3 + kKeys) * 4;
+};
+
+template <typename T, int CG, int KS, bool DELTA, bool GATED, int STAGES>
+__global__ void __launch_bounds__(32 * CG * KS) walk_kernel(WalkArgs a) {
+    using L = Layout<T, CG, KS, DELTA, STAGES>;
+    constexpr int PARTS = L::kParts;
+    constexpr int KT = kKeys / KS / 8;               // groups of 8 keys of a warp
+    constexpr int GROUPS = kTokens / 8;              // groups of 8 tokens
+    constexpr int OWN = KS <= GROUPS ? GROUPS / KS : 1;       // groups that a warp finishes
+    constexpr bool HALVES = KS > GROUPS;             // some warps finish the values, others the read-outs
+    static_assert(KT % 2 == 0 && (KS <= GROUPS || (KS == 2 * GROUPS && DELTA)), "whole steps");
+    pdl_launch_dependents();
+    pdl_wait();
+    extern __shared__ __align__(16) unsigned char mem[];
+    float4* shares = reinterpret_cast<float4*>(mem + STAGES * L::kStage);
+    float* alpha_s = reinterpret_cast<float*>(mem + STAGES * L::kStage + L::kShares);     // gated: per token
+    float* beta_s = alpha_s + kTokens;
+    float* under_s = beta_s + kTokens;
+    float* n_s = under_s + kTokens;
+    const int slab = blockIdx.x, head = blockIdx.y, seq = blockIdx.z;
+    const int row0 = a.cu_seqlens[seq], n_tokens = a.cu_seqlens[seq + 1] - row0;
+    if (n_tokens <= 0) return;
+    const int slot = a.slots[seq], unit = head / a.heads_per_unit;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int cg = warp / KS, ks = warp % KS, key0 = ks * (kKeys / KS);
+    const int group0 = HALVES ? ks % GROUPS : ks * OWN;      // the first group of tokens that this warp finishes
+    const bool fixes = !HALVES || ks < GROUPS, reads = !HALVES || ks >= GROUPS;
+    const int col0 = slab * L::kColumns;
+    const __nv_bfloat16* q_src = a.q + unit * a.key_unit + row0 * a.key_row;
+    const __nv_bfloat16* k_src = a.k + unit * a.key_unit + row0 * a.key_row;
+    const long long w_plane = (long long)a.n_rows * kKeyRow, g_plane = (long long)a.n_rows * kScoreRow;
+    const __nv_bfloat16* w_src = DELTA ? a.w + head * 3 * w_plane + (long long)row0 * kKeyRow : nullptr;
+    const __nv_bfloat16* g_src = a.scores + head * 3 * g_plane + (long long)row0 * kScoreRow;
+    const T* v_src = static_cast<const T*>(a.v) + row0 * a.v_row + head * a.v_head + col0;
+    const float4* scalar_src = a.scalars + (long long)head * a.n_rows + row0;
+
+    auto issue = [&](int chunk) {
+        unsigned char* dst = mem + (chunk % STAGES) * L::kStage;
+        const int first = chunk * kTokens, n_here = min(kTokens, n_tokens - first);
+        __nv_bfloat16* q_dst = reinterpret_cast<__nv_bfloat16*>(dst + L::kQ);
+        __nv_bfloat16* k_dst = reinterpret_cast<__nv_bfloat16*>(dst + L::kK);
+        if (PARTS == 3) {
+#pragma unroll
+            for (int p = 0; p < PARTS; ++p) {
+                copy_rows<kKeyRow, L::kThreads>(q_dst + p * L::kKeyPlane, q_src + p * a.key_plane + (long long)first * kKeyRow, n_here);
+                copy_rows<kKeyRow, L::kThreads>(k_dst + p * L::kKeyPlane, k_src + p * a.key_plane + (long long)first * kKeyRow, n_here);
+            }
+        } else {
+            for (int e = threadIdx.x; e < kTokens * (kKeys / 8); e += L::kThreads) {
+                const int i = e / (kKeys / 8), c = e % (kKeys / 8) * 8;
+                const bool there = i < n_here;
+                const long long at = (there ? first + i : 0) * a.key_row + c;
+                copy16(q_dst + i * kKeyRow + c, q_src + at, there);
+                copy16(k_dst + i * kKeyRow + c, k_src + at, there);
+            }
+        }
+#pragma unroll
+        for (int p = 0; p < 3; ++p) {
+            if (DELTA)
+                copy_rows<kKeyRow, L::kThreads>(reinterpret_cast<__nv_bfloat16*>(dst + L::kW) + p * L::kKeyPlane,
+                                                w_src + p * w_plane + (long long)first * kKeyRow, n_here);
+            copy_rows<kScoreRow, L::kThreads>(reinterpret_cast<__nv_bfloat16*>(dst + L::kG) + p * L::kScorePlane,
+                                              g_src + p * g_plane + (long long)first * kScoreRow, n_here);
+        }
+        constexpr int kPer16 = 16 / (int)sizeof(T), kValueCopies = L::kColumns / kPer16;
+        for (int e = threadIdx.x; e < kTokens * kValueCopies; e += L::kThreads) {
+            const int i = e / kValueCopies, c = e % kValueCopies * kPer16;
+            const bool there = i < n_here;
+            copy16(dst + L::kV + (i * L::kValueRow + c) * (int)sizeof(T), v_src + (there ? first + i : 0) * a.v_row + c, there);
+        }
+        for (int i = threadIdx.x; i < kTokens; i += L::kThreads)
+            copy16(dst + L::kScalars + i * 16, scalar_src + (i < n_here ? first + i : 0), i < n_here);
+        copy_commit();
+    };
+    issue(0);
+
+    // S^T: s[j][0], s[j][1]: column g, keys 8j + 2t and the one after; s[j][2], s[j][3]: column g + 8
+    float s[KT][4];
+    float* S = a.state + (((size_t)slot * a.n_heads + head) * a.value_dim + col0 + cg * 16) * kKeys + key0;
+#pragma unroll
+    for (int j = 0; j < KT; ++j) {
+        const float2 x = *reinterpret_cast<const float2*>(S + g * kKeys + 8 * j + 2 * t);
+        const float2 y = *reinterpret_cast<const float2*>(S + (g + 8) * kKeys + 8 * j + 2 * t);
+        s[j][0] = x.x; s[j][1] = x.y; s[j][2] = y.x; s[j][3] = y.y;
+    }
+    float m = 0.f;
+    float* nm = nullptr;
+    if (GATED) {
+        nm = a.normaliser + (((size_t)slot * a.n_heads + head) * (a.value_dim / 16) + slab * CG) * (kKeys + 1);
+        for (int d = threadIdx.x; d < kKeys; d += L::kThreads) n_s[d] = nm[d];
+        m = nm[kKeys];
+    }
+    const int key_at = b_tile(lane, kKeyRow) + key0;          // this lane's address in a tile of 16 tokens and 16 keys
+    const int key_at_transposed = a_tile(lane, kKeyRow) + key0;
+
+    const int n_chunks = (n_tokens + kTokens - 1) / kTokens;
+    for (int chunk = 0; chunk < n_chunks; ++chunk) {
+        if (STAGES == 1 && chunk > 0) {
+            __syncthreads();           // the only stage is free again
+            issue(chunk);
+        }
+        copy_wait_all();
+        __syncthreads();               // this chunk is in place; the other stage, and the shares, are free again
+        if (STAGES > 1 && chunk + 1 < n_chunks) issue(chunk + 1);
+        unsigned char* stage = mem + (chunk % STAGES) * L::kStage;
+        const __nv_bfloat16* q_s = reinterpret_cast<const __nv_bfloat16*>(stage + L::kQ);
+        const __nv_bfloat16* k_s = reinterpret_cast<const __nv_bfloat16*>(stage + L::kK);
+        const __nv_bfloat16* w_s = reinterpret_cast<const __nv_bfloat16*>(stage + L::kW);
+        const __nv_bfloat16* g_s = reinterpret_cast<const __nv_bfloat16*>(stage + L::kG);
+        T* v_s = reinterpret_cast<T*>(stage + L::kV) + cg * 16;
+        const float4* scalars = reinterpret_cast<const float4*>(stage + L::kScalars);
+        const int first = chunk * kTokens, n_here = min(kTokens, n_tokens - first);
+
+        if (GATED) {
+            // alpha, beta and the denominators of the chunk's tokens; four threads share a token's n . q
+            static_assert(!GATED || L::kThreads >= kTokens * 4, "four threads per token");
+            if (threadIdx.x < kTokens * 4) {
+                const int i = threadIdx.x >> 2, part = threadIdx.x & 3;
+                const float4 sc = scalars[i];
+                const float top = fmaxf(sc.x + m, sc.y);
+                const float alpha = expf(sc.x + m - top), beta = expf(sc.y - top);
+                float dot0 = 0.f, dot1 = 0.f;
+#pragma unroll
+                for (int d = 0; d < kKeys / 8; ++d) {
+                    const float2 q = pair_of(q_s + i * kKeyRow + 2 * (part + 4 * d));
+                    const float2 n = pair_of(n_s + 2 * (part + 4 * d));
+                    dot0 = fmaf(q.x, n.x, dot0);
+                    dot1 = fmaf(q.y, n.y, dot1);
+                }
+                float dot = dot0 + dot1;
+                dot += __shfl_xor_sync(0xffffffffu, dot, 1);
+                dot += __shfl_xor_sync(0xffffffffu, dot, 2);
+                if (part == 0) {
+                    alpha_s[i] = alpha;
+                    beta_s[i] = beta;
+                    under_s[i] = fmaxf(fabsf((alpha * dot + beta * sc.w) * a.scale), expf(-top)) + a.floor_;
+                }
+            }
+        }
+
+        // this warp's keys of S0^T q (and W S0): over the chunk's tokens, columns 16 cg ..
+        float read[4][4], fixed[4][4];
+#pragma unroll
+        for (int j = 0; j < KT; j += 2) {
+            const Parts p = parts_of(make_float2(s[j][0], s[j][1]), make_float2(s[j][2], s[j][3]),
+                                     make_float2(s[j + 1][0], s[j + 1][1]), make_float2(s[j + 1][2], s[j + 1][3]));
+            const int at = key_at + 8 * j;
+            auto share = [&](float (&sum)[4][4], const auto& columns) {
+                float large[4][4], small[4][4];
+                clear(large);
+                clear(small);
+                multiply(large, small, p, columns);
+#pragma unroll
+                for (int n = 0; n < 4; ++n)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) sum[n][i] = j == 0 ? joined(large[n][i], small[n][i]) : sum[n][i] + joined(large[n][i], small[n][i]);
+            };
+            if constexpr (DELTA) {
+                const Columns<3> w[2] = {columns_of<3>(w_s + at, L::kKeyPlane), columns_of<3>(w_s + at + 16 * kKeyRow, L::kKeyPlane)};
+                share(fixed, w);
+            }
+            const Columns<PARTS> q[2] = {columns_of<PARTS>(q_s + at, L::kKeyPlane), columns_of<PARTS>(q_s + at + 16 * kKeyRow, L::kKeyPlane)};
+            share(read, q);
+        }
+        constexpr int WHICH = DELTA ? 2 : 1;
+        if (KS > 1) {
+            float4* own = shares + (size_t)(ks * CG + cg) * WHICH * 4 * 32 + lane;
+#pragma unroll
+            for (int n = 0; n < 4; ++n) {
+                own[n * 32] = make_float4(read[n][0], read[n][1], read[n][2], read[n][3]);
+                if (DELTA) own[(4 + n) * 32] = make_float4(fixed[n][0], fixed[n][1], fixed[n][2], fixed[n][3]);
+            }
+        }
+        if (KS > 1 || GATED) __syncthreads();
+        if (KS > 1) {
+            // (the sums are taken in the order of the keys, whoever takes them)
+#pragma unroll
+            for (int n = 0; n < OWN; ++n) {
+#pragma unroll
+                for (int which = 0; which < WHICH; ++which) {
+                    if (HALVES && (which == 0 ? !reads : !fixes)) continue;
+                    float (&dst)[4] = which == 0 ? read[n] : fixed[n];
+                    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                    for (int other = 0; other < KS; ++other) {
+                        const float4 x = shares[((size_t)(other * CG + cg) * WHICH * 4 + which * 4 + group0 + n) * 32 + lane];
+                        sum.x += x.x; sum.y += x.y; sum.z += x.z; sum.w += x.w;
+                    }
+                    dst[0] = sum.x; dst[1] = sum.y; dst[2] = sum.z; dst[3] = sum.w;
+                }
+            }
+        }
+        if constexpr (DELTA) {
+            // v = u - W S0, in place of u
+            if (fixes) {
+#pragma unroll
+                for (int n = 0; n < OWN; ++n) {
+                    T* v = v_s + (8 * (group0 + n) + 2 * t) * L::kValueRow + g;
+                    v[0] -= fixed[n][0];
+                    v[L::kValueRow] -= fixed[n][1];
+                    v[8] -= fixed[n][2];
+                    v[L::kValueRow + 8] -= fixed[n][3];
+                }
+            }
+            if (KS > 1) __syncthreads();
+            else __syncwarp();
+        }
+        // the chunk's values as A operands: columns by tokens, as they are and times w
+        Parts plain[kTokens / 16], scaled[kTokens / 16];
+#pragma unroll
+        for (int j = 0; j < kTokens / 16; ++j) {
+            const float4* sc = scalars + 16 * j + 2 * t;
+            const float w0 = sc[0].z, w1 = sc[1].z, w8 = sc[8].z, w9 = sc[9].z;
+            float2 v[4];        // column g, g + 8 at tokens 2t, 2t + 1; the same at 2t + 8, 2t + 9
+            if constexpr (PARTS == 1) {
+                load_matrices_transposed(plain[j].part[0], v_s + 16 * j * L::kValueRow + b_tile(lane, L::kValueRow));
+#pragma unroll
+                for (int i = 0; i < 4; ++i) v[i] = make_float2(low_half(plain[j].part[0][i]), high_half(plain[j].part[0][i]));
+            } else {
+                const T* src = v_s + (16 * j + 2 * t) * L::kValueRow + g;
+                v[0] = make_float2(src[0], src[L::kValueRow]);
+                v[1] = make_float2(src[8], src[L::kValueRow + 8]);
+                src += 8 * L::kValueRow;
+                v[2] = make_float2(src[0], src[L::kValueRow]);
+                v[3] = make_float2(src[8], src[L::kValueRow + 8]);
+                plain[j] = parts_of(v[0], v[1], v[2], v[3]);
+            }
+            scaled[j] = parts_of(make_float2(v[0].x * w0, v[0].y * w1), make_float2(v[1].x * w0, v[1].y * w1),
+                                 make_float2(v[2].x * w8, v[2].y * w9), make_float2(v[3].x * w8, v[3].y * w9));
+        }
+        // the state behind the chunk
+        const float keep = GATED ? alpha_s[n_here - 1] : scalars[n_here - 1].x, take = GATED ? beta_s[n_here - 1] : 1.f;
+        constexpr int KP = KT >= 4 ? 2 : 1;          // pairs of groups of keys at a time
+#pragma unroll
+        for (int n = 0; n < KT; n += 2 * KP) {
+            float sum[2 * KP][4];
+#pragma unroll
+            for (int j = 0; j < kTokens / 16; ++j) {
+                const __nv_bfloat16* p = k_s + key_at_transposed + 16 * j * kKeyRow + 8 * n;
+                Columns<PARTS> k[KP];
+#pragma unroll
+                for (int o = 0; o < KP; ++o) k[o] = columns_transposed<PARTS>(p + 16 * o, L::kKeyPlane);
+                float large[2 * KP][4], small[2 * KP][4];
+                clear(large);
+                clear(small);
+                multiply(large, small, scaled[j], k);
+#pragma unroll
+                for (int o = 0; o < 2 * KP; ++o)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) sum[o][i] = j == 0 ? joined(large[o][i], small[o][i]) : sum[o][i] + joined(large[o][i], small[o][i]);
+            }
+#pragma unroll
+            for (int o = 0; o < 2 * KP; ++o)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) s[n + o][i] = fmaf(keep, s[n + o][i], take * sum[o][i]);
+        }
+        // sum_j G_ij v_j for this warp's tokens, and the read-outs
+        if (reads) {
+            // (G's rows are loaded for 16 tokens at a time; with one group of tokens a warp, two warps share them)
+            constexpr int kPairs = OWN >= 2 ? OWN / 2 : 1;
+            float inner[kPairs][2][4];
+            const int pair0 = group0 / 2;
+#pragma unroll
+            for (int pair = 0; pair < kPairs; ++pair) {
+                clear(inner[pair]);
+#pragma unroll
+                for (int j = 0; j < kTokens / 16; ++j) {
+                    if (j > pair0 + pair) continue;
+                    const Columns<3> row[1] = {columns_of<3>(g_s + b_tile(lane, kScoreRow) + 16 * (pair0 + pair) * kScoreRow + 16 * j, L::kScorePlane)};
+                    float large[2][4], small[2][4];
+                    clear(large);
+                    clear(small);
+                    multiply<PARTS>(large, small, plain[j], row);
+#pragma unroll
+                    for (int o = 0; o < 2; ++o)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) inner[pair][o][i] += joined(large[o][i], small[o][i]);
+                }
+            }
+#pragma unroll
+            for (int n = 0; n < OWN; ++n) {
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int i = 8 * (group0 + n) + 2 * t + half;
+                    if (i >= n_here) continue;
+                    const int o = OWN == 1 ? group0 & 1 : n & 1;
+                    const float in0 = o ? inner[n / 2][1][half] : inner[n / 2][0][half];
+                    const float in1 = o ? inner[n / 2][1][2 + half] : inner[n / 2][0][2 + half];
+                    const float alpha = GATED ? alpha_s[i] : scalars[i].x, beta = GATED ? beta_s[i] : 1.f;
+                    float y0 = (alpha * read[n][half] + beta * in0) * a.scale;
+                    float y1 = (alpha * read[n][2 + half] + beta * in1) * a.scale;
+                    if (GATED) {
+                        y0 /= under_s[i];
+                        y1 /= under_s[i];
+                    }
+                    float* dst = a.o + ((size_t)(row0 + first + i) * a.n_heads + head) * a.value_dim + col0 + cg * 16 + g;
+                    dst[0] = y0;
+                    dst[8] = y1;
+                }
+            }
+        }
+        if (GATED) {
+            const float4 sc = scalars[n_here - 1];
+            m = fmaxf(sc.x + m, sc.y);
+            // (every n . q of the chunk was taken ahead of the barrier above; the next chunk's wait behind one too)
+            const float* sums = a.key_sums + (((size_t)seq * a.max_chunks + chunk) * a.n_heads + head) * kKeys;
+            for (int d = threadIdx.x; d < kKeys; d += L::kThreads) n_s[d] = fmaf(keep, n_s[d], take * sums[d]);
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < KT; ++j) {
+        *reinterpret_cast<float2*>(S + g * kKeys + 8 * j + 2 * t) = make_float2(s[j][0], s[j][1]);
+        *reinterpret_cast<float2*>(S + (g + 8) * kKeys + 8 * j + 2 * t) = make_float2(s[j][2], s[j][3]);
+    }
+    if (GATED) {
+        for (int copy = 0; copy < CG; ++copy) {       // (a thread stores the entries of n that it holds)
+            for (int d = threadIdx.x; d < kKeys; d += L::kThreads) nm[copy * (kKeys + 1) + d] = n_s[d];
+            if (threadIdx.x == 0) nm[copy * (kKeys + 1) + kKeys] = m;
+        }
+    }
+}
+
+template <typename T, int CG, int KS, bool DELTA, bool GATED, int STAGES>
+void launch_walk(const WalkArgs& a, int n_seqs, cudaStream_t stream) {
+    using L = Layout<T, CG, KS, DELTA, STAGES>;
+    auto kernel = walk_kernel<T, CG, KS, DELTA, GATED, STAGES>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
+    thn_launch_ordered(kernel, dim3(a.value_dim / L::kColumns, a.n_heads, n_seqs), L::kThreads, L::kBytes, stream, a);
+}
+
+// ---------------------------------------------------------------- what the mixers' own kernels share
+
+// Inclusive sum over the lanes of a warp.
+__device__ __forceinline__ double lanes_cumulative(double v, int lane) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double x = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += x;
+    }
+    return v;
+}
+// The logarithm of a decay in [0, 1]; a decay of zero gets one whose exponential is zero in float32.
+__device__ __forceinline__ double log_decay(float a) { return a > 0.f ? log((double)a) : -200.0; }
+
+// Rows 16 m_tile .. of x times all 32 rows of y, both planes of kKeys in shared memory: out[n][..] are
+// the products of rows (g, g, g + 8, g + 8) with rows 8n + (2t, 2t + 1, 2t, 2t + 1); groups of y that lie
+// behind all of x's rows are left out (zero).
+template <int PARTS>
+__device__ __forceinline__ void dots(float (&out)[4][4], const __nv_bfloat16* x, const __nv_bfloat16* y, int m_tile, int lane) {
+    constexpr int kPlane = kTokens * kKeyRow;
+    const __nv_bfloat16* xa = x + 16 * m_tile * kKeyRow + a_tile(lane, kKeyRow);
+    const __nv_bfloat16* yb = y + b_tile(lane, kKeyRow);
+    clear(out);
+#pragma unroll
+    for (int j = 0; j < kKeys / 16; ++j) {
+        Parts p;
+#pragma unroll
+        for (int i = 0; i < PARTS; ++i) load_matrices(p.part[i], xa + i * kPlane + 16 * j);
+#pragma unroll
+        for (int pair = 0; pair < 2; ++pair) {
+            if (pair > m_tile) continue;
+            float large[2][4], small[2][4];
+            clear(large);
+            clear(small);
+            const Columns<PARTS> c[1] = {columns_of<PARTS>(yb + 16 * pair * kKeyRow + 16 * j, kPlane)};
+            multiply<PARTS>(large, small, p, c);
+#pragma unroll
+            for (int o = 0; o < 2; ++o)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) out[2 * pair + o][i] += joined(large[o][i], small[o][i]);
+        }
+    }
+}
+
+// Two neighbouring entries of a row, in three planes.
+__device__ __forceinline__ void store_split(__nv_bfloat16* p, long long plane, float x, float y) {
+    const Split s = split(x, y);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) *reinterpret_cast<uint32_t*>(p + i * plane) = s.part[i];
+}
+
+}  // namespace chunk

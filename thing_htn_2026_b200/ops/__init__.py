@@ -126,6 +126,9 @@ _SIGNATURES = {
                           c_float, c_int, c_void_p],
     "thn_delta_recurrence": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                              c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+    "thn_delta_chunks": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                         c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
+                         c_void_p],
     "thn_delta_conv_ring_update": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                    c_int, c_int, c_int, c_void_p],
     "thn_delta_decode": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -198,6 +201,8 @@ def lib():
         loaded.thn_linear_attention_scratch_floats.restype = c_longlong
         loaded.thn_set_recurrence_columns.argtypes = [c_int]
         loaded.thn_set_recurrence_columns.restype = None
+        loaded.thn_delta_chunks_scratch_bytes.argtypes = [c_int, c_int, c_int, c_int]
+        loaded.thn_delta_chunks_scratch_bytes.restype = c_longlong
         loaded.thn_wkv_scratch_floats.argtypes = [c_int, c_int, c_int]
         loaded.thn_wkv_scratch_floats.restype = c_longlong
         loaded.thn_state_space_scratch_floats.argtypes = [c_int, c_int, c_int, c_int, c_int]
@@ -1395,6 +1400,19 @@ DELTA_LANES = int(os.environ.get("THN_DELTA_LANES", 0))     # 8 or 32 lanes per 
 FUSE_DELTA_DECODE = os.environ.get("THN_FUSE_DELTA_DECODE", "1").strip().lower() not in ("0", "false", "no", "off")
 
 
+CHUNK_KEYS = 128           # the key size that the chunk kernels are built for
+CHUNK_MIN_TOKENS = 16      # fewer tokens a sequence are as fast one by one (60 against 66 us at 16)
+
+
+def _delta_in_chunks(proj: torch.Tensor, conv_w: torch.Tensor, state: torch.Tensor, ring: torch.Tensor, rows: StepRows,
+                     s: "DeltaShape") -> bool:
+    """Whether a step's recurrence is walked in chunks of tokens on the tensor cores."""
+    return proj.dtype == torch.bfloat16 and s.key_dim == CHUNK_KEYS and s.value_dim % 16 == 0 and s.taps == 4 \
+        and DELTA_LANES == 0 and rows.max_q_len >= CHUNK_MIN_TOKENS and s.proj_width % 4 == 0 and rows.n_rows <= 8 * 65535 \
+        and max(s.n_heads, rows.n_seqs) <= 65535 \
+        and (state.data_ptr() | conv_w.data_ptr()) % 16 == 0 and (proj.data_ptr() | ring.data_ptr()) % 8 == 0
+
+
 def delta_rule(proj: torch.Tensor, conv_w: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor,
                state: torch.Tensor, ring: torch.Tensor, rows: StepRows, seq_lens: torch.Tensor, shape: DeltaShape,
                unit_eps: float) -> torch.Tensor:
@@ -1405,8 +1423,9 @@ def delta_rule(proj: torch.Tensor, conv_w: torch.Tensor, a_log: torch.Tensor, dt
     ``ring`` [slots, taps, channels] (the raw projection of position p at p mod taps) are read
     and updated; ``seq_lens`` holds the tokens each slot held before the step.  Returns the
     read-out, float32 [rows, heads, value_dim].  Steps of one token per sequence run as one
-    kernel; others as three (prepare, recurrence, ring update).  With float32 activations the
-    recurrence carries the state in double between a step's first and last token."""
+    kernel; others as three (prepare, recurrence, ring update), or with bfloat16 rows and keys of 128 as
+    four (prepare, what a chunk of 32 tokens needs beside the state, the walk over the chunks, ring
+    update), equal up to rounding.  With float32 activations the recurrence carries the state in double between a step's first and last token."""
     _delta_check(proj, conv_w, a_log, dt_bias, state, ring, shape, "delta_rule")
     if proj.shape[0] != rows.n_rows:
         raise KernelError(f"delta_rule: {proj.shape[0]} projected rows for a step of {rows.n_rows}")
@@ -1418,6 +1437,15 @@ def delta_rule(proj: torch.Tensor, conv_w: torch.Tensor, a_log: torch.Tensor, dt
         _call("thn_delta_decode", _ptr(o), _ptr(state), _ptr(ring), _ptr(proj), _ptr(conv_w), _ptr(a_log), _ptr(dt_bias),
               _ptr(rows.row_slot), _ptr(rows.row_pos), n, s.n_heads, s.n_kv, s.key_dim, s.value_dim, s.taps,
               s.proj_width, float(unit_eps), code, _stream())
+        return o
+    if _delta_in_chunks(proj, conv_w, state, ring, rows, s):
+        scratch = torch.empty(lib().thn_delta_chunks_scratch_bytes(n, s.n_heads, s.n_kv, s.value_dim), dtype=torch.uint8, device=dev)
+        _call("thn_delta_chunks", _ptr(o), _ptr(state), _ptr(scratch), _ptr(proj), _ptr(conv_w), _ptr(a_log), _ptr(dt_bias),
+              _ptr(ring), _ptr(rows.row_slot), _ptr(rows.row_pos), _ptr(seq_lens), _ptr(rows.cu_seqlens), _ptr(rows.slots), n,
+              rows.max_q_len, rows.n_seqs, s.n_heads, s.n_kv, s.key_dim, s.value_dim, s.taps, s.proj_width, float(unit_eps),
+              _stream())
+        _call("thn_delta_conv_ring_update", _ptr(ring), _ptr(proj), _ptr(rows.cu_seqlens), _ptr(rows.slots), _ptr(seq_lens),
+              rows.n_seqs, s.n_heads, s.n_kv, s.key_dim, s.value_dim, s.taps, s.proj_width, code, _stream())
         return o
     qn = torch.empty((n, s.n_kv, s.key_dim), dtype=torch.float32, device=dev)
     kn = torch.empty_like(qn)
