@@ -24,7 +24,9 @@
 #include <math.h>
 
 #include <algorithm>
+#include <cstdlib>
 
+#include "chunk_walk.cuh"
 #include "common.cuh"
 
 static int g_mlstm_staged = 1;       // 0: steps of several tokens run the kernel without staging too (measurement)
@@ -291,6 +293,94 @@ __global__ void __launch_bounds__(LANES * kColumns) mlstm_recurrence_staged_kern
     if (threadIdx.x == 0) nm_block[D] = m;
 }
 
+// ---------------------------------------------------------------- chunk by chunk, bfloat16
+
+// What a chunk of 32 tokens needs beside the state (chunk_walk.cuh), for one head.  With F_j the sum of the
+// chunk's log f up to token j, P_j = i_j - F_j and M_i the largest P_j of the tokens up to i, the weight of
+// token j's write in the chunk's own part of token i's read-out, under the chunk's own running maximum l_i =
+// F_i + M_i, is exp(P_j - M_i).  Out: the products q_i . k_j times these as planes, per token (F_i, l_i, its
+// write's weight at the chunk's end, the sum of its row of products), per chunk the sum of the weighted keys.
+// F, P and M are double, so that differences of long sums stay exact.
+constexpr int kChunkThreads = 128;
+
+__global__ void __launch_bounds__(kChunkThreads) mlstm_chunk_kernel(
+    __nv_bfloat16* __restrict__ scores, float4* __restrict__ scalars, float* __restrict__ key_sums,
+    const __nv_bfloat16* __restrict__ proj, int proj_width, const float* __restrict__ gate_pre, const float* __restrict__ bias_i,
+    const float* __restrict__ bias_f, float cap, const int* __restrict__ cu_seqlens, int n_rows, int n_heads) {
+    pdl_launch_dependents();
+    pdl_wait();
+    constexpr int C = chunk::kTokens;
+    __shared__ __align__(16) __nv_bfloat16 q_s[C * chunk::kKeyRow], k_s[C * chunk::kKeyRow];
+    __shared__ double p_s[C], m_s[C];
+    __shared__ float f_s[C], w_s[C];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int head = blockIdx.y, seq = blockIdx.z;
+    const int begin = cu_seqlens[seq], row0 = begin + blockIdx.x * C, n_here = min(C, cu_seqlens[seq + 1] - row0);
+    if (n_here <= 0) return;
+    for (int e = tid; e < C * (chunk::kKeys / 8); e += kChunkThreads) {
+        const int i = e / (chunk::kKeys / 8), c = e % (chunk::kKeys / 8) * 8;
+        const bool there = i < n_here;
+        const __nv_bfloat16* src = proj + (size_t)(row0 + (there ? i : 0)) * proj_width + (size_t)head * chunk::kKeys + c;
+        chunk::copy16(q_s + i * chunk::kKeyRow + c, src, there);
+        chunk::copy16(k_s + i * chunk::kKeyRow + c, src + (size_t)n_heads * chunk::kKeys, there);
+    }
+    chunk::copy_commit();
+    if (warp == 0) {
+        const bool there = lane < n_here;
+        const float* pre = gate_pre + (size_t)(row0 + (there ? lane : 0)) * 2 * n_heads;
+        const double F = chunk::lanes_cumulative(there ? (double)log_forget_gate(pre[n_heads + head] + bias_f[head], cap) : 0.0, lane);
+        const double P = there ? (double)log_input_gate(pre[head] + bias_i[head], cap) - F : -1.0e300;
+        double M = P;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const double x = __shfl_up_sync(0xffffffffu, M, o);
+            if (lane >= o) M = fmax(M, x);
+        }
+        const double last = __shfl_sync(0xffffffffu, M, 31);
+        p_s[lane] = P;
+        m_s[lane] = M;
+        f_s[lane] = (float)F;
+        w_s[lane] = expf((float)(P - last));
+    }
+    chunk::copy_wait_all();
+    __syncthreads();
+    if (warp >= 2) {
+        // two keys a thread
+        const int d = 2 * (tid - 64);
+        float x = 0.f, y = 0.f;
+#pragma unroll
+        for (int j = 0; j < C; ++j) {
+            const float2 k = chunk::pair_of(k_s + j * chunk::kKeyRow + d);
+            x = fmaf(w_s[j], k.x, x);
+            y = fmaf(w_s[j], k.y, y);
+        }
+        *reinterpret_cast<float2*>(key_sums + (((size_t)seq * gridDim.x + blockIdx.x) * n_heads + head) * chunk::kKeys + d) = make_float2(x, y);
+        return;
+    }
+    float dot[4][4];
+    chunk::dots<1>(dot, q_s, k_s, warp, lane);
+    const long long plane = (long long)n_rows * chunk::kScoreRow;
+    __nv_bfloat16* dst = scores + head * 3 * plane + (long long)row0 * chunk::kScoreRow;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const int i = 16 * warp + g + 8 * half;
+        float sum = 0.f;
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+            const int j = 8 * n + 2 * t;
+            float x[2];
+#pragma unroll
+            for (int o = 0; o < 2; ++o) x[o] = j + o <= i ? expf((float)(p_s[j + o] - m_s[i])) * dot[n][2 * half + o] : 0.f;
+            sum += x[0] + x[1];
+            if (i < n_here) chunk::store_split(dst + (long long)i * chunk::kScoreRow + j, plane, x[0], x[1]);
+        }
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        if (t == 0 && i < n_here)
+            scalars[(size_t)head * n_rows + row0 + i] = make_float4(f_s[i], (float)((double)f_s[i] + m_s[i]), w_s[i], sum);
+    }
+}
+
 template <typename T>
 int launch_recurrence(float* o, float* S, float* nm, const void* proj, int proj_width, const float* gates,
                       const float* bias_i, const float* bias_f, float cap, int raw_gates, const int* cu_seqlens,
@@ -398,4 +488,51 @@ THN_API int thn_mlstm_recurrence(float* o, float* S, float* nm, const void* proj
                                                 slots, n_seqs, n_heads, key_dim, value_dim, q_scale, floor_, stream);
     THN_CHECK_ARG(false, "mlstm_recurrence: unknown dtype %d", dtype);
     return THN_OK;
+}
+
+// Bytes of the scratch that thn_mlstm_chunks needs.
+THN_API long long thn_mlstm_chunks_scratch_bytes(int n_rows, int max_tokens, int n_seqs, int n_heads) {
+    const long long chunks = (max_tokens + chunk::kTokens - 1) / chunk::kTokens;
+    return (long long)n_heads * n_rows * (3 * chunk::kScoreRow * 2 + 16) + chunks * n_seqs * n_heads * chunk::kKeys * 4;
+}
+
+// The recurrence of a step chunk by chunk: bfloat16 rows whose q, k and v parts start on 16-byte boundaries, keys of
+// 128, values of whole groups of 16 columns; max_tokens: the most rows of a sequence; gate_pre as the
+// pre-activations of thn_mlstm_gates.
+THN_API int thn_mlstm_chunks(float* o, float* S, float* nm, void* scratch, const void* proj, int proj_width, const float* gate_pre,
+                             const float* bias_i, const float* bias_f, float cap, const int* cu_seqlens, const int* slots, int n_rows,
+                             int max_tokens, int n_seqs, int n_heads, int key_dim, int value_dim, float q_scale, float floor_,
+                             cudaStream_t stream) {
+    THN_CHECK_ARG(n_seqs >= 0 && n_heads > 0 && cap > 0.f && proj_width >= n_heads * (2 * key_dim + value_dim), "mlstm_chunks: bad sizes");
+    THN_UNSUPPORTED_IF(key_dim != chunk::kKeys || value_dim <= 0 || value_dim % 16 != 0 || proj_width % 8 != 0,
+                       "mlstm_chunks: keys of %d, values of %d, rows of %d", key_dim, value_dim, proj_width);
+    THN_UNSUPPORTED_IF(n_heads > 65535 || n_seqs > 65535, "mlstm_chunks: %d heads, %d sequences", n_heads, n_seqs);
+    THN_CHECK_ARG(scratch && (((uintptr_t)S | (uintptr_t)scratch | (uintptr_t)proj) & 15) == 0, "mlstm_chunks: operands are not 16-byte aligned");
+    if (n_seqs == 0 || n_rows <= 0 || max_tokens <= 0) return THN_OK;
+    const int chunks = (max_tokens + chunk::kTokens - 1) / chunk::kTokens;
+    __nv_bfloat16* scores = static_cast<__nv_bfloat16*>(scratch);
+    float4* scalars = reinterpret_cast<float4*>(scores + (size_t)n_heads * 3 * n_rows * chunk::kScoreRow);
+    float* key_sums = reinterpret_cast<float*>(scalars + (size_t)n_heads * n_rows);
+    const __nv_bfloat16* rows = static_cast<const __nv_bfloat16*>(proj);
+    thn_launch(mlstm_chunk_kernel, dim3(chunks, n_heads, n_seqs), kChunkThreads, 0, stream, scores, scalars, key_sums, rows, proj_width,
+               gate_pre, bias_i, bias_f, cap, cu_seqlens, n_rows, n_heads);
+    chunk::WalkArgs a{};
+    a.o = o; a.state = S;
+    a.q = rows; a.k = rows + (size_t)n_heads * key_dim;
+    a.key_plane = 0; a.key_unit = key_dim; a.key_row = proj_width;
+    a.v = rows + (size_t)2 * n_heads * key_dim; a.v_row = proj_width; a.v_head = value_dim;
+    a.scores = scores; a.scalars = scalars;
+    a.cu_seqlens = cu_seqlens; a.slots = slots;
+    a.n_rows = n_rows; a.n_heads = n_heads; a.heads_per_unit = 1; a.value_dim = value_dim; a.scale = q_scale;
+    a.normaliser = nm; a.key_sums = key_sums; a.max_chunks = chunks; a.floor_ = floor_;
+    using T = __nv_bfloat16;
+    const long long pairs = (long long)n_seqs * n_heads;
+    const char* env = getenv("WALK_SHAPE");
+    const int force = env ? atoi(env) : 0;
+    if (force == 41 && value_dim % 64 == 0) chunk::launch_walk<T, 4, 1, false, true, 2>(a, n_seqs, stream);
+    else if (force ? force == 42 : (value_dim % 64 == 0 && pairs * (value_dim / 64) >= 128)) chunk::launch_walk<T, 4, 2, false, true, 2>(a, n_seqs, stream);
+    else if (force == 22) chunk::launch_walk<T, 2, 2, false, true, 2>(a, n_seqs, stream);
+    else if (force ? force == 24 : (value_dim % 32 == 0 && pairs * (value_dim / 32) >= 128)) chunk::launch_walk<T, 2, 4, false, true, 2>(a, n_seqs, stream);
+    else chunk::launch_walk<T, 1, 4, false, true, 2>(a, n_seqs, stream);
+    return thn_launch_status("mlstm_chunks");
 }

@@ -21,7 +21,9 @@
 // double and rounded once (exp_of, silu_of, softplus_of in common.cuh).
 #include <math.h>
 
+#include "chunk_walk.cuh"
 #include "linear_attention.cuh"
+#include <cstdlib>
 
 namespace {
 
@@ -142,6 +144,156 @@ __global__ void __launch_bounds__(kPrepareThreads) state_space_prepare_kernel(
                                                       n > 2 ? silu_of<T>(acc.z) : 0.f, n > 3 ? silu_of<T>(acc.w) : 0.f);
     }
 }
+
+// The same for the walk in chunks (bfloat16, four taps, a state of 128, whole groups of four entries): the raw inputs
+// ahead of a thread's rows are loaded together, B and C go out in three planes of bfloat16 (chunk_walk.cuh)
+// [group][B | C][plane][rows][kKeyRow], x as [heads][rows][vdim], the step sizes as [heads][rows].
+constexpr int kChunkTaps = 4;
+
+__global__ void __launch_bounds__(kPrepareThreads) state_space_prepare_chunks_kernel(
+    __nv_bfloat16* __restrict__ planes, float* __restrict__ values, float* __restrict__ steps, const __nv_bfloat16* __restrict__ proj,
+    int proj_width, int offset, const float* __restrict__ conv_w, const float* __restrict__ conv_b,
+    const __nv_bfloat16* __restrict__ ring, const float* __restrict__ dt_pre, const float* __restrict__ dt_bias,
+    const int* __restrict__ row_slot, const int* __restrict__ row_pos, const int* __restrict__ seq_lens, int n_rows, SpaceShape shape) {
+    pdl_launch_dependents();
+    const int item = blockIdx.x * kPrepareThreads + threadIdx.x;
+    const int C = shape.channels(), c = item * 4;
+    const int first = blockIdx.y * kRunRows, n_here = min(kRunRows, n_rows - first);
+    if (c >= C) {
+        const int head = item - C / 4;
+        if (head >= shape.n_heads) return;
+        pdl_wait();
+        for (int r = 0; r < n_here; ++r)
+            steps[(size_t)head * n_rows + first + r] = softplus_of<__nv_bfloat16>(dt_pre[(size_t)(first + r) * shape.n_heads + head] + dt_bias[head]);
+        return;
+    }
+    float w[4][kChunkTaps], b[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float4 v = *reinterpret_cast<const float4*>(conv_w + (size_t)(c + i) * kChunkTaps);
+        w[i][0] = v.x; w[i][1] = v.y; w[i][2] = v.z; w[i][3] = v.w;
+        b[i] = conv_b[c + i];
+    }
+    pdl_wait();
+    const __nv_bfloat16* src = proj + (size_t)first * proj_width + offset + c;
+    uint2 raw[kRunRows + kChunkTaps - 1];       // raw[j]: the row j - 3 rows after `first`
+#pragma unroll
+    for (int j = 0; j < kRunRows + kChunkTaps - 1; ++j) {
+        const int back = kChunkTaps - 1 - j;
+        raw[j] = back <= first && -back < n_here ? *reinterpret_cast<const uint2*>(src - (long long)back * proj_width) : make_uint2(0, 0);
+    }
+    int slot[kRunRows], pos[kRunRows], local[kRunRows];
+#pragma unroll
+    for (int r = 0; r < kRunRows; ++r) {
+        slot[r] = row_slot[first + min(r, n_here - 1)];
+        pos[r] = row_pos[first + min(r, n_here - 1)];
+    }
+#pragma unroll
+    for (int r = 0; r < kRunRows; ++r) local[r] = pos[r] - seq_lens[slot[r]];
+    const bool is_value = c < shape.inner();
+    const int kc = is_value ? 0 : c - shape.inner(), which = kc / (shape.n_groups * chunk::kKeys), in_part = kc % (shape.n_groups * chunk::kKeys);
+    const long long plane = (long long)n_rows * chunk::kKeyRow;
+    __nv_bfloat16* key_dst = planes + ((in_part / chunk::kKeys) * 2 + which) * 3 * plane + (long long)first * chunk::kKeyRow + in_part % chunk::kKeys;
+    float* value_dst = values + ((size_t)(is_value ? c / shape.vdim : 0) * n_rows + first) * shape.vdim + (is_value ? c % shape.vdim : 0);
+#pragma unroll
+    for (int r = 0; r < kRunRows; ++r) {
+        if (r >= n_here) break;
+        uint2 in[kChunkTaps];
+#pragma unroll
+        for (int j = 0; j < kChunkTaps; ++j) in[j] = raw[r + j];
+        if (local[r] < kChunkTaps - 1) {
+#pragma unroll
+            for (int back = 1; back < kChunkTaps; ++back) {
+                if (back <= local[r]) continue;
+                in[kChunkTaps - 1 - back] = back > pos[r] ? make_uint2(0, 0)           // before the sequence's start
+                    : *reinterpret_cast<const uint2*>(ring + ((size_t)slot[r] * kChunkTaps + (pos[r] - back) % kChunkTaps) * C + c);
+            }
+        }
+        float y[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            float acc = b[i];
+#pragma unroll
+            for (int j = 0; j < kChunkTaps; ++j) {
+                if (kChunkTaps - 1 - j > pos[r]) continue;
+                const uint32_t two = i < 2 ? in[j].x : in[j].y;
+                acc += w[i][j] * (i & 1 ? chunk::high_half(two) : chunk::low_half(two));
+            }
+            y[i] = silu_of<__nv_bfloat16>(acc);
+        }
+        if (is_value) {
+            *reinterpret_cast<float4*>(value_dst + (size_t)r * shape.vdim) = make_float4(y[0], y[1], y[2], y[3]);
+        } else {
+            const chunk::Split lo = chunk::split(y[0], y[1]), hi = chunk::split(y[2], y[3]);
+#pragma unroll
+            for (int p = 0; p < 3; ++p)
+                *reinterpret_cast<uint2*>(key_dst + p * plane + (long long)r * chunk::kKeyRow) = make_uint2(lo.part[p], hi.part[p]);
+        }
+    }
+}
+
+// What a chunk of 32 tokens needs beside the state, for all heads of a group: G_ij = exp(c_i - c_j) t_j C_i . B_j with
+// c the sum of the chunk's log decays -rate t (in double), plus the skip's factor on the diagonal; per token
+// (exp(c_i), -, t_i exp(c_last - c_i), -).  One block per (chunk, group, sequence): two warps take the products, then
+// each warp's lanes are the tokens j of some of the group's heads.
+__global__ void __launch_bounds__(128) state_space_chunk_kernel(
+    __nv_bfloat16* __restrict__ scores, float4* __restrict__ scalars, const __nv_bfloat16* __restrict__ planes,
+    const float* __restrict__ steps, const float* __restrict__ rate, const float* __restrict__ skip, const int* __restrict__ cu_seqlens,
+    int n_rows, int heads_per_group) {
+    pdl_launch_dependents();
+    pdl_wait();
+    constexpr int C = chunk::kTokens, kPlane = C * chunk::kKeyRow;
+    extern __shared__ __align__(16) unsigned char space_mem[];
+    __nv_bfloat16* b_s = reinterpret_cast<__nv_bfloat16*>(space_mem);      // [3][C][kKeyRow]
+    __nv_bfloat16* c_s = b_s + 3 * kPlane;                                 // [3][C][kKeyRow]
+    float* dot_s = reinterpret_cast<float*>(c_s + 3 * kPlane);             // [C][C + 1]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int group = blockIdx.y, seq = blockIdx.z;
+    const int begin = cu_seqlens[seq], row0 = begin + blockIdx.x * C, n_here = min(C, cu_seqlens[seq + 1] - row0);
+    if (n_here <= 0) return;
+    const long long plane = (long long)n_rows * chunk::kKeyRow, at0 = (long long)row0 * chunk::kKeyRow;
+#pragma unroll
+    for (int p = 0; p < 3; ++p) {
+        chunk::copy_rows<chunk::kKeyRow, 128>(b_s + p * kPlane, planes + ((long long)group * 6 + p) * plane + at0, n_here);
+        chunk::copy_rows<chunk::kKeyRow, 128>(c_s + p * kPlane, planes + ((long long)group * 6 + 3 + p) * plane + at0, n_here);
+    }
+    chunk::copy_commit();
+    chunk::copy_wait_all();
+    __syncthreads();
+    if (warp < 2) {
+        float dot[4][4];
+        chunk::dots<3>(dot, c_s, b_s, warp, lane);
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) dot_s[(16 * warp + g + 8 * (i >> 1)) * (C + 1) + 8 * n + 2 * t + (i & 1)] = dot[n][i];
+    }
+    __syncthreads();
+    const long long score_plane = (long long)n_rows * chunk::kScoreRow;
+    for (int h = warp; h < heads_per_group; h += 4) {
+        const int head = group * heads_per_group + h;
+        const bool there = lane < n_here;
+        const float step = there ? steps[(size_t)head * n_rows + row0 + lane] : 0.f;
+        const double c = chunk::lanes_cumulative(-(double)rate[head] * step, lane);
+        const double c_last = __shfl_sync(0xffffffffu, c, 31);            // (tokens beyond the step's add nothing)
+        const float d = skip[head];
+        if (there)
+            scalars[(size_t)head * n_rows + row0 + lane] = make_float4(expf((float)c), 0.f, step * expf((float)(c_last - c)), 0.f);
+        __nv_bfloat16* dst = scores + head * 3 * score_plane + (long long)row0 * chunk::kScoreRow + lane;
+        for (int i = 0; i < n_here; ++i) {
+            const double ci = __shfl_sync(0xffffffffu, c, i);
+            float x = lane <= i ? expf((float)(ci - c)) * step * dot_s[i * (C + 1) + lane] : 0.f;
+            if (lane == i) x += d;
+#pragma unroll
+            for (int p = 0; p < 3; ++p) {
+                const __nv_bfloat16 part = __float2bfloat16_rn(x);
+                dst[p * score_plane + (long long)i * chunk::kScoreRow] = part;
+                x -= __bfloat162float(part);
+            }
+        }
+    }
+}
+constexpr size_t kSpaceChunkBytes = (size_t)6 * chunk::kTokens * chunk::kKeyRow * 2 + chunk::kTokens * (chunk::kTokens + 1) * sizeof(float);
 
 constexpr int kDecodeThreads = 256;
 constexpr int kDecodeLanes = 8;            // lanes that share a column of S
@@ -318,6 +470,61 @@ void launch_prepare(float* keys, float* values, const void* proj, int proj_width
 // Floats of the scratch that thn_state_space needs for a step of n_rows rows.
 THN_API long long thn_state_space_scratch_floats(int n_rows, int n_heads, int vdim, int n_state, int n_groups) {
     return (long long)n_rows * ((long long)n_groups * 2 * padded_keys(n_state) + (long long)n_heads * (padded_values(vdim) + kRecurrenceTail));
+}
+
+// Bytes of the scratch that thn_state_space_chunks needs for a step of n_rows rows.
+THN_API long long thn_state_space_chunks_scratch_bytes(int n_rows, int n_heads, int vdim, int n_groups) {
+    return (long long)n_rows * (6ll * n_groups * chunk::kKeyRow * 2 + (long long)n_heads * (3 * chunk::kScoreRow * 2 + 16 + vdim * 4 + 4));
+}
+
+// thn_state_space chunk by chunk: bfloat16 rows in whole 8-byte pieces, four taps, a state of 128, vdim a multiple of 16;
+// max_tokens: the most rows of a sequence.
+THN_API int thn_state_space_chunks(float* y, float* state, void* scratch, const void* proj, int proj_width, int offset,
+                                   const float* conv_w, const float* conv_b, const void* ring, const float* dt_pre,
+                                   const float* dt_bias, const float* rate, const float* skip, const int* row_slot, const int* row_pos,
+                                   const int* seq_lens, const int* cu_seqlens, const int* slots, int n_rows, int max_tokens, int n_seqs,
+                                   int n_heads, int vdim, int n_state, int n_groups, int taps, cudaStream_t stream) {
+    const SpaceShape s{n_heads, vdim, n_state, n_groups, taps};
+    if (int status = check_shape("state_space_chunks", s, proj_width, offset)) return status;
+    THN_UNSUPPORTED_IF(n_state != chunk::kKeys || vdim % 16 != 0 || taps != kChunkTaps || proj_width % 4 != 0 || offset % 4 != 0,
+                       "state_space_chunks: a state of %d, values of %d, %d taps, rows of %d from %d", n_state, vdim, taps, proj_width, offset);
+    THN_UNSUPPORTED_IF(n_heads > 65535 || n_seqs > 65535 || (n_rows + kRunRows - 1) / kRunRows > 65535,
+                       "state_space_chunks: %d heads, %d sequences, %d rows", n_heads, n_seqs, n_rows);
+    THN_CHECK_ARG(scratch && (((uintptr_t)state | (uintptr_t)scratch | (uintptr_t)conv_w) & 15) == 0 &&
+                      (((uintptr_t)proj | (uintptr_t)ring) & 7) == 0,
+                  "state_space_chunks: operands are not aligned");
+    if (n_seqs <= 0 || n_rows <= 0 || max_tokens <= 0) return THN_OK;
+    const long long plane = (long long)n_rows * chunk::kKeyRow;
+    __nv_bfloat16* planes = static_cast<__nv_bfloat16*>(scratch);
+    __nv_bfloat16* scores = planes + 6 * n_groups * plane;
+    float4* scalars = reinterpret_cast<float4*>(scores + (size_t)3 * n_heads * n_rows * chunk::kScoreRow);
+    float* values = reinterpret_cast<float*>(scalars + (size_t)n_heads * n_rows);
+    float* steps = values + (size_t)n_heads * n_rows * vdim;
+    const int items = s.channels() / 4 + n_heads;
+    thn_launch(state_space_prepare_chunks_kernel, dim3((items + kPrepareThreads - 1) / kPrepareThreads, (n_rows + kRunRows - 1) / kRunRows),
+               kPrepareThreads, 0, stream, planes, values, steps, (const __nv_bfloat16*)proj, proj_width, offset, conv_w, conv_b,
+               (const __nv_bfloat16*)ring, dt_pre, dt_bias, row_slot, row_pos, seq_lens, n_rows, s);
+    cudaFuncSetAttribute(state_space_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSpaceChunkBytes);
+    thn_launch(state_space_chunk_kernel, dim3((max_tokens + chunk::kTokens - 1) / chunk::kTokens, n_groups, n_seqs), 128, kSpaceChunkBytes,
+               stream, scores, scalars, planes, steps, rate, skip, cu_seqlens, n_rows, n_heads / n_groups);
+    chunk::WalkArgs a{};
+    a.o = y; a.state = state;
+    a.k = planes; a.q = planes + 3 * plane;
+    a.key_plane = plane; a.key_unit = 6 * plane; a.key_row = chunk::kKeyRow;
+    a.v = values; a.v_row = vdim; a.v_head = (long long)n_rows * vdim;
+    a.scores = scores; a.scalars = scalars;
+    a.cu_seqlens = cu_seqlens; a.slots = slots;
+    a.n_rows = n_rows; a.n_heads = n_heads; a.heads_per_unit = n_heads / n_groups; a.value_dim = vdim; a.scale = 1.f;
+    const long long pairs = (long long)n_seqs * n_heads;
+    const char* env = getenv("WALK_SHAPE");
+    const int force = env ? atoi(env) : 0;
+    if (force == 41) chunk::launch_walk<float, 4, 1, false, false, 1>(a, n_seqs, stream);
+    else if (force == 42) chunk::launch_walk<float, 4, 2, false, false, 1>(a, n_seqs, stream);
+    else if (force == 412) chunk::launch_walk<float, 4, 1, false, false, 2>(a, n_seqs, stream);
+    else if (force ? force == 422 : (vdim % 64 == 0 && pairs * (vdim / 64) >= 128)) chunk::launch_walk<float, 4, 2, false, false, 2>(a, n_seqs, stream);
+    else if (force ? force == 242 : (vdim % 32 == 0 && pairs * (vdim / 32) >= 128)) chunk::launch_walk<float, 2, 4, false, false, 2>(a, n_seqs, stream);
+    else chunk::launch_walk<float, 1, 4, false, false, 2>(a, n_seqs, stream);
+    return thn_launch_status("state_space_chunks");
 }
 
 // y float32 [rows, heads, vdim]; state float32 [slots, heads, vdim, n_state], read and updated; the raw

@@ -96,6 +96,9 @@ _SIGNATURES = {
     "thn_state_space": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                         c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                         c_int, c_int, c_int, c_int, c_void_p],
+    "thn_state_space_chunks": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
+                               c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
+                               c_int, c_int, c_int, c_int, c_int, c_void_p],
     "thn_state_space_decode": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                c_void_p],
@@ -114,6 +117,8 @@ _SIGNATURES = {
     "thn_mlstm_gates": [c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_int, c_int, c_void_p],
     "thn_mlstm_recurrence": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_float, c_int,
                              c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_void_p],
+    "thn_mlstm_chunks": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_float, c_void_p,
+                         c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p],
     "thn_moe_route": [c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_float,
                       c_int, c_int, c_float, c_void_p],
     "thn_routed_gelu": [c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p],
@@ -203,6 +208,10 @@ def lib():
         loaded.thn_set_recurrence_columns.restype = None
         loaded.thn_delta_chunks_scratch_bytes.argtypes = [c_int, c_int, c_int, c_int]
         loaded.thn_delta_chunks_scratch_bytes.restype = c_longlong
+        loaded.thn_mlstm_chunks_scratch_bytes.argtypes = [c_int, c_int, c_int, c_int]
+        loaded.thn_mlstm_chunks_scratch_bytes.restype = c_longlong
+        loaded.thn_state_space_chunks_scratch_bytes.argtypes = [c_int, c_int, c_int, c_int]
+        loaded.thn_state_space_chunks_scratch_bytes.restype = c_longlong
         loaded.thn_wkv_scratch_floats.argtypes = [c_int, c_int, c_int]
         loaded.thn_wkv_scratch_floats.restype = c_longlong
         loaded.thn_state_space_scratch_floats.argtypes = [c_int, c_int, c_int, c_int, c_int]
@@ -1536,10 +1545,23 @@ def mlstm_column_blocks(value_dim: int) -> int:
     return -(-int(value_dim) // MLSTM_COLUMNS_PER_BLOCK)
 
 
+_mlstm_chosen = "THN_MLSTM_STAGED" in os.environ or "THN_MLSTM_LANES" in os.environ      # a token-by-token kernel was asked for
+
+
 def set_mlstm_kernel(staged: bool = True, lanes: int = 0) -> None:
     """Which kernel steps of several tokens take (tests and measurement): the one that stages
-    tokens in shared memory or the plain one; 8, 16 or 32 lanes per column, or 0: by the step's size."""
+    tokens in shared memory or the plain one; 8, 16 or 32 lanes per column, or 0: by the step's size.
+    Staged with 0 lanes also lets steps that can be walked in chunks be."""
+    global _mlstm_chosen
+    _mlstm_chosen = not staged or lanes != 0
     lib().thn_set_mlstm_staged(int(bool(staged)), int(lanes))
+
+
+def _mlstm_in_chunks(proj: torch.Tensor, state: torch.Tensor, rows: StepRows, n_heads: int, key_dim: int, value_dim: int) -> bool:
+    """Whether a step's recurrence is walked in chunks of tokens on the tensor cores."""
+    return proj.dtype == torch.bfloat16 and key_dim == CHUNK_KEYS and value_dim % 16 == 0 and not _mlstm_chosen \
+        and rows.max_q_len >= CHUNK_MIN_TOKENS and proj.shape[1] % 8 == 0 and max(n_heads, rows.n_seqs) <= 65535 \
+        and proj.shape[1] >= n_heads * (2 * key_dim + value_dim) and (state.data_ptr() | proj.data_ptr()) % 16 == 0
 
 
 def mlstm(proj: torch.Tensor, gate_pre: torch.Tensor, bias_i: torch.Tensor, bias_f: torch.Tensor, cap: float,
@@ -1566,6 +1588,13 @@ def mlstm(proj: torch.Tensor, gate_pre: torch.Tensor, bias_i: torch.Tensor, bias
                           f"{tuple(state.shape)}, normaliser {tuple(normaliser.shape)} do not fit {n_heads} heads of "
                           f"{key_dim} x {value_dim}")
     o = torch.empty((n, n_heads, value_dim), dtype=torch.float32, device=proj.device)
+    if _mlstm_in_chunks(proj, state, rows, n_heads, key_dim, value_dim):
+        scratch = torch.empty(lib().thn_mlstm_chunks_scratch_bytes(n, rows.max_q_len, rows.n_seqs, n_heads), dtype=torch.uint8,
+                              device=proj.device)
+        _call("thn_mlstm_chunks", _ptr(o), _ptr(state), _ptr(normaliser), _ptr(scratch), _ptr(proj), proj.shape[1], _ptr(gate_pre),
+              _ptr(bias_i), _ptr(bias_f), float(cap), _ptr(rows.cu_seqlens), _ptr(rows.slots), n, rows.max_q_len, rows.n_seqs, n_heads,
+              key_dim, value_dim, float(q_scale), float(floor), _stream())
+        return o
     raw = rows.max_q_len == 1
     gates = gate_pre
     if not raw:
@@ -1932,6 +1961,14 @@ class StateSpace:
         return self.conv_w.shape[1]
 
 
+def _space_in_chunks(proj: torch.Tensor, offset: int, state: torch.Tensor, ring: torch.Tensor, rows: StepRows, s: StateSpace) -> bool:
+    """Whether a step's recurrence is walked in chunks of tokens on the tensor cores."""
+    return proj.dtype == torch.bfloat16 and s.n_state == CHUNK_KEYS and s.vdim % 16 == 0 and s.taps == 4 \
+        and rows.max_q_len >= CHUNK_MIN_TOKENS and proj.shape[1] % 4 == 0 and offset % 4 == 0 and rows.n_rows <= 8 * 65535 \
+        and max(s.n_heads, rows.n_seqs) <= 65535 and 0 <= offset <= proj.shape[1] - s.channels \
+        and (state.data_ptr() | s.conv_w.data_ptr()) % 16 == 0 and (proj.data_ptr() | ring.data_ptr()) % 8 == 0
+
+
 def state_space(proj: torch.Tensor, offset: int, dt_pre: torch.Tensor, shape: StateSpace, state: torch.Tensor,
                 ring: torch.Tensor, rows: StepRows, seq_lens: torch.Tensor) -> torch.Tensor:
     """State-space duality over a step's rows: the short causal convolution (bias, silu) over the
@@ -1961,6 +1998,15 @@ def state_space(proj: torch.Tensor, offset: int, dt_pre: torch.Tensor, shape: St
         _call("thn_state_space_decode", _ptr(y), _ptr(state), _ptr(proj), proj.shape[1], int(offset), _ptr(s.conv_w),
               _ptr(s.conv_b), _ptr(ring), _ptr(dt_pre), _ptr(s.dt_bias), _ptr(s.rate), _ptr(s.skip), _ptr(rows.row_slot),
               _ptr(rows.row_pos), n, s.n_heads, s.vdim, s.n_state, s.n_groups, s.taps, code, _stream())
+        return y
+    if _space_in_chunks(proj, offset, state, ring, rows, s):
+        scratch = torch.empty(lib().thn_state_space_chunks_scratch_bytes(n, s.n_heads, s.vdim, s.n_groups), dtype=torch.uint8,
+                              device=proj.device)
+        _call("thn_state_space_chunks", _ptr(y), _ptr(state), _ptr(scratch), _ptr(proj), proj.shape[1], int(offset), _ptr(s.conv_w),
+              _ptr(s.conv_b), _ptr(ring), _ptr(dt_pre), _ptr(s.dt_bias), _ptr(s.rate), _ptr(s.skip), _ptr(rows.row_slot),
+              _ptr(rows.row_pos), _ptr(seq_lens), _ptr(rows.cu_seqlens), _ptr(rows.slots), n, rows.max_q_len, rows.n_seqs, s.n_heads,
+              s.vdim, s.n_state, s.n_groups, s.taps, _stream())
+        conv_ring_update(ring, proj, offset, rows, seq_lens)
         return y
     scratch = torch.empty(lib().thn_state_space_scratch_floats(n, s.n_heads, s.vdim, s.n_state, s.n_groups), dtype=torch.float32,
                           device=proj.device)
