@@ -70,3 +70,81 @@ def test_delta_matches_64_bits(lens, held, n_heads, n_kv, vdim):
     for i, slot in enumerate(slots):
         for r in range(max(cu[i], cu[i + 1] - (taps - 1)), cu[i + 1]):
             assert torch.equal(got_ring[slot, (held + r - cu[i]) % taps].cpu(), proj[r, :shape.conv_channels])
+
+
+@pytest.mark.parametrize("lens,n_heads,vdim", [
+    ([16], 2, 128), ([31, 1, 33], 3, 16), ([32, 64, 65, 2], 2, 48), ([97], 4, 256), ([40] * 8, 16, 128), ([70, 35], 1, 64)])
+def test_matrix_memory_matches_64_bits(lens, n_heads, vdim):
+    g = torch.Generator().manual_seed(sum(lens) + vdim)
+    rows, _, cu, slots = step(lens)
+    dev, key, cap, scale = rows.slots.device, 128, 15.0, 128 ** -0.5
+    draw = lambda *s: torch.randn(*s, generator=g)
+    proj = draw(cu[-1], n_heads * (2 * key + vdim) + 8 * (n_heads % 2)).to(BF16)
+    pre, bias_i, bias_f = draw(cu[-1], 2 * n_heads) * 3, draw(n_heads) * 2, draw(n_heads) * 2 + 1
+    state = draw(len(lens) + 1, n_heads, vdim, key)
+    normaliser = draw(len(lens) + 1, n_heads, 1, key + 1).expand(-1, -1, vdim // 16, -1).contiguous()
+    got_state, got_normaliser = state.to(dev), normaliser.to(dev)
+    assert ops._mlstm_in_chunks(proj.to(dev), got_state, rows, n_heads, key, vdim)
+    got = ops.mlstm(proj.to(dev), pre.to(dev), bias_i.to(dev), bias_f.to(dev), cap, got_state, got_normaliser, rows, n_heads, key,
+                    vdim, scale).cpu()
+    gi = cap * torch.tanh((pre[:, :n_heads].double() + bias_i.double()) / cap)
+    gf = torch.nn.functional.logsigmoid(cap * torch.tanh((pre[:, n_heads:].double() + bias_f.double()) / cap))
+    parts = proj.double()
+    for i, slot in enumerate(slots):
+        S, n, m = state[slot].double(), normaliser[slot, :, 0, :key].double(), normaliser[slot, :, 0, key].double()
+        for r in range(cu[i], cu[i + 1]):
+            q, k = parts[r, :n_heads * key].view(n_heads, key) * scale, parts[r, n_heads * key:2 * n_heads * key].view(n_heads, key)
+            v = parts[r, 2 * n_heads * key:n_heads * (2 * key + vdim)].view(n_heads, vdim)
+            top = torch.maximum(gf[r] + m, gi[r])
+            keep, take, m = torch.exp(gf[r] + m - top), torch.exp(gi[r] - top), top
+            S = keep[:, None, None] * S + take[:, None, None] * v[:, :, None] * k[:, None, :]
+            n = keep[:, None] * n + take[:, None] * k
+            below = torch.maximum((n * q).sum(-1).abs(), torch.exp(-m)) + 1e-6
+            want = torch.einsum("hek,hk->he", S, q) / below[:, None]
+            # the maximum is of the order of ten, so its roundings (2^-21 a step) weigh on every exponential; a denominator
+            # that cancels magnifies the error of n . q by |n| |q| over itself
+            slack = (1 + (n.norm(dim=-1) * q.norm(dim=-1) / below))[:, None] * want.abs().amax(dim=-1, keepdim=True)
+            assert ((got[r].double() - want).abs() <= (64 + 2 * len(range(cu[i], r + 1))) * 2 ** -23 * slack).all()
+        scale_s = S.abs().amax()
+        bound = (64 + 2 * lens[i]) * 2 ** -23
+        assert (got_state[slot].cpu().double() - S).abs().max() <= bound * scale_s
+        copies = got_normaliser[slot].cpu().double()
+        assert (copies[:, :, :key] - n[:, None]).abs().max() <= bound * n.abs().amax()
+        assert (copies[:, :, key] - m[:, None]).abs().max() <= bound * m.abs().amax().clamp(min=1)
+
+
+@pytest.mark.parametrize("lens,held,n_heads,groups,vdim", [
+    ([112], 0, 4, 2, 64), ([1, 129, 33], 0, 2, 2, 16), ([160, 2], 3, 8, 1, 96), ([115, 64], 1, 64, 8, 128), ([113] * 3, 0, 128, 4, 64)])
+def test_state_space_matches_64_bits(lens, held, n_heads, groups, vdim):
+    g = torch.Generator().manual_seed(sum(lens) + vdim)
+    rows, seq_lens, cu, slots = step(lens, held)
+    dev, n, taps, offset = rows.slots.device, 128, 4, 8
+    draw = lambda *s: torch.randn(*s, generator=g)
+    inner = n_heads * vdim
+    channels = inner + 2 * groups * n
+    shape = ops.StateSpace(n_heads, vdim, n, groups, draw(channels, taps) * 0.5, draw(channels) * 0.1, draw(n_heads) - 2,
+                           torch.exp(draw(n_heads)), draw(n_heads))
+    there = ops.StateSpace(n_heads, vdim, n, groups, *(t.to(dev) for t in (shape.conv_w, shape.conv_b, shape.dt_bias, shape.rate, shape.skip)))
+    proj, dt = draw(cu[-1], offset + channels).to(BF16), draw(cu[-1], n_heads)
+    state, ring = draw(len(lens) + 1, n_heads, vdim, n) * 0.2, draw(len(lens) + 1, taps, channels).to(BF16)
+    got_state, got_ring = state.to(dev), ring.to(dev)
+    assert ops._space_in_chunks(proj.to(dev), offset, got_state, got_ring, rows, there)
+    got = ops.state_space(proj.to(dev), offset, dt.to(dev), there, got_state, got_ring, rows, seq_lens)
+    want, want_state = torch.zeros(cu[-1], n_heads, vdim, dtype=torch.float64), state.double()
+    size = torch.nn.functional.softplus(dt.double() + shape.dt_bias.double())
+    decay = torch.exp(-shape.rate.double() * size)
+    for i, slot in enumerate(slots):
+        S = want_state[slot]
+        for r in range(cu[i], cu[i + 1]):
+            pos, acc = held + r - cu[i], shape.conv_b.double()
+            for back in range(min(taps - 1, pos) + 1):
+                raw = proj[r - back, offset:] if back <= r - cu[i] else ring[slot, (pos - back) % taps]
+                acc = acc + shape.conv_w[:, taps - 1 - back].double() * raw.double()
+            y = torch.nn.functional.silu(acc)
+            x = y[:inner].view(n_heads, vdim)
+            B, C = (y[inner + a * groups * n:inner + (a + 1) * groups * n].view(groups, n).repeat_interleave(n_heads // groups, 0) for a in (0, 1))
+            S = decay[r][:, None, None] * S + (size[r][:, None] * x)[:, :, None] * B[:, None, :]
+            want[r] = torch.einsum("hek,hk->he", S, C) + shape.skip.double()[:, None] * x
+        want_state[slot] = S
+    close(got.cpu(), want, max(lens))
+    close(got_state.cpu()[1:], want_state[1:], max(lens))

@@ -206,7 +206,7 @@ struct Layout {
 };
 
 template <typename T, int CG, int KS, bool DELTA, bool GATED, int STAGES>
-__global__ void __launch_bounds__(32 * CG * KS) walk_kernel(WalkArgs a) {
+__global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * KS) : 1) walk_kernel(WalkArgs a) {
     using L = Layout<T, CG, KS, DELTA, STAGES>;
     constexpr int PARTS = L::kParts;
     constexpr int KT = kKeys / KS / 8;               // groups of 8 keys of a warp
