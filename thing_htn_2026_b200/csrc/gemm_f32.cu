@@ -72,72 +72,72 @@ THN_API int thn_gemm_f32(float* C, const float* A, const float* W, int M, int N,
 //
 // C[M, N] float32 = A[M, K] bfloat16 @ W[N, K]^T bfloat16 for a weight of few rows (a router, a
 // gate of one number per token): the products that vendor libraries serve worst, since N is
-// neither large nor a multiple of eight.  A block of eight warps takes ROWS rows of A and walks
-// the outputs four at a time: a thread's 16-byte pieces k = t, t + 256, ... of the rows and of
-// four weight rows are loaded side by side (one round trip to memory), multiplied in float32,
-// summed over the warp by shuffles and over the warps in a fixed order.  A row's result depends on
-// nothing but K, whatever ROWS is.  K is a multiple of eight and both operands are 16-byte aligned.
+// neither large nor a multiple of eight.  A block takes 16 rows and 8 TILES columns; its eight warps deal out
+// K in steps of 32 on the tensor cores, each step into a fresh accumulator (the tensor core's accumulation
+// rounds towards zero, the sum over the steps is float32 additions).  A lane loads its operands straight from
+// memory, 16 bytes of a row at k = 32 s + 8 t: which k a lane's pair stands for does not matter as long as
+// both operands agree.  The warps' sums meet in shared memory in a fixed order, so a row's result depends on
+// nothing but K, whatever M, N and TILES are.  K is a multiple of eight and both operands are 16-byte aligned.
+// 2,251 rows, 32 columns over 2,048 on B200: 31 us in float32 multiply-adds, four rows a block (each block
+// reads the whole weight; a quarter as many do here).
 namespace {
 constexpr int kSkinnyThreads = 256;
 
-__device__ __forceinline__ float dot8(const uint4& a, const uint4& b, float acc) {
-    const __nv_bfloat162* x = reinterpret_cast<const __nv_bfloat162*>(&a);
-    const __nv_bfloat162* y = reinterpret_cast<const __nv_bfloat162*>(&b);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float2 u = __bfloat1622float2(x[i]), v = __bfloat1622float2(y[i]);
-        acc = fmaf(u.x, v.x, acc);
-        acc = fmaf(u.y, v.y, acc);
-    }
-    return acc;
+__device__ __forceinline__ void skinny_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-template <int ROWS>
+template <int TILES>
 __global__ void __launch_bounds__(kSkinnyThreads) linear_skinny_kernel(float* __restrict__ C,
                                                                        const __nv_bfloat16* __restrict__ A,
                                                                        const __nv_bfloat16* __restrict__ W, int M, int N,
                                                                        int vecs) {
     pdl_launch_dependents();
     pdl_wait();
-    __shared__ float part[kSkinnyThreads / 32][ROWS * 4];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int m0 = blockIdx.x * ROWS;
+    constexpr int kWarps = kSkinnyThreads / 32;
+    __shared__ __align__(16) float part[kWarps][TILES][32][4];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int m0 = blockIdx.x * 16, n0 = blockIdx.y * 8 * TILES;
     const uint4* a = reinterpret_cast<const uint4*>(A);
     const uint4* w = reinterpret_cast<const uint4*>(W);
     const uint4 zero = make_uint4(0, 0, 0, 0);
-    for (int n0 = blockIdx.y * 4; n0 < N; n0 += gridDim.y * 4) {        // four columns at a time
-        float acc[ROWS][4];
+    const bool lo = m0 + g < M, hi = m0 + g + 8 < M;
+    const size_t at_lo = (size_t)(m0 + g) * vecs, at_hi = (size_t)(m0 + g + 8) * vecs;
+    float acc[TILES][4];
 #pragma unroll
-        for (int r = 0; r < ROWS; ++r)
+    for (int n = 0; n < TILES; ++n)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) acc[r][j] = 0.f;
-        for (int i = threadIdx.x; i < vecs; i += kSkinnyThreads) {
-            uint4 av[ROWS], wv[4];
+        for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
+    const int steps = (vecs + 3) / 4;
+#pragma unroll 4
+    for (int s = warp; s < steps; s += kWarps) {
+        const int v = 4 * s + t;                     // this lane's 16 bytes of a row
+        const bool in = v < vecs;
+        const uint4 x = in && lo ? a[at_lo + v] : zero, y = in && hi ? a[at_hi + v] : zero;
+        uint4 z[TILES];
 #pragma unroll
-            for (int r = 0; r < ROWS; ++r) av[r] = m0 + r < M ? a[(size_t)(m0 + r) * vecs + i] : zero;
+        for (int n = 0; n < TILES; ++n) z[n] = in && n0 + 8 * n + g < N ? __ldg(w + (size_t)(n0 + 8 * n + g) * vecs + v) : zero;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) wv[j] = n0 + j < N ? __ldg(w + (size_t)(n0 + j) * vecs + i) : zero;
+        for (int n = 0; n < TILES; ++n) {
+            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+            skinny_mma(sum, x.x, y.x, x.y, y.y, z[n].x, z[n].y);
+            skinny_mma(sum, x.z, y.z, x.w, y.w, z[n].z, z[n].w);
 #pragma unroll
-            for (int r = 0; r < ROWS; ++r)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[r][j] = dot8(av[r], wv[j], acc[r][j]);
+            for (int i = 0; i < 4; ++i) acc[n][i] += sum[i];
         }
+    }
 #pragma unroll
-        for (int r = 0; r < ROWS; ++r)
+    for (int n = 0; n < TILES; ++n) *reinterpret_cast<float4*>(part[warp][n][lane]) = make_float4(acc[n][0], acc[n][1], acc[n][2], acc[n][3]);
+    __syncthreads();
+    for (int e = threadIdx.x; e < TILES * 128; e += kSkinnyThreads) {
+        const int n = e >> 7, l = e >> 2 & 31, i = e & 3;
+        float total = 0.f;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float total = warp_sum(acc[r][j]);
-                if (lane == 0) part[warp][r * 4 + j] = total;
-            }
-        __syncthreads();
-        if (threadIdx.x < ROWS * 4) {
-            const int r = threadIdx.x >> 2, j = threadIdx.x & 3;
-            float total = 0.f;
-#pragma unroll
-            for (int k = 0; k < kSkinnyThreads / 32; ++k) total += part[k][threadIdx.x];
-            if (m0 + r < M && n0 + j < N) C[(size_t)(m0 + r) * N + n0 + j] = total;
-        }
-        __syncthreads();
+        for (int k = 0; k < kWarps; ++k) total += part[k][n][l][i];
+        const int row = m0 + (l >> 2) + 8 * (i >> 1), col = n0 + 8 * n + 2 * (l & 3) + (i & 1);
+        if (row < M && col < N) C[(size_t)row * N + col] = total;
     }
 }
 }  // namespace
@@ -148,13 +148,13 @@ THN_API int thn_linear_skinny_bf16(float* C, const void* A, const void* W, int M
     THN_CHECK_ARG(M >= 0 && thn_linear_skinny_supported(N, K), "linear_skinny: bad sizes M=%d N=%d K=%d", M, N, K);
     THN_CHECK_ARG((((uintptr_t)A | (uintptr_t)W) & 15) == 0, "linear_skinny: operands must be 16-byte aligned (M=%d)", M);
     if (M == 0) return THN_OK;
-    if (M >= 1024) {    // enough rows to fill the SMs four at a time: the weight's rows are read a quarter as often
-        thn_launch(linear_skinny_kernel<4>, (M + 3) / 4, kSkinnyThreads, 0, stream, C, (const __nv_bfloat16*)A,
+    // four tiles of columns a block read A a quarter as often; one tile a block where that leaves multiprocessors idle
+    const int row_blocks = (M + 15) / 16, tiles = (N + 7) / 8;
+    if (row_blocks * ((tiles + 3) / 4) >= 120)
+        thn_launch(linear_skinny_kernel<4>, dim3(row_blocks, (tiles + 3) / 4), kSkinnyThreads, 0, stream, C, (const __nv_bfloat16*)A,
                    (const __nv_bfloat16*)W, M, N, K / 8);
-    } else {            // few rows: the columns are dealt out as well, until there are about two blocks per SM
-        const int groups = (N + 3) / 4, want = (2 * 148 + M - 1) / M;
-        thn_launch(linear_skinny_kernel<1>, dim3(M, groups < want ? groups : want), kSkinnyThreads, 0, stream, C, (const __nv_bfloat16*)A,
+    else
+        thn_launch(linear_skinny_kernel<1>, dim3(row_blocks, tiles), kSkinnyThreads, 0, stream, C, (const __nv_bfloat16*)A,
                    (const __nv_bfloat16*)W, M, N, K / 8);
-    }
     return thn_launch_status("linear_skinny");
 }

@@ -207,6 +207,67 @@ __global__ void __launch_bounds__(256) latent_assemble_vec_kernel(
     // work items of a head: plain pieces, turned pieces (pairs of them for half pairs), value pieces
     const int plain_items = plain / 8, turned_items = interleaved ? rot / 8 : half / 8, value_items = DV / 8;
     const int per_head = plain_items + turned_items + value_items;
+    if (blockDim.x % per_head == 0) {
+        // a thread does the same piece of every head that it comes to: four heads' loads at a time, ahead of their stores
+        // (a store may alias a later load as far as the compiler knows); the shared key part is turned once
+        const int i = threadIdx.x % per_head, step = gridDim.y * blockDim.x / per_head;
+        const int h0 = (blockIdx.y * blockDim.x + threadIdx.x) / per_head;
+        const int j = i < plain_items ? i * 8 : i < plain_items + turned_items ? (i - plain_items) * 8 : (i - plain_items - turned_items) * 8;
+        const bool is_plain = i < plain_items, is_turned = !is_plain && i < plain_items + turned_items;
+        if (!is_plain && !is_turned && !cache) return;
+        uint4 key_lo = make_uint4(0, 0, 0, 0), key_hi = key_lo;
+        if (is_turned && cache) {
+            if (interleaved) key_lo = turn_four_pairs(piece(k_shared + j), c_row + j / 2, s_row + j / 2);
+            else turn_eight(piece(k_shared + j), piece(k_shared + half + j), c_row + j, s_row + j, key_lo, key_hi);
+        }
+        constexpr int U = 4;
+        for (int first = h0; first < n_heads; first += U * step) {
+            uint4 x[U], y[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int h = first + u * step;
+                if (h >= n_heads) continue;
+                const __nv_bfloat16* q = q_row + (size_t)h * D;
+                if (is_plain) {
+                    x[u] = piece(q + j);
+                    if (cache) y[u] = piece(up_row + (size_t)h * plain + j);
+                } else if (is_turned) {
+                    x[u] = piece(q + plain + j);
+                    if (!interleaved) y[u] = piece(q + plain + half + j);
+                } else {
+                    x[u] = j < value_src ? piece(up_row + (size_t)n_heads * plain + (size_t)h * value_src + j) : make_uint4(0, 0, 0, 0);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int h = first + u * step;
+                if (h >= n_heads) continue;
+                __nv_bfloat16* dst = q_out + ((size_t)m * n_heads + h) * D;
+                __nv_bfloat16* key = cache ? cache + keys0 + h * key_step : nullptr;
+                if (is_plain) {
+                    put(dst + j, x[u]);
+                    if (key) put(key + j, y[u]);
+                } else if (is_turned) {
+                    if (interleaved) {
+                        put(dst + plain + j, turn_four_pairs(x[u], c_row + j / 2, s_row + j / 2));
+                        if (key) put(key + plain + j, key_lo);
+                    } else {
+                        uint4 a, b;
+                        turn_eight(x[u], y[u], c_row + j, s_row + j, a, b);
+                        put(dst + plain + j, a);
+                        put(dst + plain + half + j, b);
+                        if (key) {
+                            put(key + plain + j, key_lo);
+                            put(key + plain + half + j, key_hi);
+                        }
+                    }
+                } else {
+                    put(cache + values0 + h * value_step + j, x[u]);
+                }
+            }
+        }
+        return;
+    }
     for (int item = blockIdx.y * blockDim.x + threadIdx.x; item < n_heads * per_head; item += gridDim.y * blockDim.x) {
         const int h = item / per_head, i = item - h * per_head;
         const __nv_bfloat16* q = q_row + (size_t)h * D;

@@ -100,6 +100,44 @@ __global__ void linear_attention_prepare_kernel(float* __restrict__ prepared, co
     prepared[e] = v;
 }
 
+// The same for bfloat16 rows in whole groups of four entries: a thread per group, 8 bytes in and 16 out (1,531 rows
+// of 32 heads of 128 with gated decays on B200: 137 us above, with 2-byte accesses and two divisions an entry).
+__global__ void __launch_bounds__(256) linear_attention_prepare_vec_kernel(
+    float* __restrict__ prepared, const __nv_bfloat16* __restrict__ proj, int proj_width, int q_offset, int k_offset, int v_offset,
+    const float* __restrict__ gate, int gate_width, const float* __restrict__ gate_bias, float inv_tau, int n_heads, int key_dim,
+    int value_dim, int kp, int vp, int parts, int silu_inputs) {
+    pdl_launch_dependents();
+    pdl_wait();
+    using T = __nv_bfloat16;
+    const int per_head = parts * kp + vp, item = (blockIdx.y * 256 + threadIdx.x) * 4;
+    if (item >= n_heads * per_head) return;
+    const int head = item / per_head, c = item - head * per_head;
+    const long long row = blockIdx.x;
+    const int part = c >= parts * kp ? 3 : c / kp;              // k, q, decay, v
+    const int d = part == 3 ? c - parts * kp : c - part * kp;
+    float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (part == 2) {
+        if (d < key_dim) {
+            const int at = head * key_dim + d;
+            out = *reinterpret_cast<const float4*>(gate + row * gate_width + at);
+            if (gate_bias) {
+                const float4 b = *reinterpret_cast<const float4*>(gate_bias + at);
+                out.x += b.x; out.y += b.y; out.z += b.z; out.w += b.w;
+            }
+            out.x = logistic_power<T>(out.x, inv_tau); out.y = logistic_power<T>(out.y, inv_tau);
+            out.z = logistic_power<T>(out.z, inv_tau); out.w = logistic_power<T>(out.w, inv_tau);
+        }
+    } else if (d < (part == 3 ? value_dim : key_dim)) {
+        const T* src = proj + row * proj_width + (part == 3 ? v_offset + head * value_dim : (part == 0 ? k_offset : q_offset) + head * key_dim) + d;
+        const uint2 raw = *reinterpret_cast<const uint2*>(src);
+        const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+        const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+        out = make_float4(lo.x, lo.y, hi.x, hi.y);
+        if (silu_inputs) out = make_float4(silu_of<T>(out.x), silu_of<T>(out.y), silu_of<T>(out.z), silu_of<T>(out.w));
+    }
+    *reinterpret_cast<float4*>(prepared + row * n_heads * per_head + item) = out;
+}
+
 // PER: key channels per lane (a multiple of 4); KP = 16 * PER: the padded key size.  COLS: columns per lane.
 template <int PER, int COLS, int KIND>
 __global__ void __launch_bounds__(kLanes * kColumns / COLS) linear_attention_kernel(
@@ -325,7 +363,14 @@ int launch(float* o, float* state, float* prepared, const void* proj, int proj_w
            float q_scale, int mode, int silu_inputs, cudaStream_t stream) {
     const int kp = padded_keys(key_dim), vp = padded_values(value_dim), parts = key_parts(mode), per_head = parts * kp + vp;
     const long long n = (long long)n_rows * n_heads * per_head;
-    thn_launch(linear_attention_prepare_kernel<T>, (unsigned)((n + 255) / 256), 256, 0, stream, prepared, (const T*)proj,
+    const long long blocks = ((long long)n_heads * per_head / 4 + 255) / 256;
+    if (sizeof(T) == 2 && (key_dim | value_dim | proj_width | q_offset | k_offset | v_offset | gate_width) % 4 == 0 && blocks <= 65535 &&
+        ((uintptr_t)proj & 7) == 0 && (((uintptr_t)gate | (uintptr_t)gate_bias) & 15) == 0)
+        thn_launch(linear_attention_prepare_vec_kernel, dim3(n_rows, (unsigned)blocks), 256, 0, stream, prepared, (const __nv_bfloat16*)proj,
+                   proj_width, q_offset, k_offset, v_offset, gate, gate_width, gate_bias, inv_tau, n_heads, key_dim, value_dim, kp, vp,
+                   parts, silu_inputs);
+    else
+        thn_launch(linear_attention_prepare_kernel<T>, (unsigned)((n + 255) / 256), 256, 0, stream, prepared, (const T*)proj,
                proj_width, q_offset, k_offset, v_offset, gate, gate_width, gate_bias, inv_tau, n, n_heads, key_dim, value_dim, kp,
                vp, parts, silu_inputs);
     return launch_recurrence(mode, RecurrenceArgs{o, state, prepared, per_head, n_heads, prepared + parts * kp, per_head, decay,

@@ -437,6 +437,53 @@ __global__ void __launch_bounds__(256) gated_group_norm_kernel(T* __restrict__ o
     for (int i = threadIdx.x; i < size; i += blockDim.x) dst[i] = from_f32<T>(src[i] * silu_of<T>(to_f32<T>(g[i])) * rstd * w[i]);
 }
 
+// The same for bfloat16 and parts of whole groups of 128 entries, up to 1,024: a warp per (row, part), the gated entries in
+// registers between the sum and the result, no barrier.  (4,096 rows of eight parts of 1,024 on B200: 95 us above.)
+__global__ void __launch_bounds__(256) gated_group_norm_warp_kernel(__nv_bfloat16* __restrict__ out, const float* __restrict__ y,
+                                                                    const __nv_bfloat16* __restrict__ gate, long long gate_stride,
+                                                                    const float* __restrict__ gain, float eps, int rows, int width,
+                                                                    int size, int parts) {
+    pdl_launch_dependents();
+    pdl_wait();
+    using T = __nv_bfloat16;
+    const long long unit = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (unit >= (long long)rows * parts) return;
+    const long long row = unit / parts;
+    const int part = (int)(unit - row * parts), lane = threadIdx.x & 31;
+    const float* src = y + row * width + (long long)part * size + lane * 4;
+    const T* g = gate + row * gate_stride + (long long)part * size + lane * 4;
+    const float* w = gain + (long long)part * size + lane * 4;
+    constexpr int kGroups = 8;
+    float4 kept[kGroups];
+    uint2 z[kGroups];
+#pragma unroll
+    for (int j = 0; j < kGroups; ++j)
+        if (j * 128 < size) {
+            kept[j] = *reinterpret_cast<const float4*>(src + j * 128);
+            z[j] = *reinterpret_cast<const uint2*>(g + j * 128);
+        }
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < kGroups; ++j)
+        if (j * 128 < size) {
+            const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&z[j].x));
+            const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&z[j].y));
+            kept[j].x *= silu_of<T>(lo.x); kept[j].y *= silu_of<T>(lo.y); kept[j].z *= silu_of<T>(hi.x); kept[j].w *= silu_of<T>(hi.y);
+            ss += kept[j].x * kept[j].x + kept[j].y * kept[j].y + kept[j].z * kept[j].z + kept[j].w * kept[j].w;
+        }
+    const float rstd = 1.0f / sqrtf(warp_sum(ss) / (float)size + eps);
+    T* dst = out + row * width + (long long)part * size + lane * 4;
+#pragma unroll
+    for (int j = 0; j < kGroups; ++j)
+        if (j * 128 < size) {
+            const float4 gw = *reinterpret_cast<const float4*>(w + j * 128);
+            uint2 packed;
+            *reinterpret_cast<__nv_bfloat162*>(&packed.x) = __floats2bfloat162_rn(kept[j].x * rstd * gw.x, kept[j].y * rstd * gw.y);
+            *reinterpret_cast<__nv_bfloat162*>(&packed.y) = __floats2bfloat162_rn(kept[j].z * rstd * gw.z, kept[j].w * rstd * gw.w);
+            *reinterpret_cast<uint2*>(dst + j * 128) = packed;
+        }
+}
+
 int check_shape(const char* what, const SpaceShape& s, int proj_width, int offset) {
     THN_CHECK_ARG(s.n_heads > 0 && s.vdim > 0 && s.n_state > 0 && s.n_groups > 0 && s.n_heads % s.n_groups == 0 && s.taps > 0,
                   "%s: %d heads of %d in %d groups, state %d, %d taps", what, s.n_heads, s.vdim, s.n_groups, s.n_state, s.taps);
@@ -596,6 +643,13 @@ THN_API int thn_gated_group_norm(void* out, const float* y, const void* gate, lo
     const size_t element = dtype == THN_BF16 ? 2 : 4;
     const int vec = size % 4 == 0 && gate_stride % 4 == 0 && (((uintptr_t)y | (uintptr_t)gain) & 15) == 0 &&
                     (((uintptr_t)gate | (uintptr_t)out) & (4 * element - 1)) == 0;
+    // (few parts are faster with a block each)
+    const long long units = (long long)rows * parts;
+    if (dtype == THN_BF16 && vec && size % 128 == 0 && size <= 1024 && units >= 1184) {
+        thn_launch(gated_group_norm_warp_kernel, (unsigned)((units + 7) / 8), 256, 0, stream, (__nv_bfloat16*)out, y,
+                   (const __nv_bfloat16*)gate, gate_stride, gain, eps, rows, width, size, parts);
+        return thn_launch_status("gated_group_norm");
+    }
     const dim3 grid(rows, parts);
     const int threads = size >= 1024 ? 256 : (size / 4 + 31) / 32 * 32 < 32 ? 32 : (size / 4 + 31) / 32 * 32;
     if (dtype == THN_F32)
