@@ -72,16 +72,15 @@ THN_API int thn_gemm_f32(float* C, const float* A, const float* W, int M, int N,
 //
 // C[M, N] float32 = A[M, K] bfloat16 @ W[N, K]^T bfloat16 for a weight of few rows (a router, a
 // gate of one number per token): the products that vendor libraries serve worst, since N is
-// neither large nor a multiple of eight.  A block takes 16 rows and 8 TILES columns; its eight warps deal out
-// K in steps of 32 on the tensor cores, each step into a fresh accumulator (the tensor core's accumulation
-// rounds towards zero, the sum over the steps is float32 additions).  A lane loads its operands straight from
-// memory, 16 bytes of a row at k = 32 s + 8 t: which k a lane's pair stands for does not matter as long as
-// both operands agree.  The warps' sums meet in shared memory in a fixed order, so a row's result depends on
-// nothing but K, whatever M, N and TILES are.  K is a multiple of eight and both operands are 16-byte aligned.
-// 2,251 rows, 32 columns over 2,048 on B200: 31 us in float32 multiply-adds, four rows a block (each block
-// reads the whole weight; a quarter as many do here).
+// neither large nor a multiple of eight.  A block takes 16 rows and 8 TILES columns; its sixteen warps deal out
+// K in steps of 32 on the tensor cores, each product into a fresh accumulator (the tensor core's accumulation
+// rounds towards zero, by kLean of the result on average, which is put back at the end; the sum over the steps is
+// float32 additions).  A lane loads its operands straight from memory, 16 bytes of a row at k = 32 s + 8 t: which
+// k a lane's pair stands for does not matter as long as both operands agree; the loads of four steps are issued
+// together.  The warps' sums meet in shared memory in a fixed order, so a row's result depends on nothing but K,
+// whatever M, N and TILES are.  K is a multiple of eight and both operands are 16-byte aligned.
 namespace {
-constexpr int kSkinnyThreads = 256;
+constexpr int kSkinnyThreads = 512;
 
 __device__ __forceinline__ void skinny_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%0,%1,%2,%3};"
@@ -96,48 +95,56 @@ __global__ void __launch_bounds__(kSkinnyThreads) linear_skinny_kernel(float* __
                                                                        int vecs) {
     pdl_launch_dependents();
     pdl_wait();
-    constexpr int kWarps = kSkinnyThreads / 32;
+    constexpr int kWarps = kSkinnyThreads / 32, kBatch = 4;
+    constexpr double kLean = 4.3e-8;
     __shared__ __align__(16) float part[kWarps][TILES][32][4];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int m0 = blockIdx.x * 16, n0 = blockIdx.y * 8 * TILES;
-    const uint4* a = reinterpret_cast<const uint4*>(A);
-    const uint4* w = reinterpret_cast<const uint4*>(W);
     const uint4 zero = make_uint4(0, 0, 0, 0);
-    const bool lo = m0 + g < M, hi = m0 + g + 8 < M;
-    const size_t at_lo = (size_t)(m0 + g) * vecs, at_hi = (size_t)(m0 + g + 8) * vecs;
+    // (rows and columns beyond the last repeat it; their results are not stored)
+    const uint4* a_lo = reinterpret_cast<const uint4*>(A) + (size_t)min(m0 + g, M - 1) * vecs;
+    const uint4* a_hi = reinterpret_cast<const uint4*>(A) + (size_t)min(m0 + g + 8, M - 1) * vecs;
+    const uint4* w[TILES];
+#pragma unroll
+    for (int n = 0; n < TILES; ++n) w[n] = reinterpret_cast<const uint4*>(W) + (size_t)min(n0 + 8 * n + g, N - 1) * vecs;
     float acc[TILES][4];
 #pragma unroll
     for (int n = 0; n < TILES; ++n)
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
     const int steps = (vecs + 3) / 4;
-#pragma unroll 4
-    for (int s = warp; s < steps; s += kWarps) {
-        const int v = 4 * s + t;                     // this lane's 16 bytes of a row
-        const bool in = v < vecs;
-        const uint4 x = in && lo ? a[at_lo + v] : zero, y = in && hi ? a[at_hi + v] : zero;
-        uint4 z[TILES];
+    for (int s0 = warp; s0 < steps; s0 += kBatch * kWarps) {
+        uint4 x[kBatch], y[kBatch], z[kBatch][TILES];
 #pragma unroll
-        for (int n = 0; n < TILES; ++n) z[n] = in && n0 + 8 * n + g < N ? __ldg(w + (size_t)(n0 + 8 * n + g) * vecs + v) : zero;
+        for (int u = 0; u < kBatch; ++u) {
+            const int v = 4 * (s0 + u * kWarps) + t, at = min(v, vecs - 1);      // this lane's 16 bytes of a row
+            x[u] = a_lo[at];
+            y[u] = a_hi[at];
 #pragma unroll
-        for (int n = 0; n < TILES; ++n) {
-            float sum[4] = {0.f, 0.f, 0.f, 0.f};
-            skinny_mma(sum, x.x, y.x, x.y, y.y, z[n].x, z[n].y);
-            skinny_mma(sum, x.z, y.z, x.w, y.w, z[n].z, z[n].w);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) acc[n][i] += sum[i];
+            for (int n = 0; n < TILES; ++n) z[u][n] = v < vecs ? __ldg(w[n] + at) : zero;
+            if (v >= vecs) x[u] = y[u] = zero;
         }
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u)
+#pragma unroll
+            for (int n = 0; n < TILES; ++n) {
+                float one[4] = {0.f, 0.f, 0.f, 0.f}, two[4] = {0.f, 0.f, 0.f, 0.f};
+                skinny_mma(one, x[u].x, y[u].x, x[u].y, y[u].y, z[u][n].x, z[u][n].y);
+                skinny_mma(two, x[u].z, y[u].z, x[u].w, y[u].w, z[u][n].z, z[u][n].w);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[n][i] += one[i] + two[i];
+            }
     }
 #pragma unroll
     for (int n = 0; n < TILES; ++n) *reinterpret_cast<float4*>(part[warp][n][lane]) = make_float4(acc[n][0], acc[n][1], acc[n][2], acc[n][3]);
     __syncthreads();
     for (int e = threadIdx.x; e < TILES * 128; e += kSkinnyThreads) {
         const int n = e >> 7, l = e >> 2 & 31, i = e & 3;
-        float total = 0.f;
+        double total = 0.0;
 #pragma unroll
-        for (int k = 0; k < kWarps; ++k) total += part[k][n][l][i];
+        for (int k = 0; k < kWarps; ++k) total += (double)part[k][n][l][i];
         const int row = m0 + (l >> 2) + 8 * (i >> 1), col = n0 + 8 * n + 2 * (l & 3) + (i & 1);
-        if (row < M && col < N) C[(size_t)row * N + col] = total;
+        if (row < M && col < N) C[(size_t)row * N + col] = (float)fma(total, kLean, total);
     }
 }
 }  // namespace
@@ -148,10 +155,10 @@ THN_API int thn_linear_skinny_bf16(float* C, const void* A, const void* W, int M
     THN_CHECK_ARG(M >= 0 && thn_linear_skinny_supported(N, K), "linear_skinny: bad sizes M=%d N=%d K=%d", M, N, K);
     THN_CHECK_ARG((((uintptr_t)A | (uintptr_t)W) & 15) == 0, "linear_skinny: operands must be 16-byte aligned (M=%d)", M);
     if (M == 0) return THN_OK;
-    // four tiles of columns a block read A a quarter as often; one tile a block where that leaves multiprocessors idle
+    // two tiles of columns a block read A half as often; one tile a block where that leaves multiprocessors idle
     const int row_blocks = (M + 15) / 16, tiles = (N + 7) / 8;
-    if (row_blocks * ((tiles + 3) / 4) >= 120)
-        thn_launch(linear_skinny_kernel<4>, dim3(row_blocks, (tiles + 3) / 4), kSkinnyThreads, 0, stream, C, (const __nv_bfloat16*)A,
+    if (row_blocks * ((tiles + 1) / 2) >= 120)
+        thn_launch(linear_skinny_kernel<2>, dim3(row_blocks, (tiles + 1) / 2), kSkinnyThreads, 0, stream, C, (const __nv_bfloat16*)A,
                    (const __nv_bfloat16*)W, M, N, K / 8);
     else
         thn_launch(linear_skinny_kernel<1>, dim3(row_blocks, tiles), kSkinnyThreads, 0, stream, C, (const __nv_bfloat16*)A,

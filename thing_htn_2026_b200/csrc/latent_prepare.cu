@@ -206,97 +206,62 @@ __global__ void __launch_bounds__(256) latent_assemble_vec_kernel(
     const long long key_step = (long long)kv.page_size * D, value_step = (long long)kv.page_size * DV;
     // work items of a head: plain pieces, turned pieces (pairs of them for half pairs), value pieces
     const int plain_items = plain / 8, turned_items = interleaved ? rot / 8 : half / 8, value_items = DV / 8;
-    const int per_head = plain_items + turned_items + value_items;
-    if (blockDim.x % per_head == 0) {
-        // a thread does the same piece of every head that it comes to: four heads' loads at a time, ahead of their stores
-        // (a store may alias a later load as far as the compiler knows); the shared key part is turned once
-        const int i = threadIdx.x % per_head, step = gridDim.y * blockDim.x / per_head;
-        const int h0 = (blockIdx.y * blockDim.x + threadIdx.x) / per_head;
-        const int j = i < plain_items ? i * 8 : i < plain_items + turned_items ? (i - plain_items) * 8 : (i - plain_items - turned_items) * 8;
-        const bool is_plain = i < plain_items, is_turned = !is_plain && i < plain_items + turned_items;
-        if (!is_plain && !is_turned && !cache) return;
-        uint4 key_lo = make_uint4(0, 0, 0, 0), key_hi = key_lo;
-        if (is_turned && cache) {
-            if (interleaved) key_lo = turn_four_pairs(piece(k_shared + j), c_row + j / 2, s_row + j / 2);
-            else turn_eight(piece(k_shared + j), piece(k_shared + half + j), c_row + j, s_row + j, key_lo, key_hi);
+    // Every thread takes a plain, a turned and two value pieces a round, each kind over all heads, so that a warp does one
+    // thing at a time, and loads all four ahead of its stores (which may alias a later load as far as the compiler knows).
+    // 2,532 rows of 32 heads on B200: 48 us with the kinds side by side in a warp and a piece at a time.
+    const int stride = gridDim.y * blockDim.x;
+    const int n_plain = n_heads * plain_items, n_turned = n_heads * turned_items, n_values = cache ? n_heads * value_items : 0;
+    const __nv_bfloat16* up_values = up_row + (size_t)n_heads * plain;
+    for (int e = blockIdx.y * blockDim.x + threadIdx.x, ev = e; e < n_plain || e < n_turned || ev < n_values; e += stride, ev += 2 * stride) {
+        const bool has_plain = e < n_plain, has_turned = e < n_turned;
+        uint4 q_plain, k_plain, q_lo, q_hi, v[2];
+        int hp = 0, jp = 0, ht = 0, jt = 0, hv[2], jv[2];
+        if (has_plain) {
+            hp = e / plain_items;
+            jp = (e - hp * plain_items) * 8;
+            q_plain = piece(q_row + (size_t)hp * D + jp);
+            if (cache) k_plain = piece(up_row + (size_t)hp * plain + jp);
         }
-        constexpr int U = 4;
-        for (int first = h0; first < n_heads; first += U * step) {
-            uint4 x[U], y[U];
+        if (has_turned) {
+            ht = e / turned_items;
+            jt = (e - ht * turned_items) * 8;
+            q_lo = piece(q_row + (size_t)ht * D + plain + jt);
+            if (!interleaved) q_hi = piece(q_row + (size_t)ht * D + plain + half + jt);
+        }
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int h = first + u * step;
-                if (h >= n_heads) continue;
-                const __nv_bfloat16* q = q_row + (size_t)h * D;
-                if (is_plain) {
-                    x[u] = piece(q + j);
-                    if (cache) y[u] = piece(up_row + (size_t)h * plain + j);
-                } else if (is_turned) {
-                    x[u] = piece(q + plain + j);
-                    if (!interleaved) y[u] = piece(q + plain + half + j);
-                } else {
-                    x[u] = j < value_src ? piece(up_row + (size_t)n_heads * plain + (size_t)h * value_src + j) : make_uint4(0, 0, 0, 0);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int h = first + u * step;
-                if (h >= n_heads) continue;
-                __nv_bfloat16* dst = q_out + ((size_t)m * n_heads + h) * D;
-                __nv_bfloat16* key = cache ? cache + keys0 + h * key_step : nullptr;
-                if (is_plain) {
-                    put(dst + j, x[u]);
-                    if (key) put(key + j, y[u]);
-                } else if (is_turned) {
-                    if (interleaved) {
-                        put(dst + plain + j, turn_four_pairs(x[u], c_row + j / 2, s_row + j / 2));
-                        if (key) put(key + plain + j, key_lo);
-                    } else {
-                        uint4 a, b;
-                        turn_eight(x[u], y[u], c_row + j, s_row + j, a, b);
-                        put(dst + plain + j, a);
-                        put(dst + plain + half + j, b);
-                        if (key) {
-                            put(key + plain + j, key_lo);
-                            put(key + plain + half + j, key_hi);
-                        }
-                    }
-                } else {
-                    put(cache + values0 + h * value_step + j, x[u]);
-                }
+        for (int u = 0; u < 2; ++u) {
+            const int at = ev + u * stride;
+            if (at < n_values) {
+                hv[u] = at / value_items;
+                jv[u] = (at - hv[u] * value_items) * 8;
+                v[u] = jv[u] < value_src ? piece(up_values + (size_t)hv[u] * value_src + jv[u]) : make_uint4(0, 0, 0, 0);
             }
         }
-        return;
-    }
-    for (int item = blockIdx.y * blockDim.x + threadIdx.x; item < n_heads * per_head; item += gridDim.y * blockDim.x) {
-        const int h = item / per_head, i = item - h * per_head;
-        const __nv_bfloat16* q = q_row + (size_t)h * D;
-        __nv_bfloat16* dst = q_out + ((size_t)m * n_heads + h) * D;
-        __nv_bfloat16* key = cache ? cache + keys0 + h * key_step : nullptr;
-        if (i < plain_items) {
-            put(dst + i * 8, piece(q + i * 8));
-            if (key) put(key + i * 8, piece(up_row + (size_t)h * plain + i * 8));
-        } else if (i < plain_items + turned_items) {
-            const int j = (i - plain_items) * 8;
+        if (has_plain) {
+            put(q_out + ((size_t)m * n_heads + hp) * D + jp, q_plain);
+            if (cache) put(cache + keys0 + hp * key_step + jp, k_plain);
+        }
+        if (has_turned) {
+            __nv_bfloat16* dst = q_out + ((size_t)m * n_heads + ht) * D + plain + jt;
+            __nv_bfloat16* key = cache ? cache + keys0 + ht * key_step + plain + jt : nullptr;
             if (interleaved) {
-                put(dst + plain + j, turn_four_pairs(piece(q + plain + j), c_row + j / 2, s_row + j / 2));
-                if (key) put(key + plain + j, turn_four_pairs(piece(k_shared + j), c_row + j / 2, s_row + j / 2));
+                put(dst, turn_four_pairs(q_lo, c_row + jt / 2, s_row + jt / 2));
+                if (key) put(key, turn_four_pairs(piece(k_shared + jt), c_row + jt / 2, s_row + jt / 2));
             } else {
                 uint4 x, y;
-                turn_eight(piece(q + plain + j), piece(q + plain + half + j), c_row + j, s_row + j, x, y);
-                put(dst + plain + j, x);
-                put(dst + plain + half + j, y);
+                turn_eight(q_lo, q_hi, c_row + jt, s_row + jt, x, y);
+                put(dst, x);
+                put(dst + half, y);
                 if (key) {
-                    turn_eight(piece(k_shared + j), piece(k_shared + half + j), c_row + j, s_row + j, x, y);
-                    put(key + plain + j, x);
-                    put(key + plain + half + j, y);
+                    turn_eight(piece(k_shared + jt), piece(k_shared + half + jt), c_row + jt, s_row + jt, x, y);
+                    put(key, x);
+                    put(key + half, y);
                 }
             }
-        } else if (cache) {
-            const int j = (i - plain_items - turned_items) * 8;
-            put(cache + values0 + h * value_step + j,
-                j < value_src ? piece(up_row + (size_t)n_heads * plain + (size_t)h * value_src + j) : make_uint4(0, 0, 0, 0));
         }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            if (ev + u * stride < n_values) put(cache + values0 + hv[u] * value_step + jv[u], v[u]);
     }
 }
 
