@@ -200,7 +200,8 @@ struct Layout {
     static constexpr int kG = kW + (DELTA ? 3 * kKeyPlane * 2 : 0);
     static constexpr int kV = kG + 3 * kScorePlane * 2;
     static constexpr int kScalars = kV + kTokens * kValueRow * (int)sizeof(T);
-    static constexpr int kStage = kScalars + kTokens * 16;
+    static constexpr int kSums = kScalars + kTokens * 16;                                    // gated: the chunk's sum of keys
+    static constexpr int kStage = kSums + (kParts == 1 ? kKeys * 4 : 0);
     static constexpr int kShares = KS > 1 ? KS * CG * (DELTA ? 2 : 1) * 4 * 32 * 16 : 0;    // [ks][cg][which][8 tokens][lane] float4
     static constexpr int kBytes = STAGES * kStage + kShares + (kTokens * 3 + kKeys) * 4;
 };
@@ -251,13 +252,22 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
                 copy_rows<kKeyRow, L::kThreads>(k_dst + p * L::kKeyPlane, k_src + p * a.key_plane + (long long)first * kKeyRow, n_here);
             }
         } else {
-            for (int e = threadIdx.x; e < kTokens * (kKeys / 8); e += L::kThreads) {
-                const int i = e / (kKeys / 8), c = e % (kKeys / 8) * 8;
-                const bool there = i < n_here;
-                const long long at = (there ? first + i : 0) * a.key_row + c;
-                copy16(q_dst + i * kKeyRow + c, q_src + at, there);
-                copy16(k_dst + i * kKeyRow + c, k_src + at, there);
+            // (a thread copies the same column of some rows, the same distance apart in every chunk)
+            constexpr int kRowsApart = L::kThreads / (kKeys / 8);
+            const int i0 = threadIdx.x / (kKeys / 8), c = threadIdx.x % (kKeys / 8) * 8;
+            const __nv_bfloat16* q_from = q_src + c + (first + i0) * a.key_row;
+            const __nv_bfloat16* k_from = k_src + c + (first + i0) * a.key_row;
+#pragma unroll
+            for (int u = 0; u < kTokens / kRowsApart; ++u) {
+                const bool there = i0 + u * kRowsApart < n_here;
+                copy16(q_dst + (i0 + u * kRowsApart) * kKeyRow + c, there ? q_from : q_src, there);
+                copy16(k_dst + (i0 + u * kRowsApart) * kKeyRow + c, there ? k_from : k_src, there);
+                q_from += kRowsApart * a.key_row;
+                k_from += kRowsApart * a.key_row;
             }
+            if (GATED && threadIdx.x < kKeys / 4)
+                copy16(dst + L::kSums + threadIdx.x * 16,
+                       a.key_sums + (((size_t)seq * a.max_chunks + chunk) * a.n_heads + head) * kKeys + threadIdx.x * 4, true);
         }
 #pragma unroll
         for (int p = 0; p < 3; ++p) {
@@ -395,16 +405,30 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
                 }
             }
         }
+        // The delta rule's values v = u - W S0, as they are and times w, go out as planes [column][token] over the chunk's queries
+        // and W, which no warp reads any more: split by the warps that finish them, once.
+        constexpr int kSplitRow = kTokens + 8, kSplitPlane = 16 * kSplitRow;
+        __nv_bfloat16* plain_s = reinterpret_cast<__nv_bfloat16*>(stage + L::kQ) + cg * 3 * kSplitPlane;
+        __nv_bfloat16* scaled_s = reinterpret_cast<__nv_bfloat16*>(stage + L::kW) + cg * 3 * kSplitPlane;
         if constexpr (DELTA) {
-            // v = u - W S0, in place of u
+            if (KS == 1) __syncthreads();
             if (fixes) {
 #pragma unroll
                 for (int n = 0; n < OWN; ++n) {
-                    T* v = v_s + (8 * (group0 + n) + 2 * t) * L::kValueRow + g;
-                    v[0] -= fixed[n][0];
-                    v[L::kValueRow] -= fixed[n][1];
-                    v[8] -= fixed[n][2];
-                    v[L::kValueRow + 8] -= fixed[n][3];
+                    const int i = 8 * (group0 + n) + 2 * t;
+                    const T* u = v_s + i * L::kValueRow + g;
+                    const float w0 = scalars[i].z, w1 = scalars[i + 1].z;
+                    const float v[4] = {u[0] - fixed[n][0], u[L::kValueRow] - fixed[n][1], u[8] - fixed[n][2], u[L::kValueRow + 8] - fixed[n][3]};
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) {
+                        const int at = (g + 8 * half) * kSplitRow + i;
+                        const Split as_is = split(v[2 * half], v[2 * half + 1]), by_w = split(v[2 * half] * w0, v[2 * half + 1] * w1);
+#pragma unroll
+                        for (int p = 0; p < 3; ++p) {
+                            *reinterpret_cast<uint32_t*>(plain_s + p * kSplitPlane + at) = as_is.part[p];
+                            *reinterpret_cast<uint32_t*>(scaled_s + p * kSplitPlane + at) = by_w.part[p];
+                        }
+                    }
                 }
             }
             if (KS > 1) __syncthreads();
@@ -414,6 +438,15 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
         Parts plain[kTokens / 16], scaled[kTokens / 16];
 #pragma unroll
         for (int j = 0; j < kTokens / 16; ++j) {
+            if constexpr (DELTA) {
+                const int at = a_tile(lane, kSplitRow) + 16 * j;
+#pragma unroll
+                for (int p = 0; p < 3; ++p) {
+                    load_matrices(scaled[j].part[p], scaled_s + p * kSplitPlane + at);
+                    if (reads) load_matrices(plain[j].part[p], plain_s + p * kSplitPlane + at);
+                }
+                continue;
+            }
             const float4* sc = scalars + 16 * j + 2 * t;
             const float w0 = sc[0].z, w1 = sc[1].z, w8 = sc[8].z, w9 = sc[9].z;
             float2 v[4];        // column g, g + 8 at tokens 2t, 2t + 1; the same at 2t + 8, 2t + 9
@@ -508,7 +541,7 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
             const float4 sc = scalars[n_here - 1];
             m = fmaxf(sc.x + m, sc.y);
             // (every n . q of the chunk was taken ahead of the barrier above; the next chunk's wait behind one too)
-            const float* sums = a.key_sums + (((size_t)seq * a.max_chunks + chunk) * a.n_heads + head) * kKeys;
+            const float* sums = reinterpret_cast<const float*>(stage + L::kSums);
             for (int d = threadIdx.x; d < kKeys; d += L::kThreads) n_s[d] = fmaf(keep, n_s[d], take * sums[d]);
         }
     }

