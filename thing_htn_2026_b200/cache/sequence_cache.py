@@ -161,7 +161,9 @@ class SequenceCache:
         if count > self.book.slots.n_free:
             raise CacheFull(f"need {count} slots, {self.book.slots.n_free} of {self.max_slots} are free")
         slots = [self.book.open() for _ in range(count)]
-        index = torch.tensor(slots, dtype=torch.int64, device=self.device)
+        # (a copy that does not wait for the device: made on the device, the tensor would hold the host until
+        # every step in flight has ended)
+        index = torch.tensor(slots, dtype=torch.int64).to(self.device, non_blocking=True)
         self.seq_lens.index_fill_(0, index, 0)
         for tensor in self._named_state.values():
             tensor.index_fill_(0, index, 0)
