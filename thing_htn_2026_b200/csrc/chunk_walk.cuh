@@ -212,9 +212,8 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
     constexpr int PARTS = L::kParts;
     constexpr int KT = kKeys / KS / 8;               // groups of 8 keys of a warp
     constexpr int GROUPS = kTokens / 8;              // groups of 8 tokens
-    constexpr int OWN = KS <= GROUPS ? GROUPS / KS : 1;       // groups that a warp finishes
-    constexpr bool HALVES = KS > GROUPS;             // some warps finish the values, others the read-outs
-    static_assert(KT % 2 == 0 && (KS <= GROUPS || (KS == 2 * GROUPS && DELTA)), "whole steps");
+    constexpr int OWN = GROUPS / KS;                 // groups that a warp finishes
+    static_assert(KT % 4 == 0 && OWN >= 1, "whole steps");
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ __align__(16) unsigned char mem[];
@@ -229,8 +228,7 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
     const int slot = a.slots[seq], unit = head / a.heads_per_unit;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int cg = warp / KS, ks = warp % KS, key0 = ks * (kKeys / KS);
-    const int group0 = HALVES ? ks % GROUPS : ks * OWN;      // the first group of tokens that this warp finishes
-    const bool fixes = !HALVES || ks < GROUPS, reads = !HALVES || ks >= GROUPS;
+    const int group0 = ks * OWN;                     // the first group of tokens that this warp finishes
     const int col0 = slab * L::kColumns;
     const __nv_bfloat16* q_src = a.q + unit * a.key_unit + row0 * a.key_row;
     const __nv_bfloat16* k_src = a.k + unit * a.key_unit + row0 * a.key_row;
@@ -393,7 +391,6 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
             for (int n = 0; n < OWN; ++n) {
 #pragma unroll
                 for (int which = 0; which < WHICH; ++which) {
-                    if (HALVES && (which == 0 ? !reads : !fixes)) continue;
                     float (&dst)[4] = which == 0 ? read[n] : fixed[n];
                     float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
@@ -406,28 +403,27 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
             }
         }
         // The delta rule's values v = u - W S0, as they are and times w, go out as planes [column][token] over the chunk's queries
-        // and W, which no warp reads any more: split by the warps that finish them, once.
+        // and W, which no warp reads any more: split by the warps that finish them, once (one prompt of 2,048 tokens of 32
+        // heads 397 -> 362 us against every warp splitting them).
         constexpr int kSplitRow = kTokens + 8, kSplitPlane = 16 * kSplitRow;
         __nv_bfloat16* plain_s = reinterpret_cast<__nv_bfloat16*>(stage + L::kQ) + cg * 3 * kSplitPlane;
         __nv_bfloat16* scaled_s = reinterpret_cast<__nv_bfloat16*>(stage + L::kW) + cg * 3 * kSplitPlane;
         if constexpr (DELTA) {
             if (KS == 1) __syncthreads();
-            if (fixes) {
 #pragma unroll
-                for (int n = 0; n < OWN; ++n) {
-                    const int i = 8 * (group0 + n) + 2 * t;
-                    const T* u = v_s + i * L::kValueRow + g;
-                    const float w0 = scalars[i].z, w1 = scalars[i + 1].z;
-                    const float v[4] = {u[0] - fixed[n][0], u[L::kValueRow] - fixed[n][1], u[8] - fixed[n][2], u[L::kValueRow + 8] - fixed[n][3]};
+            for (int n = 0; n < OWN; ++n) {
+                const int i = 8 * (group0 + n) + 2 * t;
+                const T* u = v_s + i * L::kValueRow + g;
+                const float w0 = scalars[i].z, w1 = scalars[i + 1].z;
+                const float v[4] = {u[0] - fixed[n][0], u[L::kValueRow] - fixed[n][1], u[8] - fixed[n][2], u[L::kValueRow + 8] - fixed[n][3]};
 #pragma unroll
-                    for (int half = 0; half < 2; ++half) {
-                        const int at = (g + 8 * half) * kSplitRow + i;
-                        const Split as_is = split(v[2 * half], v[2 * half + 1]), by_w = split(v[2 * half] * w0, v[2 * half + 1] * w1);
+                for (int half = 0; half < 2; ++half) {
+                    const int at = (g + 8 * half) * kSplitRow + i;
+                    const Split as_is = split(v[2 * half], v[2 * half + 1]), by_w = split(v[2 * half] * w0, v[2 * half + 1] * w1);
 #pragma unroll
-                        for (int p = 0; p < 3; ++p) {
-                            *reinterpret_cast<uint32_t*>(plain_s + p * kSplitPlane + at) = as_is.part[p];
-                            *reinterpret_cast<uint32_t*>(scaled_s + p * kSplitPlane + at) = by_w.part[p];
-                        }
+                    for (int p = 0; p < 3; ++p) {
+                        *reinterpret_cast<uint32_t*>(plain_s + p * kSplitPlane + at) = as_is.part[p];
+                        *reinterpret_cast<uint32_t*>(scaled_s + p * kSplitPlane + at) = by_w.part[p];
                     }
                 }
             }
@@ -443,7 +439,7 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
 #pragma unroll
                 for (int p = 0; p < 3; ++p) {
                     load_matrices(scaled[j].part[p], scaled_s + p * kSplitPlane + at);
-                    if (reads) load_matrices(plain[j].part[p], plain_s + p * kSplitPlane + at);
+                    load_matrices(plain[j].part[p], plain_s + p * kSplitPlane + at);
                 }
                 continue;
             }
@@ -468,7 +464,7 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
         }
         // the state behind the chunk
         const float keep = GATED ? alpha_s[n_here - 1] : scalars[n_here - 1].x, take = GATED ? beta_s[n_here - 1] : 1.f;
-        constexpr int KP = KT >= 4 ? 2 : 1;          // pairs of groups of keys at a time
+        constexpr int KP = 2;                        // pairs of groups of keys at a time
 #pragma unroll
         for (int n = 0; n < KT; n += 2 * KP) {
             float sum[2 * KP][4];
@@ -493,48 +489,46 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
                 for (int i = 0; i < 4; ++i) s[n + o][i] = fmaf(keep, s[n + o][i], take * sum[o][i]);
         }
         // sum_j G_ij v_j for this warp's tokens, and the read-outs
-        if (reads) {
-            // (G's rows are loaded for 16 tokens at a time; with one group of tokens a warp, two warps share them)
-            constexpr int kPairs = OWN >= 2 ? OWN / 2 : 1;
-            float inner[kPairs][2][4];
-            const int pair0 = group0 / 2;
+        // (G's rows are loaded for 16 tokens at a time; with one group of tokens a warp, two warps share them)
+        constexpr int kPairs = OWN >= 2 ? OWN / 2 : 1;
+        float inner[kPairs][2][4];
+        const int pair0 = group0 / 2;
 #pragma unroll
-            for (int pair = 0; pair < kPairs; ++pair) {
-                clear(inner[pair]);
+        for (int pair = 0; pair < kPairs; ++pair) {
+            clear(inner[pair]);
 #pragma unroll
-                for (int j = 0; j < kTokens / 16; ++j) {
-                    if (j > pair0 + pair) continue;
-                    const Columns<3> row[1] = {columns_of<3>(g_s + b_tile(lane, kScoreRow) + 16 * (pair0 + pair) * kScoreRow + 16 * j, L::kScorePlane)};
-                    float large[2][4], small[2][4];
-                    clear(large);
-                    clear(small);
-                    multiply<PARTS>(large, small, plain[j], row);
+            for (int j = 0; j < kTokens / 16; ++j) {
+                if (j > pair0 + pair) continue;
+                const Columns<3> row[1] = {columns_of<3>(g_s + b_tile(lane, kScoreRow) + 16 * (pair0 + pair) * kScoreRow + 16 * j, L::kScorePlane)};
+                float large[2][4], small[2][4];
+                clear(large);
+                clear(small);
+                multiply<PARTS>(large, small, plain[j], row);
 #pragma unroll
-                    for (int o = 0; o < 2; ++o)
+                for (int o = 0; o < 2; ++o)
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) inner[pair][o][i] += joined(large[o][i], small[o][i]);
-                }
+                    for (int i = 0; i < 4; ++i) inner[pair][o][i] += joined(large[o][i], small[o][i]);
             }
+        }
 #pragma unroll
-            for (int n = 0; n < OWN; ++n) {
+        for (int n = 0; n < OWN; ++n) {
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    const int i = 8 * (group0 + n) + 2 * t + half;
-                    if (i >= n_here) continue;
-                    const int o = OWN == 1 ? group0 & 1 : n & 1;
-                    const float in0 = o ? inner[n / 2][1][half] : inner[n / 2][0][half];
-                    const float in1 = o ? inner[n / 2][1][2 + half] : inner[n / 2][0][2 + half];
-                    const float alpha = GATED ? alpha_s[i] : scalars[i].x, beta = GATED ? beta_s[i] : 1.f;
-                    float y0 = (alpha * read[n][half] + beta * in0) * a.scale;
-                    float y1 = (alpha * read[n][2 + half] + beta * in1) * a.scale;
-                    if (GATED) {
-                        y0 /= under_s[i];
-                        y1 /= under_s[i];
-                    }
-                    float* dst = a.o + ((size_t)(row0 + first + i) * a.n_heads + head) * a.value_dim + col0 + cg * 16 + g;
-                    dst[0] = y0;
-                    dst[8] = y1;
+            for (int half = 0; half < 2; ++half) {
+                const int i = 8 * (group0 + n) + 2 * t + half;
+                if (i >= n_here) continue;
+                const int o = OWN == 1 ? group0 & 1 : n & 1;
+                const float in0 = o ? inner[n / 2][1][half] : inner[n / 2][0][half];
+                const float in1 = o ? inner[n / 2][1][2 + half] : inner[n / 2][0][2 + half];
+                const float alpha = GATED ? alpha_s[i] : scalars[i].x, beta = GATED ? beta_s[i] : 1.f;
+                float y0 = (alpha * read[n][half] + beta * in0) * a.scale;
+                float y1 = (alpha * read[n][2 + half] + beta * in1) * a.scale;
+                if (GATED) {
+                    y0 /= under_s[i];
+                    y1 /= under_s[i];
                 }
+                float* dst = a.o + ((size_t)(row0 + first + i) * a.n_heads + head) * a.value_dim + col0 + cg * 16 + g;
+                dst[0] = y0;
+                dst[8] = y1;
             }
         }
         if (GATED) {

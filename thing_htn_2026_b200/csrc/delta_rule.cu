@@ -853,8 +853,8 @@ THN_API long long thn_delta_chunks_scratch_bytes(int n_rows, int n_heads, int n_
 // prepare and recurrence of a step chunk by chunk, the state carried in float32: bfloat16 rows, four taps, keys of
 // 128, values of whole groups of 16 columns; max_tokens: the most rows of a sequence.  scratch:
 // thn_delta_chunks_scratch_bytes(...), 16-byte aligned, as the state and the taps must be; the rows and the
-// ring are read in pieces of 8 bytes.  One prompt of 2,048 tokens, 16 heads of 128 x 128, on B200: 251 us
-// against 655 token by token; 32 heads 397 / 839; 8 x 512 tokens of 16 heads 339 / 571.  The read-out's error
+// ring are read in pieces of 8 bytes.  One prompt of 2,048 tokens, 16 heads of 128 x 128, on B200: 241 us
+// against 655 token by token; 32 heads 362 / 839; 8 x 512 tokens of 16 heads 341 / 571.  The read-out's error
 // against 64 bits is 1.4e-7 (1.3e-7 token by token), the state's 1.3e-7 (1.3e-7).
 THN_API int thn_delta_chunks(float* o, float* state, void* scratch, const void* proj, const float* conv_w, const float* a_log,
                              const float* dt_bias, const void* ring, const int* row_slot, const int* row_pos, const int* seq_lens,
@@ -899,7 +899,7 @@ THN_API int thn_delta_chunks(float* o, float* state, void* scratch, const void* 
     const long long pairs = (long long)n_seqs * n_heads;
     if (dv % 64 == 0 && pairs * (dv / 64) >= 128) chunk::launch_walk<float, 4, 2, true, false, 2>(a, n_seqs, stream);
     else if (dv % 32 == 0 && pairs * (dv / 32) >= 128) chunk::launch_walk<float, 2, 4, true, false, 2>(a, n_seqs, stream);
-    else chunk::launch_walk<float, 1, 8, true, false, 2>(a, n_seqs, stream);
+    else chunk::launch_walk<float, 1, 4, true, false, 2>(a, n_seqs, stream);
     return thn_launch_status("delta_chunks");
 }
 
