@@ -69,3 +69,17 @@ def test_conv_matches_64_bits(channels, offset, lens, held, bias):
             want[r] = torch.nn.functional.silu(acc)
     # four products and a silu in float32 (2^-20 of the sums' size), one rounding to bfloat16
     assert ((got.cpu().double() - want).abs() <= 2 ** -8 * want.abs() + 2 ** -18 * 16).all()
+
+
+@pytest.mark.parametrize("rows,heads,size,kind,own_gain", [
+    (4096, 1, 128, "silu", False), (1025, 4, 64, "logistic", True), (683, 6, 128, "logistic", True), (2049, 2, 64, "silu", False)])
+def test_gated_head_norm_of_many_pairs(rows, heads, size, kind, own_gain):
+    g = torch.Generator().manual_seed(rows)
+    dev = torch.device("cuda", 0)
+    o, gate = torch.randn(rows, heads, size, generator=g), torch.randn(rows, heads * size + 8, generator=g).to(BF16)
+    w = torch.randn(heads * size if own_gain else size, generator=g)
+    got = ops.gated_head_norm(o.to(dev), gate.to(dev), 4, w.to(dev), 1e-6, heads, size, BF16, kind)
+    x, z = o.double(), gate[:, 4:4 + heads * size].double().view(rows, heads, size)
+    want = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-6) * w.double().view(-1, size) * (torch.sigmoid(z) if kind == "logistic" else torch.nn.functional.silu(z))
+    # float32 throughout and one rounding to bfloat16
+    assert ((got.cpu().double().view(rows, heads, size) - want).abs() <= 2 ** -8 * want.abs() + 1e-7).all()

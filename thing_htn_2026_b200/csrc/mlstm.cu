@@ -21,6 +21,7 @@
 //   mlstm_recurrence   the recurrence; with raw_gates it transforms x, y itself (single-token
 //                      steps: one kernel); steps of several tokens take the kernel that stages
 //                      the tokens in shared memory where the rows' alignment allows it
+//   mlstm_chunk, and the walk of chunk_walk.cuh   bfloat16 prompts with keys of 128, chunk by chunk
 #include <math.h>
 
 #include <algorithm>

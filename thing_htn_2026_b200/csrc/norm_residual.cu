@@ -356,6 +356,49 @@ __global__ void gated_head_norm_kernel(T* __restrict__ out, const float* __restr
             from_f32<T>(src[i] * rstd * wh[i] * (gate_kind ? logistic : z * logistic) * scale);
     }
 }
+// The same for bfloat16 and heads of 64 or 128 entries when there are many: LANES = size / 4 lanes take four neighbouring
+// (row, head) pairs, 16 bytes of each, all loads ahead of the first sum.  Bounded by what it moves.  B200: 1,531 rows of 32
+// heads of 128 22 us with a pair a warp; with the logistic gate 2,251 rows of 16 heads 20 with 4-byte accesses.
+constexpr int kManyPairs = 4;
+constexpr long long kManyUnits = 4096;
+template <int LANES>
+__global__ void __launch_bounds__(128) gated_head_norm_many_kernel(__nv_bfloat16* __restrict__ out, const float* __restrict__ o,
+                                                                   const __nv_bfloat16* __restrict__ gate, long long gate_stride,
+                                                                   const float* __restrict__ w, float eps, unsigned n_units,
+                                                                   unsigned n_heads, int w_stride, int gate_kind,
+                                                                   long long out_stride, float scale) {
+    pdl_launch_dependents();
+    pdl_wait();
+    constexpr int kSize = LANES * 4;
+    const unsigned first = (blockIdx.x * (128 / LANES) + threadIdx.x / LANES) * kManyPairs;
+    const int d = threadIdx.x % LANES * 4;
+    float4 v[kManyPairs], gain[kManyPairs];
+    uint2 z[kManyPairs];
+    long long at[kManyPairs];
+#pragma unroll
+    for (int u = 0; u < kManyPairs; ++u) {
+        const unsigned unit = min(first + u, n_units - 1), m = unit / n_heads, head = unit - m * n_heads;     // (beyond the last: it again, not stored)
+        v[u] = *reinterpret_cast<const float4*>(o + (size_t)unit * kSize + d);
+        z[u] = *reinterpret_cast<const uint2*>(gate + m * gate_stride + (size_t)head * kSize + d);
+        gain[u] = *reinterpret_cast<const float4*>(w + (size_t)head * w_stride + d);
+        at[u] = m * out_stride + (long long)head * kSize + d;
+    }
+#pragma unroll
+    for (int u = 0; u < kManyPairs; ++u) {
+        float ss = v[u].x * v[u].x + v[u].y * v[u].y + v[u].z * v[u].z + v[u].w * v[u].w;
+#pragma unroll
+        for (int off = LANES / 2; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+        const float rstd = 1.0f / sqrtf(ss / (float)kSize + eps);
+        const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&z[u].x));
+        const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&z[u].y));
+        auto one = [&](float x, float g, float zz) { return x * rstd * g * ((gate_kind ? 1.0f : zz) / (1.0f + expf(-zz))) * scale; };
+        uint2 packed;
+        *reinterpret_cast<__nv_bfloat162*>(&packed.x) = __floats2bfloat162_rn(one(v[u].x, gain[u].x, lo.x), one(v[u].y, gain[u].y, lo.y));
+        *reinterpret_cast<__nv_bfloat162*>(&packed.y) = __floats2bfloat162_rn(one(v[u].z, gain[u].z, hi.x), one(v[u].w, gain[u].w, hi.y));
+        if (first + u < n_units) *reinterpret_cast<uint2*>(out + at[u]) = packed;
+    }
+}
+
 // One "head" that is a whole long row (one norm over all heads together): a block of 256 threads
 // per row instead of a warp, four consecutive entries per thread where the sizes allow.  The
 // order of additions depends on the size only.
@@ -569,6 +612,15 @@ THN_API int thn_gated_head_norm(void* out, const float* o, const void* gate, lon
     const int w_stride = w_per_head ? size : 0;
     if (out_stride <= 0) out_stride = (long long)n_heads * size;
     THN_CHECK_ARG(out_stride >= (long long)n_heads * size, "gated_head_norm: output rows %lld apart are too short", out_stride);
+    if (dtype == THN_BF16 && (size == 64 || size == 128) && units >= kManyUnits && units < (1ll << 31) && gate_stride % 4 == 0 &&
+        out_stride % 4 == 0 && ((((uintptr_t)o | (uintptr_t)w) & 15) | (((uintptr_t)gate | (uintptr_t)out) & 7)) == 0) {
+        const unsigned per_block = 128 / (size / 4) * kManyPairs;
+        auto kernel = size == 128 ? gated_head_norm_many_kernel<32> : gated_head_norm_many_kernel<16>;
+        thn_launch(kernel, (unsigned)((units + per_block - 1) / per_block), 128, 0, stream, (__nv_bfloat16*)out, o,
+                   (const __nv_bfloat16*)gate, gate_stride, w, eps, (unsigned)units, (unsigned)n_heads, w_stride, gate_kind, out_stride,
+                   scale);
+        return thn_launch_status("gated_head_norm");
+    }
     if (dtype == THN_BF16 && gate_kind == 0 && size % 4 == 0 && gate_stride % 4 == 0 && scale == 1.0f &&
         out_stride == (long long)n_heads * size &&
         ((((uintptr_t)o | (uintptr_t)w) & 15) | (((uintptr_t)gate | (uintptr_t)out) & 7)) == 0) {

@@ -12,6 +12,8 @@
 //                    for the shared recurrence (linear_attention.cuh, kSteppedDecay): [B | C] per row
 //                    and group, [x | a, t] per row and head.  A thread takes four neighbouring
 //                    channels over a run of rows, keeping the last raw inputs in registers.
+//   state_space_prepare_chunks, state_space_chunk, and the walk of chunk_walk.cuh   the same for long bfloat16
+//                    prompts over a state of 128, chunk by chunk.
 //   state_space_decode    a single token per sequence: convolution, ring, step size, decay, recurrence
 //                    and skip in one kernel, one block per (row, head).
 //   gated_group_norm   y silu(z), divided by its root mean square over equal consecutive parts, times a
@@ -279,18 +281,21 @@ __global__ void __launch_bounds__(kSpaceThreads) state_space_chunk_kernel(
         const float d = skip[head];
         if (there)
             scalars[(size_t)head * n_rows + row0 + lane] = make_float4(expf((float)c), 0.f, step * expf((float)(c_last - c)), 0.f);
-        __nv_bfloat16* dst = scores + head * 3 * score_plane + (long long)row0 * chunk::kScoreRow + lane;
+        // a half warp takes a row, a lane two neighbouring tokens j of it
+        const int j = 2 * (lane & 15);
+        const double c0 = __shfl_sync(0xffffffffu, c, j), c1 = __shfl_sync(0xffffffffu, c, j + 1);
+        const float t0 = __shfl_sync(0xffffffffu, step, j), t1 = __shfl_sync(0xffffffffu, step, j + 1);
+        __nv_bfloat16* dst = scores + head * 3 * score_plane + (long long)row0 * chunk::kScoreRow + j;
 #pragma unroll 4
-        for (int i = 0; i < n_here; ++i) {
+        for (int i0 = 0; i0 < n_here; i0 += 2) {
+            const int i = i0 + (lane >> 4);
             const double ci = __shfl_sync(0xffffffffu, c, i);
-            float x = lane <= i ? expf((float)(ci - c)) * step * dot_s[i * (C + 1) + lane] : 0.f;
-            if (lane == i) x += d;
-#pragma unroll
-            for (int p = 0; p < 3; ++p) {
-                const __nv_bfloat16 part = __float2bfloat16_rn(x);
-                dst[p * score_plane + (long long)i * chunk::kScoreRow] = part;
-                x -= __bfloat162float(part);
-            }
+            if (i >= n_here) continue;
+            float x = j <= i ? expf((float)(ci - c0)) * t0 * dot_s[i * (C + 1) + j] : 0.f;
+            float y = j + 1 <= i ? expf((float)(ci - c1)) * t1 * dot_s[i * (C + 1) + j + 1] : 0.f;
+            if (j == i) x += d;
+            if (j + 1 == i) y += d;
+            chunk::store_split(dst + (long long)i * chunk::kScoreRow, score_plane, x, y);
         }
     }
 }
