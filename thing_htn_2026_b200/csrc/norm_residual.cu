@@ -358,7 +358,7 @@ __global__ void gated_head_norm_kernel(T* __restrict__ out, const float* __restr
 }
 // The same for bfloat16 and heads of 64 or 128 entries when there are many: LANES = size / 4 lanes take four neighbouring
 // (row, head) pairs, 16 bytes of each, all loads ahead of the first sum.  Bounded by what it moves.  B200: 1,531 rows of 32
-// heads of 128 22 us with a pair a warp; with the logistic gate 2,251 rows of 16 heads 20 with 4-byte accesses.
+// heads of 128 15 us, 22 with a pair a warp; with the logistic gate 2,251 rows of 16 heads 12, 20 with 4-byte accesses.
 constexpr int kManyPairs = 4;
 constexpr long long kManyUnits = 4096;
 template <int LANES>

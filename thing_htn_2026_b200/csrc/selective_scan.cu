@@ -335,22 +335,6 @@ __global__ void __launch_bounds__(kScanThreads) selective_scan_kernel(
 constexpr int kWalkThreads = 128;          // threads of each of the two halves of a block
 constexpr int kWalkStage = 16;
 
-__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
-    unsigned long long v;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
-    return v;
-}
-__device__ __forceinline__ void unpack2(unsigned long long v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-    unsigned long long v;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
-    return v;
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long v;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
-    return v;
-}
 // the hardware's base-2 exponential (as Decay above; what would be below 2^-126 is zero)
 __device__ __forceinline__ float decay_exp2(float x) {
     float y;
