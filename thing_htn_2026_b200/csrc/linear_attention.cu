@@ -202,7 +202,9 @@ __global__ void __launch_bounds__(kLanes * kColumns / COLS) linear_attention_ker
     }
 
     const bool whole = key_dim % 4 == 0 && ((uintptr_t)state & 15) == 0;
-    using pair = unsigned long long;                    // two neighbouring channels of a column: every operation is two wide
+    // Two neighbouring channels of a column: every operation is two wide, half as many to issue (the whole call for 1,531
+    // tokens of 32 heads of 128 x 128: gated decays 286 -> 267 us, a constant decay 278 -> 241).
+    using pair = unsigned long long;
     pair s[COLS][PER / 2];
 #pragma unroll
     for (int c = 0; c < COLS; ++c) {
