@@ -76,8 +76,8 @@ THN_API int thn_gemm_f32(float* C, const float* A, const float* W, int M, int N,
 // K in steps of 32 on the tensor cores, each product into a fresh accumulator (the tensor core's accumulation
 // rounds towards zero, by kLean of the result on average, which is put back at the end; the sum over the steps is
 // float32 additions).  A lane loads its operands straight from memory, 16 bytes of a row at k = 32 s + 8 t: which
-// k a lane's pair stands for does not matter as long as both operands agree; the loads of four steps are issued
-// together.  The warps' sums meet in shared memory in a fixed order, so a row's result depends on nothing but K,
+// k a lane's pair stands for does not matter as long as both operands agree; the loads of four or eight steps are
+// issued together.  The warps' sums meet in shared memory in a fixed order, so a row's result depends on nothing but K,
 // whatever M, N and TILES are.  K is a multiple of eight and both operands are 16-byte aligned.
 // B200, against a warp's float32 multiply-adds over four rows and four columns at a time: 2,251 rows, 32 columns over 2,048
 // 8 us / 31, 4,096 rows over 4,096 25 / 84, 1 to 64 rows the same; the error against 64 bits 6.5e-8 to 7.6e-8 / 7.9e-8 to 8.5e-8.
@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(kSkinnyThreads) linear_skinny_kernel(float* __
                                                                        int vecs) {
     pdl_launch_dependents();
     pdl_wait();
-    constexpr int kWarps = kSkinnyThreads / 32, kBatch = 4;
+    constexpr int kWarps = kSkinnyThreads / 32, kBatch = TILES == 1 ? 8 : 4;
     constexpr double kLean = 4.3e-8;
     __shared__ __align__(16) float part[kWarps][TILES][32][4];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
@@ -119,6 +119,7 @@ __global__ void __launch_bounds__(kSkinnyThreads) linear_skinny_kernel(float* __
         uint4 x[kBatch], y[kBatch], z[kBatch][TILES];
 #pragma unroll
         for (int u = 0; u < kBatch; ++u) {
+            if (s0 + u * kWarps >= steps) continue;
             const int v = 4 * (s0 + u * kWarps) + t, at = min(v, vecs - 1);      // this lane's 16 bytes of a row
             x[u] = a_lo[at];
             y[u] = a_hi[at];
@@ -127,7 +128,8 @@ __global__ void __launch_bounds__(kSkinnyThreads) linear_skinny_kernel(float* __
             if (v >= vecs) x[u] = y[u] = zero;
         }
 #pragma unroll
-        for (int u = 0; u < kBatch; ++u)
+        for (int u = 0; u < kBatch; ++u) {
+            if (s0 + u * kWarps >= steps) continue;
 #pragma unroll
             for (int n = 0; n < TILES; ++n) {
                 float one[4] = {0.f, 0.f, 0.f, 0.f}, two[4] = {0.f, 0.f, 0.f, 0.f};
@@ -136,15 +138,17 @@ __global__ void __launch_bounds__(kSkinnyThreads) linear_skinny_kernel(float* __
 #pragma unroll
                 for (int i = 0; i < 4; ++i) acc[n][i] += one[i] + two[i];
             }
+        }
     }
 #pragma unroll
     for (int n = 0; n < TILES; ++n) *reinterpret_cast<float4*>(part[warp][n][lane]) = make_float4(acc[n][0], acc[n][1], acc[n][2], acc[n][3]);
     __syncthreads();
     for (int e = threadIdx.x; e < TILES * 128; e += kSkinnyThreads) {
         const int n = e >> 7, l = e >> 2 & 31, i = e & 3;
-        double total = 0.0;
+        double sum[4] = {0.0, 0.0, 0.0, 0.0};            // (four short chains)
 #pragma unroll
-        for (int k = 0; k < kWarps; ++k) total += (double)part[k][n][l][i];
+        for (int k = 0; k < kWarps; ++k) sum[k & 3] += (double)part[k][n][l][i];
+        const double total = (sum[0] + sum[1]) + (sum[2] + sum[3]);
         const int row = m0 + (l >> 2) + 8 * (i >> 1), col = n0 + 8 * n + 2 * (l & 3) + (i & 1);
         if (row < M && col < N) C[(size_t)row * N + col] = (float)fma(total, kLean, total);
     }
