@@ -202,74 +202,56 @@ __global__ void __launch_bounds__(kLanes * kColumns / COLS) linear_attention_ker
     }
 
     const bool whole = key_dim % 4 == 0 && ((uintptr_t)state & 15) == 0;
-    // Two neighbouring channels of a column: every operation is two wide, half as many to issue (the whole call for 1,531
-    // tokens of 32 heads of 128 x 128: gated decays 286 -> 267 us, a constant decay 278 -> 241).
-    using pair = unsigned long long;
-    pair s[COLS][PER / 2];
+    float s[COLS][PER];
 #pragma unroll
     for (int c = 0; c < COLS; ++c) {
         const float* src = S + (size_t)min(own_col + c, value_dim - 1) * key_dim;     // idle columns mirror the last one and store nothing
 #pragma unroll
         for (int i = 0; i < PER; i += 4) {
             const int d = (i / 4) * (4 * kLanes) + lane * 4;
-            float x[4];
             if (whole) {                      // a run of four is inside the key or outside as a whole
-                const float4 v = d < key_dim ? *reinterpret_cast<const float4*>(src + d) : make_float4(0.f, 0.f, 0.f, 0.f);
-                x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+                const float4 x = d < key_dim ? *reinterpret_cast<const float4*>(src + d) : make_float4(0.f, 0.f, 0.f, 0.f);
+                s[c][i] = x.x; s[c][i + 1] = x.y; s[c][i + 2] = x.z; s[c][i + 3] = x.w;
             } else {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) x[j] = d + j < key_dim ? src[d + j] : 0.f;
+                for (int j = 0; j < 4; ++j) s[c][i + j] = d + j < key_dim ? src[d + j] : 0.f;
             }
-            s[c][i / 2] = pack2(x[0], x[1]);
-            s[c][i / 2 + 1] = pack2(x[2], x[3]);
         }
     }
     const float own = per_head != nullptr ? per_head[head] : 0.f;      // the constant decay, or the skip's factor
 
     // one token: the sums of its read-out over this lane's channels, and the state behind it
     auto advance = [&](const float* tok, float (&sums)[COLS]) {
-        pair v[COLS], sum[COLS];
-        float decay = own, step = 1.f;
+        float v[COLS];
+#pragma unroll
+        for (int c = 0; c < COLS; ++c) {
+            v[c] = tok[V_AT + group * COLS + c];
+            sums[c] = 0.f;
+        }
+        float decay = own;
         if (KIND == kSteppedDecay) {
             const float2 tail = *reinterpret_cast<const float2*>(tok + TAIL_AT);
             decay = tail.x;
-            step = tail.y;
-        }
 #pragma unroll
-        for (int c = 0; c < COLS; ++c) {
-            float x = tok[V_AT + group * COLS + c];
-            if (KIND == kSteppedDecay) x *= step;
-            v[c] = pack2(x, x);
-            sum[c] = 0;                       // (two zeros)
+            for (int c = 0; c < COLS; ++c) v[c] *= tail.y;
         }
 #pragma unroll
         for (int i = 0; i < PER; i += 4) {
             const int d = (i / 4) * (4 * kLanes) + lane * 4;
-            const ulonglong2 k = *reinterpret_cast<const ulonglong2*>(tok + d);
-            const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(tok + KP + d);
-            ulonglong2 a;
-            if (PARTS == 3) a = *reinterpret_cast<const ulonglong2*>(tok + 2 * KP + d);
-            else a.x = a.y = pack2(decay, decay);
+            const float4 k = *reinterpret_cast<const float4*>(tok + d);
+            const float4 q = *reinterpret_cast<const float4*>(tok + KP + d);
+            float4 a = make_float4(decay, decay, decay, decay);
+            if (PARTS == 3) a = *reinterpret_cast<const float4*>(tok + 2 * KP + d);
 #pragma unroll
             for (int c = 0; c < COLS; ++c) {
-                pair* x = s[c] + i / 2;
-                if (KIND == kBonusRead) {
-                    sum[c] = fma2(x[0], q.x, sum[c]);
-                    sum[c] = fma2(x[1], q.y, sum[c]);
-                }
-                x[0] = fma2(a.x, x[0], mul2(k.x, v[c]));      // (one multiply-add links a token's state to the next)
-                x[1] = fma2(a.y, x[1], mul2(k.y, v[c]));
-                if (KIND != kBonusRead) {
-                    sum[c] = fma2(x[0], q.x, sum[c]);
-                    sum[c] = fma2(x[1], q.y, sum[c]);
-                }
+                float* x = s[c] + i;
+                if (KIND == kBonusRead) sums[c] += x[0] * q.x + x[1] * q.y + x[2] * q.z + x[3] * q.w;
+                x[0] = fmaf(a.x, x[0], k.x * v[c]);      // (one multiply-add links a token's state to the next)
+                x[1] = fmaf(a.y, x[1], k.y * v[c]);
+                x[2] = fmaf(a.z, x[2], k.z * v[c]);
+                x[3] = fmaf(a.w, x[3], k.w * v[c]);
+                if (KIND != kBonusRead) sums[c] += x[0] * q.x + x[1] * q.y + x[2] * q.z + x[3] * q.w;
             }
-        }
-#pragma unroll
-        for (int c = 0; c < COLS; ++c) {
-            float lo, hi;
-            unpack2(sum[c], lo, hi);
-            sums[c] = lo + hi;
         }
     };
     float* own_share = shares + (size_t)group * COLS * SHARE + lane;
@@ -326,15 +308,12 @@ __global__ void __launch_bounds__(kLanes * kColumns / COLS) linear_attention_ker
 #pragma unroll
         for (int i = 0; i < PER; i += 4) {
             const int d = (i / 4) * (4 * kLanes) + lane * 4;
-            float x[4];
-            unpack2(s[c][i / 2], x[0], x[1]);
-            unpack2(s[c][i / 2 + 1], x[2], x[3]);
             if (whole) {
-                if (d < key_dim) *reinterpret_cast<float4*>(dst + d) = make_float4(x[0], x[1], x[2], x[3]);
+                if (d < key_dim) *reinterpret_cast<float4*>(dst + d) = make_float4(s[c][i], s[c][i + 1], s[c][i + 2], s[c][i + 3]);
             } else {
 #pragma unroll
                 for (int j = 0; j < 4; ++j)
-                    if (d + j < key_dim) dst[d + j] = x[j];
+                    if (d + j < key_dim) dst[d + j] = s[c][i + j];
             }
         }
     }
