@@ -72,6 +72,23 @@ def test_delta_matches_64_bits(lens, held, n_heads, n_kv, vdim):
             assert torch.equal(got_ring[slot, (held + r - cu[i]) % taps].cpu(), proj[r, :shape.conv_channels])
 
 
+@pytest.mark.parametrize("n_seqs,held", [(65535, 3), (65537, 2)])
+def test_the_ring_of_very_many_sequences(n_seqs, held):
+    """Two rows a sequence, as many sequences as a grid's second and third axes cannot count."""
+    dev = torch.device("cuda", 0)
+    shape, lens = ops.DeltaShape(1, 1, 4, 4, 4), torch.full((n_seqs,), held, dtype=torch.int32, device=dev)
+    rows = ops.step_rows(torch.arange(0, 2 * n_seqs + 1, 2, dtype=torch.int32, device=dev), torch.arange(n_seqs, dtype=torch.int32, device=dev),
+                         lens, 2 * n_seqs, 2)
+    g = torch.Generator(device=dev).manual_seed(n_seqs)
+    draw = lambda *s: torch.randn(*s, generator=g, device=dev)
+    proj, ring = draw(2 * n_seqs, shape.proj_width).to(BF16), draw(n_seqs, 4, shape.conv_channels).to(BF16)
+    want = ring.clone()
+    for i in range(2):
+        want[:, (held + i) % 4] = proj[i::2, :shape.conv_channels]
+    ops.delta_rule(proj, draw(shape.conv_channels, 4), draw(1), draw(1), torch.zeros(n_seqs, 1, 4, 4, device=dev), ring, rows, lens, shape, 1e-6)
+    assert torch.equal(ring, want)
+
+
 @pytest.mark.parametrize("lens,n_heads,vdim", [
     ([16], 2, 128), ([31, 1, 33], 3, 16), ([32, 64, 65, 2], 2, 48), ([97], 4, 256), ([40] * 8, 16, 128), ([70, 35], 1, 64)])
 def test_matrix_memory_matches_64_bits(lens, n_heads, vdim):

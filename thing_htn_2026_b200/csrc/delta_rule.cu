@@ -603,15 +603,16 @@ constexpr size_t kDeltaChunkBytes = (size_t)6 * chunk::kTokens * chunk::kKeyRow 
                                     (chunk::kTokens * kValueRow + chunk::kTokens * kSquare + 4 * chunk::kTokens) * sizeof(float);
 
 // After a step: the raw projections of the step's last taps - 1 positions go into the ring
-// (position p at p mod taps).  A thread per channel (one block per sequence took 20 us for 3,072 channels, this 3).  Nothing reads the ring while this
-// runs: the kernels of the step that read it have ended.
+// (position p at p mod taps).  A thread per channel (one block per sequence took 20 us for 3,072 channels, this 3);
+// the sequences lie along x, the grid's axis that takes more than 65,535.  Nothing reads the ring while this runs: the
+// kernels of the step that read it have ended.
 template <typename T>
 __global__ void conv_ring_update_kernel(T* __restrict__ ring, const T* __restrict__ proj,
                                         const int* __restrict__ cu_seqlens, const int* __restrict__ slots,
                                         const int* __restrict__ seq_lens, DeltaShape s) {
     pdl_launch_dependents();
     pdl_wait();
-    const int seq = blockIdx.y;
+    const int seq = blockIdx.x;
     const int row0 = cu_seqlens[seq], n = cu_seqlens[seq + 1] - row0;
     const int slot = slots[seq], start = seq_lens[slot];
     const int C = s.conv_channels();
@@ -619,7 +620,7 @@ __global__ void conv_ring_update_kernel(T* __restrict__ ring, const T* __restric
     T* dst = ring + (size_t)slot * s.taps * C;
     for (int t = n - keep; t < n; ++t) {
         const int p = start + t;
-        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < C; c += gridDim.x * blockDim.x)
+        for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < C; c += gridDim.y * blockDim.x)
             dst[(size_t)(p % s.taps) * C + c] = proj[(size_t)(row0 + t) * s.proj_width + c];
     }
 }
@@ -909,8 +910,8 @@ THN_API int thn_delta_conv_ring_update(void* ring, const void* proj, const int* 
     DeltaShape s{n_heads, n_kv, dk, dv, taps, proj_width};
     if (int status = check_shape(s, "delta_conv_ring_update")) return status;
     if (n_seqs <= 0 || taps <= 1) return THN_OK;
-    THN_UNSUPPORTED_IF(n_seqs > 65535, "delta_conv_ring_update: %d sequences", n_seqs);
-    const dim3 ring_grid((unsigned)((s.conv_channels() + 255) / 256), (unsigned)n_seqs);
+    const int channel_blocks = (s.conv_channels() + 255) / 256;
+    const dim3 ring_grid((unsigned)n_seqs, (unsigned)(channel_blocks < 65535 ? channel_blocks : 65535));
     if (dtype == THN_F32)
         thn_launch(conv_ring_update_kernel<float>, ring_grid, 256, 0, stream, (float*)ring, (const float*)proj, cu_seqlens,
                    slots, seq_lens, s);
