@@ -165,3 +165,93 @@ def test_state_space_matches_64_bits(lens, held, n_heads, groups, vdim):
         want_state[slot] = S
     close(got.cpu(), want, max(lens))
     close(got_state.cpu()[1:], want_state[1:], max(lens))
+
+
+# What is not finite must reach what it reaches token by token and nothing else: in particular no token ahead of it.
+BAD = (float("nan"), float("inf"))
+
+
+def same_reach(chunks, tokens):
+    """The same entries are finite, and those are close: two float32 ways to take the same sums."""
+    for a, b in zip(chunks, tokens):
+        there = torch.isfinite(b)
+        assert torch.equal(torch.isfinite(a), there) and there.any()
+        assert (a[there] - b[there]).abs().max() <= 2 ** -16 * b[there].abs().max()
+
+
+@pytest.mark.parametrize("bad", BAD)
+@pytest.mark.parametrize("what", ["q", "k", "v", "b", "a", "a_log"])
+@pytest.mark.parametrize("lens,at,vdim", [([70, 40], 37, 128), ([33], 16, 16), ([40], 31, 160)])
+def test_delta_keeps_what_is_not_finite_to_itself(monkeypatch, bad, what, lens, at, vdim):
+    rows, seq_lens, cu, _ = step(lens)
+    dev, shape = rows.slots.device, ops.DeltaShape(4, 2, 128, vdim, 4)
+    g = torch.Generator(device=dev).manual_seed(at)
+    draw = lambda *s: torch.randn(*s, generator=g, device=dev)
+    proj, w, a_log, dt_bias = draw(cu[-1], shape.proj_width).to(BF16), draw(shape.conv_channels, 4) * 0.5, draw(4), draw(4)
+    gate_end = shape.gate_offset + 4 * vdim
+    column = {"q": 5, "k": 256 + 128 + 7, "v": 512 + vdim + 3, "b": gate_end + 1, "a": gate_end + 4 + 2}.get(what)
+    if column is None:
+        a_log[1] = bad          # an infinite one is a decay of zero, a NaN a NaN
+    else:
+        proj[at, column] = bad
+    state, ring = draw(len(lens) + 1, 4, vdim, 128) * 0.2, torch.zeros(len(lens) + 1, 4, shape.conv_channels, dtype=BF16, device=dev)
+    results = []
+    for lanes in (0, 8):
+        monkeypatch.setattr(ops, "DELTA_LANES", lanes)
+        s = state.clone()
+        assert ops._delta_in_chunks(proj, w, s, ring, rows, shape) == (lanes == 0)
+        results.append((ops.delta_rule(proj, w, a_log, dt_bias, s, ring.clone(), rows, seq_lens, shape, 1e-6), s))
+    same_reach(*results)
+
+
+@pytest.mark.parametrize("bad", BAD)
+@pytest.mark.parametrize("what", ["q", "k", "v", "i", "f"])
+@pytest.mark.parametrize("lens,at,heads,vdim", [([70, 40], 37, 2, 128), ([33], 16, 2, 16), ([40] * 8, 50, 16, 128)])
+def test_matrix_memory_keeps_what_is_not_finite_to_itself(bad, what, lens, at, heads, vdim):
+    rows, _, cu, _ = step(lens)
+    dev = rows.slots.device
+    g = torch.Generator(device=dev).manual_seed(at)
+    draw = lambda *s: torch.randn(*s, generator=g, device=dev)
+    proj, pre = draw(cu[-1], heads * (256 + vdim)).to(BF16), draw(cu[-1], 2 * heads)
+    if what in "if":
+        pre[at, 1 + (heads if what == "f" else 0)] = bad       # (the cap makes a large number of an infinity)
+    else:
+        proj[at, {"q": 128 + 5, "k": (heads + 1) * 128 + 7, "v": heads * 256 + vdim + 3}[what]] = bad
+    state, normaliser = draw(len(lens) + 1, heads, vdim, 128), draw(len(lens) + 1, heads, 1, 129).expand(-1, -1, vdim // 16, -1).contiguous()
+    results = []
+    for lanes in (0, 8):
+        ops.set_mlstm_kernel(True, lanes)
+        try:
+            s, n = state.clone(), normaliser.clone()
+            assert ops._mlstm_in_chunks(proj, s, rows, heads, 128, vdim) == (lanes == 0)
+            results.append((ops.mlstm(proj, pre, torch.zeros(heads, device=dev), torch.ones(heads, device=dev), 15.0, s, n, rows, heads,
+                                      128, vdim, 128 ** -0.5), s, n[..., :128]))     # (behind a NaN gate the maximum says nothing)
+        finally:
+            ops.set_mlstm_kernel(True, 0)
+    same_reach(*results)
+
+
+@pytest.mark.parametrize("bad", BAD)
+@pytest.mark.parametrize("what", ["x", "B", "C", "step", "rate"])
+@pytest.mark.parametrize("lens,at,heads,groups,vdim", [([130, 40], 37, 4, 2, 64), ([113], 63, 2, 1, 16), ([128] * 8, 200, 64, 8, 64)])
+def test_state_space_keeps_what_is_not_finite_to_itself(monkeypatch, bad, what, lens, at, heads, groups, vdim):
+    rows, seq_lens, cu, _ = step(lens)
+    dev, inner = rows.slots.device, heads * vdim
+    g = torch.Generator(device=dev).manual_seed(at)
+    draw = lambda *s: torch.randn(*s, generator=g, device=dev)
+    channels = inner + 256 * groups
+    shape = ops.StateSpace(heads, vdim, 128, groups, draw(channels, 4) * 0.5, draw(channels) * 0.1, draw(heads) - 2, torch.exp(draw(heads)), draw(heads))
+    proj, dt = draw(cu[-1], channels).to(BF16), draw(cu[-1], heads)
+    if what == "rate":
+        shape.rate[1] = bad     # an infinite one is a decay of zero
+    elif what == "step":
+        dt[at, 1] = bad
+    else:
+        proj[at, {"x": vdim + 3, "B": inner + 7, "C": inner + groups * 128 + 9}[what]] = bad
+    state, ring = draw(len(lens) + 1, heads, vdim, 128) * 0.2, torch.zeros(len(lens) + 1, 4, channels, dtype=BF16, device=dev)
+    results = []
+    for in_chunks in (True, False):
+        monkeypatch.setattr(ops, "_space_in_chunks", lambda *a, answer=in_chunks: answer)
+        s = state.clone()
+        results.append((ops.state_space(proj, 0, dt, shape, s, ring.clone(), rows, seq_lens), s))
+    same_reach(*results)

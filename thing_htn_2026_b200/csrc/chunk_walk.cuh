@@ -86,6 +86,10 @@ __device__ __forceinline__ uint32_t pack_bf16(float x, float y) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
     return *reinterpret_cast<const uint32_t*>(&v);
 }
+// Nonzero where one of the two halves is an infinity or a NaN.
+__device__ __forceinline__ uint32_t not_finite(uint32_t two) { return ((two & 0x7f807f80u) + 0x00800080u) & 0x80008000u; }
+__device__ __forceinline__ bool finite(float x) { return (__float_as_uint(x) & 0x7f800000u) != 0x7f800000u; }
+__device__ __forceinline__ float not_a_number() { return __uint_as_float(0x7fffffffu); }
 __device__ __forceinline__ float low_half(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float high_half(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 // two floats in three parts each: part[0] + part[1] + part[2], exactly
@@ -462,6 +466,36 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
             scaled[j] = parts_of(make_float2(v[0].x * w0, v[0].y * w1), make_float2(v[1].x * w0, v[1].y * w1),
                                  make_float2(v[2].x * w8, v[2].y * w9), make_float2(v[3].x * w8, v[3].y * w9));
         }
+        // Where G is zero the products still multiply, and zero times an infinity or a NaN is NaN: such a value would reach
+        // the tokens ahead of its own.  It is left out of the products with G, and its column's read-outs are NaN from its
+        // token on.  (The state takes it as it is.)
+        int lost[2] = {kTokens, kTokens};            // the first such token of columns g and g + 8
+        {
+            uint32_t any = 0;
+#pragma unroll
+            for (int j = 0; j < kTokens / 16; ++j)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) any |= not_finite(plain[j].part[0][i]);
+            if (__any_sync(0xffffffffu, any != 0)) {
+#pragma unroll
+                for (int j = 0; j < kTokens / 16; ++j)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const uint32_t which = not_finite(plain[j].part[0][i]);
+                        const int token = 16 * j + 8 * (i >> 1) + 2 * t;
+                        if (which & 0x80000000u) lost[i & 1] = min(lost[i & 1], token + 1);
+                        if (which & 0x00008000u) lost[i & 1] = min(lost[i & 1], token);
+                        const uint32_t kept = (which & 0x80000000u ? 0u : 0xffff0000u) | (which & 0x00008000u ? 0u : 0x0000ffffu);
+#pragma unroll
+                        for (int p = 0; p < (PARTS == 1 ? 1 : 3); ++p) plain[j].part[p][i] &= kept;
+                    }
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    lost[c] = min(lost[c], __shfl_xor_sync(0xffffffffu, lost[c], 1));
+                    lost[c] = min(lost[c], __shfl_xor_sync(0xffffffffu, lost[c], 2));
+                }
+            }
+        }
         // the state behind the chunk
         const float keep = GATED ? alpha_s[n_here - 1] : scalars[n_here - 1].x, take = GATED ? beta_s[n_here - 1] : 1.f;
         constexpr int KP = 2;                        // pairs of groups of keys at a time
@@ -517,8 +551,8 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
                 const int i = 8 * (group0 + n) + 2 * t + half;
                 if (i >= n_here) continue;
                 const int o = OWN == 1 ? group0 & 1 : n & 1;
-                const float in0 = o ? inner[n / 2][1][half] : inner[n / 2][0][half];
-                const float in1 = o ? inner[n / 2][1][2 + half] : inner[n / 2][0][2 + half];
+                const float in0 = i >= lost[0] ? not_a_number() : o ? inner[n / 2][1][half] : inner[n / 2][0][half];
+                const float in1 = i >= lost[1] ? not_a_number() : o ? inner[n / 2][1][2 + half] : inner[n / 2][0][2 + half];
                 const float alpha = GATED ? alpha_s[i] : scalars[i].x, beta = GATED ? beta_s[i] : 1.f;
                 float y0 = (alpha * read[n][half] + beta * in0) * a.scale;
                 float y1 = (alpha * read[n][2 + half] + beta * in1) * a.scale;
@@ -571,8 +605,10 @@ __device__ __forceinline__ double lanes_cumulative(double v, int lane) {
     }
     return v;
 }
-// The logarithm of a decay in [0, 1]; a decay of zero gets one whose exponential is zero in float32.
-__device__ __forceinline__ double log_decay(float a) { return a > 0.f ? log((double)a) : -200.0; }
+// The logarithm of a decay in [0, 1]; a decay of zero gets one whose exponential is zero in float32, so that differences of
+// sums of logarithms stay numbers.  A NaN stays one.
+constexpr double kLogOfNothing = -200.0;
+__device__ __forceinline__ double log_decay(float a) { return a <= 0.f ? kLogOfNothing : log((double)a); }
 
 // Rows 16 m_tile .. of x times all 32 rows of y, both planes of kKeys in shared memory: out[n][..] are
 // the products of rows (g, g, g + 8, g + 8) with rows 8n + (2t, 2t + 1, 2t, 2t + 1); groups of y that lie

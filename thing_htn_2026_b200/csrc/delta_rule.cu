@@ -427,6 +427,10 @@ __global__ void __launch_bounds__(128) delta_prepare_chunks_kernel(
 // of W and U.  Products on the tensor cores in three parts, T in float32 multiply-adds; the log decays are
 // summed in double, so that differences of large sums stay exact.  Out: U in place of the values, W and
 // D_ij q_i . k_j as planes, the scalars.
+// T is zero above the diagonal, but a product multiplies there too, and zero times a NaN is NaN.  So that tokens ahead
+// of one with a key, b or decay that is not finite do not see it, its key and factors are zero in the products, and its
+// row of U is NaN (the walk spreads that to the tokens behind it); a value that is not finite is zero in the products, and
+// its own entry of U is NaN.
 constexpr int kChunkThreads = 128;
 constexpr int kSquare = chunk::kTokens + 8;            // row of a 32 x 32 matrix of floats
 constexpr int kValueRow = 128 + 4;
@@ -446,6 +450,7 @@ __global__ void __launch_bounds__(kChunkThreads) delta_chunk_kernel(
     float* e_s = a_s + C * kSquare;                                        // [C] exp(c)
     float* b_s = e_s + C;                                                  // [C]
     double* c_s = reinterpret_cast<double*>(b_s + C);                      // [C]
+    __shared__ unsigned lost_s;                                            // bit i: token i has a key, b or decay that is not finite
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int head = blockIdx.y, seq = blockIdx.z, unit = head / (s.n_heads / s.n_kv);
     const int begin = cu_seqlens[seq], row0 = begin + blockIdx.x * C, n_here = min(C, cu_seqlens[seq + 1] - row0);
@@ -472,9 +477,13 @@ __global__ void __launch_bounds__(kChunkThreads) delta_chunk_kernel(
         const bool there = lane < n_here;
         const double c = chunk::lanes_cumulative(there ? chunk::log_decay(decay[at]) : 0.0, lane);
         const double c_last = __shfl_sync(0xffffffffu, c, n_here - 1);
+        const float b = there ? beta[at] : 0.f;
+        const bool is_lost = isnan(c) || !chunk::finite(b);
+        const unsigned all_lost = __ballot_sync(0xffffffffu, is_lost);
+        if (lane == 0) lost_s = all_lost;
         c_s[lane] = c;
-        e_s[lane] = expf((float)c);
-        b_s[lane] = there ? beta[at] : 0.f;
+        e_s[lane] = is_lost ? 0.f : expf((float)c);
+        b_s[lane] = is_lost ? 0.f : b;
         if (there) scalars[(size_t)head * n_rows + row0 + lane] = make_float4(e_s[lane], 0.f, expf((float)(c_last - c)), 0.f);
     }
     chunk::copy_wait_all();
@@ -492,6 +501,7 @@ __global__ void __launch_bounds__(kChunkThreads) delta_chunk_kernel(
             for (int half = 0; half < 2; ++half) {
                 const int i = 16 * m_tile + g + 8 * half, j = 8 * n + 2 * t;
                 float x[2];
+                if (of_keys && (i & ~1) == j && !chunk::finite(i & 1 ? dot[n][2 * half + 1] : dot[n][2 * half])) atomicOr(&lost_s, 1u << i);      // k_i . k_i
 #pragma unroll
                 for (int o = 0; o < 2; ++o)
                     x[o] = j + o <= i ? expf((float)(c_s[i] - c_s[j + o])) * dot[n][2 * half + o] : 0.f;
@@ -502,6 +512,10 @@ __global__ void __launch_bounds__(kChunkThreads) delta_chunk_kernel(
             }
     }
     __syncthreads();
+    const unsigned lost = lost_s;
+    if (lost)
+        for (int e = tid; e < 3 * kPlane; e += kChunkThreads)
+            if (lost >> (e % kPlane / chunk::kKeyRow) & 1) k_s[e] = __float2bfloat16_rn(0.f);
     if (warp == 0) {
         // (I + A)^-1 column by column: lane j holds column j
         float column[C];
@@ -520,7 +534,7 @@ __global__ void __launch_bounds__(kChunkThreads) delta_chunk_kernel(
         }
         __syncwarp();
 #pragma unroll
-        for (int i = 0; i < C; ++i) a_s[i * kSquare + lane] = column[i] * b_s[lane];
+        for (int i = 0; i < C; ++i) a_s[i * kSquare + lane] = lane <= i ? column[i] * b_s[lane] : 0.f;
     }
     __syncthreads();
     // T diag(b) (exp(c) for W) as A operands: tokens by tokens; [0]: rows 0-15, [1], [2]: rows 16-31 by tokens 0-15, 16-31
@@ -580,21 +594,31 @@ __global__ void __launch_bounds__(kChunkThreads) delta_chunk_kernel(
             chunk::copy_wait_all();
             __syncthreads();
         }
+        bool some_lost = lost != 0;             // of the warp
         by_rows(a,
                 [&](int n, int j) {
                     chunk::Columns<3> b;
+                    bool own_lost = false;
 #pragma unroll
                     for (int o = 0; o < 2; ++o)
 #pragma unroll
                         for (int half = 0; half < 2; ++half) {
                             const float* p = v_s + (16 * j + 8 * half + 2 * t) * kValueRow + 32 * warp + 8 * (n + o) + g;
-                            const chunk::Split x = chunk::split(p[0], p[kValueRow]);
+                            const bool ok0 = chunk::finite(p[0]), ok1 = chunk::finite(p[kValueRow]);
+                            own_lost |= !ok0 || !ok1;
+                            const chunk::Split x = chunk::split(ok0 ? p[0] : 0.f, ok1 ? p[kValueRow] : 0.f);
 #pragma unroll
                             for (int i = 0; i < 3; ++i) b.part[i][2 * o + half] = x.part[i];
                         }
+                    some_lost |= __any_sync(0xffffffffu, own_lost);
                     return b;
                 },
                 [&](int i, int d, float x, float y) {
+                    if (some_lost) {
+                        const bool row = lost >> i & 1;
+                        if (row || !chunk::finite(v_s[i * kValueRow + d])) x = chunk::not_a_number();
+                        if (row || !chunk::finite(v_s[i * kValueRow + d + 1])) y = chunk::not_a_number();
+                    }
                     if (e0 + d < s.dv) *reinterpret_cast<float2*>(own_values + (size_t)i * s.dv + e0 + d) = make_float2(x, y);
                 });
     }

@@ -276,7 +276,8 @@ __global__ void __launch_bounds__(kSpaceThreads) state_space_chunk_kernel(
         const int head = group * heads_per_group + h;
         const bool there = lane < n_here;
         const float step = there ? steps[(size_t)head * n_rows + row0 + lane] : 0.f;
-        const double c = chunk::lanes_cumulative(-(double)rate[head] * step, lane);
+        const double log_own = there ? -(double)rate[head] * step : 0.0;      // (an infinite one, as of an infinite rate, is one of a decay of zero)
+        const double c = chunk::lanes_cumulative(log_own < chunk::kLogOfNothing ? chunk::kLogOfNothing : log_own, lane);
         const double c_last = __shfl_sync(0xffffffffu, c, 31);            // (tokens beyond the step's add nothing)
         const float d = skip[head];
         if (there)
