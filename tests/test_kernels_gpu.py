@@ -101,6 +101,37 @@ def test_a_few_float32_outputs_per_row(m, n, k):
     assert torch.equal(alone[0], got[m // 2])
 
 
+@pytest.mark.parametrize("m, n, k", [(1, 1, 8), (3, 5, 72), (17, 9, 2048), (300, 33, 4104), (1000, 64, 4104), (2100, 33, 1024), (1921, 16, 72)])
+def test_a_few_float32_outputs_per_row_that_float32_holds_exactly(m, n, k):
+    """Sums of small whole numbers, and rows of one entry: whatever order they are taken in, nothing is rounded."""
+    g = torch.Generator().manual_seed(m + n + k)
+    whole = lambda *s: torch.randint(-8, 9, s, generator=g).to(torch.bfloat16)       # |sums| < 2^6 k < 2^24
+    one = torch.zeros(m, k, dtype=torch.bfloat16).scatter_(1, torch.randint(0, k, (m, 1), generator=g), rand((m, 1), torch.bfloat16, 3))
+    for x, w in ((whole(m, k), whole(n, k)), (one, rand((n, k), torch.bfloat16, 4))):
+        got = ops().linear(x.to(DEV), w.to(DEV), out_dtype=torch.float32).cpu()
+        assert torch.equal(got.double(), x.double() @ w.double().t())
+
+
+@pytest.mark.parametrize("m, n, k", [(2100, 33, 1024), (1000, 64, 4104), (1921, 16, 72)])
+@pytest.mark.parametrize("kind", ["normal", "positive", "cancelling"])
+def test_many_rows_of_a_few_float32_outputs(m, n, k, kind):
+    """Two tiles of columns a block and several blocks of columns: every entry, and a row alone has the same bits."""
+    x, w = rand((m, k), torch.bfloat16, 1), rand((n, k), torch.bfloat16, 2, 0.3)
+    if kind == "positive":
+        x, w = x.abs(), w.abs()
+    elif kind == "cancelling":
+        x[:, k // 2:] = x[:, :k // 2]
+        w[:, k // 2:] = -w[:, :k // 2]
+    got = ops().linear(x.to(DEV), w.to(DEV), out_dtype=torch.float32).cpu()
+    size = x.double().abs() @ w.double().abs().t()
+    # of the sum of the products' sizes: a product of 16 loses at most 2^-22 of its largest partial sum, and of the at
+    # most 11 additions behind it (8 in a warp, 3 over the warps in double and one rounding) each at most 2^-24
+    assert ((got.double() - x.double() @ w.double().t()).abs() <= (2 ** -22 + 12 * 2 ** -24) * size).all()
+    for row in (0, m // 2, m - 1):
+        alone = ops().linear(x[row:row + 1].to(DEV).contiguous(), w.to(DEV), out_dtype=torch.float32).cpu()
+        assert torch.equal(alone[0], got[row])
+
+
 def test_rope_table_matches_formula():
     from thing_htn_2026_b200.config.base import PartSpec
     from thing_htn_2026_b200.parts import Runtime, part_class

@@ -73,14 +73,19 @@ THN_API int thn_gemm_f32(float* C, const float* A, const float* W, int M, int N,
 // C[M, N] float32 = A[M, K] bfloat16 @ W[N, K]^T bfloat16 for a weight of few rows (a router, a
 // gate of one number per token): the products that vendor libraries serve worst, since N is
 // neither large nor a multiple of eight.  A block takes 16 rows and 8 TILES columns; its sixteen warps deal out
-// K in steps of 32 on the tensor cores, each product into a fresh accumulator (the tensor core's accumulation
-// rounds towards zero, by kLean of the result on average, which is put back at the end; the sum over the steps is
-// float32 additions).  A lane loads its operands straight from memory, 16 bytes of a row at k = 32 s + 8 t: which
+// K in steps of 32 on the tensor cores, each product of 16 into a fresh accumulator (the tensor core's accumulation
+// rounds towards zero; the sum over the products is float32 additions, over the warps double ones).  A sum that float32
+// holds exactly comes out exactly.  A lane loads its operands straight from memory, 16 bytes of a row at k = 32 s + 8 t: which
 // k a lane's pair stands for does not matter as long as both operands agree; the loads of four or eight steps are
 // issued together.  The warps' sums meet in shared memory in a fixed order, so a row's result depends on nothing but K,
 // whatever M, N and TILES are.  K is a multiple of eight and both operands are 16-byte aligned.
-// B200, against a warp's float32 multiply-adds over four rows and four columns at a time: 2,251 rows, 32 columns over 2,048
-// 8 us / 31, 4,096 rows over 4,096 25 / 84, 1 to 64 rows the same; the error against 64 bits 6.5e-8 to 7.6e-8 / 7.9e-8 to 8.5e-8.
+// B200, against a warp's float32 multiply-adds over four rows and four columns at a time, which it took the place of: 2,251
+// rows, 32 columns over 2,048 5.8 us / 27.4, 4,096 rows, 64 columns over 4,096 30 / 143; few rows the same with the weight
+// in HBM (8 rows, 32 columns over 4,096: 8.2 / 10.2), 0.1 to 1.1 us more back to back with everything in L2 (2.2 / 1.8 for 8
+// rows, 32 columns over 2,048; the number of rows may not choose the kernel, since a row's bits would follow it).  Error against 64 bits,
+// 2-norms: 5.8e-8 to 7.3e-8 / 7.9e-8 to 9.2e-8 over 2,048 and 4,096 normal entries, 2.8e-8 / 4.8e-8 where all are positive,
+// 7.3e-8 / 9.1e-8 where they spread over forty powers of two.  (Scaling the result up by the
+// accumulation's mean loss, 4.3e-8, changes sums that were exact.)
 namespace {
 constexpr int kSkinnyThreads = 512;
 
@@ -98,7 +103,6 @@ __global__ void __launch_bounds__(kSkinnyThreads) linear_skinny_kernel(float* __
     pdl_launch_dependents();
     pdl_wait();
     constexpr int kWarps = kSkinnyThreads / 32, kBatch = TILES == 1 ? 8 : 4;
-    constexpr double kLean = 4.3e-8;
     __shared__ __align__(16) float part[kWarps][TILES][32][4];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const int m0 = blockIdx.x * 16, n0 = blockIdx.y * 8 * TILES;
@@ -150,7 +154,7 @@ __global__ void __launch_bounds__(kSkinnyThreads) linear_skinny_kernel(float* __
         for (int k = 0; k < kWarps; ++k) sum[k & 3] += (double)part[k][n][l][i];
         const double total = (sum[0] + sum[1]) + (sum[2] + sum[3]);
         const int row = m0 + (l >> 2) + 8 * (i >> 1), col = n0 + 8 * n + 2 * (l & 3) + (i & 1);
-        if (row < M && col < N) C[(size_t)row * N + col] = (float)fma(total, kLean, total);
+        if (row < M && col < N) C[(size_t)row * N + col] = (float)total;
     }
 }
 }  // namespace

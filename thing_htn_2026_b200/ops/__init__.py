@@ -905,7 +905,8 @@ def linear_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, err: Optional[torch.
 
 # The product of few columns re-reads its weight for every 16 rows: with many rows and more than a few
 # columns a caller that does not need a row's result to be independent of its neighbours gets the vendor
-# library's product.
+# library's product.  (B200, 64 columns over 2,048 entries, this kernel against the library: 256 rows 2.9 / 6.3 us,
+# 1,024 5.9 / 6.3, 2,048 10.9 / 6.4; 16 columns, 2,048 rows 3.7 / 6.3.  The two meet at about 1,000 rows of 64 columns.)
 SKINNY_MAX_ROWS = 256
 SKINNY_ANY_ROWS_COLUMNS = 16
 
