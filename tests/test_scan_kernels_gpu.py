@@ -47,6 +47,12 @@ def test_scan_matches_64_bits(channels, state, lens):
     assert ((y.cpu().double() - want).abs() <= 2 ** -8 * want.abs() + 2 ** -14 * want.abs().amax()).all()
 
 
+@pytest.mark.parametrize("channels,state,lens", [(2400, 16, [3] + [1] * 40), (4096, 16, [2] + [1] * 8), (4100, 9, [17] + [1] * 20), (2400, 32, [2] * 30)])
+def test_scan_of_a_few_tokens_among_single_ones(channels, state, lens):
+    """Steps that are cheaper token by token."""
+    test_scan_matches_64_bits(channels, state, lens)
+
+
 @pytest.mark.parametrize("channels,offset,lens,held,bias", [
     (4, 0, [1], 0, True), (12, 4, [9, 2, 8], 0, True), (516, 8, [7, 17], 2, False), (64, 0, [1, 3, 24], 5, True),
     (6, 0, [9], 3, True), (64, 2, [9], 3, True)])

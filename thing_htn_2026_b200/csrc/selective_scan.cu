@@ -17,12 +17,16 @@
 //   selective_scan     a channel's state is held by 4 lanes (8 for states above 32; entry n by lane
 //                 n mod lanes); one block per (sequence, 64 or 32 channels) walks the sequence's tokens of the step in order;
 //                 the tokens come through shared memory, sixteen at a time in two buffers.
+//   selective_scan_walk     the same for bfloat16 prompts with states up to 32 (walk_pays): half of a block's warps walk the
+//                 state, the others load, transform and write beside them.
 //
 // float32 after the loads: the step size with its softplus, the decay with its exponential, the
 // state, the sums, the gate.  The convolution is summed in float32 and rounded once after silu.
 // With float32 activations the exponentials and logarithms are computed in double and rounded once
 // (exp_of, silu_of, softplus_of in common.cuh).
 #include <math.h>
+
+#include <algorithm>
 
 #include "common.cuh"
 
@@ -518,6 +522,20 @@ int launch_walk(void* y, float* state, const void* x, const float* dt_pre, const
     return thn_launch_status("selective_scan");
 }
 
+// Whether a step's rows are walked by the kernel above.  It takes a sequence's tokens sixteen at a time, so that one token
+// costs as much as sixteen: a few prompts among many single tokens are cheaper token by token.  What the two take, in us on
+// B200, to within a fifth of what was measured (4,096 channels, 16 entries, token by token / walked):
+// two tokens of one sequence 6.3 / 4.8, beside 8 single tokens 7.7 / 11.9; 16 beside 8 10.4 / 12.3, beside 60 39 / 61; 128 beside
+// 8 55 / 21, beside 60 57 / 66; 2,048 beside 60 770 / 205; 64 sequences of 2 59 / 66, of 4 70 / 66, of 16 133 / 70.
+bool walk_pays(int n_rows, int max_tokens, int n_seqs, int channels) {
+    const float width = channels / 4096.f;
+    const long long longest = (max_tokens + kWalkStage - 1) / kWalkStage;
+    const long long stages = std::min((long long)n_seqs * longest, n_rows / kWalkStage + (long long)n_seqs);      // at most
+    const float by_token = 0.5f + std::max(0.37f * max_tokens, (0.09f * n_rows + 0.6f * n_seqs) * width);
+    const float walked = std::max(1.1f * longest, 0.95f * stages * width);
+    return max_tokens > 1 && walked <= by_token;
+}
+
 template <typename T>
 int launch_scan(void* y, float* state, const void* x, const float* dt_pre, const float* dt_bias, const void* bc,
                 int bc_width, const float* A, const float* D, const void* z, int z_stride, const int* cu_seqlens,
@@ -595,7 +613,7 @@ THN_API int thn_conv_ring_update(void* ring, const void* proj, int proj_width, i
 // (negative); D float32 [channels]; z of the activation type, rows z_stride apart.
 THN_API int thn_selective_scan(void* y, float* state, const void* x, const float* dt_pre, const float* dt_bias,
                                const void* bc, int bc_width, const float* A, const float* D, const void* z, int z_stride,
-                               const int* cu_seqlens, const int* slots, int n_rows, int n_seqs, int channels, int n_state, int dtype,
+                               const int* cu_seqlens, const int* slots, int n_rows, int max_tokens, int n_seqs, int channels, int n_state, int dtype,
                                cudaStream_t stream) {
     THN_CHECK_ARG(n_seqs >= 0 && channels > 0 && n_state > 0 && bc_width >= 2 * n_state && z_stride >= channels,
                   "selective_scan: bad sizes");
@@ -605,8 +623,7 @@ THN_API int thn_selective_scan(void* y, float* state, const void* x, const float
     if (dtype == THN_F32)
         return launch_scan<float>(y, state, x, dt_pre, dt_bias, bc, bc_width, A, D, z, z_stride, cu_seqlens, slots, n_seqs,
                                   channels, n_state, stream);
-    // (steps of one token per sequence move a state and nothing else: the kernel above reads it without a stage)
-    if (dtype == THN_BF16 && n_state <= 32 && n_rows > n_seqs)
+    if (dtype == THN_BF16 && n_state <= 32 && walk_pays(n_rows, max_tokens, n_seqs, channels))
         return launch_walk(y, state, x, dt_pre, dt_bias, bc, bc_width, A, D, z, z_stride, cu_seqlens, slots, n_seqs, channels,
                            n_state, stream);
     if (dtype == THN_BF16)

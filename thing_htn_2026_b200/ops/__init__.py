@@ -77,7 +77,7 @@ _SIGNATURES = {
     "thn_conv_ring_update": [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                              c_void_p],
     "thn_selective_scan": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
-                           c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p],
+                           c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "thn_rotate_gate": [c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_int, c_int, c_int,
                         c_void_p, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p],
     "thn_add_bias_f32": [c_void_p, c_void_p, c_int, c_int, c_float, c_void_p],
@@ -1855,7 +1855,7 @@ def selective_scan(x: torch.Tensor, dt_pre: torch.Tensor, dt_bias: torch.Tensor,
     y = torch.empty_like(x)
     _call("thn_selective_scan", _ptr(y), _ptr(state), _ptr(x), _ptr(dt_pre), _ptr(dt_bias), _ptr(bc), bc.shape[1], _ptr(a),
           _ptr(d), gate.data_ptr() + gate_offset * gate.element_size(), gate.shape[1], _ptr(rows.cu_seqlens),
-          _ptr(rows.slots), n_rows, rows.n_seqs, channels, n_state, _code(x, "selective_scan"), _stream())
+          _ptr(rows.slots), n_rows, rows.max_q_len, rows.n_seqs, channels, n_state, _code(x, "selective_scan"), _stream())
     return y
 
 
