@@ -24,7 +24,7 @@ def step(lens, held=0):
 @pytest.mark.parametrize("channels,state,lens", [
     (5, 3, [2]), (33, 8, [15, 16, 17, 1]), (64, 9, [33]), (100, 16, [31, 48, 2]), (16, 16, [1, 1, 2]),
     (2400, 16, [18, 33]), (70, 17, [40]), (40, 32, [16, 5]), (40, 40, [16, 5])])
-def test_scan_matches_64_bits(channels, state, lens):
+def test_scan_matches_64_bits(channels, state, lens, infinite=False):
     g = torch.Generator().manual_seed(channels * 31 + state)
     rows, _, cu = step(lens)
     total, dev = cu[-1], rows.slots.device
@@ -32,6 +32,8 @@ def test_scan_matches_64_bits(channels, state, lens):
     x, bc, gate = draw(total, channels).to(BF16), draw(total, 2 * state + 2).to(BF16), draw(total, channels + 3).to(BF16)
     dt, bias, d, start = draw(total, channels) * 2, draw(channels) * 0.1, draw(channels), draw(len(lens), channels, state)
     a = -torch.exp(draw(channels, state))
+    if infinite:
+        a[::2, state // 2] = -float("inf")
     held = start.to(dev)
     y = ops.selective_scan(x.to(dev), dt.to(dev), bias.to(dev), bc.to(dev), a.to(dev), d.to(dev), gate.to(dev), 3, held, rows)
     want, want_state = torch.zeros(total, channels, dtype=torch.float64), start.double()
@@ -51,6 +53,12 @@ def test_scan_matches_64_bits(channels, state, lens):
 def test_scan_of_a_few_tokens_among_single_ones(channels, state, lens):
     """Steps that are cheaper token by token."""
     test_scan_matches_64_bits(channels, state, lens)
+
+
+@pytest.mark.parametrize("channels,state,lens", [(33, 8, [18, 16, 5]), (2400, 16, [18, 33]), (70, 17, [40]), (2400, 16, [3] + [1] * 40)])
+def test_scan_with_decays_of_zero(channels, state, lens):
+    """An infinite rate: a state that holds the last token alone, also where the tokens do not fill a stage."""
+    test_scan_matches_64_bits(channels, state, lens, infinite=True)
 
 
 @pytest.mark.parametrize("channels,offset,lens,held,bias", [

@@ -346,6 +346,13 @@ __device__ __forceinline__ float decay_exp2(float x) {
     return y;
 }
 
+// A in base 2.  An infinite one (a decay of zero) becomes the largest number: times the step size of zero of the tokens that
+// fill up a stage it must be zero, not a NaN.
+__device__ __forceinline__ float bounded_rate(float a) {
+    const float x = a * 1.4426950408889634f;
+    return x < -3.4e38f ? -3.4e38f : x;
+}
+
 template <int LANES, int PER>
 __global__ void __launch_bounds__(2 * kWalkThreads) selective_scan_walk_kernel(
     __nv_bfloat16* __restrict__ y, float* __restrict__ state, const __nv_bfloat16* __restrict__ x,
@@ -377,8 +384,8 @@ __global__ void __launch_bounds__(2 * kWalkThreads) selective_scan_walk_kernel(
         for (int i = 0; i < PAIRS; ++i) {
             const int n = lane * PER + 2 * i;
             s[i] = pack2(n < n_state ? S[n] : 0.f, n + 1 < n_state ? S[n + 1] : 0.f);
-            a[i] = pack2(n < n_state ? A[(size_t)c * n_state + n] * 1.4426950408889634f : 0.f,
-                         n + 1 < n_state ? A[(size_t)c * n_state + n + 1] * 1.4426950408889634f : 0.f);
+            a[i] = pack2(n < n_state ? bounded_rate(A[(size_t)c * n_state + n]) : 0.f,
+                         n + 1 < n_state ? bounded_rate(A[(size_t)c * n_state + n + 1]) : 0.f);
         }
         __syncthreads();                       // the first stage is in place
         for (int stage = 0; stage < n_stages; ++stage) {
