@@ -353,6 +353,10 @@ __device__ __forceinline__ float bounded_rate(float a) {
     return x < -3.4e38f ? -3.4e38f : x;
 }
 
+// The barrier at which the two halves of a block meet.  They wait for one another at different places of the program, which
+// __syncthreads() does not allow: a numbered barrier of all the block's threads does.
+__device__ __forceinline__ void halves_meet() { asm volatile("barrier.cta.sync 1, %0;" ::"n"(2 * kWalkThreads) : "memory"); }
+
 template <int LANES, int PER>
 __global__ void __launch_bounds__(2 * kWalkThreads) selective_scan_walk_kernel(
     __nv_bfloat16* __restrict__ y, float* __restrict__ state, const __nv_bfloat16* __restrict__ x,
@@ -387,7 +391,7 @@ __global__ void __launch_bounds__(2 * kWalkThreads) selective_scan_walk_kernel(
             a[i] = pack2(n < n_state ? bounded_rate(A[(size_t)c * n_state + n]) : 0.f,
                          n + 1 < n_state ? bounded_rate(A[(size_t)c * n_state + n + 1]) : 0.f);
         }
-        __syncthreads();                       // the first stage is in place
+        halves_meet();                       // the first stage is in place
         for (int stage = 0; stage < n_stages; ++stage) {
             const int buf = stage & 1;
             // (tokens beyond the step's have a step size of zero and leave the state as it is)
@@ -407,7 +411,7 @@ __global__ void __launch_bounds__(2 * kWalkThreads) selective_scan_walk_kernel(
                 unpack2(sum, s0, s1);
                 share_mem[buf][t][threadIdx.x] = s0 + s1;
             }
-            __syncthreads();
+            halves_meet();
         }
         if (!live) return;
 #pragma unroll
@@ -492,18 +496,18 @@ __global__ void __launch_bounds__(2 * kWalkThreads) selective_scan_walk_kernel(
     fetch(0);
     transform(0, 0, skipped[0], gate[0]);
     if (1 < n_stages) fetch(1);
-    __syncthreads();
+    halves_meet();
     for (int stage = 0; stage < n_stages; stage += 2) {
         // the walk is at `stage`: read out the one before, prepare the one after
         if (stage > 0) finish(stage - 1, 1, skipped[1], gate[1]);
         if (stage + 1 < n_stages) transform(stage + 1, 1, skipped[1], gate[1]);
         if (stage + 2 < n_stages) fetch(stage + 2);
-        __syncthreads();
+        halves_meet();
         if (stage + 1 >= n_stages) break;
         finish(stage, 0, skipped[0], gate[0]);
         if (stage + 2 < n_stages) transform(stage + 2, 0, skipped[0], gate[0]);
         if (stage + 3 < n_stages) fetch(stage + 3);
-        __syncthreads();
+        halves_meet();
     }
     if (n_stages & 1) finish(n_stages - 1, 0, skipped[0], gate[0]);
     else finish(n_stages - 1, 1, skipped[1], gate[1]);
