@@ -130,6 +130,13 @@ def test_matrix_memory_matches_64_bits(lens, n_heads, vdim):
         assert (copies[:, :, key] - m[:, None]).abs().max() <= bound * m.abs().amax().clamp(min=1)
 
 
+def test_matrix_memory_of_many_short_sequences():
+    """What a step of long and short sequences needs grows with its rows, not with the longest times their number."""
+    bytes_for = ops.lib().thn_mlstm_chunks_scratch_bytes
+    assert bytes_for(100999, 1000, 16) <= 1.05 * bytes_for(100999, 1, 16)
+    test_matrix_memory_matches_64_bits([33] + [1] * 9 + [70, 32, 1, 64], 2, 64)
+
+
 @pytest.mark.parametrize("lens,held,n_heads,groups,vdim", [
     ([112], 0, 4, 2, 64), ([1, 129, 33], 0, 2, 2, 16), ([160, 2], 3, 8, 1, 96), ([115, 64], 1, 64, 8, 128), ([113] * 3, 0, 128, 4, 64)])
 def test_state_space_matches_64_bits(lens, held, n_heads, groups, vdim):

@@ -37,6 +37,11 @@ constexpr int kKeys = 128;
 // rows of the planes, in bfloat16: eight rows of 16 bytes lie on distinct banks
 constexpr int kKeyRow = kKeys + 8, kScoreRow = kTokens + 8;
 
+// Where the chunks of a sequence stand among the chunks of all, counted from its first row on; chunk_places: how many places
+// there are.  (A sequence of n rows from row0 on takes (n + 31) / 32 places, never more than lie ahead of the next one's.)
+__host__ __device__ inline size_t chunk_place(int row0, int seq) { return (size_t)row0 / kTokens + seq; }
+inline long long chunk_places(int n_rows, int n_seqs) { return n_rows / kTokens + (long long)n_seqs; }
+
 struct WalkArgs {
     float* o;                  // [rows, heads, value_dim]
     float* state;              // [slots, heads, value_dim, kKeys], read and updated
@@ -56,8 +61,7 @@ struct WalkArgs {
     float scale;               // on every read-out
     // the gated matrix memory
     float* normaliser;         // [slots, heads, value_dim / 16, kKeys + 1]: copies of n, then m
-    const float* key_sums;     // [sequences, chunks, heads, kKeys]: sum_j w_j k_j of every chunk
-    int max_chunks;
+    const float* key_sums;     // [chunk_place, heads, kKeys]: sum_j w_j k_j of every chunk
     float floor_;
 };
 
@@ -269,7 +273,7 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
             }
             if (GATED && threadIdx.x < kKeys / 4)
                 copy16(dst + L::kSums + threadIdx.x * 16,
-                       a.key_sums + (((size_t)seq * a.max_chunks + chunk) * a.n_heads + head) * kKeys + threadIdx.x * 4, true);
+                       a.key_sums + ((chunk_place(row0, seq) + chunk) * a.n_heads + head) * kKeys + threadIdx.x * 4, true);
         }
 #pragma unroll
         for (int p = 0; p < 3; ++p) {

@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(kChunkThreads) mlstm_chunk_kernel(
             x = fmaf(w_s[j], k.x, x);
             y = fmaf(w_s[j], k.y, y);
         }
-        *reinterpret_cast<float2*>(key_sums + (((size_t)seq * gridDim.x + blockIdx.x) * n_heads + head) * chunk::kKeys + d) = make_float2(x, y);
+        *reinterpret_cast<float2*>(key_sums + ((chunk::chunk_place(begin, seq) + blockIdx.x) * n_heads + head) * chunk::kKeys + d) = make_float2(x, y);
         return;
     }
     float dot[4][4];
@@ -491,9 +491,8 @@ THN_API int thn_mlstm_recurrence(float* o, float* S, float* nm, const void* proj
 }
 
 // Bytes of the scratch that thn_mlstm_chunks needs.
-THN_API long long thn_mlstm_chunks_scratch_bytes(int n_rows, int max_tokens, int n_seqs, int n_heads) {
-    const long long chunks = (max_tokens + chunk::kTokens - 1) / chunk::kTokens;
-    return (long long)n_heads * n_rows * (3 * chunk::kScoreRow * 2 + 16) + chunks * n_seqs * n_heads * chunk::kKeys * 4;
+THN_API long long thn_mlstm_chunks_scratch_bytes(int n_rows, int n_seqs, int n_heads) {
+    return (long long)n_heads * n_rows * (3 * chunk::kScoreRow * 2 + 16) + chunk::chunk_places(n_rows, n_seqs) * n_heads * chunk::kKeys * 4;
 }
 
 // The recurrence of a step chunk by chunk: bfloat16 rows whose q, k and v parts start on 16-byte boundaries, keys of
@@ -526,7 +525,7 @@ THN_API int thn_mlstm_chunks(float* o, float* S, float* nm, void* scratch, const
     a.scores = scores; a.scalars = scalars;
     a.cu_seqlens = cu_seqlens; a.slots = slots;
     a.n_rows = n_rows; a.n_heads = n_heads; a.heads_per_unit = 1; a.value_dim = value_dim; a.scale = q_scale;
-    a.normaliser = nm; a.key_sums = key_sums; a.max_chunks = chunks; a.floor_ = floor_;
+    a.normaliser = nm; a.key_sums = key_sums; a.floor_ = floor_;
     using T = __nv_bfloat16;
     // Wide blocks share the loads of a chunk's keys and queries, narrow ones give more blocks, whose four warps split
     // the keys; us of the whole call with 64 / 16 columns: 8 x 512 tokens of 16 heads 132 / 155, one prompt of 2,048 tokens

@@ -208,7 +208,7 @@ def lib():
         loaded.thn_set_recurrence_columns.restype = None
         loaded.thn_delta_chunks_scratch_bytes.argtypes = [c_int, c_int, c_int, c_int]
         loaded.thn_delta_chunks_scratch_bytes.restype = c_longlong
-        loaded.thn_mlstm_chunks_scratch_bytes.argtypes = [c_int, c_int, c_int, c_int]
+        loaded.thn_mlstm_chunks_scratch_bytes.argtypes = [c_int, c_int, c_int]
         loaded.thn_mlstm_chunks_scratch_bytes.restype = c_longlong
         loaded.thn_state_space_chunks_scratch_bytes.argtypes = [c_int, c_int, c_int, c_int]
         loaded.thn_state_space_chunks_scratch_bytes.restype = c_longlong
@@ -1590,7 +1590,7 @@ def mlstm(proj: torch.Tensor, gate_pre: torch.Tensor, bias_i: torch.Tensor, bias
                           f"{key_dim} x {value_dim}")
     o = torch.empty((n, n_heads, value_dim), dtype=torch.float32, device=proj.device)
     if _mlstm_in_chunks(proj, state, rows, n_heads, key_dim, value_dim):
-        scratch = torch.empty(lib().thn_mlstm_chunks_scratch_bytes(n, rows.max_q_len, rows.n_seqs, n_heads), dtype=torch.uint8,
+        scratch = torch.empty(lib().thn_mlstm_chunks_scratch_bytes(n, rows.n_seqs, n_heads), dtype=torch.uint8,
                               device=proj.device)
         _call("thn_mlstm_chunks", _ptr(o), _ptr(state), _ptr(normaliser), _ptr(scratch), _ptr(proj), proj.shape[1], _ptr(gate_pre),
               _ptr(bias_i), _ptr(bias_f), float(cap), _ptr(rows.cu_seqlens), _ptr(rows.slots), n, rows.max_q_len, rows.n_seqs, n_heads,
