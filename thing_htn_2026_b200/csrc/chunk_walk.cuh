@@ -196,6 +196,30 @@ __device__ __forceinline__ void clear(float (&d)[N][4]) {
 __device__ __forceinline__ float2 pair_of(const float* p) { return *reinterpret_cast<const float2*>(p); }
 __device__ __forceinline__ float2 pair_of(const __nv_bfloat16* p) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p)); }
 
+// Of a chunk's values as A operands (columns by tokens), those that are not finite become zero; from[0], from[1]: the first
+// token of columns g and g + 8 that had one.
+template <int PARTS>
+__device__ __forceinline__ void leave_out(Parts (&values)[kTokens / 16], int (&from)[2], int t) {
+    from[0] = from[1] = kTokens;
+#pragma unroll
+    for (int j = 0; j < kTokens / 16; ++j)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t which = not_finite(values[j].part[0][i]);
+            const int token = 16 * j + 8 * (i >> 1) + 2 * t;
+            if (which & 0x80000000u) from[i & 1] = min(from[i & 1], token + 1);
+            if (which & 0x00008000u) from[i & 1] = min(from[i & 1], token);
+            const uint32_t kept = (which & 0x80000000u ? 0u : 0xffff0000u) | (which & 0x00008000u ? 0u : 0x0000ffffu);
+#pragma unroll
+            for (int p = 0; p < (PARTS == 1 ? 1 : 3); ++p) values[j].part[p][i] &= kept;
+        }
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        from[c] = min(from[c], __shfl_xor_sync(0xffffffffu, from[c], 1));
+        from[c] = min(from[c], __shfl_xor_sync(0xffffffffu, from[c], 2));
+    }
+}
+
 template <typename T, int CG, int KS, bool DELTA, int STAGES>
 struct Layout {
     static constexpr int kParts = sizeof(T) == 2 ? 1 : 3;
@@ -211,7 +235,7 @@ struct Layout {
     static constexpr int kSums = kScalars + kTokens * 16;                                    // gated: the chunk's sum of keys
     static constexpr int kStage = kSums + (kParts == 1 ? kKeys * 4 : 0);
     static constexpr int kShares = KS > 1 ? KS * CG * (DELTA ? 2 : 1) * 4 * 32 * 16 : 0;    // [ks][cg][which][8 tokens][lane] float4
-    static constexpr int kBytes = STAGES * kStage + kShares + (kTokens * 3 + kKeys) * 4;
+    static constexpr int kBytes = STAGES * kStage + kShares + (kTokens * 3 + kKeys + 4) * 4;
 };
 
 template <typename T, int CG, int KS, bool DELTA, bool GATED, int STAGES>
@@ -222,6 +246,7 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
     constexpr int GROUPS = kTokens / 8;              // groups of 8 tokens
     constexpr int OWN = GROUPS / KS;                 // groups that a warp finishes
     static_assert(KT % 4 == 0 && OWN >= 1, "whole steps");
+    static_assert(!DELTA || KS > 1, "the barrier ahead of the shares frees the chunk's queries and W");
     pdl_launch_dependents();
     pdl_wait();
     extern __shared__ __align__(16) unsigned char mem[];
@@ -230,7 +255,9 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
     float* beta_s = alpha_s + kTokens;
     float* under_s = beta_s + kTokens;
     float* n_s = under_s + kTokens;
+    int* lost_s = reinterpret_cast<int*>(n_s + kKeys);      // delta: a value was not finite, in this chunk or ahead of it
     const int slab = blockIdx.x, head = blockIdx.y, seq = blockIdx.z;
+    if (DELTA && threadIdx.x == 0) *lost_s = 0;
     const int row0 = a.cu_seqlens[seq], n_tokens = a.cu_seqlens[seq + 1] - row0;
     if (n_tokens <= 0) return;
     const int slot = a.slots[seq], unit = head / a.heads_per_unit;
@@ -417,7 +444,7 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
         __nv_bfloat16* plain_s = reinterpret_cast<__nv_bfloat16*>(stage + L::kQ) + cg * 3 * kSplitPlane;
         __nv_bfloat16* scaled_s = reinterpret_cast<__nv_bfloat16*>(stage + L::kW) + cg * 3 * kSplitPlane;
         if constexpr (DELTA) {
-            if (KS == 1) __syncthreads();
+            uint32_t own_lost = 0;
 #pragma unroll
             for (int n = 0; n < OWN; ++n) {
                 const int i = 8 * (group0 + n) + 2 * t;
@@ -428,6 +455,7 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
                 for (int half = 0; half < 2; ++half) {
                     const int at = (g + 8 * half) * kSplitRow + i;
                     const Split as_is = split(v[2 * half], v[2 * half + 1]), by_w = split(v[2 * half] * w0, v[2 * half + 1] * w1);
+                    own_lost |= not_finite(as_is.part[0]);
 #pragma unroll
                     for (int p = 0; p < 3; ++p) {
                         *reinterpret_cast<uint32_t*>(plain_s + p * kSplitPlane + at) = as_is.part[p];
@@ -435,8 +463,8 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
                     }
                 }
             }
-            if (KS > 1) __syncthreads();
-            else __syncwarp();
+            if (own_lost) *lost_s = 1;
+            __syncthreads();
         }
         // the chunk's values as A operands: columns by tokens, as they are and times w
         Parts plain[kTokens / 16], scaled[kTokens / 16];
@@ -470,36 +498,6 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
             scaled[j] = parts_of(make_float2(v[0].x * w0, v[0].y * w1), make_float2(v[1].x * w0, v[1].y * w1),
                                  make_float2(v[2].x * w8, v[2].y * w9), make_float2(v[3].x * w8, v[3].y * w9));
         }
-        // Where G is zero the products still multiply, and zero times an infinity or a NaN is NaN: such a value would reach
-        // the tokens ahead of its own.  It is left out of the products with G, and its column's read-outs are NaN from its
-        // token on.  (The state takes it as it is.)
-        int lost[2] = {kTokens, kTokens};            // the first such token of columns g and g + 8
-        {
-            uint32_t any = 0;
-#pragma unroll
-            for (int j = 0; j < kTokens / 16; ++j)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) any |= not_finite(plain[j].part[0][i]);
-            if (__any_sync(0xffffffffu, any != 0)) {
-#pragma unroll
-                for (int j = 0; j < kTokens / 16; ++j)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const uint32_t which = not_finite(plain[j].part[0][i]);
-                        const int token = 16 * j + 8 * (i >> 1) + 2 * t;
-                        if (which & 0x80000000u) lost[i & 1] = min(lost[i & 1], token + 1);
-                        if (which & 0x00008000u) lost[i & 1] = min(lost[i & 1], token);
-                        const uint32_t kept = (which & 0x80000000u ? 0u : 0xffff0000u) | (which & 0x00008000u ? 0u : 0x0000ffffu);
-#pragma unroll
-                        for (int p = 0; p < (PARTS == 1 ? 1 : 3); ++p) plain[j].part[p][i] &= kept;
-                    }
-#pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    lost[c] = min(lost[c], __shfl_xor_sync(0xffffffffu, lost[c], 1));
-                    lost[c] = min(lost[c], __shfl_xor_sync(0xffffffffu, lost[c], 2));
-                }
-            }
-        }
         // the state behind the chunk
         const float keep = GATED ? alpha_s[n_here - 1] : scalars[n_here - 1].x, take = GATED ? beta_s[n_here - 1] : 1.f;
         constexpr int KP = 2;                        // pairs of groups of keys at a time
@@ -531,22 +529,52 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
         constexpr int kPairs = OWN >= 2 ? OWN / 2 : 1;
         float inner[kPairs][2][4];
         const int pair0 = group0 / 2;
+        auto take_inner = [&] {
 #pragma unroll
-        for (int pair = 0; pair < kPairs; ++pair) {
-            clear(inner[pair]);
+            for (int pair = 0; pair < kPairs; ++pair) {
+                clear(inner[pair]);
 #pragma unroll
-            for (int j = 0; j < kTokens / 16; ++j) {
-                if (j > pair0 + pair) continue;
-                const Columns<3> row[1] = {columns_of<3>(g_s + b_tile(lane, kScoreRow) + 16 * (pair0 + pair) * kScoreRow + 16 * j, L::kScorePlane)};
-                float large[2][4], small[2][4];
-                clear(large);
-                clear(small);
-                multiply<PARTS>(large, small, plain[j], row);
+                for (int j = 0; j < kTokens / 16; ++j) {
+                    if (j > pair0 + pair) continue;
+                    const Columns<3> row[1] = {columns_of<3>(g_s + b_tile(lane, kScoreRow) + 16 * (pair0 + pair) * kScoreRow + 16 * j, L::kScorePlane)};
+                    float large[2][4], small[2][4];
+                    clear(large);
+                    clear(small);
+                    multiply<PARTS>(large, small, plain[j], row);
+#pragma unroll
+                    for (int o = 0; o < 2; ++o)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) inner[pair][o][i] += joined(large[o][i], small[o][i]);
+                }
+            }
+        };
+        take_inner();
+        // Where G is zero the products multiply all the same, and zero times an infinity or a NaN is NaN: such a value would
+        // reach the tokens ahead of its own.  Where a warp has one, the products are taken again without it, and the column's
+        // sums are NaN from its token on.  (The state has taken it as it is.)  The delta rule's values are looked at by the warps that
+        // finish them.
+        bool lost;
+        if constexpr (DELTA) {
+            lost = *reinterpret_cast<volatile int*>(lost_s) != 0;
+        } else {
+            uint32_t own = 0;
+#pragma unroll
+            for (int j = 0; j < kTokens / 16; ++j)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) own |= not_finite(plain[j].part[0][i]);
+            lost = __any_sync(0xffffffffu, own != 0);
+        }
+        if (lost) {
+            int from[2];
+            leave_out<PARTS>(plain, from, t);
+            take_inner();
+#pragma unroll
+            for (int pair = 0; pair < kPairs; ++pair)
 #pragma unroll
                 for (int o = 0; o < 2; ++o)
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) inner[pair][o][i] += joined(large[o][i], small[o][i]);
-            }
+                    for (int i = 0; i < 4; ++i)
+                        if (16 * (pair0 + pair) + 8 * o + 2 * t + (i & 1) >= from[i >> 1]) inner[pair][o][i] = not_a_number();
         }
 #pragma unroll
         for (int n = 0; n < OWN; ++n) {
@@ -555,8 +583,8 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
                 const int i = 8 * (group0 + n) + 2 * t + half;
                 if (i >= n_here) continue;
                 const int o = OWN == 1 ? group0 & 1 : n & 1;
-                const float in0 = i >= lost[0] ? not_a_number() : o ? inner[n / 2][1][half] : inner[n / 2][0][half];
-                const float in1 = i >= lost[1] ? not_a_number() : o ? inner[n / 2][1][2 + half] : inner[n / 2][0][2 + half];
+                const float in0 = o ? inner[n / 2][1][half] : inner[n / 2][0][half];
+                const float in1 = o ? inner[n / 2][1][2 + half] : inner[n / 2][0][2 + half];
                 const float alpha = GATED ? alpha_s[i] : scalars[i].x, beta = GATED ? beta_s[i] : 1.f;
                 float y0 = (alpha * read[n][half] + beta * in0) * a.scale;
                 float y1 = (alpha * read[n][2 + half] + beta * in1) * a.scale;
