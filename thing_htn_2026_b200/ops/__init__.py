@@ -9,7 +9,7 @@ from __future__ import annotations
 import ctypes
 import os
 from dataclasses import dataclass
-from typing import Dict, Optional, Tuple
+from typing import Dict, NamedTuple, Optional, Tuple
 
 import torch
 
@@ -1411,7 +1411,39 @@ FUSE_DELTA_DECODE = os.environ.get("THN_FUSE_DELTA_DECODE", "1").strip().lower()
 
 
 CHUNK_KEYS = 128           # the key size that the chunk kernels are built for
-CHUNK_MIN_TOKENS = 16      # fewer tokens a sequence are as fast one by one (60 against 66 us at 16)
+CHUNK_TOKENS = 32
+CHUNK_MIN_TOKENS = 16      # fewer tokens a sequence are as fast one by one (delta rule 60 against 66 us at 16)
+
+
+class _ChunkCost(NamedTuple):
+    """What a step costs token by token and in chunks, in us on B200: the chain of a sequence's tokens or chunks, and what
+    all of them take together, per head of the size named.  A chunk costs as much with one token as with 32, so that
+    single tokens beside a prompt, or many short prompts, are cheaper one by one."""
+    token_chain: float       # a token of the longest sequence
+    row: float               # a row, per head
+    sequence: float          # a sequence's state, per head
+    chunk_chain: float       # a chunk of the longest sequence
+    chunk: float             # a chunk, per head
+    lead: float              # by how much the kernels around the walk are cheaper than those around the tokens
+    size: int                # the value size that the figures are for
+
+    def chunks_pay(self, rows: StepRows, n_heads: int, value_dim: int) -> bool:
+        heads, longest = n_heads * value_dim / self.size, -(-rows.max_q_len // CHUNK_TOKENS)
+        chunks = min(rows.n_seqs * longest, rows.n_rows // CHUNK_TOKENS + rows.n_seqs)       # at most
+        by_token = max(self.token_chain * rows.max_q_len, (self.row * rows.n_rows + self.sequence * rows.n_seqs) * heads)
+        return max(self.chunk_chain * longest, self.chunk * chunks * heads) <= by_token + self.lead
+
+
+# Measured on B200, token by token / in chunks, us of the whole call; "a + b": one prompt of a tokens beside b single ones.
+#   delta rule, 16 heads of 128: 16 + 0 65 / 52, 16 + 60 91 / 187, 128 + 8 116 / 79, 128 + 60 142 / 192, 512 + 60 296 / 224,
+#     2,048 + 0 658 / 241, 2,048 + 60 1,054 / 542, 64 prompts of 33 tokens 294 / 319, 32 of 128 511 / 341
+_DELTA_COST = _ChunkCost(0.4, 0.007, 0.02, 3.0, 0.14, 12.0, 128)
+#   matrix memory, 16 heads of 128: 16 + 0 17 / 15, 16 + 60 52 / 69, 33 + 60 62 / 71, 128 + 60 116 / 73, 2,048 + 60 1,223 / 390,
+#     64 prompts of 16 tokens 173 / 77
+_MLSTM_COST = _ChunkCost(0.5, 0.009, 0.03, 1.8, 0.055, 0.0, 128)
+#   state-space duality, 64 heads of 64: 96 + 0 38 / 43, 128 + 0 44 / 42, 128 + 60 108 / 171, 512 + 8 142 / 122, 512 + 60 151 / 198,
+#     2,048 + 60 517 / 460, 32 prompts of 128 tokens 568 / 349
+_SPACE_COST = _ChunkCost(0.205, 0.0021, 0.016, 3.1, 0.035, -10.0, 64)
 
 
 def _delta_in_chunks(proj: torch.Tensor, conv_w: torch.Tensor, state: torch.Tensor, ring: torch.Tensor, rows: StepRows,
@@ -1420,7 +1452,8 @@ def _delta_in_chunks(proj: torch.Tensor, conv_w: torch.Tensor, state: torch.Tens
     return proj.dtype == torch.bfloat16 and s.key_dim == CHUNK_KEYS and s.value_dim % 16 == 0 and s.taps == 4 \
         and DELTA_LANES == 0 and rows.max_q_len >= CHUNK_MIN_TOKENS and s.proj_width % 4 == 0 and rows.n_rows <= 8 * 65535 \
         and max(s.n_heads, rows.n_seqs) <= 65535 \
-        and (state.data_ptr() | conv_w.data_ptr()) % 16 == 0 and (proj.data_ptr() | ring.data_ptr()) % 8 == 0
+        and (state.data_ptr() | conv_w.data_ptr()) % 16 == 0 and (proj.data_ptr() | ring.data_ptr()) % 8 == 0 \
+        and _DELTA_COST.chunks_pay(rows, s.n_heads, s.value_dim)
 
 
 def delta_rule(proj: torch.Tensor, conv_w: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor,
@@ -1562,7 +1595,8 @@ def _mlstm_in_chunks(proj: torch.Tensor, state: torch.Tensor, rows: StepRows, n_
     """Whether a step's recurrence is walked in chunks of tokens on the tensor cores."""
     return proj.dtype == torch.bfloat16 and key_dim == CHUNK_KEYS and value_dim % 16 == 0 and not _mlstm_chosen \
         and rows.max_q_len >= CHUNK_MIN_TOKENS and proj.shape[1] % 8 == 0 and max(n_heads, rows.n_seqs) <= 65535 \
-        and proj.shape[1] >= n_heads * (2 * key_dim + value_dim) and (state.data_ptr() | proj.data_ptr()) % 16 == 0
+        and proj.shape[1] >= n_heads * (2 * key_dim + value_dim) and (state.data_ptr() | proj.data_ptr()) % 16 == 0 \
+        and _MLSTM_COST.chunks_pay(rows, n_heads, value_dim)
 
 
 def mlstm(proj: torch.Tensor, gate_pre: torch.Tensor, bias_i: torch.Tensor, bias_f: torch.Tensor, cap: float,
@@ -1962,7 +1996,7 @@ class StateSpace:
         return self.conv_w.shape[1]
 
 
-SPACE_CHUNK_MIN_TOKENS = 112     # tokens a sequence from which the chunks are as fast (96: 43 against 38 us; 128: 44 both)
+SPACE_CHUNK_MIN_TOKENS = 112     # tokens of the longest sequence from which the chunks are as fast
 
 
 def _space_in_chunks(proj: torch.Tensor, offset: int, state: torch.Tensor, ring: torch.Tensor, rows: StepRows, s: StateSpace) -> bool:
@@ -1970,7 +2004,8 @@ def _space_in_chunks(proj: torch.Tensor, offset: int, state: torch.Tensor, ring:
     return proj.dtype == torch.bfloat16 and s.n_state == CHUNK_KEYS and s.vdim % 16 == 0 and s.taps == 4 \
         and rows.max_q_len >= SPACE_CHUNK_MIN_TOKENS and proj.shape[1] % 4 == 0 and offset % 4 == 0 and rows.n_rows <= 8 * 65535 \
         and max(s.n_heads, rows.n_seqs) <= 65535 and 0 <= offset <= proj.shape[1] - s.channels \
-        and (state.data_ptr() | s.conv_w.data_ptr()) % 16 == 0 and (proj.data_ptr() | ring.data_ptr()) % 8 == 0
+        and (state.data_ptr() | s.conv_w.data_ptr()) % 16 == 0 and (proj.data_ptr() | ring.data_ptr()) % 8 == 0 \
+        and _SPACE_COST.chunks_pay(rows, s.n_heads, s.vdim)
 
 
 def state_space(proj: torch.Tensor, offset: int, dt_pre: torch.Tensor, shape: StateSpace, state: torch.Tensor,
