@@ -97,3 +97,26 @@ def test_gated_head_norm_of_many_pairs(rows, heads, size, kind, own_gain):
     want = x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-6) * w.double().view(-1, size) * (torch.sigmoid(z) if kind == "logistic" else torch.nn.functional.silu(z))
     # float32 throughout and one rounding to bfloat16
     assert ((got.cpu().double().view(rows, heads, size) - want).abs() <= 2 ** -8 * want.abs() + 1e-7).all()
+
+
+@pytest.mark.parametrize("rows,heads", [(12287, 1), (12288, 1), (768, 16), (1025, 12)])
+def test_gated_head_norm_at_the_line_of_the_silu_gate(rows, heads):
+    test_gated_head_norm_of_many_pairs(rows, heads, 128, "silu", False)
+
+
+@pytest.mark.parametrize("gated", [True, False])
+def test_linear_attention_of_one_step_and_of_two(gated):
+    """Many rows are prepared four entries a thread, few an entry a thread, with the same bits."""
+    heads, size, dev = 2, 64, torch.device("cuda", 0)
+    g = torch.Generator(device=dev).manual_seed(5)
+    draw = lambda *s: torch.randn(*s, generator=g, device=dev)
+    proj, gate, bias = draw(130, 3 * heads * size).to(BF16), draw(130, heads * size), draw(heads * size)
+    results = []
+    for cuts in ([0, 130], [0, 65, 130]):
+        state, out = torch.zeros(1, heads, size, size, device=dev), []
+        for a, b in zip(cuts, cuts[1:]):
+            rows, _, _ = step([b - a])
+            how = dict(gate=gate[a:b].contiguous(), gate_bias=bias, tau=16.0) if gated else dict(decay=torch.tensor([0.9, 0.99], device=dev), silu_inputs=True)
+            out.append(ops.linear_attention(proj[a:b].contiguous(), (0, heads * size, 2 * heads * size), state, rows, heads, size, size, **how))
+        results.append((torch.cat(out), state))
+    assert all(torch.equal(x, y) for x, y in zip(*results))
