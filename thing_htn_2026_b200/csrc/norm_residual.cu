@@ -359,8 +359,11 @@ __global__ void gated_head_norm_kernel(T* __restrict__ out, const float* __restr
 // The same for bfloat16 and heads of 64 or 128 entries when there are many: LANES = size / 4 lanes take four neighbouring
 // (row, head) pairs, 16 bytes of each, all loads ahead of the first sum.  Bounded by what it moves.  B200: 1,531 rows of 32
 // heads of 128 15 us, 22 with a pair a warp; with the logistic gate 2,251 rows of 16 heads 12, 20 with 4-byte accesses.
+// Fewer pairs leave it too few warps: in us, a pair a warp / this, back to back, 4,096 pairs 4.4 / 4.1 (logistic gate) and 3.5 / 3.3
+// (64 entries); with the silu gate and 128 entries, for which the other kernel loads four at a time too, 8,192 pairs 4.0 / 5.0, 12,288
+// 5.4 / 5.4, 16,384 6.8 / 5.5.
 constexpr int kManyPairs = 4;
-constexpr long long kManyUnits = 4096;
+constexpr long long many_units(int size, int gate_kind) { return size == 128 && gate_kind == 0 ? 12288 : 4096; }
 template <int LANES>
 __global__ void __launch_bounds__(128) gated_head_norm_many_kernel(__nv_bfloat16* __restrict__ out, const float* __restrict__ o,
                                                                    const __nv_bfloat16* __restrict__ gate, long long gate_stride,
@@ -612,7 +615,7 @@ THN_API int thn_gated_head_norm(void* out, const float* o, const void* gate, lon
     const int w_stride = w_per_head ? size : 0;
     if (out_stride <= 0) out_stride = (long long)n_heads * size;
     THN_CHECK_ARG(out_stride >= (long long)n_heads * size, "gated_head_norm: output rows %lld apart are too short", out_stride);
-    if (dtype == THN_BF16 && (size == 64 || size == 128) && units >= kManyUnits && units < (1ll << 31) && gate_stride % 4 == 0 &&
+    if (dtype == THN_BF16 && (size == 64 || size == 128) && units >= many_units(size, gate_kind) && units < (1ll << 31) && gate_stride % 4 == 0 &&
         out_stride % 4 == 0 && ((((uintptr_t)o | (uintptr_t)w) & 15) | (((uintptr_t)gate | (uintptr_t)out) & 7)) == 0) {
         const unsigned per_block = 128 / (size / 4) * kManyPairs;
         auto kernel = size == 128 ? gated_head_norm_many_kernel<32> : gated_head_norm_many_kernel<16>;
