@@ -279,6 +279,23 @@ def test_the_gate_ahead_of_a_grouped_norm(dtype, width, parts):
     close(got, (p / torch.sqrt((p * p).mean(-1, keepdim=True) + eps)).reshape(5, width) * gain, dtype, "aligned rows")
 
 
+@pytest.mark.parametrize("rows, parts, size", [(1184, 1, 128), (1183, 1, 128), (148, 8, 256), (192, 8, 512), (1021, 3, 1024), (769, 4, 1024), (767, 4, 1024), (500, 8, 384)])
+def test_the_gate_ahead_of_a_grouped_norm_of_many_parts(rows, parts, size):
+    """A warp per part, and on the other side of the line a block per part: sizes of whole 128s, parts that do not fill
+    the last block."""
+    from thing_htn_2026_b200 import ops
+    eps, width = 1e-5, parts * size
+    g = torch.Generator().manual_seed(rows)
+    y = torch.randn(rows, width, generator=g) * torch.logspace(-2, 2, parts).repeat_interleave(size)
+    proj, gain = torch.randn(rows, width + 8, generator=g).to(torch.bfloat16), torch.randn(width, generator=g)
+    got = ops.gated_group_norm(y.to(DEV), proj.to(DEV), 8, gain.to(DEV), eps, parts, torch.bfloat16).cpu().double()
+    z = proj.double()[:, 8:]
+    p = (y.double() * z * torch.sigmoid(z)).reshape(rows, parts, size)
+    want = (p / torch.sqrt((p * p).mean(-1, keepdim=True) + eps)).reshape(rows, width) * gain
+    # float32 throughout (sums of at most 32 a lane and five over the lanes) and one rounding to bfloat16
+    assert ((got - want).abs() <= (2 ** -8 + 2 ** -18) * want.abs() + 1e-30).all()
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("shape", [(3, 7), (5, 64), (2, 4096)])
 def test_squared_relu(dtype, shape):

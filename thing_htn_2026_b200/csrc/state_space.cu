@@ -649,9 +649,11 @@ THN_API int thn_gated_group_norm(void* out, const float* y, const void* gate, lo
     const size_t element = dtype == THN_BF16 ? 2 : 4;
     const int vec = size % 4 == 0 && gate_stride % 4 == 0 && (((uintptr_t)y | (uintptr_t)gain) & 15) == 0 &&
                     (((uintptr_t)gate | (uintptr_t)out) & (4 * element - 1)) == 0;
-    // (few parts are faster with a block each)
+    // Few parts are faster with a block each, the more so the longer they are.  In us, a block / a warp each, back to back: parts of
+    // 1,024: 1,184 of them 4.3 / 4.6, 2,048 6.3 / 6.7, 3,072 8.9 / 6.7; of 512: 1,184 2.9 / 3.0, 2,048 4.1 / 3.9; of 256: 1,184 2.9 / 2.4.
     const long long units = (long long)rows * parts;
-    if (dtype == THN_BF16 && vec && size % 128 == 0 && size <= 1024 && units >= 1184) {
+    const long long enough = 3ll * size < 1184 ? 1184 : 3ll * size;
+    if (dtype == THN_BF16 && vec && size % 128 == 0 && size <= 1024 && units >= enough) {
         thn_launch(gated_group_norm_warp_kernel, (unsigned)((units + 7) / 8), 256, 0, stream, (__nv_bfloat16*)out, y,
                    (const __nv_bfloat16*)gate, gate_stride, gain, eps, rows, width, size, parts);
         return thn_launch_status("gated_group_norm");
