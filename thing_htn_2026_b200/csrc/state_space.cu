@@ -533,7 +533,7 @@ THN_API long long thn_state_space_chunks_scratch_bytes(int n_rows, int n_heads, 
 
 // thn_state_space chunk by chunk: bfloat16 rows in whole 8-byte pieces, four taps, a state of 128, vdim a multiple of 16;
 // max_tokens: the most rows of a sequence.  On B200, us against token by token: 8 x 512 tokens of 128 heads of 64 over a
-// state of 128 613 / 1,074, one prompt of 2,048 tokens of 64 heads 220 / 365, 128 tokens 44 / 44.  The error against 64 bits:
+// state of 128 620 / 1,074, one prompt of 2,048 tokens of 64 heads 226 / 368, 128 tokens 42 / 44.  The error against 64 bits:
 // y 1.2e-7 (1.2e-7 to 1.3e-7), the state 1.1e-7 (1.2e-7).
 THN_API int thn_state_space_chunks(float* y, float* state, void* scratch, const void* proj, int proj_width, int offset,
                                    const float* conv_w, const float* conv_b, const void* ring, const float* dt_pre,
