@@ -890,9 +890,10 @@ THN_API long long thn_delta_chunks_scratch_bytes(int n_rows, int n_heads, int n_
 // prepare and recurrence of a step chunk by chunk, the state carried in float32: bfloat16 rows, four taps, keys of
 // 128, values of whole groups of 16 columns; max_tokens: the most rows of a sequence.  scratch:
 // thn_delta_chunks_scratch_bytes(...), 16-byte aligned, as the state and the taps must be; the rows and the
-// ring are read in pieces of 8 bytes.  One prompt of 2,048 tokens, 16 heads of 128 x 128, on B200: 241 us
-// against 655 token by token; 32 heads 362 / 839; 8 x 512 tokens of 16 heads 341 / 571.  The read-out's error
-// against 64 bits is 1.4e-7 (1.3e-7 token by token), the state's 1.3e-7 (1.3e-7).
+// ring are read in pieces of 8 bytes.  One prompt of 2,048 tokens, 16 heads of 128 x 128, on B200: 243 us
+// against 658 token by token; 32 heads 368 / 839; 8 x 512 tokens of 16 heads 333 / 571; steps of long and short sequences beside
+// the rule in ops (_DELTA_COST).  The read-out's error
+// against 64 bits is 1.37e-7 to 1.41e-7 (1.33e-7 to 1.36e-7 token by token), the state's 1.2e-7 to 1.4e-7 (1.1e-7 to 1.3e-7).
 THN_API int thn_delta_chunks(float* o, float* state, void* scratch, const void* proj, const float* conv_w, const float* a_log,
                              const float* dt_bias, const void* ring, const int* row_slot, const int* row_pos, const int* seq_lens,
                              const int* cu_seqlens, const int* slots, int n_rows, int max_tokens, int n_seqs, int n_heads, int n_kv,
