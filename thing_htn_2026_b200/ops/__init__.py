@@ -7,6 +7,7 @@ else, and every product of the 32-bit path, is this library's own kernel.
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 from dataclasses import dataclass
 from typing import Dict, NamedTuple, Optional, Tuple
@@ -122,6 +123,10 @@ _SIGNATURES = {
     "thn_moe_route": [c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_float,
                       c_int, c_int, c_float, c_void_p],
     "thn_routed_gelu": [c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p],
+    "thn_moe_grouped_supported": [c_int, c_int, c_int, c_int],
+    "thn_moe_grouped_bf16": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p,
+                             c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float,
+                             c_float, c_int, c_void_p, c_void_p],
     "thn_clamped_glu": [c_void_p, c_void_p, c_longlong, c_int, c_int, c_float, c_float, c_int, c_void_p],
     "thn_qk_prepare": [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_float, c_float, c_void_p, c_void_p,
                        c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
@@ -1724,6 +1729,62 @@ def routed_gelu(u: torch.Tensor, routing: Routing, ff: int, shared_ff: int,
     return out
 
 
+# Where the chosen experts are multiplied alone: products of this many rows (below, both forms wait for the weights) and
+# operations that leaving the other experts out saves.  (B200, grouped / dense in us, cold weights.  8 experts of 1,024 over 2,048, top 2, a
+# shared one, gated: 512 rows 78 / 65, 1,024 88 / 99, 2,048 121 / 163, 4,096 176 / 318; gelu: 1,024 74 / 75, 2,048 100 / 122.  Of 2,048 over 4,096: 256
+# rows 131 / 134, 2,048 313 / 585; gelu: 512 129 / 124, 1,024 154 / 204.  64 of 512 over 2,048, top 6: 256 rows 127 / 140, 2,048 180 / 587.  16 of 1,024,
+# top 4, none shared: 256 rows 74 / 81, 2,048 148 / 280.  4 of 512 over 1,024, top 2: 4,096 rows 64 / 60.)
+GROUPED_MIN_ROWS = 256
+GROUPED_MIN_SAVED = {True: 60e9, False: 100e9}       # gated, gelu
+
+
+def experts_in_groups(x: torch.Tensor, n_experts: int, top: int, ff: int, shared_ff: int, gated: bool) -> bool:
+    """Whether ``grouped_experts`` takes these sizes and is the faster form."""
+    rows, hidden = x.shape
+    saved = (6.0 if gated else 4.0) * rows * (n_experts - top) * ff * hidden
+    return (x.dtype == torch.bfloat16 and rows >= GROUPED_MIN_ROWS and saved >= GROUPED_MIN_SAVED[gated] and rows * top <= 1 << 30
+            and x.data_ptr() % 16 == 0 and bool(lib().thn_moe_grouped_supported(hidden, n_experts, ff, shared_ff)))
+
+
+def grouped_experts(x: torch.Tensor, routing: Routing, w_up: torch.Tensor, w_down: torch.Tensor, ff: int, shared_ff: int,
+                    glu: Optional[Tuple[float, float, float, float, str]] = None, shared_logit: Optional[torch.Tensor] = None,
+                    logit_column: int = 0, err: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """The weighted sum of the chosen experts' outputs and the shared expert's, ``[rows, hidden]`` in bfloat16, as products of
+    the chosen experts alone (tcgen05; csrc/moe_grouped.cu).  ``glu`` (limit, shared limit, alpha, up shift, weight at): experts of the form
+    of ``routed_clamped_glu``, ``w_up`` [2 * (experts * ff + shared_ff), hidden]; without it those of ``routed_gelu``,
+    ``w_up`` [experts * ff + shared_ff, hidden].  ``w_down`` [hidden, experts * ff + shared_ff].  ``err``: the step's device error
+    word for the kernels' bounded waits."""
+    _need(x, "grouped_experts x", torch.bfloat16)
+    _need(w_up, "grouped_experts w_up", torch.bfloat16)
+    _need(w_down, "grouped_experts w_down", torch.bfloat16)
+    _need(routing.dense, "grouped_experts weights", torch.float32)
+    _need(routing.chosen, "grouped_experts choices", torch.int32)
+    rows, hidden = x.shape
+    n_experts, top = routing.dense.shape[1], routing.chosen.shape[1]
+    width = n_experts * ff + shared_ff
+    if tuple(w_up.shape) != ((1 if glu is None else 2) * width, hidden) or tuple(w_down.shape) != (hidden, width) \
+            or routing.dense.shape[0] != rows or routing.chosen.shape[0] != rows:
+        raise KernelError(f"grouped_experts: x {tuple(x.shape)}, w_up {tuple(w_up.shape)}, w_down {tuple(w_down.shape)}, "
+                          f"{n_experts} experts of {ff} and {shared_ff}, {routing.dense.shape[0]} rows of weights")
+    limit, shared_limit, alpha, up_shift, weight_at = glu or (1.0, 1.0, 1.0, 0.0, "output")
+    if weight_at not in ("input", "output"):
+        raise KernelError(f"grouped_experts: weight_at {weight_at!r} is neither 'input' nor 'output'")
+    logit_ptr, stride = None, 0
+    if shared_logit is not None:
+        _need(shared_logit, "grouped_experts gate logits", torch.float32)
+        logit_ptr, stride = shared_logit.data_ptr() + 4 * logit_column, shared_logit.shape[1]
+    n, new = rows * top, functools.partial(torch.empty, device=x.device)
+    sorted_x, act, shared_act = (new(shape, dtype=x.dtype) for shape in ((n, hidden), (n, ff), (rows, shared_ff)))
+    partial, weights = new((n, hidden), dtype=torch.float32), new(n, dtype=torch.float32)
+    ints = new(2 * n + n_experts + 1, dtype=torch.int32)
+    out = torch.empty_like(x)
+    _call("thn_moe_grouped_bf16", _ptr(out), _ptr(x), _ptr(routing.chosen), _ptr(routing.dense), _ptr(w_up), _ptr(w_down), logit_ptr, stride,
+          _ptr(sorted_x), _ptr(act), _ptr(shared_act), _ptr(partial), _ptr(ints), _ptr(weights), rows, hidden, n_experts, top, ff, shared_ff,
+          int(glu is not None), float(limit), float(shared_limit or 1.0), float(alpha), float(up_shift), int(weight_at == "output"),
+          _ptr(err), _stream())
+    return out
+
+
 # ------------------------------------------------------------------ hyper-connections
 
 
@@ -2146,5 +2207,5 @@ def gather_i32(src: torch.Tensor, index: torch.Tensor, out: Optional[torch.Tenso
 __all__ = [
     "KernelError", "KernelLibraryError", "KVView", "RotaryTables", "RowTiles", "StepRows", "row_tiles_of", "prompt_attention_tile", "linear_stream", "linear_swiglu", "linear_tcgen05", "add_rmsnorm", "advance",
     "ROW_TILE", "attention", "attention_decode_bf16", "attention_generic", "attention_prefill_bf16", "attention_prefill_tcgen05", "decode_splits", "choose_tokens", "gather_i32", "gather_rows", "lib", "linear", "new_error_word",
-    "qk_norm_rope_cache", "qk_prepare", "Gain", "STREAM_AS_IS", "residual_norm", "gather_rows_scaled", "logistic_gate", "latent_norm", "latent_assemble", "mlstm", "mlstm_column_blocks", "set_mlstm_kernel", "Routing", "moe_route", "routed_gelu", "gated_head_norm", "clamped_glu", "routed_clamped_glu", "polynorm", "scale_", "ScoreShape", "PLAIN_SCORES", "DeltaShape", "delta_rule", "qkv_attention", "raise_on_device_error", "rmsnorm", "StreamNumbers", "hyper_norm", "linear_attention", "set_recurrence_columns", "causal_conv", "conv_ring_update", "selective_scan", "PairTable", "embed_rows", "squared_relu", "linear_batched", "token_shift", "tanh_rows", "wkv", "wkv_decode", "StateSpace", "state_space", "gated_group_norm", "rotate_gate", "rope_table", "scatter_i32", "step_rows", "swiglu",
+    "qk_norm_rope_cache", "qk_prepare", "Gain", "STREAM_AS_IS", "residual_norm", "gather_rows_scaled", "logistic_gate", "latent_norm", "latent_assemble", "mlstm", "mlstm_column_blocks", "set_mlstm_kernel", "Routing", "moe_route", "routed_gelu", "gated_head_norm", "clamped_glu", "routed_clamped_glu", "experts_in_groups", "grouped_experts", "polynorm", "scale_", "ScoreShape", "PLAIN_SCORES", "DeltaShape", "delta_rule", "qkv_attention", "raise_on_device_error", "rmsnorm", "StreamNumbers", "hyper_norm", "linear_attention", "set_recurrence_columns", "causal_conv", "conv_ring_update", "selective_scan", "PairTable", "embed_rows", "squared_relu", "linear_batched", "token_shift", "tanh_rows", "wkv", "wkv_decode", "StateSpace", "state_space", "gated_group_norm", "rotate_gate", "rope_table", "scatter_i32", "step_rows", "swiglu",
 ]

@@ -15,7 +15,8 @@ the same form runs for every token and is added, multiplied by ``logistic(shared
 number per token; ``shared_gated`` False: added as it is).  The up-projections of all experts are
 one product, the activation carries the routing weights (zero for an expert that was not chosen),
 and one down-projection over all experts' columns sums the chosen ones: the result does not
-depend on the other rows of the step.  Kernels: csrc/moe.cu.
+depend on the other rows of the step.  With many rows the chosen experts are multiplied alone, over the rows sorted by
+expert (``ops.experts_in_groups``).  Kernels: csrc/moe.cu, csrc/moe_grouped.cu.
 
 ``polynorm``: ``down(act(up(x)))`` with ``act(z) = a N(z) + b N(z^2) + c N(z^3) + e``, powers
 taken entry by entry and ``N`` the division of a token's vector by its root mean square (``eps``
@@ -146,6 +147,9 @@ class RoutedExperts:
         err = getattr(ctx, "err", None)
         z = ops.linear(x, self.w_route, out_dtype=torch.float32, err=err)
         routing = ops.moe_route(z, self.n_experts, self.groups, self.keep, self.top, self.scale)
+        if ops.experts_in_groups(x, self.n_experts, self.top, self.ff, self.shared_ff, False):
+            return ops.grouped_experts(x, routing, self.w_up, self.w_down, self.ff, self.shared_ff, None,
+                                       z if self.shared_gated else None, self.n_experts, err)
         u = ops.linear(x, self.w_up, err=err)
         a = ops.routed_gelu(u, routing, self.ff, self.shared_ff, z if self.shared_gated else None, self.n_experts)
         return ops.linear(a, self.w_down, err=err)
@@ -248,6 +252,10 @@ class RoutedClampedExperts:
         err = getattr(ctx, "err", None)
         z = ops.linear(x, self.w_route, out_dtype=torch.float32, err=err)
         routing = ops.moe_route(z, self.n_experts, 1, 1, self.top, 1.0, scoring=self.scoring, renormalise=self.renormalise)
+        if ops.experts_in_groups(x, self.n_experts, self.top, self.ff, self.shared_ff, True):
+            glu = (self.limit, self.shared_limit, self.slope, self.up_shift, self.weight_at)
+            return ops.grouped_experts(x, routing, self.w_gate_up, self.w_down, self.ff, self.shared_ff, glu,
+                                       z if self.shared_gated else None, self.n_experts, err)
         gu = ops.linear(x, self.w_gate_up, err=err)
         y = ops.routed_clamped_glu(gu, routing, self.ff, self.shared_ff, self.limit, self.shared_limit, self.slope,
                                    z if self.shared_gated else None, self.n_experts, weight_at=self.weight_at, up_shift=self.up_shift)
