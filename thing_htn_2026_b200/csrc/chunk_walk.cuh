@@ -1,5 +1,5 @@
-// Recurrences over a matrix state S [128 keys, values] whose decay is one number per head and token,
-// walked a chunk of 32 tokens at a time, for prompts with bfloat16 activations.  Token by token such a
+// Recurrences over a matrix state S [128 keys, values] whose decay is one number per head and token, or one
+// per head, token and key, walked a chunk of 32 tokens at a time, for prompts with bfloat16 activations.  Token by token such a
 // kernel is a chain of thousands of dependent steps.  Inside a chunk the sums can be taken in any order:
 //
 //     o_i  = alpha_i S0^T q_i + beta_i sum_{j <= i} G_ij v_j
@@ -9,7 +9,8 @@
 // products q_i . k_j with the decays between the two tokens, zero for j > i) and the numbers per token;
 // what is left to walk is three products per chunk.  The delta rule's values are v = u - W S0 with rows u
 // and W that its kernel has worked out too.  The gated matrix memory keeps the logarithms' running maximum
-// m, a number that only the walk knows: alpha and beta come from it, and a vector n beside S.
+// m, a number that only the walk knows: alpha and beta come from it, and a vector n beside S.  With a decay
+// per key the mixer's kernel has multiplied it into the queries, the keys and G, and S is decayed by a number per key.
 //
 // The products run on the tensor cores in bfloat16 with operands split into three parts, x = h + m + l exactly (24
 // bits), and the six products of parts that reach 2^-24: h h; and, in an accumulator of their own, h m, m h, m m,
@@ -61,7 +62,7 @@ struct WalkArgs {
     float scale;               // on every read-out
     // the gated matrix memory
     float* normaliser;         // [slots, heads, value_dim / 16, kKeys + 1]: copies of n, then m
-    const float* key_sums;     // [chunk_place, heads, kKeys]: sum_j w_j k_j of every chunk
+    const float* key_sums;     // [chunk_place, heads, kKeys]: sum_j w_j k_j of every chunk; a decay per key: the chunk's decay of S
     float floor_;
 };
 
@@ -220,9 +221,18 @@ __device__ __forceinline__ void leave_out(Parts (&values)[kTokens / 16], int (&f
     }
 }
 
-template <typename T, int CG, int KS, bool DELTA, int STAGES>
+// What the mixer's recurrence is.
+enum Kind {
+    kPlain,        // a decay per token
+    kDelta,        // values less what the state holds
+    kGated,        // a running maximum beside it, read-outs divided
+    kPerKey        // a decay per token and key, already in the queries, the keys and G
+};
+
+template <typename T, int CG, int KS, Kind KIND, int STAGES>
 struct Layout {
-    static constexpr int kParts = sizeof(T) == 2 ? 1 : 3;
+    static constexpr bool DELTA = KIND == kDelta;
+    static constexpr int kParts = sizeof(T) == 2 && KIND != kPerKey ? 1 : 3;      // of queries and keys
     static constexpr int kThreads = 32 * CG * KS, kColumns = 16 * CG;
     static constexpr int kValueRow = kColumns + (sizeof(T) == 2 ? 8 : 4);
     static constexpr int kKeyPlane = kTokens * kKeyRow, kScorePlane = kTokens * kScoreRow;      // elements
@@ -233,15 +243,16 @@ struct Layout {
     static constexpr int kV = kG + 3 * kScorePlane * 2;
     static constexpr int kScalars = kV + kTokens * kValueRow * (int)sizeof(T);
     static constexpr int kSums = kScalars + kTokens * 16;                                    // gated: the chunk's sum of keys
-    static constexpr int kStage = kSums + (kParts == 1 ? kKeys * 4 : 0);
+    static constexpr int kStage = kSums + (KIND == kGated || KIND == kPerKey ? kKeys * 4 : 0);
     static constexpr int kShares = KS > 1 ? KS * CG * (DELTA ? 2 : 1) * 4 * 32 * 16 : 0;    // [ks][cg][which][8 tokens][lane] float4
     static constexpr int kBytes = STAGES * kStage + kShares + (kTokens * 3 + kKeys + 4) * 4;
 };
 
-template <typename T, int CG, int KS, bool DELTA, bool GATED, int STAGES>
+template <typename T, int CG, int KS, Kind KIND, int STAGES>
 __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * KS) : 1) walk_kernel(WalkArgs a) {
-    using L = Layout<T, CG, KS, DELTA, STAGES>;
-    constexpr int PARTS = L::kParts;
+    using L = Layout<T, CG, KS, KIND, STAGES>;
+    constexpr bool DELTA = KIND == kDelta, GATED = KIND == kGated, PER_KEY = KIND == kPerKey;
+    constexpr int PARTS = L::kParts, VALUE_PARTS = sizeof(T) == 2 ? 1 : 3;
     constexpr int KT = kKeys / KS / 8;               // groups of 8 keys of a warp
     constexpr int GROUPS = kTokens / 8;              // groups of 8 tokens
     constexpr int OWN = GROUPS / KS;                 // groups that a warp finishes
@@ -298,10 +309,10 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
                 q_from += kRowsApart * a.key_row;
                 k_from += kRowsApart * a.key_row;
             }
-            if (GATED && threadIdx.x < kKeys / 4)
-                copy16(dst + L::kSums + threadIdx.x * 16,
-                       a.key_sums + ((chunk_place(row0, seq) + chunk) * a.n_heads + head) * kKeys + threadIdx.x * 4, true);
         }
+        if ((GATED || PER_KEY) && threadIdx.x < kKeys / 4)
+            copy16(dst + L::kSums + threadIdx.x * 16,
+                   a.key_sums + ((chunk_place(row0, seq) + chunk) * a.n_heads + head) * kKeys + threadIdx.x * 4, true);
 #pragma unroll
         for (int p = 0; p < 3; ++p) {
             if (DELTA)
@@ -316,7 +327,7 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
             const bool there = i < n_here;
             copy16(dst + L::kV + (i * L::kValueRow + c) * (int)sizeof(T), v_src + (there ? first + i : 0) * a.v_row + c, there);
         }
-        for (int i = threadIdx.x; i < kTokens; i += L::kThreads)
+        for (int i = threadIdx.x; !PER_KEY && i < kTokens; i += L::kThreads)
             copy16(dst + L::kScalars + i * 16, scalar_src + (i < n_here ? first + i : 0), i < n_here);
         copy_commit();
     };
@@ -479,10 +490,8 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
                 }
                 continue;
             }
-            const float4* sc = scalars + 16 * j + 2 * t;
-            const float w0 = sc[0].z, w1 = sc[1].z, w8 = sc[8].z, w9 = sc[9].z;
             float2 v[4];        // column g, g + 8 at tokens 2t, 2t + 1; the same at 2t + 8, 2t + 9
-            if constexpr (PARTS == 1) {
+            if constexpr (VALUE_PARTS == 1) {
                 load_matrices_transposed(plain[j].part[0], v_s + 16 * j * L::kValueRow + b_tile(lane, L::kValueRow));
 #pragma unroll
                 for (int i = 0; i < 4; ++i) v[i] = make_float2(low_half(plain[j].part[0][i]), high_half(plain[j].part[0][i]));
@@ -495,11 +504,14 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
                 v[3] = make_float2(src[8], src[L::kValueRow + 8]);
                 plain[j] = parts_of(v[0], v[1], v[2], v[3]);
             }
+            if constexpr (PER_KEY) continue;
+            const float4* sc = scalars + 16 * j + 2 * t;
+            const float w0 = sc[0].z, w1 = sc[1].z, w8 = sc[8].z, w9 = sc[9].z;
             scaled[j] = parts_of(make_float2(v[0].x * w0, v[0].y * w1), make_float2(v[1].x * w0, v[1].y * w1),
                                  make_float2(v[2].x * w8, v[2].y * w9), make_float2(v[3].x * w8, v[3].y * w9));
         }
         // the state behind the chunk
-        const float keep = GATED ? alpha_s[n_here - 1] : scalars[n_here - 1].x, take = GATED ? beta_s[n_here - 1] : 1.f;
+        const float keep = PER_KEY ? 1.f : GATED ? alpha_s[n_here - 1] : scalars[n_here - 1].x, take = GATED ? beta_s[n_here - 1] : 1.f;
         constexpr int KP = 2;                        // pairs of groups of keys at a time
 #pragma unroll
         for (int n = 0; n < KT; n += 2 * KP) {
@@ -513,16 +525,20 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
                 float large[2 * KP][4], small[2 * KP][4];
                 clear(large);
                 clear(small);
-                multiply(large, small, scaled[j], k);
+                if constexpr (PER_KEY) multiply<VALUE_PARTS>(large, small, plain[j], k);
+                else multiply(large, small, scaled[j], k);
 #pragma unroll
                 for (int o = 0; o < 2 * KP; ++o)
 #pragma unroll
                     for (int i = 0; i < 4; ++i) sum[o][i] = j == 0 ? joined(large[o][i], small[o][i]) : sum[o][i] + joined(large[o][i], small[o][i]);
             }
 #pragma unroll
-            for (int o = 0; o < 2 * KP; ++o)
+            for (int o = 0; o < 2 * KP; ++o) {
+                float2 by_key = make_float2(keep, keep);
+                if constexpr (PER_KEY) by_key = pair_of(reinterpret_cast<const float*>(stage + L::kSums) + key0 + 8 * (n + o) + 2 * t);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) s[n + o][i] = fmaf(keep, s[n + o][i], take * sum[o][i]);
+                for (int i = 0; i < 4; ++i) s[n + o][i] = fmaf(i & 1 ? by_key.y : by_key.x, s[n + o][i], take * sum[o][i]);
+            }
         }
         // sum_j G_ij v_j for this warp's tokens, and the read-outs
         // (G's rows are loaded for 16 tokens at a time; with one group of tokens a warp, two warps share them)
@@ -540,7 +556,7 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
                     float large[2][4], small[2][4];
                     clear(large);
                     clear(small);
-                    multiply<PARTS>(large, small, plain[j], row);
+                    multiply<VALUE_PARTS>(large, small, plain[j], row);
 #pragma unroll
                     for (int o = 0; o < 2; ++o)
 #pragma unroll
@@ -566,7 +582,7 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
         }
         if (lost) {
             int from[2];
-            leave_out<PARTS>(plain, from, t);
+            leave_out<VALUE_PARTS>(plain, from, t);
             take_inner();
 #pragma unroll
             for (int pair = 0; pair < kPairs; ++pair)
@@ -585,7 +601,7 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
                 const int o = OWN == 1 ? group0 & 1 : n & 1;
                 const float in0 = o ? inner[n / 2][1][half] : inner[n / 2][0][half];
                 const float in1 = o ? inner[n / 2][1][2 + half] : inner[n / 2][0][2 + half];
-                const float alpha = GATED ? alpha_s[i] : scalars[i].x, beta = GATED ? beta_s[i] : 1.f;
+                const float alpha = PER_KEY ? 1.f : GATED ? alpha_s[i] : scalars[i].x, beta = GATED ? beta_s[i] : 1.f;
                 float y0 = (alpha * read[n][half] + beta * in0) * a.scale;
                 float y1 = (alpha * read[n][2 + half] + beta * in1) * a.scale;
                 if (GATED) {
@@ -618,10 +634,10 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
     }
 }
 
-template <typename T, int CG, int KS, bool DELTA, bool GATED, int STAGES>
+template <typename T, int CG, int KS, Kind KIND, int STAGES>
 void launch_walk(const WalkArgs& a, int n_seqs, cudaStream_t stream) {
-    using L = Layout<T, CG, KS, DELTA, STAGES>;
-    auto kernel = walk_kernel<T, CG, KS, DELTA, GATED, STAGES>;
+    using L = Layout<T, CG, KS, KIND, STAGES>;
+    auto kernel = walk_kernel<T, CG, KS, KIND, STAGES>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
     thn_launch_ordered(kernel, dim3(a.value_dim / L::kColumns, a.n_heads, n_seqs), L::kThreads, L::kBytes, stream, a);
 }

@@ -935,9 +935,9 @@ THN_API int thn_delta_chunks(float* o, float* state, void* scratch, const void* 
     // once they reach nearly every multiprocessor.  us of the whole call, 16 / 32 / 64 columns: one prompt of
     // 2,048 tokens, 16 heads 247 / 310 / 415, 32 heads 464 / 379 / 480; 8 x 512 tokens of 16 heads 427 / 375 / 316.
     const long long pairs = (long long)n_seqs * n_heads;
-    if (dv % 64 == 0 && pairs * (dv / 64) >= 128) chunk::launch_walk<float, 4, 2, true, false, 2>(a, n_seqs, stream);
-    else if (dv % 32 == 0 && pairs * (dv / 32) >= 128) chunk::launch_walk<float, 2, 4, true, false, 2>(a, n_seqs, stream);
-    else chunk::launch_walk<float, 1, 4, true, false, 2>(a, n_seqs, stream);
+    if (dv % 64 == 0 && pairs * (dv / 64) >= 128) chunk::launch_walk<float, 4, 2, chunk::kDelta, 2>(a, n_seqs, stream);
+    else if (dv % 32 == 0 && pairs * (dv / 32) >= 128) chunk::launch_walk<float, 2, 4, chunk::kDelta, 2>(a, n_seqs, stream);
+    else chunk::launch_walk<float, 1, 4, chunk::kDelta, 2>(a, n_seqs, stream);
     return thn_launch_status("delta_chunks");
 }
 

@@ -28,8 +28,14 @@
 // shared memory, and once a stage of tokens is through, each lane adds up the 16 shares of some
 // (token, column) pairs and writes their results.  A row's result depends on its sequence's own
 // tokens only, in an order fixed by the sizes.
+//
+// Prompts with gated decays, bfloat16 rows and keys of 128 go in chunks of 32 tokens instead: linear_attention_chunk_kernel works out what
+// a chunk needs beside the state, the walk of chunk_walk.cuh takes the chunks on the tensor cores.
 #include <math.h>
 
+#include <algorithm>
+
+#include "chunk_walk.cuh"
 #include "linear_attention.cuh"
 
 namespace {
@@ -51,7 +57,7 @@ template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.
 
 // logistic(z)^(1 / tau) = exp(-softplus(-z) / tau), without overflow; in double on the 32-bit path
 template <typename T> __device__ __forceinline__ float logistic_power(float z, float inv_tau) {
-    const float log_logistic = z >= 0.f ? -log1pf(expf(-z)) : z - log1pf(expf(z));
+    const float log_logistic = fminf(z, 0.f) - log1pf(expf(-fabsf(z)));      // (one way for either sign: no lane waits for another)
     return expf(log_logistic * inv_tau);
 }
 template <> __device__ __forceinline__ float logistic_power<float>(float z, float inv_tau) {
@@ -136,6 +142,157 @@ __global__ void __launch_bounds__(256) linear_attention_prepare_vec_kernel(
         if (silu_inputs) out = make_float4(silu_of<T>(out.x), silu_of<T>(out.y), silu_of<T>(out.z), silu_of<T>(out.w));
     }
     *reinterpret_cast<float4*>(prepared + row * n_heads * per_head + item) = out;
+}
+
+// ---------------------------------------------------------------- chunk by chunk, bfloat16
+
+// What a chunk of 32 tokens needs beside the state (chunk_walk.cuh), for one head with a decay per key channel.  Eight threads hold two
+// tokens' keys and multiply them by the decay of every token that follows, as the state is token by token, so that no logarithm is taken and
+// no product can overflow: what they hold at token i times its query is G_ij, what is left at the chunk's end is what the token adds to
+// the state.  Out: G, the queries times the decays up to their token and those keys as planes, the chunk's decay of the state.
+// Bound by its 60 KB of planes a chunk and by issue: the decays' logarithms and exponentials, and the 528 pairs of tokens by 128
+// channels, which are taken two channels an instruction.  (A key a thread loaded its queries and decays from shared memory twice as often.)  The
+// sums over the channels of eight tokens are taken together, by halving (seven exchanges for eight sums).  Six blocks on a multiprocessor: 1,531
+// tokens of 32 heads on B200 56 us (five, in three waves: 63; a key a thread: 66).  The whole call 187 us, token by token 278.  The error against 64 bits is the
+// same: read-out 7.4e-7 over 300 tokens, 1.63e-6 over 2,000 (token by token 7.4e-7, 1.66e-6), state 1.09e-6 and 1.75e-6 (1.08e-6, 1.78e-6).
+constexpr int kChunkThreads = 128, kChunkParts = 8;
+
+__global__ void __launch_bounds__(kChunkThreads, 6) linear_attention_chunk_kernel(
+    __nv_bfloat16* __restrict__ scores, __nv_bfloat16* __restrict__ queries, __nv_bfloat16* __restrict__ keys, float* __restrict__ decays,
+    const __nv_bfloat16* __restrict__ proj, int proj_width, int q_offset, int k_offset, const float* __restrict__ gate, int gate_width,
+    const float* __restrict__ gate_bias, float inv_tau, const int* __restrict__ cu_seqlens, int n_rows, int n_heads) {
+    pdl_launch_dependents();
+    pdl_wait();
+    constexpr int C = chunk::kTokens, D = chunk::kKeys;
+    __shared__ __align__(16) float a_s[C][D], q_s[C][D], g_s[C][C + 1];
+    const int tid = threadIdx.x, j0 = tid / kChunkParts * 2, part = tid % kChunkParts, warp = tid >> 5;
+    const int head = blockIdx.y, seq = blockIdx.z;
+    const int begin = cu_seqlens[seq], row0 = begin + blockIdx.x * C, n_here = min(C, cu_seqlens[seq + 1] - row0);
+    if (n_here <= 0) return;
+
+    // decays, queries and keys of tokens j0 and j0 + 1: channels 4 part + 32 r .. + 3 are this thread's, as two pairs (rows beyond
+    // the sequence's: no decay, zeros)
+    unsigned long long key[2][8];
+    float4 bias[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+        bias[r] = gate_bias ? *reinterpret_cast<const float4*>(gate_bias + head * D + 4 * part + 32 * r) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int o = 0; o < 2; ++o) {
+        const int j = j0 + o;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int d = 4 * part + 32 * r;
+            float4 a = make_float4(1.f, 1.f, 1.f, 1.f), q = make_float4(0.f, 0.f, 0.f, 0.f);
+            uint2 kv = make_uint2(0u, 0u);
+            if (j < n_here) {
+                const size_t row = row0 + j;
+                const __nv_bfloat16* src = proj + row * proj_width + (size_t)head * D + d;
+                const uint2 qv = *reinterpret_cast<const uint2*>(src + q_offset);
+                kv = *reinterpret_cast<const uint2*>(src + k_offset);
+                a = *reinterpret_cast<const float4*>(gate + row * gate_width + head * D + d);
+                a.x = logistic_power<__nv_bfloat16>(a.x + bias[r].x, inv_tau); a.y = logistic_power<__nv_bfloat16>(a.y + bias[r].y, inv_tau);
+                a.z = logistic_power<__nv_bfloat16>(a.z + bias[r].z, inv_tau); a.w = logistic_power<__nv_bfloat16>(a.w + bias[r].w, inv_tau);
+                q = make_float4(chunk::low_half(qv.x), chunk::high_half(qv.x), chunk::low_half(qv.y), chunk::high_half(qv.y));
+            }
+            key[o][2 * r] = pack2(chunk::low_half(kv.x), chunk::high_half(kv.x));
+            key[o][2 * r + 1] = pack2(chunk::low_half(kv.y), chunk::high_half(kv.y));
+            *reinterpret_cast<float4*>(&a_s[j][d]) = a;
+            *reinterpret_cast<float4*>(&q_s[j][d]) = q;
+        }
+    }
+    __syncthreads();
+
+    // G, eight tokens i at a time, from the eight on whose keys this warp holds
+    const int first = 8 * warp;
+    auto eight = [&](int i0, bool own) {
+        float sum[2][8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int i = i0 + u;
+            unsigned long long dot[2] = {pack2(0.f, 0.f), pack2(0.f, 0.f)};
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(&q_s[i][4 * part + 32 * r]);
+                const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(&a_s[i][4 * part + 32 * r]);
+#pragma unroll
+                for (int o = 0; o < 2; ++o) {
+                    if (!own || i > j0 + o) {      // (only the decays of tokens behind the key's)
+                        key[o][2 * r] = mul2(key[o][2 * r], a.x);
+                        key[o][2 * r + 1] = mul2(key[o][2 * r + 1], a.y);
+                    }
+                    dot[o] = fma2(q.x, key[o][2 * r], dot[o]);
+                    dot[o] = fma2(q.y, key[o][2 * r + 1], dot[o]);
+                }
+            }
+#pragma unroll
+            for (int o = 0; o < 2; ++o) {
+                float x, y;
+                unpack2(dot[o], x, y);
+                sum[o][u] = x + y;
+            }
+        }
+        // the eight threads' shares: thread p ends up with token i0 + p
+#pragma unroll
+        for (int w = 4; w > 0; w >>= 1) {
+            const bool upper = part & w;
+#pragma unroll
+            for (int o = 0; o < 2; ++o)
+#pragma unroll
+                for (int u = 0; u < w; ++u) {
+                    const float give = upper ? sum[o][u] : sum[o][u + w];
+                    const float got = __shfl_xor_sync(0xffffffffu, give, w);
+                    sum[o][u] = (upper ? sum[o][u + w] : sum[o][u]) + got;
+                }
+        }
+        g_s[i0 + part][j0] = sum[0][0];
+        g_s[i0 + part][j0 + 1] = sum[1][0];
+    };
+    eight(first, true);
+#pragma unroll 1
+    for (int i0 = first + 8; i0 < C; i0 += 8) eight(i0, false);
+
+    const long long plane = (long long)n_rows * chunk::kKeyRow, score_plane = (long long)n_rows * chunk::kScoreRow;
+    auto store = [&](__nv_bfloat16* planes, int j, int r, float4 v) {
+        const chunk::Split lo = chunk::split(v.x, v.y), hi = chunk::split(v.z, v.w);
+        __nv_bfloat16* dst = planes + head * 3 * plane + (size_t)(row0 + j) * chunk::kKeyRow + 4 * part + 32 * r;
+#pragma unroll
+        for (int p = 0; p < 3; ++p) *reinterpret_cast<uint2*>(dst + p * plane) = make_uint2(lo.part[p], hi.part[p]);
+    };
+#pragma unroll
+    for (int o = 0; o < 2; ++o)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            float4 k;
+            unpack2(key[o][2 * r], k.x, k.y);
+            unpack2(key[o][2 * r + 1], k.z, k.w);
+            if (j0 + o < n_here) store(keys, j0 + o, r, k);
+        }
+    __syncthreads();
+    // the decays up to each token, a channel a thread, over the decays themselves
+    float upto = 1.f;
+#pragma unroll 8
+    for (int i = 0; i < C; ++i) {
+        upto *= a_s[i][tid];
+        a_s[i][tid] = upto;
+    }
+    decays[((chunk::chunk_place(begin, seq) + blockIdx.x) * n_heads + head) * D + tid] = upto;
+    __nv_bfloat16* dst = scores + head * 3 * score_plane + (long long)row0 * chunk::kScoreRow;
+#pragma unroll
+    for (int e = tid; e < C * C / 2; e += kChunkThreads) {
+        const int i = e / (C / 2), c = e % (C / 2) * 2;
+        if (i < n_here)
+            chunk::store_split(dst + i * chunk::kScoreRow + c, score_plane, c <= i ? g_s[i][c] : 0.f, c + 1 <= i ? g_s[i][c + 1] : 0.f);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int o = 0; o < 2; ++o)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int j = j0 + o, d = 4 * part + 32 * r;
+            const float4 q = *reinterpret_cast<const float4*>(&q_s[j][d]), a = *reinterpret_cast<const float4*>(&a_s[j][d]);
+            if (j < n_here) store(queries, j, r, make_float4(q.x * a.x, q.y * a.y, q.z * a.z, q.w * a.w));
+        }
 }
 
 // PER: key channels per lane (a multiple of 4); KP = 16 * PER: the padded key size.  COLS: columns per lane.
@@ -440,4 +597,62 @@ THN_API int thn_linear_attention(float* o, float* state, float* scratch, const v
                                      mode, silu_inputs, stream);
     THN_CHECK_ARG(false, "linear_attention: unknown dtype %d", dtype);
     return THN_OK;
+}
+
+// Bytes of the scratch that thn_linear_attention_chunks needs.
+THN_API long long thn_linear_attention_chunks_scratch_bytes(int n_rows, int n_seqs, int n_heads) {
+    return (long long)n_heads * n_rows * 3 * (2 * chunk::kKeyRow + chunk::kScoreRow) * 2 + chunk::chunk_places(n_rows, n_seqs) * n_heads * chunk::kKeys * 4;
+}
+
+// The recurrence of a step with gated decays chunk by chunk: bfloat16 rows as thn_linear_attention takes them (no silu), keys of
+// 128, values of whole groups of 16; v's columns start on 16-byte boundaries, q's and k's on 8-byte ones, gate and its bias on
+// 16-byte ones; max_tokens: the most rows of a sequence.  shape: 0, or which blocks walk (tests and measurement).
+THN_API int thn_linear_attention_chunks(float* o, float* state, void* scratch, const void* proj, int proj_width, int q_offset, int k_offset,
+                                        int v_offset, const float* gate, int gate_width, const float* gate_bias, float tau,
+                                        const int* cu_seqlens, const int* slots, int n_rows, int max_tokens, int n_seqs, int n_heads,
+                                        int key_dim, int value_dim, float q_scale, int shape, cudaStream_t stream) {
+    THN_CHECK_ARG(n_seqs >= 0 && n_heads > 0 && gate != nullptr && tau > 0.f && gate_width >= n_heads * key_dim, "linear_attention_chunks: bad sizes");
+    THN_UNSUPPORTED_IF(key_dim != chunk::kKeys || value_dim <= 0 || value_dim % 16 != 0 || proj_width % 8 != 0 || v_offset % 8 != 0 ||
+                           (q_offset | k_offset | gate_width) % 4 != 0,
+                       "linear_attention_chunks: keys of %d, values of %d, rows of %d, columns %d, %d, %d", key_dim, value_dim, proj_width,
+                       q_offset, k_offset, v_offset);
+    THN_CHECK_ARG(q_offset >= 0 && k_offset >= 0 && v_offset >= 0 && q_offset + n_heads * key_dim <= proj_width &&
+                      k_offset + n_heads * key_dim <= proj_width && v_offset + n_heads * value_dim <= proj_width,
+                  "linear_attention_chunks: q, k, v do not lie inside rows of %d", proj_width);
+    THN_UNSUPPORTED_IF(n_heads > 65535 || n_seqs > 65535, "linear_attention_chunks: %d heads, %d sequences", n_heads, n_seqs);
+    THN_CHECK_ARG(scratch && (((uintptr_t)state | (uintptr_t)scratch | (uintptr_t)proj | (uintptr_t)gate | (uintptr_t)gate_bias) & 15) == 0,
+                  "linear_attention_chunks: operands are not 16-byte aligned");
+    if (n_seqs == 0 || n_rows <= 0 || max_tokens <= 0) return THN_OK;
+    const int chunks = (max_tokens + chunk::kTokens - 1) / chunk::kTokens;
+    const size_t plane = (size_t)n_rows * chunk::kKeyRow;
+    __nv_bfloat16* queries = static_cast<__nv_bfloat16*>(scratch);
+    __nv_bfloat16* keys = queries + 3 * n_heads * plane;
+    __nv_bfloat16* scores = keys + 3 * n_heads * plane;
+    float* decays = reinterpret_cast<float*>(scores + (size_t)3 * n_heads * n_rows * chunk::kScoreRow);
+    const __nv_bfloat16* rows = static_cast<const __nv_bfloat16*>(proj);
+    cudaFuncSetAttribute(linear_attention_chunk_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    thn_launch(linear_attention_chunk_kernel, dim3(chunks, n_heads, n_seqs), kChunkThreads, 0, stream, scores, queries, keys, decays, rows,
+               proj_width, q_offset, k_offset, gate, gate_width, gate_bias, 1.0f / tau, cu_seqlens, n_rows, n_heads);
+    chunk::WalkArgs a{};
+    a.o = o; a.state = state;
+    a.q = queries; a.k = keys;
+    a.key_plane = plane; a.key_unit = 3 * plane; a.key_row = chunk::kKeyRow;
+    a.v = rows + v_offset; a.v_row = proj_width; a.v_head = value_dim;
+    a.scores = scores; a.key_sums = decays;
+    a.cu_seqlens = cu_seqlens; a.slots = slots;
+    a.n_rows = n_rows; a.n_heads = n_heads; a.heads_per_unit = 1; a.value_dim = value_dim; a.scale = q_scale;
+    using T = __nv_bfloat16;
+    // Few sequences: narrow blocks, whose four warps split the keys; more: wide ones, which share a chunk's keys and queries, with one
+    // buffer where two blocks on a multiprocessor cover each other's loads.  By the sequences that are walked at once for the longest one's time
+    // (or, with many short ones beside it, by all there are), us of the whole call with shapes 1 / 2 / 3 / 4: one prompt of 2,048 tokens of 16 heads
+    // SHAPES16, of 32 heads SHAPES32, 2 x 512 of 32 heads SHAPES64, 8 x 512 of 32 heads SHAPES256.
+    const double busy = (double)n_heads * value_dim / chunk::kKeys * std::max((double)n_rows / max_tokens, n_seqs / 30.0);
+    if (shape == 0) shape = busy <= 18 ? 1 : busy <= 48 ? 2 : busy <= 100 ? 3 : 4;
+    if (value_dim % 64 != 0) shape = std::min(shape, 2);
+    if (value_dim % 32 != 0) shape = 1;
+    if (shape == 4) chunk::launch_walk<T, 4, 2, chunk::kPerKey, 1>(a, n_seqs, stream);
+    else if (shape == 3) chunk::launch_walk<T, 4, 2, chunk::kPerKey, 2>(a, n_seqs, stream);
+    else if (shape == 2) chunk::launch_walk<T, 2, 4, chunk::kPerKey, 2>(a, n_seqs, stream);
+    else chunk::launch_walk<T, 1, 4, chunk::kPerKey, 2>(a, n_seqs, stream);
+    return thn_launch_status("linear_attention_chunks");
 }

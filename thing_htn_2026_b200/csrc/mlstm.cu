@@ -531,7 +531,7 @@ THN_API int thn_mlstm_chunks(float* o, float* S, float* nm, void* scratch, const
     // the keys; us of the whole call with 64 / 16 columns: 8 x 512 tokens of 16 heads 132 / 155, one prompt of 2,048 tokens
     // of 16 heads 357 / 140, of 32 heads 370 / 179, four of up to 1,000 tokens 191 / 110.
     const long long pairs = (long long)n_seqs * n_heads;
-    if (value_dim % 64 == 0 && pairs * (value_dim / 64) >= 256) chunk::launch_walk<T, 4, 1, false, true, 2>(a, n_seqs, stream);
-    else chunk::launch_walk<T, 1, 4, false, true, 2>(a, n_seqs, stream);
+    if (value_dim % 64 == 0 && pairs * (value_dim / 64) >= 256) chunk::launch_walk<T, 4, 1, chunk::kGated, 2>(a, n_seqs, stream);
+    else chunk::launch_walk<T, 1, 4, chunk::kGated, 2>(a, n_seqs, stream);
     return thn_launch_status("mlstm_chunks");
 }

@@ -574,10 +574,10 @@ THN_API int thn_state_space_chunks(float* y, float* state, void* scratch, const 
     // us of the whole call with blocks of 64 columns and two to a multiprocessor, 64 with two buffers, 32: 8 x 512 tokens of
     // 128 heads 613 / 624 / 736, one prompt of 2,048 tokens of 128 heads 415 / 349 / 410, of 64 heads 372 / 306 / 220.
     const long long pairs = (long long)n_seqs * n_heads;
-    if (vdim % 64 == 0 && pairs * (vdim / 64) >= 384) chunk::launch_walk<float, 4, 2, false, false, 1>(a, n_seqs, stream);
-    else if (vdim % 64 == 0 && pairs * (vdim / 64) >= 128) chunk::launch_walk<float, 4, 2, false, false, 2>(a, n_seqs, stream);
-    else if (vdim % 32 == 0) chunk::launch_walk<float, 2, 4, false, false, 2>(a, n_seqs, stream);
-    else chunk::launch_walk<float, 1, 4, false, false, 2>(a, n_seqs, stream);
+    if (vdim % 64 == 0 && pairs * (vdim / 64) >= 384) chunk::launch_walk<float, 4, 2, chunk::kPlain, 1>(a, n_seqs, stream);
+    else if (vdim % 64 == 0 && pairs * (vdim / 64) >= 128) chunk::launch_walk<float, 4, 2, chunk::kPlain, 2>(a, n_seqs, stream);
+    else if (vdim % 32 == 0) chunk::launch_walk<float, 2, 4, chunk::kPlain, 2>(a, n_seqs, stream);
+    else chunk::launch_walk<float, 1, 4, chunk::kPlain, 2>(a, n_seqs, stream);
     return thn_launch_status("state_space_chunks");
 }
 

@@ -70,6 +70,9 @@ _SIGNATURES = {
                             c_int, c_longlong, c_float, c_int, c_void_p],
     "thn_hyper_norm": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_float,
                        c_int, c_int, c_int, c_int, c_void_p],
+    "thn_linear_attention_chunks_scratch_bytes": [c_int, c_int, c_int],
+    "thn_linear_attention_chunks": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_float,
+                                    c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p],
     "thn_linear_attention": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
                              c_void_p, c_float, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int,
                              c_int, c_void_p],
@@ -1449,6 +1452,10 @@ _MLSTM_COST = _ChunkCost(0.5, 0.009, 0.03, 1.8, 0.055, 0.0, 128)
 #   state-space duality, 64 heads of 64: 96 + 0 38 / 43, 128 + 0 44 / 42, 128 + 60 108 / 171, 512 + 8 142 / 122, 512 + 60 151 / 198,
 #     2,048 + 60 517 / 460, 32 prompts of 128 tokens 568 / 349
 _SPACE_COST = _ChunkCost(0.205, 0.0021, 0.016, 3.1, 0.035, -10.0, 64)
+#   linear attention with gated decays, 32 heads of 128: 16 + 0 15 / 24, 64 + 0 24 / 28, 128 + 0 36 / 32, 300 + 0 65 / 50, 2,048 + 0 368 / 222,
+#     16 + 60 103 / 155, 512 + 60 181 / 241, 2,048 + 60 419 / 439, 64 prompts of 16 tokens 247 / 183; 16 heads: 128 + 0 28 / 30, 300 + 0 50 / 42,
+#     2,048 + 0 263 / 155, 2,048 + 60 335 / 259
+_LINEAR_COST = _ChunkCost(0.128, 0.0055, 0.045, 2.6, 0.082, -12.0, 128)
 
 
 def _delta_in_chunks(proj: torch.Tensor, conv_w: torch.Tensor, state: torch.Tensor, ring: torch.Tensor, rows: StepRows,
@@ -1850,6 +1857,20 @@ def set_recurrence_columns(columns: int = 0) -> None:
     lib().thn_set_recurrence_columns(int(columns))
 
 
+LINEAR_CHUNK_SHAPE = 0      # which blocks walk the chunks: 0 a rule of sizes, 1 to 4 one of them (tests and measurement)
+
+
+def _linear_in_chunks(proj: torch.Tensor, offsets: Tuple[int, int, int], state: torch.Tensor, rows: StepRows, n_heads: int, key_dim: int,
+                      value_dim: int, gate: torch.Tensor, gate_bias: Optional[torch.Tensor]) -> bool:
+    """Whether a step's recurrence with gated decays is walked in chunks of tokens on the tensor cores."""
+    return proj.dtype == torch.bfloat16 and key_dim == CHUNK_KEYS and value_dim % 16 == 0 and rows.max_q_len >= CHUNK_MIN_TOKENS \
+        and proj.shape[1] % 8 == 0 and offsets[2] % 8 == 0 and (offsets[0] | offsets[1] | gate.shape[1]) % 4 == 0 \
+        and max(n_heads, rows.n_seqs) <= 65535 and max(offsets[0], offsets[1]) + n_heads * key_dim <= proj.shape[1] \
+        and min(offsets) >= 0 and offsets[2] + n_heads * value_dim <= proj.shape[1] \
+        and (state.data_ptr() | proj.data_ptr() | gate.data_ptr() | (0 if gate_bias is None else gate_bias.data_ptr())) % 16 == 0 \
+        and _LINEAR_COST.chunks_pay(rows, n_heads, value_dim)
+
+
 def linear_attention(proj: torch.Tensor, offsets: Tuple[int, int, int], state: torch.Tensor, rows: StepRows,
                      n_heads: int, key_dim: int, value_dim: int, *, decay: Optional[torch.Tensor] = None,
                      gate: Optional[torch.Tensor] = None, gate_bias: Optional[torch.Tensor] = None, tau: float = 1.0,
@@ -1862,7 +1883,8 @@ def linear_attention(proj: torch.Tensor, offsets: Tuple[int, int, int], state: t
     ``logistic(gate + gate_bias) ** (1 / tau)`` with ``gate`` float32 ``[rows, >= heads * key_dim]``.
     ``state`` float32 [slots, heads, value_dim, key_dim] is read and updated.  Returns the read-out,
     float32 [rows, heads, value_dim].  Two kernels: the inputs' activations and the decays once per
-    entry into float32 scratch rows, then the recurrence."""
+    entry into float32 scratch rows, then the recurrence; or, prompts with gated decays, bfloat16 rows and keys of 128, what a
+    chunk of 32 tokens needs beside the state, then the walk over the chunks, equal up to rounding."""
     _need(proj, "linear_attention proj")
     _need(state, "linear_attention state", torch.float32)
     if (decay is None) == (gate is None):
@@ -1883,6 +1905,13 @@ def linear_attention(proj: torch.Tensor, offsets: Tuple[int, int, int], state: t
             if gate_bias.shape[0] != n_heads * key_dim:
                 raise KernelError(f"linear_attention: gate bias {tuple(gate_bias.shape)}")
     o = torch.empty((rows.n_rows, n_heads, value_dim), dtype=torch.float32, device=proj.device)
+    if gate is not None and not silu_inputs and _linear_in_chunks(proj, offsets, state, rows, n_heads, key_dim, value_dim, gate, gate_bias):
+        scratch = torch.empty(lib().thn_linear_attention_chunks_scratch_bytes(rows.n_rows, rows.n_seqs, n_heads), dtype=torch.uint8,
+                              device=proj.device)
+        _call("thn_linear_attention_chunks", _ptr(o), _ptr(state), _ptr(scratch), _ptr(proj), proj.shape[1], int(offsets[0]), int(offsets[1]),
+              int(offsets[2]), _ptr(gate), gate.shape[1], _ptr(gate_bias), float(tau), _ptr(rows.cu_seqlens), _ptr(rows.slots), rows.n_rows,
+              rows.max_q_len, rows.n_seqs, n_heads, key_dim, value_dim, float(q_scale), LINEAR_CHUNK_SHAPE, _stream())
+        return o
     mode = 0 if decay is not None else 1
     scratch = torch.empty(lib().thn_linear_attention_scratch_floats(rows.n_rows, n_heads, key_dim, value_dim, mode),
                           dtype=torch.float32, device=proj.device)
