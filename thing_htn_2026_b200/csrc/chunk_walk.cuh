@@ -24,9 +24,15 @@
 // A block walks one sequence, head and 16 CG columns of values.  S^T lives in the accumulator registers of
 // its warps: warp (cg, ks) holds 16 columns and 128 / KS keys; the accumulator layout of two groups of eight
 // keys is the A operand's layout, so S never moves.  With KS > 1 the warps' shares of W S0 and S0^T q meet in
-// shared memory, each warp then finishes some of the tokens.  The next chunk's operands travel by
-// asynchronous copies into the other of STAGES buffers (with one buffer, other blocks of the
-// multiprocessor cover the wait); rows beyond the sequence's are filled with zeros.
+// shared memory, each warp then finishes some of the tokens.  The next chunk's operands travel into the other of STAGES
+// buffers (with one buffer, other blocks of the multiprocessor cover the wait); rows beyond the sequence's are zeros.
+//
+// Who brings them: the warps themselves, by asynchronous copies of 16 bytes, or (BROUGHT, where the operands lie in planes) four more
+// warps, by bulk copies of whole planes.  The first hold every warp up for as long as a chunk takes to come from L2 (1,765 of a chunk's
+// 4,630 clocks for the delta rule of 16 heads, 1,225 of 3,700 for 32 heads with a decay per key), but start sooner and leave room for more
+// blocks: they stay where blocks are many and short.  (One more warp takes 1,200 clocks to start a chunk's bulk copies, most of the time that the others
+// need for it.)  The wait for what is brought is bounded: after kWaitLimitNs by the global timer the block sets
+// THN_ERR_WAIT_TIMEOUT and returns.
 #pragma once
 
 #include "common.cuh"
@@ -64,6 +70,7 @@ struct WalkArgs {
     float* normaliser;         // [slots, heads, value_dim / 16, kKeys + 1]: copies of n, then m
     const float* key_sums;     // [chunk_place, heads, kKeys]: sum_j w_j k_j of every chunk; a decay per key: the chunk's decay of S
     float floor_;
+    int* err;                  // the caller's error word, or null
 };
 
 __device__ __forceinline__ void copy16(void* smem, const void* gmem, bool there) {
@@ -86,6 +93,60 @@ __device__ __forceinline__ void copy_rows(__nv_bfloat16* smem, const __nv_bfloat
         if (kPieces % THREADS == 0 || i < kPieces) copy16(smem + i * 8, gmem + (i < end ? i * 8 : 0), i < end);
     }
 }
+
+constexpr unsigned long long kWaitLimitNs = 20ull * 1000 * 1000;
+__device__ __forceinline__ uint32_t shared_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(shared_addr(bar)), "r"(count));
+}
+__device__ __forceinline__ void mbar_expect(uint64_t* bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_addr(bar)), "r"(bytes) : "memory");
+}
+// Bounded wait for the phase with the given parity.  Returns false when it gave up.
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
+    WaitClock clock;
+    for (int spin = 0;; ++spin) {
+        uint32_t done;
+        asm volatile(
+            "{\n"
+            ".reg .pred p;\n"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+            "selp.u32 %0, 1, 0, p;\n"
+            "}\n"
+            : "=r"(done)
+            : "r"(shared_addr(bar)), "r"(parity)
+            : "memory");
+        if (done) return true;
+        if ((spin & 15) == 15 && clock.ran_out(kWaitLimitNs)) return false;
+    }
+}
+// 16-byte aligned on both sides, whole pieces of 16 bytes; counted by `bar`.
+__device__ __forceinline__ void copy_bulk(void* smem, const void* gmem, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(shared_addr(smem)), "l"(gmem), "r"(bytes), "r"(shared_addr(bar)) : "memory");
+}
+// The barrier hears of this thread's copies of 16 bytes when they have landed.
+__device__ __forceinline__ void copies_arrive(uint64_t* bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(shared_addr(bar)) : "memory");
+}
+__device__ __forceinline__ void barrier_sync(int id, int threads) { asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+// Whether all threads of the block say yes, and a barrier.
+__device__ __forceinline__ bool all_agree(bool yes) {
+    uint32_t all;
+    asm volatile(
+        "{\n"
+        ".reg .pred p, q;\n"
+        "setp.ne.u32 p, %1, 0;\n"
+        "barrier.cta.red.and.pred q, 0, p;\n"
+        "selp.u32 %0, 1, 0, q;\n"
+        "}\n"
+        : "=r"(all)
+        : "r"((uint32_t)yes)
+        : "memory");
+    return all != 0;
+}
+// What threads have written to shared memory stands ahead of the bulk copies that are started behind the next barrier.
+__device__ __forceinline__ void writes_ahead_of_copies() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t pack_bf16(float x, float y) {
     const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
@@ -229,11 +290,13 @@ enum Kind {
     kPerKey        // a decay per token and key, already in the queries, the keys and G
 };
 
-template <typename T, int CG, int KS, Kind KIND, int STAGES>
+template <typename T, int CG, int KS, Kind KIND, int STAGES, bool BROUGHT>
 struct Layout {
     static constexpr bool DELTA = KIND == kDelta;
     static constexpr int kParts = sizeof(T) == 2 && KIND != kPerKey ? 1 : 3;      // of queries and keys
     static constexpr int kThreads = 32 * CG * KS, kColumns = 16 * CG;
+    static constexpr int kBringers = BROUGHT ? 128 : 0;            // threads that bring the operands
+    static_assert(!BROUGHT || (kParts == 3 && STAGES == 2), "planes, two buffers");
     static constexpr int kValueRow = kColumns + (sizeof(T) == 2 ? 8 : 4);
     static constexpr int kKeyPlane = kTokens * kKeyRow, kScorePlane = kTokens * kScoreRow;      // elements
     static constexpr int kQ = 0;
@@ -245,12 +308,12 @@ struct Layout {
     static constexpr int kSums = kScalars + kTokens * 16;                                    // gated: the chunk's sum of keys
     static constexpr int kStage = kSums + (KIND == kGated || KIND == kPerKey ? kKeys * 4 : 0);
     static constexpr int kShares = KS > 1 ? KS * CG * (DELTA ? 2 : 1) * 4 * 32 * 16 : 0;    // [ks][cg][which][8 tokens][lane] float4
-    static constexpr int kBytes = STAGES * kStage + kShares + (kTokens * 3 + kKeys + 4) * 4;
+    static constexpr int kBytes = STAGES * kStage + kShares + (kTokens * 3 + kKeys + 4) * 4 + STAGES * 8;
 };
 
-template <typename T, int CG, int KS, Kind KIND, int STAGES>
-__global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * KS) : 1) walk_kernel(WalkArgs a) {
-    using L = Layout<T, CG, KS, KIND, STAGES>;
+template <typename T, int CG, int KS, Kind KIND, int STAGES, bool BROUGHT>
+__global__ void __launch_bounds__(32 * CG * KS + (BROUGHT ? 128 : 0), STAGES == 1 ? 512 / (32 * CG * KS) : 1) walk_kernel(WalkArgs a) {
+    using L = Layout<T, CG, KS, KIND, STAGES, BROUGHT>;
     constexpr bool DELTA = KIND == kDelta, GATED = KIND == kGated, PER_KEY = KIND == kPerKey;
     constexpr int PARTS = L::kParts, VALUE_PARTS = sizeof(T) == 2 ? 1 : 3;
     constexpr int KT = kKeys / KS / 8;               // groups of 8 keys of a warp
@@ -267,11 +330,17 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
     float* under_s = beta_s + kTokens;
     float* n_s = under_s + kTokens;
     int* lost_s = reinterpret_cast<int*>(n_s + kKeys);      // delta: a value was not finite, in this chunk or ahead of it
+    uint64_t* full = reinterpret_cast<uint64_t*>(lost_s + 4);        // [STAGES] a chunk has landed
     const int slab = blockIdx.x, head = blockIdx.y, seq = blockIdx.z;
     if (DELTA && threadIdx.x == 0) *lost_s = 0;
+    if (BROUGHT && threadIdx.x == 0) {
+        for (int i = 0; i < STAGES; ++i) mbar_init(full + i, L::kBringers + 1);      // their copies, and the bytes' announcement
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (BROUGHT) __syncthreads();
     const int row0 = a.cu_seqlens[seq], n_tokens = a.cu_seqlens[seq + 1] - row0;
     if (n_tokens <= 0) return;
-    const int slot = a.slots[seq], unit = head / a.heads_per_unit;
+    const int slot = a.slots[seq], unit = head / a.heads_per_unit, n_chunks = (n_tokens + kTokens - 1) / kTokens;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int cg = warp / KS, ks = warp % KS, key0 = ks * (kKeys / KS);
     const int group0 = ks * OWN;                     // the first group of tokens that this warp finishes
@@ -284,6 +353,48 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
     const T* v_src = static_cast<const T*>(a.v) + row0 * a.v_row + head * a.v_head + col0;
     const float4* scalar_src = a.scalars + (long long)head * a.n_rows + row0;
 
+    if (BROUGHT && warp >= CG * KS) {
+        // ---- the warps that bring the operands: W, the queries, the keys and G, a plane a lane, and the values' rows
+        const int bringer = threadIdx.x - L::kThreads, p = min(lane, 2);
+        auto bring = [&](int chunk) {
+            unsigned char* dst = mem + (chunk % STAGES) * L::kStage;
+            uint64_t* bar = full + chunk % STAGES;
+            const int first = chunk * kTokens, n_here = min(kTokens, n_tokens - first);
+            constexpr uint32_t kRowBytes = (DELTA ? 9 : 6) * kKeyRow * 2 + 3 * kScoreRow * 2 + (PER_KEY ? 0 : 16);
+            if (bringer == 0) mbar_expect(bar, n_here * kRowBytes + (PER_KEY ? kKeys * 4 : 0));
+            const uint32_t key_bytes = n_here * kKeyRow * 2;
+            const long long key_at = (long long)first * kKeyRow;
+            if (bringer < 32) {
+                if (DELTA && lane < 3) copy_bulk(dst + L::kW + p * L::kKeyPlane * 2, w_src + p * w_plane + key_at, key_bytes, bar);
+                if (PER_KEY && lane == 0)
+                    copy_bulk(dst + L::kSums, a.key_sums + ((chunk_place(row0, seq) + chunk) * a.n_heads + head) * kKeys, kKeys * 4, bar);
+            } else if (bringer < 64) {
+                if (lane < 3) copy_bulk(dst + L::kQ + p * L::kKeyPlane * 2, q_src + p * a.key_plane + key_at, key_bytes, bar);
+            } else if (bringer < 96) {
+                if (lane < 3) copy_bulk(dst + L::kK + p * L::kKeyPlane * 2, k_src + p * a.key_plane + key_at, key_bytes, bar);
+            } else {
+                if (lane < 3)
+                    copy_bulk(dst + L::kG + p * L::kScorePlane * 2, g_src + p * g_plane + (long long)first * kScoreRow, n_here * kScoreRow * 2, bar);
+                else if (!PER_KEY && lane == 3)
+                    copy_bulk(dst + L::kScalars, scalar_src + first, n_here * 16, bar);
+            }
+            constexpr int kPer16 = 16 / (int)sizeof(T), kValueCopies = L::kColumns / kPer16;
+#pragma unroll
+            for (int e = bringer; e < kTokens * kValueCopies; e += L::kBringers) {
+                const int i = e / kValueCopies, c = e % kValueCopies * kPer16;
+                const bool there = i < n_here;
+                copy16(dst + L::kV + (i * L::kValueRow + c) * (int)sizeof(T), v_src + (there ? first + i : 0) * a.v_row + c, there);
+            }
+            copies_arrive(bar);
+        };
+        bring(0);
+        if (n_chunks > 1) bring(1);
+        for (int chunk = 0; chunk < n_chunks; ++chunk) {
+            if (!all_agree(true)) return;
+            if (chunk > 0 && chunk + 1 < n_chunks) bring(chunk + 1);      // (the chunk ahead of this one is through: its buffer is free)
+        }
+        return;
+    }
     auto issue = [&](int chunk) {
         unsigned char* dst = mem + (chunk % STAGES) * L::kStage;
         const int first = chunk * kTokens, n_here = min(kTokens, n_tokens - first);
@@ -331,7 +442,7 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
             copy16(dst + L::kScalars + i * 16, scalar_src + (i < n_here ? first + i : 0), i < n_here);
         copy_commit();
     };
-    issue(0);
+    if (!BROUGHT) issue(0);
 
     // S^T: s[j][0], s[j][1]: column g, keys 8j + 2t and the one after; s[j][2], s[j][3]: column g + 8
     float s[KT][4];
@@ -352,15 +463,22 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
     const int key_at = b_tile(lane, kKeyRow) + key0;          // this lane's address in a tile of 16 tokens and 16 keys
     const int key_at_transposed = a_tile(lane, kKeyRow) + key0;
 
-    const int n_chunks = (n_tokens + kTokens - 1) / kTokens;
     for (int chunk = 0; chunk < n_chunks; ++chunk) {
-        if (STAGES == 1 && chunk > 0) {
-            __syncthreads();           // the only stage is free again
-            issue(chunk);
+        // this chunk is in place; the other buffer, and the shares, are free again
+        if constexpr (BROUGHT) {
+            if (!all_agree(mbar_wait(full + chunk % STAGES, chunk / STAGES & 1))) {
+                if (threadIdx.x == 0 && a.err) atomicOr(a.err, THN_ERR_WAIT_TIMEOUT);
+                return;
+            }
+        } else {
+            if (STAGES == 1 && chunk > 0) {
+                __syncthreads();           // the only stage is free again
+                issue(chunk);
+            }
+            copy_wait_all();
+            __syncthreads();
+            if (STAGES > 1 && chunk + 1 < n_chunks) issue(chunk + 1);
         }
-        copy_wait_all();
-        __syncthreads();               // this chunk is in place; the other stage, and the shares, are free again
-        if (STAGES > 1 && chunk + 1 < n_chunks) issue(chunk + 1);
         unsigned char* stage = mem + (chunk % STAGES) * L::kStage;
         const __nv_bfloat16* q_s = reinterpret_cast<const __nv_bfloat16*>(stage + L::kQ);
         const __nv_bfloat16* k_s = reinterpret_cast<const __nv_bfloat16*>(stage + L::kK);
@@ -369,6 +487,21 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
         T* v_s = reinterpret_cast<T*>(stage + L::kV) + cg * 16;
         const float4* scalars = reinterpret_cast<const float4*>(stage + L::kScalars);
         const int first = chunk * kTokens, n_here = min(kTokens, n_tokens - first);
+        if (BROUGHT && n_here < kTokens) {
+            // the sequence's last chunk: zeros where rows beyond it would enter the state (queries and G's rows enter their own read-outs
+            // alone, and G's columns behind a row's token are zero)
+            auto clear_rows = [&](int at, int row_bytes) {
+                for (int e = n_here * row_bytes / 16 + threadIdx.x; e < kTokens * row_bytes / 16; e += L::kThreads)
+                    *reinterpret_cast<uint4*>(stage + at + e * 16) = make_uint4(0, 0, 0, 0);
+            };
+#pragma unroll
+            for (int p = 0; p < 3; ++p) {
+                clear_rows(L::kK + p * L::kKeyPlane * 2, kKeyRow * 2);
+                if (DELTA) clear_rows(L::kW + p * L::kKeyPlane * 2, kKeyRow * 2);
+            }
+            if (!PER_KEY) clear_rows(L::kScalars, 16);
+            barrier_sync(1, L::kThreads);
+        }
 
         if (GATED) {
             // alpha, beta and the denominators of the chunk's tokens; four threads share a token's n . q
@@ -430,7 +563,7 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
                 if (DELTA) own[(4 + n) * 32] = make_float4(fixed[n][0], fixed[n][1], fixed[n][2], fixed[n][3]);
             }
         }
-        if (KS > 1 || GATED) __syncthreads();
+        if (KS > 1 || GATED) barrier_sync(1, L::kThreads);
         if (KS > 1) {
             // (the sums are taken in the order of the keys, whoever takes them)
 #pragma unroll
@@ -475,7 +608,8 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
                 }
             }
             if (own_lost) *lost_s = 1;
-            __syncthreads();
+            if (BROUGHT) writes_ahead_of_copies();
+            barrier_sync(1, L::kThreads);
         }
         // the chunk's values as A operands: columns by tokens, as they are and times w
         Parts plain[kTokens / 16], scaled[kTokens / 16];
@@ -634,13 +768,20 @@ __global__ void __launch_bounds__(32 * CG * KS, STAGES == 1 ? 512 / (32 * CG * K
     }
 }
 
-template <typename T, int CG, int KS, Kind KIND, int STAGES>
+template <typename T, int CG, int KS, Kind KIND, int STAGES, bool BROUGHT>
 void launch_walk(const WalkArgs& a, int n_seqs, cudaStream_t stream) {
-    using L = Layout<T, CG, KS, KIND, STAGES>;
-    auto kernel = walk_kernel<T, CG, KS, KIND, STAGES>;
+    using L = Layout<T, CG, KS, KIND, STAGES, BROUGHT>;
+    static_assert(L::kBytes <= 227 * 1024, "what a block may have");
+    auto kernel = walk_kernel<T, CG, KS, KIND, STAGES, BROUGHT>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
-    thn_launch_ordered(kernel, dim3(a.value_dim / L::kColumns, a.n_heads, n_seqs), L::kThreads, L::kBytes, stream, a);
+    thn_launch_ordered(kernel, dim3(a.value_dim / L::kColumns, a.n_heads, n_seqs), L::kThreads + L::kBringers, L::kBytes, stream, a);
 }
+
+// Whether a step's sequences are so short that the blocks' starts weigh more than their chunks: the warps then copy themselves.  us of the whole
+// call, copying / brought, 16 heads of the delta rule, of a decay per key, 64 heads of state-space duality: one prompt of 2,048 tokens 245 / 206,
+// 157 / 136, 222 / 202; 1,531 tokens 216 / 161, 136 / 99, 192 / 159; 8 x 512 329 / 324, 194 / 187, 368 / 361; 32 x 128 327 / 327, 189 / 193,
+// 351 / 368; 64 x 33 306 / 318, 173 / 194, -; 2,048 tokens beside 60 single ones 519 / 493, 263 / 245, 452 / 361, 512 tokens 220 / 230, 155 / 146, 194 / 233.
+inline bool many_short(int n_rows, int n_seqs, int max_tokens) { return n_rows < 200ll * n_seqs && max_tokens < 1024; }
 
 // ---------------------------------------------------------------- what the mixers' own kernels share
 

@@ -890,14 +890,14 @@ THN_API long long thn_delta_chunks_scratch_bytes(int n_rows, int n_heads, int n_
 // prepare and recurrence of a step chunk by chunk, the state carried in float32: bfloat16 rows, four taps, keys of
 // 128, values of whole groups of 16 columns; max_tokens: the most rows of a sequence.  scratch:
 // thn_delta_chunks_scratch_bytes(...), 16-byte aligned, as the state and the taps must be; the rows and the
-// ring are read in pieces of 8 bytes.  One prompt of 2,048 tokens, 16 heads of 128 x 128, on B200: 243 us
-// against 658 token by token; 32 heads 368 / 839; 8 x 512 tokens of 16 heads 333 / 571; steps of long and short sequences beside
+// ring are read in pieces of 8 bytes.  One prompt of 2,048 tokens, 16 heads of 128 x 128, on B200: 206 us
+// against 658 token by token; 32 heads 321 / 839; 8 x 512 tokens of 16 heads 324 / 571; steps of long and short sequences beside
 // the rule in ops (_DELTA_COST).  The read-out's error
 // against 64 bits is 1.37e-7 to 1.41e-7 (1.33e-7 to 1.36e-7 token by token), the state's 1.2e-7 to 1.4e-7 (1.1e-7 to 1.3e-7).
 THN_API int thn_delta_chunks(float* o, float* state, void* scratch, const void* proj, const float* conv_w, const float* a_log,
                              const float* dt_bias, const void* ring, const int* row_slot, const int* row_pos, const int* seq_lens,
                              const int* cu_seqlens, const int* slots, int n_rows, int max_tokens, int n_seqs, int n_heads, int n_kv,
-                             int dk, int dv, int taps, int proj_width, float unit_eps, cudaStream_t stream) {
+                             int dk, int dv, int taps, int proj_width, float unit_eps, int* err, cudaStream_t stream) {
     DeltaShape s{n_heads, n_kv, dk, dv, taps, proj_width};
     if (int status = check_shape(s, "delta_chunks")) return status;
     THN_UNSUPPORTED_IF(dk != chunk::kKeys || dv % 16 != 0 || taps != kRunTaps || proj_width % 4 != 0,
@@ -924,6 +924,7 @@ THN_API int thn_delta_chunks(float* o, float* state, void* scratch, const void* 
     thn_launch(delta_chunk_kernel, dim3((max_tokens + chunk::kTokens - 1) / chunk::kTokens, n_heads, n_seqs), kChunkThreads,
                kDeltaChunkBytes, stream, values, w, scores, scalars, planes, beta, decay, cu_seqlens, n_rows, s);
     chunk::WalkArgs a{};
+    a.err = err;
     a.o = o; a.state = state;
     a.q = planes; a.k = planes + 3 * n_kv * key_plane;
     a.key_plane = key_plane; a.key_unit = 3 * key_plane; a.key_row = chunk::kKeyRow;
@@ -932,12 +933,18 @@ THN_API int thn_delta_chunks(float* o, float* state, void* scratch, const void* 
     a.cu_seqlens = cu_seqlens; a.slots = slots;
     a.n_rows = n_rows; a.n_heads = n_heads; a.heads_per_unit = n_heads / n_kv; a.value_dim = dv; a.scale = 1.f;
     // More columns a block load the chunk's keys, queries and W less often, fewer give more blocks: wide blocks
-    // once they reach nearly every multiprocessor.  us of the whole call, 16 / 32 / 64 columns: one prompt of
+    // once they reach nearly every multiprocessor.  us of the whole call, 16 / 32 / 64 columns (the warps copying themselves): one prompt of
     // 2,048 tokens, 16 heads 247 / 310 / 415, 32 heads 464 / 379 / 480; 8 x 512 tokens of 16 heads 427 / 375 / 316.
     const long long pairs = (long long)n_seqs * n_heads;
-    if (dv % 64 == 0 && pairs * (dv / 64) >= 128) chunk::launch_walk<float, 4, 2, chunk::kDelta, 2>(a, n_seqs, stream);
-    else if (dv % 32 == 0 && pairs * (dv / 32) >= 128) chunk::launch_walk<float, 2, 4, chunk::kDelta, 2>(a, n_seqs, stream);
-    else chunk::launch_walk<float, 1, 4, chunk::kDelta, 2>(a, n_seqs, stream);
+    using namespace chunk;
+    if (dv % 64 == 0 && pairs * (dv / 64) >= 128) {
+        if (many_short(n_rows, n_seqs, max_tokens)) launch_walk<float, 4, 2, kDelta, 2, false>(a, n_seqs, stream);
+        else launch_walk<float, 4, 2, kDelta, 2, true>(a, n_seqs, stream);
+    } else if (dv % 32 == 0 && pairs * (dv / 32) >= 128) {
+        launch_walk<float, 2, 4, kDelta, 2, true>(a, n_seqs, stream);
+    } else {
+        launch_walk<float, 1, 4, kDelta, 2, true>(a, n_seqs, stream);
+    }
     return thn_launch_status("delta_chunks");
 }
 

@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(256) linear_attention_prepare_vec_kernel(
 // Bound by its 60 KB of planes a chunk and by issue: the decays' logarithms and exponentials, and the 528 pairs of tokens by 128
 // channels, which are taken two channels an instruction.  (A key a thread loaded its queries and decays from shared memory twice as often.)  The
 // sums over the channels of eight tokens are taken together, by halving (seven exchanges for eight sums).  Six blocks on a multiprocessor: 1,531
-// tokens of 32 heads on B200 56 us (five, in three waves: 63; a key a thread: 66).  The whole call 187 us, token by token 278.  The error against 64 bits is the
+// tokens of 32 heads on B200 56 us (five, in three waves: 63; a key a thread: 66).  The whole call 153 us, token by token 278.  The error against 64 bits is the
 // same: read-out 7.4e-7 over 300 tokens, 1.63e-6 over 2,000 (token by token 7.4e-7, 1.66e-6), state 1.09e-6 and 1.75e-6 (1.08e-6, 1.78e-6).
 constexpr int kChunkThreads = 128, kChunkParts = 8;
 
@@ -610,7 +610,7 @@ THN_API long long thn_linear_attention_chunks_scratch_bytes(int n_rows, int n_se
 THN_API int thn_linear_attention_chunks(float* o, float* state, void* scratch, const void* proj, int proj_width, int q_offset, int k_offset,
                                         int v_offset, const float* gate, int gate_width, const float* gate_bias, float tau,
                                         const int* cu_seqlens, const int* slots, int n_rows, int max_tokens, int n_seqs, int n_heads,
-                                        int key_dim, int value_dim, float q_scale, int shape, cudaStream_t stream) {
+                                        int key_dim, int value_dim, float q_scale, int shape, int* err, cudaStream_t stream) {
     THN_CHECK_ARG(n_seqs >= 0 && n_heads > 0 && gate != nullptr && tau > 0.f && gate_width >= n_heads * key_dim, "linear_attention_chunks: bad sizes");
     THN_UNSUPPORTED_IF(key_dim != chunk::kKeys || value_dim <= 0 || value_dim % 16 != 0 || proj_width % 8 != 0 || v_offset % 8 != 0 ||
                            (q_offset | k_offset | gate_width) % 4 != 0,
@@ -634,6 +634,7 @@ THN_API int thn_linear_attention_chunks(float* o, float* state, void* scratch, c
     thn_launch(linear_attention_chunk_kernel, dim3(chunks, n_heads, n_seqs), kChunkThreads, 0, stream, scores, queries, keys, decays, rows,
                proj_width, q_offset, k_offset, gate, gate_width, gate_bias, 1.0f / tau, cu_seqlens, n_rows, n_heads);
     chunk::WalkArgs a{};
+    a.err = err;
     a.o = o; a.state = state;
     a.q = queries; a.k = keys;
     a.key_plane = plane; a.key_unit = 3 * plane; a.key_row = chunk::kKeyRow;
@@ -642,17 +643,19 @@ THN_API int thn_linear_attention_chunks(float* o, float* state, void* scratch, c
     a.cu_seqlens = cu_seqlens; a.slots = slots;
     a.n_rows = n_rows; a.n_heads = n_heads; a.heads_per_unit = 1; a.value_dim = value_dim; a.scale = q_scale;
     using T = __nv_bfloat16;
-    // Few sequences: narrow blocks, whose four warps split the keys; more: wide ones, which share a chunk's keys and queries, with one
-    // buffer where two blocks on a multiprocessor cover each other's loads.  By the sequences that are walked at once for the longest one's time
-    // (or, with many short ones beside it, by all there are), us of the whole call with shapes 1 / 2 / 3 / 4: one prompt of 2,048 tokens of 16 heads
-    // SHAPES16, of 32 heads SHAPES32, 2 x 512 of 32 heads SHAPES64, 8 x 512 of 32 heads SHAPES256.
-    const double busy = (double)n_heads * value_dim / chunk::kKeys * std::max((double)n_rows / max_tokens, n_seqs / 30.0);
-    if (shape == 0) shape = busy <= 18 ? 1 : busy <= 48 ? 2 : busy <= 100 ? 3 : 4;
+    // Few sequences: narrow blocks, whose four warps split the keys; more: wide ones, which share a chunk's keys and queries; where blocks
+    // are many and short, two on a multiprocessor with one buffer each (4).  By the sequences that are walked at once for the longest one's time
+    // (or, with many short ones beside it, by all there are), us of the whole call with shapes 1 / 2 / 3 / 4 (the warps copying themselves): one prompt
+    // of 2,048 tokens of 16 heads 155 / 181 / 245 / 294, of 32 heads 290 / 218 / 279 / 335, 2 x 512 of 32 heads 157 / 122 / 103 / 120, 8 x 512 of 32 heads
+    // 542 / 411 / 376 / 368.
+    using namespace chunk;
+    const double busy = (double)n_heads * value_dim / kKeys * std::max((double)n_rows / max_tokens, n_seqs / 30.0);
+    if (shape == 0) shape = busy <= 18 ? 1 : busy <= 48 ? 2 : busy > 100 && many_short(n_rows, n_seqs, max_tokens) ? 4 : 3;
     if (value_dim % 64 != 0) shape = std::min(shape, 2);
     if (value_dim % 32 != 0) shape = 1;
-    if (shape == 4) chunk::launch_walk<T, 4, 2, chunk::kPerKey, 1>(a, n_seqs, stream);
-    else if (shape == 3) chunk::launch_walk<T, 4, 2, chunk::kPerKey, 2>(a, n_seqs, stream);
-    else if (shape == 2) chunk::launch_walk<T, 2, 4, chunk::kPerKey, 2>(a, n_seqs, stream);
-    else chunk::launch_walk<T, 1, 4, chunk::kPerKey, 2>(a, n_seqs, stream);
+    if (shape == 4) launch_walk<T, 4, 2, kPerKey, 1, false>(a, n_seqs, stream);
+    else if (shape == 3) launch_walk<T, 4, 2, kPerKey, 2, true>(a, n_seqs, stream);
+    else if (shape == 2) launch_walk<T, 2, 4, kPerKey, 2, true>(a, n_seqs, stream);
+    else launch_walk<T, 1, 4, kPerKey, 2, true>(a, n_seqs, stream);
     return thn_launch_status("linear_attention_chunks");
 }

@@ -503,7 +503,7 @@ THN_API long long thn_mlstm_chunks_scratch_bytes(int n_rows, int n_seqs, int n_h
 THN_API int thn_mlstm_chunks(float* o, float* S, float* nm, void* scratch, const void* proj, int proj_width, const float* gate_pre,
                              const float* bias_i, const float* bias_f, float cap, const int* cu_seqlens, const int* slots, int n_rows,
                              int max_tokens, int n_seqs, int n_heads, int key_dim, int value_dim, float q_scale, float floor_,
-                             cudaStream_t stream) {
+                             int* err, cudaStream_t stream) {
     THN_CHECK_ARG(n_seqs >= 0 && n_heads > 0 && cap > 0.f && proj_width >= n_heads * (2 * key_dim + value_dim), "mlstm_chunks: bad sizes");
     THN_UNSUPPORTED_IF(key_dim != chunk::kKeys || value_dim <= 0 || value_dim % 16 != 0 || proj_width % 8 != 0,
                        "mlstm_chunks: keys of %d, values of %d, rows of %d", key_dim, value_dim, proj_width);
@@ -518,6 +518,7 @@ THN_API int thn_mlstm_chunks(float* o, float* S, float* nm, void* scratch, const
     thn_launch(mlstm_chunk_kernel, dim3(chunks, n_heads, n_seqs), kChunkThreads, 0, stream, scores, scalars, key_sums, rows, proj_width,
                gate_pre, bias_i, bias_f, cap, cu_seqlens, n_rows, n_heads);
     chunk::WalkArgs a{};
+    a.err = err;
     a.o = o; a.state = S;
     a.q = rows; a.k = rows + (size_t)n_heads * key_dim;
     a.key_plane = 0; a.key_unit = key_dim; a.key_row = proj_width;
@@ -531,7 +532,7 @@ THN_API int thn_mlstm_chunks(float* o, float* S, float* nm, void* scratch, const
     // the keys; us of the whole call with 64 / 16 columns: 8 x 512 tokens of 16 heads 132 / 155, one prompt of 2,048 tokens
     // of 16 heads 357 / 140, of 32 heads 370 / 179, four of up to 1,000 tokens 191 / 110.
     const long long pairs = (long long)n_seqs * n_heads;
-    if (value_dim % 64 == 0 && pairs * (value_dim / 64) >= 256) chunk::launch_walk<T, 4, 1, chunk::kGated, 2>(a, n_seqs, stream);
-    else chunk::launch_walk<T, 1, 4, chunk::kGated, 2>(a, n_seqs, stream);
+    if (value_dim % 64 == 0 && pairs * (value_dim / 64) >= 256) chunk::launch_walk<T, 4, 1, chunk::kGated, 2, false>(a, n_seqs, stream);
+    else chunk::launch_walk<T, 1, 4, chunk::kGated, 2, false>(a, n_seqs, stream);
     return thn_launch_status("mlstm_chunks");
 }

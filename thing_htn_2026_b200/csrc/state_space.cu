@@ -533,13 +533,13 @@ THN_API long long thn_state_space_chunks_scratch_bytes(int n_rows, int n_heads, 
 
 // thn_state_space chunk by chunk: bfloat16 rows in whole 8-byte pieces, four taps, a state of 128, vdim a multiple of 16;
 // max_tokens: the most rows of a sequence.  On B200, us against token by token: 8 x 512 tokens of 128 heads of 64 over a
-// state of 128 620 / 1,074, one prompt of 2,048 tokens of 64 heads 226 / 368, 128 tokens 42 / 44.  The error against 64 bits:
+// state of 128 617 / 1,074, one prompt of 2,048 tokens of 64 heads 202 / 368, 128 tokens 42 / 44.  The error against 64 bits:
 // y 1.2e-7 (1.2e-7 to 1.3e-7), the state 1.1e-7 (1.2e-7).
 THN_API int thn_state_space_chunks(float* y, float* state, void* scratch, const void* proj, int proj_width, int offset,
                                    const float* conv_w, const float* conv_b, const void* ring, const float* dt_pre,
                                    const float* dt_bias, const float* rate, const float* skip, const int* row_slot, const int* row_pos,
                                    const int* seq_lens, const int* cu_seqlens, const int* slots, int n_rows, int max_tokens, int n_seqs,
-                                   int n_heads, int vdim, int n_state, int n_groups, int taps, cudaStream_t stream) {
+                                   int n_heads, int vdim, int n_state, int n_groups, int taps, int* err, cudaStream_t stream) {
     const SpaceShape s{n_heads, vdim, n_state, n_groups, taps};
     if (int status = check_shape("state_space_chunks", s, proj_width, offset)) return status;
     THN_UNSUPPORTED_IF(n_state != chunk::kKeys || vdim % 16 != 0 || taps != kChunkTaps || proj_width % 4 != 0 || offset % 4 != 0,
@@ -564,6 +564,7 @@ THN_API int thn_state_space_chunks(float* y, float* state, void* scratch, const 
     thn_launch(state_space_chunk_kernel, dim3((max_tokens + chunk::kTokens - 1) / chunk::kTokens, n_groups, n_seqs), kSpaceThreads, kSpaceChunkBytes,
                stream, scores, scalars, planes, steps, rate, skip, cu_seqlens, n_rows, n_heads / n_groups);
     chunk::WalkArgs a{};
+    a.err = err;
     a.o = y; a.state = state;
     a.k = planes; a.q = planes + 3 * plane;
     a.key_plane = plane; a.key_unit = 6 * plane; a.key_row = chunk::kKeyRow;
@@ -571,13 +572,18 @@ THN_API int thn_state_space_chunks(float* y, float* state, void* scratch, const 
     a.scores = scores; a.scalars = scalars;
     a.cu_seqlens = cu_seqlens; a.slots = slots;
     a.n_rows = n_rows; a.n_heads = n_heads; a.heads_per_unit = n_heads / n_groups; a.value_dim = vdim; a.scale = 1.f;
-    // us of the whole call with blocks of 64 columns and two to a multiprocessor, 64 with two buffers, 32: 8 x 512 tokens of
-    // 128 heads 613 / 624 / 736, one prompt of 2,048 tokens of 128 heads 415 / 349 / 410, of 64 heads 372 / 306 / 220.
+    // us of the whole call with blocks of 64 columns and two to a multiprocessor, 64 with two buffers, 32 (the warps copying themselves): 8 x 512
+    // tokens of 128 heads 613 / 624 / 736, one prompt of 2,048 tokens of 128 heads 415 / 349 / 410, of 64 heads 372 / 306 / 220.
     const long long pairs = (long long)n_seqs * n_heads;
-    if (vdim % 64 == 0 && pairs * (vdim / 64) >= 384) chunk::launch_walk<float, 4, 2, chunk::kPlain, 1>(a, n_seqs, stream);
-    else if (vdim % 64 == 0 && pairs * (vdim / 64) >= 128) chunk::launch_walk<float, 4, 2, chunk::kPlain, 2>(a, n_seqs, stream);
-    else if (vdim % 32 == 0) chunk::launch_walk<float, 2, 4, chunk::kPlain, 2>(a, n_seqs, stream);
-    else chunk::launch_walk<float, 1, 4, chunk::kPlain, 2>(a, n_seqs, stream);
+    using namespace chunk;
+    if (vdim % 64 == 0 && pairs * (vdim / 64) >= 128) {
+        if (pairs * (vdim / 64) >= 384 && many_short(n_rows, n_seqs, max_tokens)) launch_walk<float, 4, 2, kPlain, 1, false>(a, n_seqs, stream);
+        else launch_walk<float, 4, 2, kPlain, 2, true>(a, n_seqs, stream);
+    } else if (vdim % 32 == 0) {
+        launch_walk<float, 2, 4, kPlain, 2, true>(a, n_seqs, stream);
+    } else {
+        launch_walk<float, 1, 4, kPlain, 2, true>(a, n_seqs, stream);
+    }
     return thn_launch_status("state_space_chunks");
 }
 

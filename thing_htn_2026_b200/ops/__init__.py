@@ -72,7 +72,7 @@ _SIGNATURES = {
                        c_int, c_int, c_int, c_int, c_void_p],
     "thn_linear_attention_chunks_scratch_bytes": [c_int, c_int, c_int],
     "thn_linear_attention_chunks": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_float,
-                                    c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p],
+                                    c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p],
     "thn_linear_attention": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
                              c_void_p, c_float, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int,
                              c_int, c_void_p],
@@ -102,7 +102,7 @@ _SIGNATURES = {
                         c_int, c_int, c_int, c_int, c_void_p],
     "thn_state_space_chunks": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
-                               c_int, c_int, c_int, c_int, c_int, c_void_p],
+                               c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "thn_state_space_decode": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                c_void_p],
@@ -122,7 +122,7 @@ _SIGNATURES = {
     "thn_mlstm_recurrence": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_float, c_int,
                              c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_void_p],
     "thn_mlstm_chunks": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_float, c_void_p,
-                         c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p],
+                         c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p],
     "thn_moe_route": [c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_float,
                       c_int, c_int, c_float, c_void_p],
     "thn_routed_gelu": [c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p],
@@ -141,7 +141,7 @@ _SIGNATURES = {
                              c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
     "thn_delta_chunks": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                          c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
-                         c_void_p],
+                         c_void_p, c_void_p],
     "thn_delta_conv_ring_update": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                    c_int, c_int, c_int, c_void_p],
     "thn_delta_decode": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -1470,7 +1470,7 @@ def _delta_in_chunks(proj: torch.Tensor, conv_w: torch.Tensor, state: torch.Tens
 
 def delta_rule(proj: torch.Tensor, conv_w: torch.Tensor, a_log: torch.Tensor, dt_bias: torch.Tensor,
                state: torch.Tensor, ring: torch.Tensor, rows: StepRows, seq_lens: torch.Tensor, shape: DeltaShape,
-               unit_eps: float) -> torch.Tensor:
+               unit_eps: float, err: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The gated delta rule over a step's rows: short causal convolutions of q, k and v with
     silu, unit norms of q (also scaled by ``key_dim ** -0.5``) and k, write strength and decay,
     and per head ``S <- g S; u = b (v - S^T k); S <- S + k u^T; o = S^T q`` from the state the
@@ -1498,7 +1498,7 @@ def delta_rule(proj: torch.Tensor, conv_w: torch.Tensor, a_log: torch.Tensor, dt
         _call("thn_delta_chunks", _ptr(o), _ptr(state), _ptr(scratch), _ptr(proj), _ptr(conv_w), _ptr(a_log), _ptr(dt_bias),
               _ptr(ring), _ptr(rows.row_slot), _ptr(rows.row_pos), _ptr(seq_lens), _ptr(rows.cu_seqlens), _ptr(rows.slots), n,
               rows.max_q_len, rows.n_seqs, s.n_heads, s.n_kv, s.key_dim, s.value_dim, s.taps, s.proj_width, float(unit_eps),
-              _stream())
+              _ptr(err), _stream())
         _call("thn_delta_conv_ring_update", _ptr(ring), _ptr(proj), _ptr(rows.cu_seqlens), _ptr(rows.slots), _ptr(seq_lens),
               rows.n_seqs, s.n_heads, s.n_kv, s.key_dim, s.value_dim, s.taps, s.proj_width, code, _stream())
         return o
@@ -1613,7 +1613,7 @@ def _mlstm_in_chunks(proj: torch.Tensor, state: torch.Tensor, rows: StepRows, n_
 
 def mlstm(proj: torch.Tensor, gate_pre: torch.Tensor, bias_i: torch.Tensor, bias_f: torch.Tensor, cap: float,
           state: torch.Tensor, normaliser: torch.Tensor, rows: StepRows, n_heads: int, key_dim: int, value_dim: int,
-          q_scale: float, floor: float = 1e-6) -> torch.Tensor:
+          q_scale: float, floor: float = 1e-6, err: Optional[torch.Tensor] = None) -> torch.Tensor:
     """The matrix-memory recurrence over a step's rows.  ``proj`` rows hold ``[q | k | v | ...]``
     (heads * key_dim, heads * key_dim, heads * value_dim); ``gate_pre`` float32 [rows, 2 * heads]
     the pre-activations of the input gates, then of the forget gates (biases are added here).
@@ -1640,7 +1640,7 @@ def mlstm(proj: torch.Tensor, gate_pre: torch.Tensor, bias_i: torch.Tensor, bias
                               device=proj.device)
         _call("thn_mlstm_chunks", _ptr(o), _ptr(state), _ptr(normaliser), _ptr(scratch), _ptr(proj), proj.shape[1], _ptr(gate_pre),
               _ptr(bias_i), _ptr(bias_f), float(cap), _ptr(rows.cu_seqlens), _ptr(rows.slots), n, rows.max_q_len, rows.n_seqs, n_heads,
-              key_dim, value_dim, float(q_scale), float(floor), _stream())
+              key_dim, value_dim, float(q_scale), float(floor), _ptr(err), _stream())
         return o
     raw = rows.max_q_len == 1
     gates = gate_pre
@@ -1874,7 +1874,7 @@ def _linear_in_chunks(proj: torch.Tensor, offsets: Tuple[int, int, int], state: 
 def linear_attention(proj: torch.Tensor, offsets: Tuple[int, int, int], state: torch.Tensor, rows: StepRows,
                      n_heads: int, key_dim: int, value_dim: int, *, decay: Optional[torch.Tensor] = None,
                      gate: Optional[torch.Tensor] = None, gate_bias: Optional[torch.Tensor] = None, tau: float = 1.0,
-                     q_scale: float = 1.0, silu_inputs: bool = False) -> torch.Tensor:
+                     q_scale: float = 1.0, silu_inputs: bool = False, err: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Linear attention with a decayed matrix state over a step's rows: per head
     ``S <- diag(a) S + k v^T``, ``o = S^T q * q_scale`` from the state the sequences' earlier steps
     left.  ``proj`` rows hold q, k (``heads * key_dim``) and v (``heads * value_dim``) from the
@@ -1910,7 +1910,7 @@ def linear_attention(proj: torch.Tensor, offsets: Tuple[int, int, int], state: t
                               device=proj.device)
         _call("thn_linear_attention_chunks", _ptr(o), _ptr(state), _ptr(scratch), _ptr(proj), proj.shape[1], int(offsets[0]), int(offsets[1]),
               int(offsets[2]), _ptr(gate), gate.shape[1], _ptr(gate_bias), float(tau), _ptr(rows.cu_seqlens), _ptr(rows.slots), rows.n_rows,
-              rows.max_q_len, rows.n_seqs, n_heads, key_dim, value_dim, float(q_scale), LINEAR_CHUNK_SHAPE, _stream())
+              rows.max_q_len, rows.n_seqs, n_heads, key_dim, value_dim, float(q_scale), LINEAR_CHUNK_SHAPE, _ptr(err), _stream())
         return o
     mode = 0 if decay is not None else 1
     scratch = torch.empty(lib().thn_linear_attention_scratch_floats(rows.n_rows, n_heads, key_dim, value_dim, mode),
@@ -2099,7 +2099,7 @@ def _space_in_chunks(proj: torch.Tensor, offset: int, state: torch.Tensor, ring:
 
 
 def state_space(proj: torch.Tensor, offset: int, dt_pre: torch.Tensor, shape: StateSpace, state: torch.Tensor,
-                ring: torch.Tensor, rows: StepRows, seq_lens: torch.Tensor) -> torch.Tensor:
+                ring: torch.Tensor, rows: StepRows, seq_lens: torch.Tensor, err: Optional[torch.Tensor] = None) -> torch.Tensor:
     """State-space duality over a step's rows: the short causal convolution (bias, silu) over the
     columns ``[offset, offset + channels)`` of ``proj``, step sizes ``t = softplus(dt_pre + dt_bias)`` and
     decays ``a = exp(-rate t)`` per head, then ``S <- a S + (t B) x^T``, ``y = S^T C + skip x`` per head (B
@@ -2135,7 +2135,7 @@ def state_space(proj: torch.Tensor, offset: int, dt_pre: torch.Tensor, shape: St
         _call("thn_state_space_chunks", _ptr(y), _ptr(state), _ptr(scratch), _ptr(proj), proj.shape[1], int(offset), _ptr(s.conv_w),
               _ptr(s.conv_b), _ptr(ring), _ptr(dt_pre), _ptr(s.dt_bias), _ptr(s.rate), _ptr(s.skip), _ptr(rows.row_slot),
               _ptr(rows.row_pos), _ptr(seq_lens), _ptr(rows.cu_seqlens), _ptr(rows.slots), n, rows.max_q_len, rows.n_seqs, s.n_heads,
-              s.vdim, s.n_state, s.n_groups, s.taps, _stream())
+              s.vdim, s.n_state, s.n_groups, s.taps, _ptr(err), _stream())
         conv_ring_update(ring, proj, offset, rows, seq_lens)
         return y
     scratch = torch.empty(lib().thn_state_space_scratch_floats(n, s.n_heads, s.vdim, s.n_state, s.n_groups), dtype=torch.float32,

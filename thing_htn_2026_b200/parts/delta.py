@@ -85,6 +85,6 @@ class GatedDelta:
         s = self.shape
         proj = ops.linear(x, self.w_in, err=ctx.err)
         o = ops.delta_rule(proj, self.conv_w, self.a_log, self.dt_bias, ctx.cache.state_view(entry.cache, 0),
-                           ctx.cache.state_view(entry.cache, 1), ctx.rows, ctx.cache.seq_lens, s, self.unit_eps)
+                           ctx.cache.state_view(entry.cache, 1), ctx.rows, ctx.cache.seq_lens, s, self.unit_eps, ctx.err)
         y = ops.gated_head_norm(o, proj, s.gate_offset, self.out_gain, self.norm_eps, s.n_heads, s.value_dim, self.dtype)
         return ops.linear(y, self.w_o, err=ctx.err)

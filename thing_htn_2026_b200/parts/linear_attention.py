@@ -121,7 +121,7 @@ class LinearAttention(PhasedMixer):
             gate = ops.linear(ops.linear(x, self.w_a1, err=ctx.err), self.w_a2, out_dtype=torch.float32, err=ctx.err)
         o = ops.linear_attention(proj, (offset, offset + h * d, offset + 2 * h * d), state, ctx.rows, h, d, e,
                                  decay=self.decay, gate=gate, gate_bias=self.a_bias, tau=self.tau or 1.0,
-                                 q_scale=self.q_scale, silu_inputs=self.silu_inputs)
+                                 q_scale=self.q_scale, silu_inputs=self.silu_inputs, err=ctx.err)
         if self.norm_all:
             ops.gated_head_norm(o, proj, offset + self.gate_offset, self.out_gain, self.norm_eps, 1, h * e, self.dtype,
                                 self.gate_kind, scale, out, out_offset)
