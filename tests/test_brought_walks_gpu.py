@@ -5,6 +5,7 @@ import pytest
 import torch
 
 from test_chunk_recurrences_gpu import BF16, step
+from test_chunk_recurrences_gpu import test_matrix_memory_matches_64_bits as matrix_memory_matches_64_bits
 from thing_htn_2026_b200 import ops
 
 pytestmark = pytest.mark.gpu
@@ -69,3 +70,12 @@ def test_state_space(heads, vdim):
     close(o, want)
     close(together[1:], states[1:])
     assert int(err.item()) == 0
+
+
+# the blocks' shapes of the matrix memory, by how many heads are walked at once: 32 columns and four warps over the keys, 64 and two,
+# 32 and two, 64 and one
+@pytest.mark.parametrize("lens,heads,vdim", [([40, 33], 16, 128), ([40] * 4, 16, 128), ([64, 31, 64, 64], 24, 96), ([40] * 6, 16, 128),
+                                             ([33, 16], 32, 64), ([40] * 9, 16, 128)])
+def test_matrix_memory(monkeypatch, lens, heads, vdim):
+    monkeypatch.setattr(ops, "_MLSTM_COST", ops._MLSTM_COST._replace(lead=1e9))
+    matrix_memory_matches_64_bits(lens, heads, vdim)

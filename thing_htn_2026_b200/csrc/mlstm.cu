@@ -528,11 +528,18 @@ THN_API int thn_mlstm_chunks(float* o, float* S, float* nm, void* scratch, const
     a.n_rows = n_rows; a.n_heads = n_heads; a.heads_per_unit = 1; a.value_dim = value_dim; a.scale = q_scale;
     a.normaliser = nm; a.key_sums = key_sums; a.floor_ = floor_;
     using T = __nv_bfloat16;
-    // Wide blocks share the loads of a chunk's keys and queries, narrow ones give more blocks, whose four warps split
-    // the keys; us of the whole call with 64 / 16 columns: 8 x 512 tokens of 16 heads 132 / 155, one prompt of 2,048 tokens
-    // of 16 heads 357 / 140, of 32 heads 370 / 179, four of up to 1,000 tokens 191 / 110.
-    const long long pairs = (long long)n_seqs * n_heads;
-    if (value_dim % 64 == 0 && pairs * (value_dim / 64) >= 256) chunk::launch_walk<T, 4, 1, chunk::kGated, 2, false>(a, n_seqs, stream);
-    else chunk::launch_walk<T, 1, 4, chunk::kGated, 2, false>(a, n_seqs, stream);
+    // Wide blocks share the loads of a chunk's keys and queries and its denominators, narrow ones give more blocks, whose four or two warps
+    // split the keys.  By the heads that are walked at once for the longest sequence's time (or, with many single tokens beside it, by all
+    // there are), us of the whole call with 16 columns and four warps a group of them / 32, four / 64, two / 32, two / 64, one: one prompt of 1,531 tokens
+    // of 16 heads 93 / 114 / 161 / 122 / 294, 2 x 512 of 16 heads 52 / 50 / 66 / 52 / 112, 2,048 beside 60 single ones 386 / 220 / 271 / 234 / 497, 4 x 512
+    // 91 / 87 / 71 / 71 / 120, 3 x 512 of 32 heads 132 / 126 / 124 / 110 / 142, 4 x 512 of 32 heads 183 / 163 / 128 / 128 / 120, 8 x 512 - / 285 / 247 / 243 / 230.
+    using namespace chunk;
+    const double busy = (double)n_heads * value_dim / kKeys * std::max((double)n_rows / max_tokens, n_seqs / 30.0);
+    const bool by32 = value_dim % 32 == 0, by64 = value_dim % 64 == 0;
+    if (busy > 110 && by64) launch_walk<T, 4, 1, kGated, 2, false>(a, n_seqs, stream);
+    else if (busy > 80 && by32) launch_walk<T, 2, 2, kGated, 2, false>(a, n_seqs, stream);
+    else if (busy > 40 && by64) launch_walk<T, 4, 2, kGated, 2, false>(a, n_seqs, stream);
+    else if (busy > 16 && by32) launch_walk<T, 2, 4, kGated, 2, false>(a, n_seqs, stream);
+    else launch_walk<T, 1, 4, kGated, 2, false>(a, n_seqs, stream);
     return thn_launch_status("mlstm_chunks");
 }
