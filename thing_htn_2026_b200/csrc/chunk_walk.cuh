@@ -125,6 +125,12 @@ __device__ __forceinline__ void copy_bulk(void* smem, const void* gmem, uint32_t
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(shared_addr(smem)), "l"(gmem), "r"(bytes), "r"(shared_addr(bar)) : "memory");
 }
+// The other way; the thread that starts such stores waits for them with stores_wait.
+__device__ __forceinline__ void store_bulk(void* gmem, const void* smem, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\ncp.async.bulk.commit_group;"
+                 ::"l"(gmem), "r"(shared_addr(smem)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void stores_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // The barrier hears of this thread's copies of 16 bytes when they have landed.
 __device__ __forceinline__ void copies_arrive(uint64_t* bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(shared_addr(bar)) : "memory");

@@ -422,58 +422,68 @@ __global__ void __launch_bounds__(128) delta_prepare_chunks_kernel(
 //     u_i = b_i (v_i - exp(c_i) S0^T k_i) - b_i sum_{j < i} D_ij (k_i . k_j) u_j
 //
 // so with A_ij = b_i D_ij k_i . k_j below the diagonal and T = (I + A)^-1 the corrections are U - W S0 with
-// U = T diag(b) V and W = T diag(b exp(c)) K.  One block per (chunk, head, sequence): four warps take the
-// products with the keys (16 tokens of q k^T or k k^T each), the first solves for T, and each takes 32 columns
-// of W and U.  Products on the tensor cores in three parts, T in float32 multiply-adds; the log decays are
+// U = T diag(b) V and W = T diag(b exp(c)) K.  One block per (chunk, HEADS neighbouring heads that share a key head, sequence): the
+// products q k^T and k k^T, which the heads share, go through shared memory; then four warps a head: the first solves for T, each takes 32
+// columns of W and U.  Products on the tensor cores in three parts, T in float32 multiply-adds; the log decays are
 // summed in double, so that differences of large sums stay exact.  Out: U in place of the values, W and
 // D_ij q_i . k_j as planes, the scalars.
 // T is zero above the diagonal, but a product multiplies there too, and zero times a NaN is NaN.  So that tokens ahead
 // of one with a key, b or decay that is not finite do not see it, its key and factors are zero in the products, and its
 // row of U is NaN (the walk spreads that to the tokens behind it); a value that is not finite is zero in the products, and
 // its own entry of U is NaN.
-constexpr int kChunkThreads = 128;
+// Bound by the products (1,152 a head of m16n8k16 in its own block, 864 in one of two) and by what it writes: a fragment stored as it lies is
+// 16 bytes a row, so W goes out through shared memory, over the queries and keys, by bulk copies.  2,048 tokens of 16 heads on B200: 57 us with a
+// block per head and fragments stored one by one (of 30,000 clocks a block the products q k^T and k k^T took 5,500, W and U 9,000 each), 37 now.
 constexpr int kSquare = chunk::kTokens + 8;            // row of a 32 x 32 matrix of floats
+constexpr int kDotRow = chunk::kTokens + 4;
 constexpr int kValueRow = 128 + 4;
 
-__global__ void __launch_bounds__(kChunkThreads) delta_chunk_kernel(
+// Shared memory, in bytes: queries and keys (planes), and a head's values, square, factors and log decays.
+constexpr int kChunkKeyBytes = 3 * chunk::kTokens * chunk::kKeyRow * 2;
+constexpr int kChunkHeadBytes = chunk::kTokens * (kValueRow + kSquare + 4) * 4;
+constexpr int delta_chunk_bytes(int heads) { return 2 * kChunkKeyBytes + heads * kChunkHeadBytes; }
+
+template <int HEADS>
+__global__ void __launch_bounds__(128 * HEADS, HEADS == 2 ? 2 : 3) delta_chunk_kernel(
     float* __restrict__ values, __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ scores, float4* __restrict__ scalars,
     const __nv_bfloat16* __restrict__ planes, const float* __restrict__ beta, const float* __restrict__ decay,
     const int* __restrict__ cu_seqlens, int n_rows, DeltaShape s) {
     pdl_launch_dependents();
     pdl_wait();
-    constexpr int C = chunk::kTokens, kPlane = C * chunk::kKeyRow;
+    constexpr int C = chunk::kTokens, kPlane = C * chunk::kKeyRow, kThreads = 128 * HEADS;
     extern __shared__ __align__(16) unsigned char chunk_mem[];
-    __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(chunk_mem);      // [3][C][kKeyRow]
-    __nv_bfloat16* k_s = q_s + 3 * kPlane;                                 // [3][C][kKeyRow]
-    float* v_s = reinterpret_cast<float*>(k_s + 3 * kPlane);               // [C][kValueRow]: 128 columns of the values
-    float* a_s = v_s + C * kValueRow;                                      // [C][kSquare]: A, then T diag(b)
-    float* e_s = a_s + C * kSquare;                                        // [C] exp(c)
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int own = threadIdx.x / 128, tid = threadIdx.x % 128, warp = tid >> 5;      // which of the block's heads, and the place among its threads
+    __nv_bfloat16* q_s = reinterpret_cast<__nv_bfloat16*>(chunk_mem);                          // [3][C][kKeyRow]; then the products, then W of the first head
+    __nv_bfloat16* k_s = reinterpret_cast<__nv_bfloat16*>(chunk_mem + kChunkKeyBytes);         // [3][C][kKeyRow]; then W of the second
+    float* qk_s = reinterpret_cast<float*>(chunk_mem);                                         // [C][kDotRow] q_i . k_j
+    float* kk_s = qk_s + C * kDotRow;                                                          // [C][kDotRow] k_i . k_j
+    float* v_s = reinterpret_cast<float*>(chunk_mem + 2 * kChunkKeyBytes + own * kChunkHeadBytes);
+    float* a_s = v_s + C * kValueRow;                                      // (v_s: [C][kValueRow], 128 columns) [C][kSquare]: A, then T diag(b)
+    double* c_s = reinterpret_cast<double*>(a_s + C * kSquare);            // [C]
+    float* e_s = reinterpret_cast<float*>(c_s + C);                        // [C] exp(c)
     float* b_s = e_s + C;                                                  // [C]
-    double* c_s = reinterpret_cast<double*>(b_s + C);                      // [C]
-    // bit i: token i has a key, b or decay that is not finite (in the padding of A's first row: with a static word the kernel took
-    // 61.8 us in place of 56.8 for 2,048 tokens of 16 heads)
-    unsigned* lost_s = reinterpret_cast<unsigned*>(a_s + C);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-    const int head = blockIdx.y, seq = blockIdx.z, unit = head / (s.n_heads / s.n_kv);
+    const int first_head = blockIdx.y * HEADS, head = first_head + own, seq = blockIdx.z, unit = first_head / (s.n_heads / s.n_kv);
     const int begin = cu_seqlens[seq], row0 = begin + blockIdx.x * C, n_here = min(C, cu_seqlens[seq + 1] - row0);
     if (n_here <= 0) return;
 
     const long long plane = (long long)n_rows * chunk::kKeyRow, at0 = (long long)row0 * chunk::kKeyRow;
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
-        chunk::copy_rows<chunk::kKeyRow, kChunkThreads>(q_s + p * kPlane, planes + ((long long)unit * 3 + p) * plane + at0, n_here);
-        chunk::copy_rows<chunk::kKeyRow, kChunkThreads>(k_s + p * kPlane, planes + ((long long)(s.n_kv + unit) * 3 + p) * plane + at0, n_here);
+        chunk::copy_rows<chunk::kKeyRow, kThreads>(q_s + p * kPlane, planes + ((long long)unit * 3 + p) * plane + at0, n_here);
+        chunk::copy_rows<chunk::kKeyRow, kThreads>(k_s + p * kPlane, planes + ((long long)(s.n_kv + unit) * 3 + p) * plane + at0, n_here);
     }
+    chunk::copy_commit();
     float* own_values = values + ((size_t)head * n_rows + row0) * s.dv;
     auto fetch_values = [&](int e0) {
-        for (int e = tid; e < C * 32; e += kChunkThreads) {
+        for (int e = tid; e < C * 32; e += 128) {
             const int i = e / 32, c = e % 32 * 4;
             const bool there = i < n_here && e0 + c < s.dv;
             chunk::copy16(v_s + i * kValueRow + c, own_values + (there ? (size_t)i * s.dv + e0 + c : 0), there);
         }
+        chunk::copy_commit();
     };
     fetch_values(0);
-    chunk::copy_commit();
     if (warp == 0) {
         const size_t at = (size_t)(row0 + lane) * s.n_heads + head;
         const bool there = lane < n_here;
@@ -481,49 +491,83 @@ __global__ void __launch_bounds__(kChunkThreads) delta_chunk_kernel(
         const double c_last = __shfl_sync(0xffffffffu, c, n_here - 1);
         const float b = there ? beta[at] : 0.f;
         const bool is_lost = isnan(c) || !chunk::finite(b);
-        const unsigned all_lost = __ballot_sync(0xffffffffu, is_lost);
-        if (lane == 0) *lost_s = all_lost;
         c_s[lane] = c;
         e_s[lane] = is_lost ? 0.f : expf((float)c);
-        b_s[lane] = is_lost ? 0.f : b;
+        b_s[lane] = is_lost ? chunk::not_a_number() : b;      // (zero once every warp knows)
         if (there) scalars[(size_t)head * n_rows + row0 + lane] = make_float4(e_s[lane], 0.f, expf((float)(c_last - c)), 0.f);
     }
-    chunk::copy_wait_all();
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");          // queries and keys
     __syncthreads();
-    {
-        const int m_tile = warp & 1;
-        const bool of_keys = warp >= 2;
-        float dot[4][4];
-        chunk::dots<3>(dot, of_keys ? k_s : q_s, k_s, m_tile, lane);
-        const long long score_plane = (long long)n_rows * chunk::kScoreRow;
-        __nv_bfloat16* score_dst = scores + head * 3 * score_plane + (long long)row0 * chunk::kScoreRow;
-        float squares[2] = {0.f, 0.f};           // k_i . k_i, in the lanes that have it
+    // q k^T and k k^T: rows 0-15 by columns 0-15, rows 16-31 by columns 0-15 and 16-31, of either
+    constexpr int kTasks = 6, kTurns = (kTasks + kThreads / 32 - 1) / (kThreads / 32);
+    float dot[kTurns][2][4];
 #pragma unroll
-        for (int n = 0; n < 4; ++n)
+    for (int turn = 0; turn < kTurns; ++turn) {
+        const int task = (threadIdx.x >> 5) + turn * (kThreads / 32), part = task % 3, m_tile = part > 0, pair = part > 1;
+        if (task >= kTasks) break;
+        const __nv_bfloat16* xa = (task >= 3 ? k_s : q_s) + 16 * m_tile * chunk::kKeyRow + chunk::a_tile(lane, chunk::kKeyRow);
+        const __nv_bfloat16* yb = k_s + 16 * pair * chunk::kKeyRow + chunk::b_tile(lane, chunk::kKeyRow);
+        chunk::clear(dot[turn]);
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                const int i = 16 * m_tile + g + 8 * half, j = 8 * n + 2 * t;
-                float x[2];
-                if ((i & ~1) == j) squares[half] = i & 1 ? dot[n][2 * half + 1] : dot[n][2 * half];
+        for (int j = 0; j < chunk::kKeys / 16; ++j) {
+            chunk::Parts p;
 #pragma unroll
-                for (int o = 0; o < 2; ++o)
-                    x[o] = j + o <= i ? expf((float)(c_s[i] - c_s[j + o])) * dot[n][2 * half + o] : 0.f;
-                if (of_keys)
-                    *reinterpret_cast<float2*>(a_s + i * kSquare + j) = make_float2(j < i ? b_s[i] * x[0] : 0.f, j + 1 < i ? b_s[i] * x[1] : 0.f);
-                else if (i < n_here)
-                    chunk::store_split(score_dst + (long long)i * chunk::kScoreRow + j, score_plane, x[0], x[1]);
-            }
-        if (of_keys) {
+            for (int i = 0; i < 3; ++i) chunk::load_matrices(p.part[i], xa + i * kPlane + 16 * j);
+            const chunk::Columns<3> c[1] = {chunk::columns_of<3>(yb + 16 * j, kPlane)};
+            float large[2][4], small[2][4];
+            chunk::clear(large);
+            chunk::clear(small);
+            chunk::multiply(large, small, p, c);
 #pragma unroll
-            for (int half = 0; half < 2; ++half)
-                if (!chunk::finite(squares[half])) atomicOr(lost_s, 1u << (16 * m_tile + g + 8 * half));
+            for (int o = 0; o < 2; ++o)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) dot[turn][o][i] += chunk::joined(large[o][i], small[o][i]);
+        }
+    }
+    __syncthreads();                           // nobody reads the queries any more
+#pragma unroll
+    for (int turn = 0; turn < kTurns; ++turn) {
+        const int task = (threadIdx.x >> 5) + turn * (kThreads / 32), part = task % 3, m_tile = part > 0, pair = part > 1;
+        if (task >= kTasks) break;
+        float* dst = (task >= 3 ? kk_s : qk_s) + (16 * m_tile + g) * kDotRow + 16 * pair + 2 * t;
+#pragma unroll
+        for (int o = 0; o < 2; ++o) {
+            *reinterpret_cast<float2*>(dst + 8 * o) = make_float2(dot[turn][o][0], dot[turn][o][1]);
+            *reinterpret_cast<float2*>(dst + 8 * kDotRow + 8 * o) = make_float2(dot[turn][o][2], dot[turn][o][3]);
         }
     }
     __syncthreads();
-    const unsigned lost = *lost_s;
-    if (lost)
-        for (int e = tid; e < 3 * kPlane; e += kChunkThreads)
-            if (lost >> (e % kPlane / chunk::kKeyRow) & 1) k_s[e] = __float2bfloat16_rn(0.f);
+    // bit i: token i's key, or its b or decay, is not finite
+    const unsigned lost_key = __ballot_sync(0xffffffffu, !chunk::finite(kk_s[lane * kDotRow + lane]));
+    const unsigned lost = lost_key | __ballot_sync(0xffffffffu, !chunk::finite(b_s[lane]));
+    {
+        // eight neighbouring entries of a row a thread: G = D q k^T in planes, A
+        const int i = tid >> 2, j0 = tid % 4 * 8;
+        float y[8], a[8];
+        const float b = lost >> i & 1 ? 0.f : b_s[i];
+#pragma unroll
+        for (int o = 0; o < 8; ++o) {
+            const int j = j0 + o;
+            const float d = j <= i ? expf((float)(c_s[i] - c_s[j])) : 0.f;
+            y[o] = j <= i ? d * qk_s[i * kDotRow + j] : 0.f;
+            a[o] = j < i ? b * (d * kk_s[i * kDotRow + j]) : 0.f;
+        }
+        *reinterpret_cast<float4*>(a_s + i * kSquare + j0) = make_float4(a[0], a[1], a[2], a[3]);
+        *reinterpret_cast<float4*>(a_s + i * kSquare + j0 + 4) = make_float4(a[4], a[5], a[6], a[7]);
+        if (i < n_here) {
+            const long long score_plane = (long long)n_rows * chunk::kScoreRow;
+            __nv_bfloat16* dst = scores + head * 3 * score_plane + (long long)(row0 + i) * chunk::kScoreRow + j0;
+            const chunk::Split x[4] = {chunk::split(y[0], y[1]), chunk::split(y[2], y[3]), chunk::split(y[4], y[5]), chunk::split(y[6], y[7])};
+#pragma unroll
+            for (int p = 0; p < 3; ++p)
+                *reinterpret_cast<uint4*>(dst + p * score_plane) = make_uint4(x[0].part[p], x[1].part[p], x[2].part[p], x[3].part[p]);
+        }
+    }
+    chunk::copy_wait_all();
+    __syncthreads();
+    if (lost_key)
+        for (int e = threadIdx.x; e < 3 * kPlane; e += kThreads)
+            if (lost_key >> (e % kPlane / chunk::kKeyRow) & 1) k_s[e] = __float2bfloat16_rn(0.f);
     if (warp == 0) {
         // (I + A)^-1 column by column: lane j holds column j
         float column[C];
@@ -541,8 +585,9 @@ __global__ void __launch_bounds__(kChunkThreads) delta_chunk_kernel(
             column[i] = (sum[0] + sum[1]) + (sum[2] + sum[3]);
         }
         __syncwarp();
+        const float b = lost >> lane & 1 ? 0.f : b_s[lane];
 #pragma unroll
-        for (int i = 0; i < C; ++i) a_s[i * kSquare + lane] = column[i] * b_s[lane];
+        for (int i = 0; i < C; ++i) a_s[i * kSquare + lane] = column[i] * b;
     }
     __syncthreads();
     // T diag(b) (exp(c) for W) as A operands: tokens by tokens; [0]: rows 0-15, [1], [2]: rows 16-31 by tokens 0-15, 16-31
@@ -556,71 +601,91 @@ __global__ void __launch_bounds__(kChunkThreads) delta_chunk_kernel(
         }
         return chunk::parts_of(x[0], x[1], x[2], x[3]);
     };
-    auto by_rows = [&](const chunk::Parts (&a)[3], auto&& columns, auto&& store) {
+    // sum[m][o]: rows 16 m .. by groups of columns n + o of this warp's 32
+    auto two_groups = [&](float (&sum)[2][2][4], const chunk::Parts (&a)[3], int n, auto&& columns) {
+        chunk::clear(sum[0]);
+        chunk::clear(sum[1]);
 #pragma unroll
-        for (int n = 0; n < 4; n += 2) {
-            float sum[2][2][4];
-            chunk::clear(sum[0]);
-            chunk::clear(sum[1]);
+        for (int j = 0; j < 2; ++j) {
+            const chunk::Columns<3> b[1] = {columns(n, j)};
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const chunk::Columns<3> b[1] = {columns(n, j)};
+            for (int m = j; m < 2; ++m) {
+                float large[2][4], small[2][4];
+                chunk::clear(large);
+                chunk::clear(small);
+                chunk::multiply(large, small, a[m + j], b);
 #pragma unroll
-                for (int m = j; m < 2; ++m) {
-                    float large[2][4], small[2][4];
-                    chunk::clear(large);
-                    chunk::clear(small);
-                    chunk::multiply(large, small, a[m + j], b);
+                for (int o = 0; o < 2; ++o)
 #pragma unroll
-                    for (int o = 0; o < 2; ++o)
-#pragma unroll
-                        for (int i = 0; i < 4; ++i) sum[m][o][i] += chunk::joined(large[o][i], small[o][i]);
-                }
+                    for (int i = 0; i < 4; ++i) sum[m][o][i] += chunk::joined(large[o][i], small[o][i]);
             }
+        }
+    };
+    {
+        const chunk::Parts a[3] = {operand(0, 0, e_s), operand(1, 0, e_s), operand(1, 1, e_s)};
+        float sum[2][2][2][4];
+#pragma unroll
+        for (int n = 0; n < 4; n += 2)
+            two_groups(sum[n / 2], a, n, [&](int n, int j) {
+                return chunk::columns_transposed<3>(k_s + chunk::a_tile(lane, chunk::kKeyRow) + 16 * j * chunk::kKeyRow + 32 * warp + 8 * n, kPlane);
+            });
+        __syncthreads();                       // nobody reads queries or keys any more
+        __nv_bfloat16* w_s = own == 0 ? q_s : k_s;
+#pragma unroll
+        for (int n = 0; n < 4; n += 2)
 #pragma unroll
             for (int m = 0; m < 2; ++m)
 #pragma unroll
                 for (int o = 0; o < 2; ++o)
 #pragma unroll
                     for (int half = 0; half < 2; ++half)
-                        if (16 * m + g + 8 * half < n_here)
-                            store(16 * m + g + 8 * half, 32 * warp + 8 * (n + o) + 2 * t, sum[m][o][2 * half], sum[m][o][2 * half + 1]);
+                        chunk::store_split(w_s + (16 * m + g + 8 * half) * chunk::kKeyRow + 32 * warp + 8 * (n + o) + 2 * t, kPlane,
+                                           sum[n / 2][m][o][2 * half], sum[n / 2][m][o][2 * half + 1]);
+        chunk::writes_ahead_of_copies();
+        __syncthreads();
+        if (threadIdx.x < 3 * HEADS) {
+            const int p = threadIdx.x % 3, h = threadIdx.x / 3;
+            const __nv_bfloat16* src = (h == 0 ? q_s : k_s) + p * kPlane;
+            chunk::store_bulk(w + ((long long)(first_head + h) * 3 + p) * plane + at0, src, n_here * chunk::kKeyRow * 2);
         }
-    };
-    {
-        const chunk::Parts a[3] = {operand(0, 0, e_s), operand(1, 0, e_s), operand(1, 1, e_s)};
-        __nv_bfloat16* dst = w + head * 3 * plane + at0;
-        by_rows(a, [&](int n, int j) { return chunk::columns_transposed<3>(k_s + chunk::a_tile(lane, chunk::kKeyRow) + 16 * j * chunk::kKeyRow + 32 * warp + 8 * n, kPlane); },
-                [&](int i, int d, float x, float y) { chunk::store_split(dst + (long long)i * chunk::kKeyRow + d, plane, x, y); });
     }
     const chunk::Parts a[3] = {operand(0, 0, nullptr), operand(1, 0, nullptr), operand(1, 1, nullptr)};
     for (int e0 = 0; e0 < s.dv; e0 += 128) {
         if (e0 > 0) {
             __syncthreads();
             fetch_values(e0);
-            chunk::copy_commit();
             chunk::copy_wait_all();
             __syncthreads();
         }
         uint32_t seen = 0;                      // values that are not finite
-        by_rows(a,
-                [&](int n, int j) {
-                    chunk::Columns<3> b;
 #pragma unroll
-                    for (int o = 0; o < 2; ++o)
+        for (int n = 0; n < 4; n += 2) {
+            float sum[2][2][4];
+            two_groups(sum, a, n, [&](int n, int j) {
+                chunk::Columns<3> b;
 #pragma unroll
-                        for (int half = 0; half < 2; ++half) {
-                            const float* p = v_s + (16 * j + 8 * half + 2 * t) * kValueRow + 32 * warp + 8 * (n + o) + g;
-                            const chunk::Split x = chunk::split(p[0], p[kValueRow]);
-                            seen |= chunk::not_finite(x.part[0]);
+                for (int o = 0; o < 2; ++o)
 #pragma unroll
-                            for (int i = 0; i < 3; ++i) b.part[i][2 * o + half] = x.part[i];
-                        }
-                    return b;
-                },
-                [&](int i, int d, float x, float y) {
-                    if (e0 + d < s.dv) *reinterpret_cast<float2*>(own_values + (size_t)i * s.dv + e0 + d) = make_float2(x, y);
-                });
+                    for (int half = 0; half < 2; ++half) {
+                        const float* p = v_s + (16 * j + 8 * half + 2 * t) * kValueRow + 32 * warp + 8 * (n + o) + g;
+                        const chunk::Split x = chunk::split(p[0], p[kValueRow]);
+                        seen |= chunk::not_finite(x.part[0]);
+#pragma unroll
+                        for (int i = 0; i < 3; ++i) b.part[i][2 * o + half] = x.part[i];
+                    }
+                return b;
+            });
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+                for (int o = 0; o < 2; ++o)
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) {
+                        const int i = 16 * m + g + 8 * half, d = e0 + 32 * warp + 8 * (n + o) + 2 * t;
+                        if (i < n_here && d < s.dv)
+                            *reinterpret_cast<float2*>(own_values + (size_t)i * s.dv + d) = make_float2(sum[m][o][2 * half], sum[m][o][2 * half + 1]);
+                    }
+        }
         if (lost || __any_sync(0xffffffffu, seen != 0)) {
             // a row of U per lane, column by column: without the values that are not finite
             __syncwarp();
@@ -634,9 +699,8 @@ __global__ void __launch_bounds__(kChunkThreads) delta_chunk_kernel(
             }
         }
     }
+    if (threadIdx.x < 3 * HEADS) chunk::stores_wait();
 }
-constexpr size_t kDeltaChunkBytes = (size_t)6 * chunk::kTokens * chunk::kKeyRow * 2 +
-                                    (chunk::kTokens * kValueRow + chunk::kTokens * kSquare + 4 * chunk::kTokens) * sizeof(float);
 
 // After a step: the raw projections of the step's last taps - 1 positions go into the ring
 // (position p at p mod taps).  A thread per channel (one block per sequence took 20 us for 3,072 channels, this 3);
@@ -890,8 +954,8 @@ THN_API long long thn_delta_chunks_scratch_bytes(int n_rows, int n_heads, int n_
 // prepare and recurrence of a step chunk by chunk, the state carried in float32: bfloat16 rows, four taps, keys of
 // 128, values of whole groups of 16 columns; max_tokens: the most rows of a sequence.  scratch:
 // thn_delta_chunks_scratch_bytes(...), 16-byte aligned, as the state and the taps must be; the rows and the
-// ring are read in pieces of 8 bytes.  One prompt of 2,048 tokens, 16 heads of 128 x 128, on B200: 206 us
-// against 658 token by token; 32 heads 321 / 839; 8 x 512 tokens of 16 heads 324 / 571; steps of long and short sequences beside
+// ring are read in pieces of 8 bytes.  One prompt of 2,048 tokens, 16 heads of 128 x 128, on B200: 187 us
+// against 658 token by token; 32 heads 308 / 839; 8 x 512 tokens of 16 heads 298 / 571; steps of long and short sequences beside
 // the rule in ops (_DELTA_COST).  The read-out's error
 // against 64 bits is 1.37e-7 to 1.41e-7 (1.33e-7 to 1.36e-7 token by token), the state's 1.2e-7 to 1.4e-7 (1.1e-7 to 1.3e-7).
 THN_API int thn_delta_chunks(float* o, float* state, void* scratch, const void* proj, const float* conv_w, const float* a_log,
@@ -920,9 +984,16 @@ THN_API int thn_delta_chunks(float* o, float* state, void* scratch, const void* 
     thn_launch(delta_prepare_chunks_kernel, dim3((items + 127) / 128, (n_rows + kRunRows - 1) / kRunRows), 128, 0, stream, planes,
                values, beta, decay, (const __nv_bfloat16*)proj, conv_w, a_log, dt_bias, (const __nv_bfloat16*)ring, row_slot, row_pos,
                seq_lens, n_rows, s, unit_eps);
-    cudaFuncSetAttribute(delta_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDeltaChunkBytes);
-    thn_launch(delta_chunk_kernel, dim3((max_tokens + chunk::kTokens - 1) / chunk::kTokens, n_heads, n_seqs), kChunkThreads,
-               kDeltaChunkBytes, stream, values, w, scores, scalars, planes, beta, decay, cu_seqlens, n_rows, s);
+    const dim3 chunks((max_tokens + chunk::kTokens - 1) / chunk::kTokens, n_heads, n_seqs);
+    if (n_heads / n_kv % 2 == 0) {
+        cudaFuncSetAttribute(delta_chunk_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, delta_chunk_bytes(2));
+        thn_launch(delta_chunk_kernel<2>, dim3(chunks.x, n_heads / 2, n_seqs), 256, delta_chunk_bytes(2), stream, values, w, scores, scalars, planes,
+                   beta, decay, cu_seqlens, n_rows, s);
+    } else {
+        cudaFuncSetAttribute(delta_chunk_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, delta_chunk_bytes(1));
+        thn_launch(delta_chunk_kernel<1>, chunks, 128, delta_chunk_bytes(1), stream, values, w, scores, scalars, planes, beta, decay, cu_seqlens,
+                   n_rows, s);
+    }
     chunk::WalkArgs a{};
     a.err = err;
     a.o = o; a.state = state;
