@@ -23,6 +23,7 @@
 #include <math.h>
 
 #include "chunk_walk.cuh"
+#include "conv_run.cuh"
 #include "common.cuh"
 
 namespace {
@@ -326,7 +327,7 @@ constexpr size_t recurrence_smem() {
 // kRunRows rows with the raw inputs ahead of a row in registers, so a warp holds one key head's 128 channels
 // and its norm is a sum over the warp.  The unit queries and keys go out in three planes of bfloat16
 // (chunk_walk.cuh), [q | k][head][plane][rows][kKeyRow], the values as float32 [heads][rows][dv].
-// 2,048 rows of 16 heads on B200: 24 us, 54 with a block per row, a thread per channel and 2-byte accesses.
+// 2,048 rows of 16 heads on B200: 18 us (conv_run.cuh), 54 with a block per row, a thread per channel and 2-byte accesses.
 constexpr int kRunRows = 8;
 constexpr int kRunTaps = 4;
 
@@ -351,58 +352,22 @@ __global__ void __launch_bounds__(128) delta_prepare_chunks_kernel(
         }
         return;
     }
-    float4 w[4];
+    float w[4][kRunTaps];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4*>(conv_w + (size_t)(c + i) * kRunTaps);
+    for (int i = 0; i < 4; ++i) {
+        const float4 v = *reinterpret_cast<const float4*>(conv_w + (size_t)(c + i) * kRunTaps);
+        w[i][0] = v.x; w[i][1] = v.y; w[i][2] = v.z; w[i][3] = v.w;
+    }
     pdl_wait();
-    const __nv_bfloat16* src = proj + (size_t)first * s.proj_width + c;
-    uint2 raw[kRunRows + kRunTaps - 1];       // raw[j]: the row j - 3 rows after `first`
-#pragma unroll
-    for (int j = 0; j < kRunRows + kRunTaps - 1; ++j) {
-        const int back = kRunTaps - 1 - j;
-        raw[j] = back <= first && -back < n_here ? *reinterpret_cast<const uint2*>(src - (long long)back * s.proj_width) : make_uint2(0, 0);
-    }
-    int slot[kRunRows], pos[kRunRows], local[kRunRows];
-#pragma unroll
-    for (int r = 0; r < kRunRows; ++r) {
-        slot[r] = row_slot[first + min(r, n_here - 1)];
-        pos[r] = row_pos[first + min(r, n_here - 1)];
-    }
-#pragma unroll
-    for (int r = 0; r < kRunRows; ++r) local[r] = pos[r] - seq_lens[slot[r]];
     const bool is_value = c >= 2 * QK;                 // (a warp's channels are all one key head's, or all values)
     const double norm_scale = c < QK ? (double)s.dk : 1.0;
     const long long plane = (long long)n_rows * chunk::kKeyRow;
     __nv_bfloat16* key_dst = planes + (c / chunk::kKeys) * 3 * plane + (long long)first * chunk::kKeyRow + c % chunk::kKeys;
     const int vc = c - 2 * QK;
     float* value_dst = values + ((size_t)(is_value ? vc / s.dv : 0) * n_rows + first) * s.dv + (is_value ? vc % s.dv : 0);
-#pragma unroll
-    for (int r = 0; r < kRunRows; ++r) {
-        if (r >= n_here) break;
-        uint2 in[kRunTaps];
-#pragma unroll
-        for (int j = 0; j < kRunTaps; ++j) in[j] = raw[r + j];
-        if (local[r] < kRunTaps - 1) {
-#pragma unroll
-            for (int back = 1; back < kRunTaps; ++back) {
-                if (back <= local[r]) continue;
-                in[kRunTaps - 1 - back] = back > pos[r] ? make_uint2(0, 0)           // before the sequence's start
-                    : *reinterpret_cast<const uint2*>(ring + ((size_t)slot[r] * kRunTaps + (pos[r] - back) % kRunTaps) * C + c);
-            }
-        }
-        float y[4];
-        const float* taps[4] = {&w[0].x, &w[1].x, &w[2].x, &w[3].x};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float acc = 0.f;
-#pragma unroll
-            for (int j = 0; j < kRunTaps; ++j) {
-                if (kRunTaps - 1 - j > pos[r]) continue;
-                const uint32_t two = i < 2 ? in[j].x : in[j].y;
-                acc = fmaf(taps[i][j], i & 1 ? chunk::high_half(two) : chunk::low_half(two), acc);
-            }
-            y[i] = silu_f(acc);
-        }
+    const float none[4] = {0.f, 0.f, 0.f, 0.f};
+    const conv_run::Source source{proj + (size_t)first * s.proj_width + c, s.proj_width, ring + c, C, row_slot, row_pos, seq_lens};
+    conv_run::run<kRunRows>(source, first, n_here, w, none, [&](int r, const float (&y)[4]) {
         if (is_value) {
             *reinterpret_cast<float4*>(value_dst + (size_t)r * s.dv) = make_float4(y[0], y[1], y[2], y[3]);
         } else {
@@ -413,7 +378,7 @@ __global__ void __launch_bounds__(128) delta_prepare_chunks_kernel(
             for (int p = 0; p < 3; ++p)
                 *reinterpret_cast<uint2*>(key_dst + p * plane + (long long)r * chunk::kKeyRow) = make_uint2(lo.part[p], hi.part[p]);
         }
-    }
+    });
 }
 
 // What a chunk of 32 tokens needs beside the state (chunk_walk.cuh), for one head.  With c_i the sum of

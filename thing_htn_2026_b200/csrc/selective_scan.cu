@@ -29,6 +29,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "conv_run.cuh"
 
 namespace {
 
@@ -85,55 +86,13 @@ __global__ void __launch_bounds__(128) causal_conv_vec_kernel(
         b[i] = bias ? bias[c + i] : 0.f;
     }
     pdl_wait();
-    const __nv_bfloat16* src = proj + (size_t)first * proj_width + offset + c;
-    // raw[j]: the row j - 3 rows after `first`
-    uint2 raw[kConvRows + kConvTaps - 1];
-#pragma unroll
-    for (int j = 0; j < kConvRows + kConvTaps - 1; ++j) {
-        const int back = kConvTaps - 1 - j;
-        raw[j] = back <= first && -back < n_here ? *reinterpret_cast<const uint2*>(src - (long long)back * proj_width)
-                                                 : make_uint2(0, 0);
-    }
-    int slot[kConvRows], pos[kConvRows], local[kConvRows];
-#pragma unroll
-    for (int t = 0; t < kConvRows; ++t) {
-        const int row = first + min(t, n_here - 1);
-        slot[t] = row_slot[row];
-        pos[t] = row_pos[row];
-    }
-#pragma unroll
-    for (int t = 0; t < kConvRows; ++t) local[t] = pos[t] - seq_lens[slot[t]];   // its index among its sequence's rows of this step
     __nv_bfloat16* dst = out + (size_t)first * channels + c;
-#pragma unroll
-    for (int t = 0; t < kConvRows; ++t) {
-        if (t >= n_here) break;
-        uint2 in[kConvTaps];
-#pragma unroll
-        for (int j = 0; j < kConvTaps; ++j) in[j] = raw[t + j];
-        if (local[t] < kConvTaps - 1) {
-#pragma unroll
-            for (int back = 1; back < kConvTaps; ++back) {
-                if (back <= local[t]) continue;
-                in[kConvTaps - 1 - back] = back > pos[t] ? make_uint2(0, 0)          // before the sequence's start
-                    : *reinterpret_cast<const uint2*>(ring + ((size_t)slot[t] * kConvTaps + (pos[t] - back) % kConvTaps) * channels + c);
-            }
-        }
-        float acc[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[i] = b[i];
-#pragma unroll
-        for (int j = 0; j < kConvTaps; ++j) {
-            if (kConvTaps - 1 - j > pos[t]) continue;
-            acc[0] += w[0][j] * __uint_as_float(in[j].x << 16);
-            acc[1] += w[1][j] * __uint_as_float(in[j].x & 0xffff0000u);
-            acc[2] += w[2][j] * __uint_as_float(in[j].y << 16);
-            acc[3] += w[3][j] * __uint_as_float(in[j].y & 0xffff0000u);
-        }
-        const __nv_bfloat162 lo = __floats2bfloat162_rn(silu_of<__nv_bfloat16>(acc[0]), silu_of<__nv_bfloat16>(acc[1]));
-        const __nv_bfloat162 hi = __floats2bfloat162_rn(silu_of<__nv_bfloat16>(acc[2]), silu_of<__nv_bfloat16>(acc[3]));
+    const conv_run::Source source{proj + (size_t)first * proj_width + offset + c, proj_width, ring + c, channels, row_slot, row_pos, seq_lens};
+    conv_run::run<kConvRows>(source, first, n_here, w, b, [&](int t, const float (&y)[4]) {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(y[0], y[1]), hi = __floats2bfloat162_rn(y[2], y[3]);
         *reinterpret_cast<uint2*>(dst + (size_t)t * channels) =
             make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-    }
+    });
 }
 
 template <typename T>

@@ -24,6 +24,7 @@
 #include <math.h>
 
 #include "chunk_walk.cuh"
+#include "conv_run.cuh"
 #include "linear_attention.cuh"
 
 namespace {
@@ -147,7 +148,7 @@ __global__ void __launch_bounds__(kPrepareThreads) state_space_prepare_kernel(
 }
 
 // The same for the walk in chunks (bfloat16, four taps, a state of 128, whole groups of four entries): the raw inputs
-// ahead of a thread's rows are loaded together (4,096 rows of 10,240 channels on B200: 98 us, 130 above), B and C go out in three planes of bfloat16 (chunk_walk.cuh)
+// ahead of a thread's rows are loaded together (conv_run.cuh; 4,096 rows of 10,240 channels on B200: 80 us, 130 above), B and C go out in three planes of bfloat16 (chunk_walk.cuh)
 // [group][B | C][plane][rows][kKeyRow], x as [heads][rows][vdim], the step sizes as [heads][rows].
 constexpr int kChunkTaps = 4;
 
@@ -176,52 +177,13 @@ __global__ void __launch_bounds__(kPrepareThreads, 6) state_space_prepare_chunks
         b[i] = conv_b[c + i];
     }
     pdl_wait();
-    const __nv_bfloat16* src = proj + (size_t)first * proj_width + offset + c;
-    uint2 raw[kRunRows + kChunkTaps - 1];       // raw[j]: the row j - 3 rows after `first`
-#pragma unroll
-    for (int j = 0; j < kRunRows + kChunkTaps - 1; ++j) {
-        const int back = kChunkTaps - 1 - j;
-        raw[j] = back <= first && -back < n_here ? *reinterpret_cast<const uint2*>(src - (long long)back * proj_width) : make_uint2(0, 0);
-    }
-    int slot[kRunRows], pos[kRunRows], local[kRunRows];
-#pragma unroll
-    for (int r = 0; r < kRunRows; ++r) {
-        slot[r] = row_slot[first + min(r, n_here - 1)];
-        pos[r] = row_pos[first + min(r, n_here - 1)];
-    }
-#pragma unroll
-    for (int r = 0; r < kRunRows; ++r) local[r] = pos[r] - seq_lens[slot[r]];
     const bool is_value = c < shape.inner();
     const int kc = is_value ? 0 : c - shape.inner(), which = kc / (shape.n_groups * chunk::kKeys), in_part = kc % (shape.n_groups * chunk::kKeys);
     const long long plane = (long long)n_rows * chunk::kKeyRow;
     __nv_bfloat16* key_dst = planes + ((in_part / chunk::kKeys) * 2 + which) * 3 * plane + (long long)first * chunk::kKeyRow + in_part % chunk::kKeys;
     float* value_dst = values + ((size_t)(is_value ? c / shape.vdim : 0) * n_rows + first) * shape.vdim + (is_value ? c % shape.vdim : 0);
-#pragma unroll
-    for (int r = 0; r < kRunRows; ++r) {
-        if (r >= n_here) break;
-        uint2 in[kChunkTaps];
-#pragma unroll
-        for (int j = 0; j < kChunkTaps; ++j) in[j] = raw[r + j];
-        if (local[r] < kChunkTaps - 1) {
-#pragma unroll
-            for (int back = 1; back < kChunkTaps; ++back) {
-                if (back <= local[r]) continue;
-                in[kChunkTaps - 1 - back] = back > pos[r] ? make_uint2(0, 0)           // before the sequence's start
-                    : *reinterpret_cast<const uint2*>(ring + ((size_t)slot[r] * kChunkTaps + (pos[r] - back) % kChunkTaps) * C + c);
-            }
-        }
-        float y[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float acc = b[i];
-#pragma unroll
-            for (int j = 0; j < kChunkTaps; ++j) {
-                if (kChunkTaps - 1 - j > pos[r]) continue;
-                const uint32_t two = i < 2 ? in[j].x : in[j].y;
-                acc += w[i][j] * (i & 1 ? chunk::high_half(two) : chunk::low_half(two));
-            }
-            y[i] = silu_of<__nv_bfloat16>(acc);
-        }
+    const conv_run::Source source{proj + (size_t)first * proj_width + offset + c, proj_width, ring + c, C, row_slot, row_pos, seq_lens};
+    conv_run::run<kRunRows>(source, first, n_here, w, b, [&](int r, const float (&y)[4]) {
         if (is_value) {
             *reinterpret_cast<float4*>(value_dst + (size_t)r * shape.vdim) = make_float4(y[0], y[1], y[2], y[3]);
         } else {
@@ -230,7 +192,7 @@ __global__ void __launch_bounds__(kPrepareThreads, 6) state_space_prepare_chunks
             for (int p = 0; p < 3; ++p)
                 *reinterpret_cast<uint2*>(key_dst + p * plane + (long long)r * chunk::kKeyRow) = make_uint2(lo.part[p], hi.part[p]);
         }
-    }
+    });
 }
 
 // What a chunk of 32 tokens needs beside the state, for all heads of a group: G_ij = exp(c_i - c_j) t_j C_i . B_j with
