@@ -17,7 +17,7 @@
 //   selective_scan     a channel's state is held by 4 lanes (8 for states above 32; entry n by lane
 //                 n mod lanes); one block per (sequence, 64 or 32 channels) walks the sequence's tokens of the step in order;
 //                 the tokens come through shared memory, sixteen at a time in two buffers.
-//   selective_scan_walk     the same for bfloat16 prompts with states up to 32 (walk_pays): half of a block's warps walk the
+//   selective_scan_walk     the same for bfloat16 prompts with states up to 32 (walk_pays): some of a block's warps walk the
 //                 state, the others load, transform and write beside them.
 //
 // float32 after the loads: the step size with its softplus, the decay with its exponential, the
@@ -285,16 +285,18 @@ __global__ void __launch_bounds__(kScanThreads) selective_scan_kernel(
 //
 // What a token costs a channel beside its state (loads, the softplus of the step size, the silu of the gate,
 // the write) is more work than the state itself, and none of it waits for the token before.  So four warps
-// of a block walk the state and nothing else, and four others run ahead of and behind them: they load a
+// of a block walk the state and nothing else, and eight (or four) others run ahead of and behind them: they load a
 // stage of tokens, leave (step size, step size * input) and B, C in shared memory a stage ahead, and add up,
 // gate and write the read-outs of the stage before.  LANES lanes hold a channel's state, PER neighbouring
 // entries each, in pairs for the two-wide multiply-add; a lane leaves its share of a token's sum in shared
 // memory for the other warps to add.  One barrier per stage, two buffers of everything.
-// What bounds it is instruction issue (58 million warp instructions for 2,048 tokens of 4,096 channels, 16
-// entries; half of them the loads, softplus and silu) with few warps to cover latencies.  B200, against the
-// kernel above, us: one prompt of 2,048 tokens, 4,096 channels 140 / 763, 8,192 channels 201 / 770; 8 x 512
-// tokens of 4,096 162 / 447; 100 tokens 14 / 46.  (One set of warps for everything took 211 for the first; cutting
-// the tokens into segments that run side by side, twice, 134, but 230 for 8 x 512: it doubles the exponentials.)
+// Either side is a chain of latencies: with four helping warps and the walk a token at a time, one prompt of 2,048 tokens and 4,096 channels
+// took 141 us, the helpers alone 134, the walk alone 107.  The walk takes GROUP tokens' loads and exponentials ahead of their chain
+// through the state, the helpers are twice as many: 118.  What bounds it now is shared memory (three quarters of its cycles) and issue.  B200,
+// against the kernel above, us: one prompt of 2,048 tokens, 4,096 channels 118 / 763, 8,192 channels 165 / 770; 8 x 512
+// tokens of 4,096 153 / 447; 100 tokens 13 / 46.  (One set of warps for everything took 211 for the first; cutting
+// the tokens into segments that run side by side doubles the exponentials; step sizes once instead of twice in shared memory 124; loads
+// two stages ahead 137.)
 constexpr int kWalkThreads = 128;          // threads of each of the two halves of a block
 constexpr int kWalkStage = 16;
 
@@ -314,10 +316,11 @@ __device__ __forceinline__ float bounded_rate(float a) {
 
 // The barrier at which the two halves of a block meet.  They wait for one another at different places of the program, which
 // __syncthreads() does not allow: a numbered barrier of all the block's threads does.
-__device__ __forceinline__ void halves_meet() { asm volatile("barrier.cta.sync 1, %0;" ::"n"(2 * kWalkThreads) : "memory"); }
+template <int THREADS>
+__device__ __forceinline__ void halves_meet() { asm volatile("barrier.cta.sync 1, %0;" ::"n"(THREADS) : "memory"); }
 
-template <int LANES, int PER>
-__global__ void __launch_bounds__(2 * kWalkThreads) selective_scan_walk_kernel(
+template <int LANES, int PER, int HELPERS, int GROUP>
+__global__ void __launch_bounds__(kWalkThreads + HELPERS, HELPERS > 128 || LANES * PER > 16 ? 2 : 3) selective_scan_walk_kernel(
     __nv_bfloat16* __restrict__ y, float* __restrict__ state, const __nv_bfloat16* __restrict__ x,
     const float* __restrict__ dt_pre, const float* __restrict__ dt_bias, const __nv_bfloat16* __restrict__ bc, int bc_width,
     const float* __restrict__ A, const float* __restrict__ D, const __nv_bfloat16* __restrict__ z, int z_stride,
@@ -350,27 +353,51 @@ __global__ void __launch_bounds__(2 * kWalkThreads) selective_scan_walk_kernel(
             a[i] = pack2(n < n_state ? bounded_rate(A[(size_t)c * n_state + n]) : 0.f,
                          n + 1 < n_state ? bounded_rate(A[(size_t)c * n_state + n + 1]) : 0.f);
         }
-        halves_meet();                       // the first stage is in place
+        halves_meet<kWalkThreads + HELPERS>();                       // the first stage is in place
         for (int stage = 0; stage < n_stages; ++stage) {
             const int buf = stage & 1;
             // (tokens beyond the step's have a step size of zero and leave the state as it is)
 #pragma unroll
-            for (int t = 0; t < ST; ++t) {
-                const ulonglong2 step = *reinterpret_cast<const ulonglong2*>(&step_mem[buf][t][group]);
-                const ull* b = reinterpret_cast<const ull*>(bc_mem[buf][t] + lane * 2 * PER);
-                ull sum = 0;
+            for (int t0 = 0; t0 < ST; t0 += GROUP) {
+                ulonglong2 step[GROUP];
+                ull b[GROUP][2 * PAIRS], decay[GROUP][PAIRS];
 #pragma unroll
-                for (int i = 0; i < PAIRS; ++i) {
-                    float e0, e1;
-                    unpack2(mul2(step.x, a[i]), e0, e1);
-                    s[i] = fma2(pack2(decay_exp2(e0), decay_exp2(e1)), s[i], mul2(step.y, b[i]));
-                    sum = i == 0 ? mul2(s[i], b[PAIRS + i]) : fma2(s[i], b[PAIRS + i], sum);
+                for (int t = 0; t < GROUP; ++t) {
+                    step[t] = *reinterpret_cast<const ulonglong2*>(&step_mem[buf][t0 + t][group]);
+#pragma unroll
+                    for (int i = 0; i < 2 * PAIRS; i += 2) {
+                        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(bc_mem[buf][t0 + t] + lane * 2 * PER + 2 * i);
+                        b[t][i] = v.x;
+                        b[t][i + 1] = v.y;
+                    }
                 }
-                float s0, s1;
-                unpack2(sum, s0, s1);
-                share_mem[buf][t][threadIdx.x] = s0 + s1;
+                if (GROUP > 1) asm volatile("" ::: "memory");
+#pragma unroll
+                for (int t = 0; t < GROUP; ++t)
+#pragma unroll
+                    for (int i = 0; i < PAIRS; ++i) {
+                        float e0, e1;
+                        unpack2(mul2(step[t].x, a[i]), e0, e1);
+                        decay[t][i] = pack2(decay_exp2(e0), decay_exp2(e1));
+                        b[t][i] = mul2(step[t].y, b[t][i]);
+                    }
+                float part[GROUP];
+#pragma unroll
+                for (int t = 0; t < GROUP; ++t) {
+                    ull sum = 0;
+#pragma unroll
+                    for (int i = 0; i < PAIRS; ++i) {
+                        s[i] = fma2(decay[t][i], s[i], b[t][i]);
+                        sum = i == 0 ? mul2(s[i], b[t][PAIRS + i]) : fma2(s[i], b[t][PAIRS + i], sum);
+                    }
+                    float s0, s1;
+                    unpack2(sum, s0, s1);
+                    part[t] = s0 + s1;
+                }
+#pragma unroll
+                for (int t = 0; t < GROUP; ++t) share_mem[buf][t0 + t][threadIdx.x] = part[t];
             }
-            halves_meet();
+            halves_meet<kWalkThreads + HELPERS>();
         }
         if (!live) return;
 #pragma unroll
@@ -386,13 +413,13 @@ __global__ void __launch_bounds__(2 * kWalkThreads) selective_scan_walk_kernel(
 
     // the other half: a thread serves one channel and every (kWalkThreads / CH)-th token of a stage
     const int tid = threadIdx.x - kWalkThreads;
-    constexpr int STRIDE = kWalkThreads / CH, OWN = ST / STRIDE;
+    constexpr int STRIDE = HELPERS / CH, OWN = ST / STRIDE;
     const int group = tid % CH, t0 = tid / CH;
     const bool live = c0 + group < channels;
     const int c = live ? c0 + group : channels - 1;
     const float skip = D[c], bias = dt_bias[c];
-    constexpr int kShare = ST * 2 * N / kWalkThreads, kShareStep = kWalkThreads / (2 * N);
-    static_assert(ST * 2 * N % kWalkThreads == 0 && kWalkThreads % (2 * N) == 0 && ST % STRIDE == 0, "whole shares");
+    constexpr int kShare = ST * 2 * N / HELPERS, kShareStep = HELPERS / (2 * N);
+    static_assert(ST * 2 * N % HELPERS == 0 && HELPERS % (2 * N) == 0 && ST % STRIDE == 0, "whole shares");
     // this thread's column of the staged B and C: lane, B or C, entry
     const int share_col = tid % (2 * N), share_t = tid / (2 * N);
     const int share_n = share_col / (2 * PER) * PER + share_col % PER, share_which = share_col % (2 * PER) / PER;
@@ -426,7 +453,7 @@ __global__ void __launch_bounds__(2 * kWalkThreads) selective_scan_walk_kernel(
     auto transform = [&](int stage, int buf, float (&skipped_)[OWN], float (&gate_)[OWN]) {
         const int left = n_tokens - stage * ST;
 #pragma unroll
-        for (int j = 0; j < kShare; ++j) (&bc_mem[buf][0][0])[tid + j * kWalkThreads] = from_raw<T>(bc_raw[j]);
+        for (int j = 0; j < kShare; ++j) (&bc_mem[buf][0][0])[tid + j * HELPERS] = from_raw<T>(bc_raw[j]);
 #pragma unroll
         for (int j = 0; j < OWN; ++j) {
             const float d = t0 + j * STRIDE < left ? softplus_of<T>(dt_raw[j] + bias) : 0.f;
@@ -455,39 +482,49 @@ __global__ void __launch_bounds__(2 * kWalkThreads) selective_scan_walk_kernel(
     fetch(0);
     transform(0, 0, skipped[0], gate[0]);
     if (1 < n_stages) fetch(1);
-    halves_meet();
+    halves_meet<kWalkThreads + HELPERS>();
     for (int stage = 0; stage < n_stages; stage += 2) {
         // the walk is at `stage`: read out the one before, prepare the one after
         if (stage > 0) finish(stage - 1, 1, skipped[1], gate[1]);
         if (stage + 1 < n_stages) transform(stage + 1, 1, skipped[1], gate[1]);
         if (stage + 2 < n_stages) fetch(stage + 2);
-        halves_meet();
+        halves_meet<kWalkThreads + HELPERS>();
         if (stage + 1 >= n_stages) break;
         finish(stage, 0, skipped[0], gate[0]);
         if (stage + 2 < n_stages) transform(stage + 2, 0, skipped[0], gate[0]);
         if (stage + 3 < n_stages) fetch(stage + 3);
-        halves_meet();
+        halves_meet<kWalkThreads + HELPERS>();
     }
     if (n_stages & 1) finish(n_stages - 1, 0, skipped[0], gate[0]);
     else finish(n_stages - 1, 1, skipped[1], gate[1]);
 }
 
 int launch_walk(void* y, float* state, const void* x, const float* dt_pre, const float* dt_bias, const void* bc, int bc_width,
-                const float* A, const float* D, const void* z, int z_stride, const int* cu_seqlens, const int* slots, int n_seqs,
+                const float* A, const float* D, const void* z, int z_stride, const int* cu_seqlens, const int* slots, int n_rows, int n_seqs,
                 int channels, int n_state, cudaStream_t stream) {
     using T = __nv_bfloat16;
-#define THN_WALK_LAUNCH(L, P)                                                                                               \
-    thn_launch_ordered(selective_scan_walk_kernel<L, P>, dim3((channels + kWalkThreads / L - 1) / (kWalkThreads / L), n_seqs), \
-                       2 * kWalkThreads, 0, stream, (T*)y, state, (const T*)x, dt_pre, dt_bias, (const T*)bc, bc_width, A, D, \
+#define THN_WALK_LAUNCH(L, P, H, G)                                                                                               \
+    thn_launch_ordered(selective_scan_walk_kernel<L, P, H, G>, dim3((channels + kWalkThreads / L - 1) / (kWalkThreads / L), n_seqs), \
+                       kWalkThreads + H, 0, stream, (T*)y, state, (const T*)x, dt_pre, dt_bias, (const T*)bc, bc_width, A, D, \
                        (const T*)z, z_stride, cu_seqlens, slots, channels, n_state)
     // Eight lanes a channel put twice as many warps on the chip and issue more for the same sums: they win while the
-    // blocks of four lanes (32 channels) do not fill it once.  us with 8 / 4 lanes: one prompt of 2,048 tokens, 4,096
-    // channels 140 / 181, 8,192 channels 284 / 201; 2 x 700 tokens of 4,096 channels 104 / 76; 8 x 512 200 / 162.
-    const bool few = (long long)channels * n_seqs <= 148ll * 32;
-    if (n_state <= 8) THN_WALK_LAUNCH(4, 2);
-    else if (n_state <= 16 && few) THN_WALK_LAUNCH(8, 2);
-    else if (n_state <= 16) THN_WALK_LAUNCH(4, 4);
-    else THN_WALK_LAUNCH(8, 4);
+    // blocks of four lanes (32 channels) do not fill it once.  Eight warps beside the four that walk: with four, these were what the
+    // walk waited for.  Very short sequences need smaller blocks more, and so do as many blocks as three, but not two, a multiprocessor hold.  us
+    // with eight lanes and eight warps / four and eight / four and four: one prompt of 2,048 tokens, 4,096 channels 118 / 132 / 177, 8,192
+    // channels 241 / 165 / 199; 2 x 700 tokens of 4,096 channels 89 / 62 / 75; 3 x 512 85 / 78 / 68; 8 x 512 185 / 153 / 164; 64 x 16 101 / 75 / 70.
+    const long long blocks = (channels + 31) / 32 * (long long)n_seqs;
+    const bool few = blocks <= 148, small = n_rows < 64ll * n_seqs || (blocks > 2 * 148 && blocks <= 3 * 148);
+    if (n_state <= 8) {
+        if (small) THN_WALK_LAUNCH(4, 2, 128, 1);
+        else THN_WALK_LAUNCH(4, 2, 256, 8);
+    } else if (n_state <= 16 && few) {
+        THN_WALK_LAUNCH(8, 2, 256, 2);
+    } else if (n_state <= 16) {
+        if (small) THN_WALK_LAUNCH(4, 4, 128, 1);
+        else THN_WALK_LAUNCH(4, 4, 256, 8);
+    } else {
+        THN_WALK_LAUNCH(8, 4, 128, 1);
+    }
 #undef THN_WALK_LAUNCH
     return thn_launch_status("selective_scan");
 }
@@ -594,7 +631,7 @@ THN_API int thn_selective_scan(void* y, float* state, const void* x, const float
         return launch_scan<float>(y, state, x, dt_pre, dt_bias, bc, bc_width, A, D, z, z_stride, cu_seqlens, slots, n_seqs,
                                   channels, n_state, stream);
     if (dtype == THN_BF16 && n_state <= 32 && walk_pays(n_rows, max_tokens, n_seqs, channels))
-        return launch_walk(y, state, x, dt_pre, dt_bias, bc, bc_width, A, D, z, z_stride, cu_seqlens, slots, n_seqs, channels,
+        return launch_walk(y, state, x, dt_pre, dt_bias, bc, bc_width, A, D, z, z_stride, cu_seqlens, slots, n_rows, n_seqs, channels,
                            n_state, stream);
     if (dtype == THN_BF16)
         return launch_scan<__nv_bfloat16>(y, state, x, dt_pre, dt_bias, bc, bc_width, A, D, z, z_stride, cu_seqlens, slots,
