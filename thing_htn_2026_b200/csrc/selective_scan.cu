@@ -320,7 +320,7 @@ template <int THREADS>
 __device__ __forceinline__ void halves_meet() { asm volatile("barrier.cta.sync 1, %0;" ::"n"(THREADS) : "memory"); }
 
 template <int LANES, int PER, int HELPERS, int GROUP>
-__global__ void __launch_bounds__(kWalkThreads + HELPERS, HELPERS > 128 || LANES * PER > 16 ? 2 : 3) selective_scan_walk_kernel(
+__global__ void __launch_bounds__(kWalkThreads + HELPERS, HELPERS > 128 ? 2 : 3) selective_scan_walk_kernel(
     __nv_bfloat16* __restrict__ y, float* __restrict__ state, const __nv_bfloat16* __restrict__ x,
     const float* __restrict__ dt_pre, const float* __restrict__ dt_bias, const __nv_bfloat16* __restrict__ bc, int bc_width,
     const float* __restrict__ A, const float* __restrict__ D, const __nv_bfloat16* __restrict__ z, int z_stride,
@@ -509,21 +509,28 @@ int launch_walk(void* y, float* state, const void* x, const float* dt_pre, const
                        (const T*)z, z_stride, cu_seqlens, slots, channels, n_state)
     // Eight lanes a channel put twice as many warps on the chip and issue more for the same sums: they win while the
     // blocks of four lanes (32 channels) do not fill it once.  Eight warps beside the four that walk: with four, these were what the
-    // walk waited for.  Very short sequences need smaller blocks more, and so do as many blocks as three, but not two, a multiprocessor hold.  us
-    // with eight lanes and eight warps / four and eight / four and four: one prompt of 2,048 tokens, 4,096 channels 118 / 132 / 177, 8,192
-    // channels 241 / 165 / 199; 2 x 700 tokens of 4,096 channels 89 / 62 / 75; 3 x 512 85 / 78 / 68; 8 x 512 185 / 153 / 164; 64 x 16 101 / 75 / 70.
-    const long long blocks = (channels + 31) / 32 * (long long)n_seqs;
-    const bool few = blocks <= 148, small = n_rows < 64ll * n_seqs || (blocks > 2 * 148 && blocks <= 3 * 148);
+    // walk waited for.  But two blocks of twelve warps share a multiprocessor where three of eight do, and a wave of two takes three
+    // quarters of the time of one of three: few waves that come out worse so take four, and so do very short sequences, which
+    // have little to walk.  us, eight lanes and eight warps / four and eight / four and four, 16 entries: one prompt of 2,048 tokens, 4,096
+    // channels 118 / 132 / 177, 8,192 channels 241 / 165 / 199; 2 x 700 tokens of 4,096 channels 89 / 62 / 75; 3 x 512 85 / 78 / 68;
+    // 8 x 512 185 / 153 / 164; 64 x 16 101 / 75 / 70.  32 entries, eight / four warps: 2 x 700 150 / 181, 3 x 512 163 / 161, 4 x 512
+    // 193 / 212, 64 x 16 171 / 133.
+    auto blocks = [&](int lanes) { return ((long long)channels * lanes + kWalkThreads - 1) / kWalkThreads * n_seqs; };
+    auto four = [&](int lanes) {
+        const long long n = blocks(lanes);
+        return n_rows < 64ll * n_seqs || (n <= 6 * 148 && (n + 295) / 296 * 3 > (n + 443) / 444 * 4);
+    };
     if (n_state <= 8) {
-        if (small) THN_WALK_LAUNCH(4, 2, 128, 1);
+        if (four(4)) THN_WALK_LAUNCH(4, 2, 128, 1);
         else THN_WALK_LAUNCH(4, 2, 256, 8);
-    } else if (n_state <= 16 && few) {
+    } else if (n_state <= 16 && blocks(4) <= 148) {
         THN_WALK_LAUNCH(8, 2, 256, 2);
     } else if (n_state <= 16) {
-        if (small) THN_WALK_LAUNCH(4, 4, 128, 1);
+        if (four(4)) THN_WALK_LAUNCH(4, 4, 128, 1);
         else THN_WALK_LAUNCH(4, 4, 256, 8);
     } else {
-        THN_WALK_LAUNCH(8, 4, 128, 1);
+        if (four(8)) THN_WALK_LAUNCH(8, 4, 128, 1);
+        else THN_WALK_LAUNCH(8, 4, 256, 2);
     }
 #undef THN_WALK_LAUNCH
     return thn_launch_status("selective_scan");
