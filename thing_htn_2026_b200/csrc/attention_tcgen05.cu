@@ -24,8 +24,8 @@
 //
 // What a softmax warp's tile of 64 keys takes (clocks, two blocks a multiprocessor, 2,048 tokens of 32 heads): 400 until S is there, 460 for the
 // load, the mask and the maximum (one load of 64 columns, a bit a key, four chains: 690 with two loads, three comparisons a key and one
-// chain), 740 for the exponentials (510 are the unit's own), 140 for P and the accumulator.  A kernel of a layer 54.6 -> 44.6 us (windowed, 2,532 rows of 32 heads 55.6 -> 45.7).  The products
-// read their operands from shared memory, Q again for every 64 keys, and keep its port busy for most of the rest.
+// chain), 740 for the exponentials (510 are the unit's own), 140 for P and the accumulator.  A
+// kernel of a layer 54.6 -> 44.6 us (windowed, 2,532 rows of 32 heads 55.6 -> 45.7).  The products read their operands from shared memory, Q again for every 64 keys, and keep its port busy for most of the rest.
 //
 // Every wait on an mbarrier is bounded (see gemm_tcgen05.cu); a waiter that gives up sets
 // THN_ERR_WAIT_TIMEOUT and all roles leave through the common exit.
