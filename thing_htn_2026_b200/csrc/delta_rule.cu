@@ -923,7 +923,7 @@ THN_API long long thn_delta_chunks_scratch_bytes(int n_rows, int n_heads, int n_
 // against 658 token by token; 32 heads 308 / 839; 8 x 512 tokens of 16 heads 298 / 571; steps of long and short sequences beside
 // the rule in ops (_DELTA_COST).  The read-out's error
 // against 64 bits is 1.37e-7 to 1.41e-7 (1.33e-7 to 1.36e-7 token by token), the state's 1.2e-7 to 1.4e-7 (1.1e-7 to 1.3e-7).
-THN_API int thn_delta_chunks(float* o, float* state, void* scratch, const void* proj, const float* conv_w, const float* a_log,
+THN_API int thn_delta_chunks(float* o, float* state, void* scratch, long long scratch_bytes, const void* proj, const float* conv_w, const float* a_log,
                              const float* dt_bias, const void* ring, const int* row_slot, const int* row_pos, const int* seq_lens,
                              const int* cu_seqlens, const int* slots, int n_rows, int max_tokens, int n_seqs, int n_heads, int n_kv,
                              int dk, int dv, int taps, int proj_width, float unit_eps, int* err, cudaStream_t stream) {
@@ -937,6 +937,8 @@ THN_API int thn_delta_chunks(float* o, float* state, void* scratch, const void* 
                       (((uintptr_t)proj | (uintptr_t)ring) & 7) == 0,
                   "delta_chunks: operands are not aligned");
     if (n_seqs <= 0 || n_rows <= 0 || max_tokens <= 0) return THN_OK;
+    const long long need = thn_delta_chunks_scratch_bytes(n_rows, n_heads, n_kv, dv);
+    THN_CHECK_ARG(scratch_bytes >= need, "delta_chunks: %lld bytes of scratch, %lld needed", scratch_bytes, need);
     const long long key_plane = (long long)n_rows * chunk::kKeyRow, score_plane = (long long)n_rows * chunk::kScoreRow;
     __nv_bfloat16* planes = static_cast<__nv_bfloat16*>(scratch);
     __nv_bfloat16* w = planes + 6 * n_kv * key_plane;

@@ -607,7 +607,7 @@ THN_API long long thn_linear_attention_chunks_scratch_bytes(int n_rows, int n_se
 // The recurrence of a step with gated decays chunk by chunk: bfloat16 rows as thn_linear_attention takes them (no silu), keys of
 // 128, values of whole groups of 16; v's columns start on 16-byte boundaries, q's and k's on 8-byte ones, gate and its bias on
 // 16-byte ones; max_tokens: the most rows of a sequence.  shape: 0, or which blocks walk (tests and measurement).
-THN_API int thn_linear_attention_chunks(float* o, float* state, void* scratch, const void* proj, int proj_width, int q_offset, int k_offset,
+THN_API int thn_linear_attention_chunks(float* o, float* state, void* scratch, long long scratch_bytes, const void* proj, int proj_width, int q_offset, int k_offset,
                                         int v_offset, const float* gate, int gate_width, const float* gate_bias, float tau,
                                         const int* cu_seqlens, const int* slots, int n_rows, int max_tokens, int n_seqs, int n_heads,
                                         int key_dim, int value_dim, float q_scale, int shape, int* err, cudaStream_t stream) {
@@ -623,6 +623,8 @@ THN_API int thn_linear_attention_chunks(float* o, float* state, void* scratch, c
     THN_CHECK_ARG(scratch && (((uintptr_t)state | (uintptr_t)scratch | (uintptr_t)proj | (uintptr_t)gate | (uintptr_t)gate_bias) & 15) == 0,
                   "linear_attention_chunks: operands are not 16-byte aligned");
     if (n_seqs == 0 || n_rows <= 0 || max_tokens <= 0) return THN_OK;
+    const long long need = thn_linear_attention_chunks_scratch_bytes(n_rows, n_seqs, n_heads);
+    THN_CHECK_ARG(scratch_bytes >= need, "linear_attention_chunks: %lld bytes of scratch, %lld needed", scratch_bytes, need);
     const int chunks = (max_tokens + chunk::kTokens - 1) / chunk::kTokens;
     const size_t plane = (size_t)n_rows * chunk::kKeyRow;
     __nv_bfloat16* queries = static_cast<__nv_bfloat16*>(scratch);

@@ -500,7 +500,7 @@ THN_API long long thn_mlstm_chunks_scratch_bytes(int n_rows, int n_seqs, int n_h
 // pre-activations of thn_mlstm_gates.  16 heads of 128 x 128 on B200, us against token by token: one prompt of 2,048
 // tokens 118 / 767, four of up to 1,000 tokens 99 / 730, 8 x 512 tokens 122 / 652, 64 tokens 17 / 36.  The error
 // against 64 bits is no larger: a median row's 1.7e-7 to 2.3e-7 (2.0e-7 to 2.9e-7), the state's 1.9e-7 to 3.0e-7 (2.8e-7 to 5.2e-7).
-THN_API int thn_mlstm_chunks(float* o, float* S, float* nm, void* scratch, const void* proj, int proj_width, const float* gate_pre,
+THN_API int thn_mlstm_chunks(float* o, float* S, float* nm, void* scratch, long long scratch_bytes, const void* proj, int proj_width, const float* gate_pre,
                              const float* bias_i, const float* bias_f, float cap, const int* cu_seqlens, const int* slots, int n_rows,
                              int max_tokens, int n_seqs, int n_heads, int key_dim, int value_dim, float q_scale, float floor_,
                              int* err, cudaStream_t stream) {
@@ -510,6 +510,8 @@ THN_API int thn_mlstm_chunks(float* o, float* S, float* nm, void* scratch, const
     THN_UNSUPPORTED_IF(n_heads > 65535 || n_seqs > 65535, "mlstm_chunks: %d heads, %d sequences", n_heads, n_seqs);
     THN_CHECK_ARG(scratch && (((uintptr_t)S | (uintptr_t)scratch | (uintptr_t)proj) & 15) == 0, "mlstm_chunks: operands are not 16-byte aligned");
     if (n_seqs == 0 || n_rows <= 0 || max_tokens <= 0) return THN_OK;
+    const long long need = thn_mlstm_chunks_scratch_bytes(n_rows, n_seqs, n_heads);
+    THN_CHECK_ARG(scratch_bytes >= need, "mlstm_chunks: %lld bytes of scratch, %lld needed", scratch_bytes, need);
     const int chunks = (max_tokens + chunk::kTokens - 1) / chunk::kTokens;
     __nv_bfloat16* scores = static_cast<__nv_bfloat16*>(scratch);
     float4* scalars = reinterpret_cast<float4*>(scores + (size_t)n_heads * 3 * n_rows * chunk::kScoreRow);

@@ -497,7 +497,7 @@ THN_API long long thn_state_space_chunks_scratch_bytes(int n_rows, int n_heads, 
 // max_tokens: the most rows of a sequence.  On B200, us against token by token: 8 x 512 tokens of 128 heads of 64 over a
 // state of 128 617 / 1,074, one prompt of 2,048 tokens of 64 heads 202 / 368, 128 tokens 42 / 44.  The error against 64 bits:
 // y 1.2e-7 (1.2e-7 to 1.3e-7), the state 1.1e-7 (1.2e-7).
-THN_API int thn_state_space_chunks(float* y, float* state, void* scratch, const void* proj, int proj_width, int offset,
+THN_API int thn_state_space_chunks(float* y, float* state, void* scratch, long long scratch_bytes, const void* proj, int proj_width, int offset,
                                    const float* conv_w, const float* conv_b, const void* ring, const float* dt_pre,
                                    const float* dt_bias, const float* rate, const float* skip, const int* row_slot, const int* row_pos,
                                    const int* seq_lens, const int* cu_seqlens, const int* slots, int n_rows, int max_tokens, int n_seqs,
@@ -512,6 +512,8 @@ THN_API int thn_state_space_chunks(float* y, float* state, void* scratch, const 
                       (((uintptr_t)proj | (uintptr_t)ring) & 7) == 0,
                   "state_space_chunks: operands are not aligned");
     if (n_seqs <= 0 || n_rows <= 0 || max_tokens <= 0) return THN_OK;
+    const long long need = thn_state_space_chunks_scratch_bytes(n_rows, n_heads, vdim, n_groups);
+    THN_CHECK_ARG(scratch_bytes >= need, "state_space_chunks: %lld bytes of scratch, %lld needed", scratch_bytes, need);
     const long long plane = (long long)n_rows * chunk::kKeyRow;
     __nv_bfloat16* planes = static_cast<__nv_bfloat16*>(scratch);
     __nv_bfloat16* scores = planes + 6 * n_groups * plane;

@@ -71,7 +71,7 @@ _SIGNATURES = {
     "thn_hyper_norm": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_float,
                        c_int, c_int, c_int, c_int, c_void_p],
     "thn_linear_attention_chunks_scratch_bytes": [c_int, c_int, c_int],
-    "thn_linear_attention_chunks": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_float,
+    "thn_linear_attention_chunks": [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_float,
                                     c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p],
     "thn_linear_attention": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
                              c_void_p, c_float, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_int,
@@ -100,7 +100,7 @@ _SIGNATURES = {
     "thn_state_space": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                         c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                         c_int, c_int, c_int, c_int, c_void_p],
-    "thn_state_space_chunks": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
+    "thn_state_space_chunks": [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
                                c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
                                c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     "thn_state_space_decode": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -121,7 +121,7 @@ _SIGNATURES = {
     "thn_mlstm_gates": [c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_int, c_int, c_void_p],
     "thn_mlstm_recurrence": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_float, c_int,
                              c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_void_p],
-    "thn_mlstm_chunks": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_float, c_void_p,
+    "thn_mlstm_chunks": [c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_float, c_void_p,
                          c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p],
     "thn_moe_route": [c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_float,
                       c_int, c_int, c_float, c_void_p],
@@ -139,7 +139,7 @@ _SIGNATURES = {
                           c_float, c_int, c_void_p],
     "thn_delta_recurrence": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                              c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
-    "thn_delta_chunks": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+    "thn_delta_chunks": [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                          c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
                          c_void_p, c_void_p],
     "thn_delta_conv_ring_update": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
@@ -172,7 +172,16 @@ _SIGNATURES = {
     "thn_attention_prefill_tcgen05": [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p,
                                       c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_int, c_float,
                                       c_int, c_int, c_int, c_float, c_float, c_int, c_void_p, c_void_p, c_void_p],
+    "thn_choose_tokens_scratch_floats": [c_int, c_int],
+    "thn_attention_decode_scratch_floats": [c_int, c_int, c_int, c_int],
+    "thn_linear_attention_scratch_floats": [c_int, c_int, c_int, c_int, c_int],
+    "thn_delta_chunks_scratch_bytes": [c_int, c_int, c_int, c_int],
+    "thn_mlstm_chunks_scratch_bytes": [c_int, c_int, c_int],
+    "thn_state_space_chunks_scratch_bytes": [c_int, c_int, c_int, c_int],
+    "thn_wkv_scratch_floats": [c_int, c_int, c_int],
+    "thn_state_space_scratch_floats": [c_int, c_int, c_int, c_int, c_int],
 }
+_SIZES = ("_scratch_bytes", "_scratch_floats")      # entry points whose result is a 64-bit size; every other one returns a status or an int
 
 _lib = None
 
@@ -184,7 +193,7 @@ def lib():
         for name, argtypes in _SIGNATURES.items():
             fn = getattr(loaded, name)
             fn.argtypes = argtypes
-            fn.restype = c_int
+            fn.restype = c_longlong if name.endswith(_SIZES) else c_int
         loaded.thn_set_pdl.argtypes = [c_int]
         loaded.thn_set_pdl.restype = None
         loaded.thn_set_pdl(0 if os.environ.get("THN_PDL", "1").strip().lower() in ("0", "false", "no", "off") else 1)
@@ -206,24 +215,8 @@ def lib():
         loaded.thn_set_mlstm_staged.restype = None
         loaded.thn_set_mlstm_staged(0 if os.environ.get("THN_MLSTM_STAGED", "1").strip() in ("0", "false", "off") else 1,
                                     int(os.environ.get("THN_MLSTM_LANES", 0)))
-        loaded.thn_choose_tokens_scratch_floats.argtypes = [c_int, c_int]
-        loaded.thn_choose_tokens_scratch_floats.restype = c_longlong
-        loaded.thn_attention_decode_scratch_floats.argtypes = [c_int, c_int, c_int, c_int]
-        loaded.thn_attention_decode_scratch_floats.restype = c_longlong
-        loaded.thn_linear_attention_scratch_floats.argtypes = [c_int, c_int, c_int, c_int, c_int]
-        loaded.thn_linear_attention_scratch_floats.restype = c_longlong
         loaded.thn_set_recurrence_columns.argtypes = [c_int]
         loaded.thn_set_recurrence_columns.restype = None
-        loaded.thn_delta_chunks_scratch_bytes.argtypes = [c_int, c_int, c_int, c_int]
-        loaded.thn_delta_chunks_scratch_bytes.restype = c_longlong
-        loaded.thn_mlstm_chunks_scratch_bytes.argtypes = [c_int, c_int, c_int]
-        loaded.thn_mlstm_chunks_scratch_bytes.restype = c_longlong
-        loaded.thn_state_space_chunks_scratch_bytes.argtypes = [c_int, c_int, c_int, c_int]
-        loaded.thn_state_space_chunks_scratch_bytes.restype = c_longlong
-        loaded.thn_wkv_scratch_floats.argtypes = [c_int, c_int, c_int]
-        loaded.thn_wkv_scratch_floats.restype = c_longlong
-        loaded.thn_state_space_scratch_floats.argtypes = [c_int, c_int, c_int, c_int, c_int]
-        loaded.thn_state_space_scratch_floats.restype = c_longlong
         _lib = loaded
     return _lib
 
@@ -1495,7 +1488,7 @@ def delta_rule(proj: torch.Tensor, conv_w: torch.Tensor, a_log: torch.Tensor, dt
         return o
     if _delta_in_chunks(proj, conv_w, state, ring, rows, s):
         scratch = torch.empty(lib().thn_delta_chunks_scratch_bytes(n, s.n_heads, s.n_kv, s.value_dim), dtype=torch.uint8, device=dev)
-        _call("thn_delta_chunks", _ptr(o), _ptr(state), _ptr(scratch), _ptr(proj), _ptr(conv_w), _ptr(a_log), _ptr(dt_bias),
+        _call("thn_delta_chunks", _ptr(o), _ptr(state), _ptr(scratch), scratch.numel(), _ptr(proj), _ptr(conv_w), _ptr(a_log), _ptr(dt_bias),
               _ptr(ring), _ptr(rows.row_slot), _ptr(rows.row_pos), _ptr(seq_lens), _ptr(rows.cu_seqlens), _ptr(rows.slots), n,
               rows.max_q_len, rows.n_seqs, s.n_heads, s.n_kv, s.key_dim, s.value_dim, s.taps, s.proj_width, float(unit_eps),
               _ptr(err), _stream())
@@ -1638,7 +1631,7 @@ def mlstm(proj: torch.Tensor, gate_pre: torch.Tensor, bias_i: torch.Tensor, bias
     if _mlstm_in_chunks(proj, state, rows, n_heads, key_dim, value_dim):
         scratch = torch.empty(lib().thn_mlstm_chunks_scratch_bytes(n, rows.n_seqs, n_heads), dtype=torch.uint8,
                               device=proj.device)
-        _call("thn_mlstm_chunks", _ptr(o), _ptr(state), _ptr(normaliser), _ptr(scratch), _ptr(proj), proj.shape[1], _ptr(gate_pre),
+        _call("thn_mlstm_chunks", _ptr(o), _ptr(state), _ptr(normaliser), _ptr(scratch), scratch.numel(), _ptr(proj), proj.shape[1], _ptr(gate_pre),
               _ptr(bias_i), _ptr(bias_f), float(cap), _ptr(rows.cu_seqlens), _ptr(rows.slots), n, rows.max_q_len, rows.n_seqs, n_heads,
               key_dim, value_dim, float(q_scale), float(floor), _ptr(err), _stream())
         return o
@@ -1908,7 +1901,7 @@ def linear_attention(proj: torch.Tensor, offsets: Tuple[int, int, int], state: t
     if gate is not None and not silu_inputs and _linear_in_chunks(proj, offsets, state, rows, n_heads, key_dim, value_dim, gate, gate_bias):
         scratch = torch.empty(lib().thn_linear_attention_chunks_scratch_bytes(rows.n_rows, rows.n_seqs, n_heads), dtype=torch.uint8,
                               device=proj.device)
-        _call("thn_linear_attention_chunks", _ptr(o), _ptr(state), _ptr(scratch), _ptr(proj), proj.shape[1], int(offsets[0]), int(offsets[1]),
+        _call("thn_linear_attention_chunks", _ptr(o), _ptr(state), _ptr(scratch), scratch.numel(), _ptr(proj), proj.shape[1], int(offsets[0]), int(offsets[1]),
               int(offsets[2]), _ptr(gate), gate.shape[1], _ptr(gate_bias), float(tau), _ptr(rows.cu_seqlens), _ptr(rows.slots), rows.n_rows,
               rows.max_q_len, rows.n_seqs, n_heads, key_dim, value_dim, float(q_scale), LINEAR_CHUNK_SHAPE, _ptr(err), _stream())
         return o
@@ -2132,7 +2125,7 @@ def state_space(proj: torch.Tensor, offset: int, dt_pre: torch.Tensor, shape: St
     if _space_in_chunks(proj, offset, state, ring, rows, s):
         scratch = torch.empty(lib().thn_state_space_chunks_scratch_bytes(n, s.n_heads, s.vdim, s.n_groups), dtype=torch.uint8,
                               device=proj.device)
-        _call("thn_state_space_chunks", _ptr(y), _ptr(state), _ptr(scratch), _ptr(proj), proj.shape[1], int(offset), _ptr(s.conv_w),
+        _call("thn_state_space_chunks", _ptr(y), _ptr(state), _ptr(scratch), scratch.numel(), _ptr(proj), proj.shape[1], int(offset), _ptr(s.conv_w),
               _ptr(s.conv_b), _ptr(ring), _ptr(dt_pre), _ptr(s.dt_bias), _ptr(s.rate), _ptr(s.skip), _ptr(rows.row_slot),
               _ptr(rows.row_pos), _ptr(seq_lens), _ptr(rows.cu_seqlens), _ptr(rows.slots), n, rows.max_q_len, rows.n_seqs, s.n_heads,
               s.vdim, s.n_state, s.n_groups, s.taps, _ptr(err), _stream())
