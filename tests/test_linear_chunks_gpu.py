@@ -23,10 +23,11 @@ def operands(lens, heads, vdim, seed, spread=2.0):
     return proj, draw(sum(lens), heads * KEY + 4) * spread, draw(heads * KEY) + 2, draw(len(lens) + 1, heads, vdim, KEY)
 
 
-def run(proj, gate, bias, state, rows, heads, vdim, tau):
-    state = state.clone()
+def run(proj, gate, bias, state, rows, heads, vdim, tau, want_bits=0):
+    state, err = state.clone(), ops.new_error_word(torch.device("cuda"))
     o = ops.linear_attention(proj, (8, 8 + heads * KEY, 16 + 2 * heads * KEY), state, rows, heads, KEY, vdim, gate=gate, gate_bias=bias, tau=tau,
-                             q_scale=KEY ** -0.5)
+                             q_scale=KEY ** -0.5, err=err)
+    assert int(err.item()) == want_bits
     return o, state
 
 
@@ -82,3 +83,18 @@ def test_what_the_rule_leaves_to_the_tokens():
     assert not ask(o=(8, 8 + 2 * KEY, 12 + 4 * KEY)) and not ask(o=(6, 8 + 2 * KEY, 16 + 4 * KEY))
     assert not ask(p=torch.empty(40, proj.shape[1] + 4, dtype=BF16, device="cuda")) and not ask(g=torch.empty(40, gate.shape[1] + 2, device="cuda"))
     assert not ask(b=torch.empty(2 * KEY + 1, device="cuda")[1:])
+
+
+@pytest.mark.parametrize("shape", [1, 2, 3])
+def test_a_wait_that_runs_out_sets_its_bit_and_the_kernel_returns(monkeypatch, shape):
+    """With nothing brought the walk's wait ends after 20 ms, the bit is set, the state stays, and the next launch is right again."""
+    rows, _, _, _ = step([70, 33])
+    proj, gate, bias, state = operands([70, 33], 2, 128, 5)
+    monkeypatch.setattr(ops, "LINEAR_CHUNK_SHAPE", shape)
+    want = run(proj, gate, bias, state, rows, 2, 128, 16.0)
+    monkeypatch.setattr(ops, "LINEAR_CHUNK_SHAPE", shape + 16)
+    _, untouched = run(proj, gate, bias, state, rows, 2, 128, 16.0, ops.ERR_WAIT_TIMEOUT)
+    assert torch.equal(untouched, state)
+    monkeypatch.setattr(ops, "LINEAR_CHUNK_SHAPE", shape)
+    again = run(proj, gate, bias, state, rows, 2, 128, 16.0)
+    assert torch.equal(again[0], want[0]) and torch.equal(again[1], want[1])

@@ -115,3 +115,20 @@ def test_sizes_and_operands_that_are_refused():
         ops.grouped_experts(x, routing, rand((2048, 96), 3).bfloat16(), rand((96, 1024), 4).bfloat16(), 128, 0, SILU)
     with pytest.raises(ops.KernelError):
         ops.grouped_experts(x, routing, rand((2048, 96), 3).bfloat16(), rand((96, 1000), 4).bfloat16(), 128, 0, SILU)
+
+
+@pytest.mark.parametrize("form, shared_ff", [("silu", 128), ("gelu", 0)])
+def test_a_wait_that_runs_out_sets_its_bit_and_the_kernels_return(form, shared_ff, monkeypatch):
+    """With no operand loaded every wait of the products ends after 20 ms, the bit is set, and the next launch is right again."""
+    from thing_htn_2026_b200 import ops
+    glu = {"silu": SILU, "gelu": None}[form]
+    x, width = rand((300, 256), 1).bfloat16(), 8 * 128 + shared_ff
+    w_up, w_down = rand(((2 if glu else 1) * width, 256), 2).bfloat16(), rand((256, width), 3).bfloat16()
+    routing = ops.moe_route(rand((300, 8), 4), 8, 1, 1, 2, 1.0, scoring="softmax_chosen")
+    err = ops.new_error_word(torch.device(DEV))
+    with monkeypatch.context() as patch:
+        patch.setattr(ops, "GROUPED_SKIP_LOADS", 1)
+        ops.grouped_experts(x, routing, w_up, w_down, 128, shared_ff, glu, err=err)
+    torch.cuda.synchronize()
+    assert int(err.item()) == ops.ERR_WAIT_TIMEOUT
+    check(300, 256, 8, 2, 128, shared_ff, glu, False)

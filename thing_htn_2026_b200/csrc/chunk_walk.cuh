@@ -32,7 +32,7 @@
 // 4,630 clocks for the delta rule of 16 heads, 1,225 of 3,700 for 32 heads with a decay per key), but start sooner and leave room for more
 // blocks: they stay where blocks are many and short.  (One more warp takes 1,200 clocks to start a chunk's bulk copies, most of the time that the others
 // need for it.)  The wait for what is brought is bounded: after kWaitLimitNs by the global timer the block sets
-// THN_ERR_WAIT_TIMEOUT and returns.
+// THN_ERR_WAIT_TIMEOUT, lets what is on its way land and returns; its results and state are then not written, those of other blocks may be.
 #pragma once
 
 #include "common.cuh"
@@ -71,6 +71,7 @@ struct WalkArgs {
     const float* key_sums;     // [chunk_place, heads, kKeys]: sum_j w_j k_j of every chunk; a decay per key: the chunk's decay of S
     float floor_;
     int* err;                  // the caller's error word, or null
+    int skip_loads;            // the test of the bounded wait: nothing is brought
 };
 
 __device__ __forceinline__ void copy16(void* smem, const void* gmem, bool there) {
@@ -363,6 +364,7 @@ __global__ void __launch_bounds__(32 * CG * KS + (BROUGHT ? 128 : 0), STAGES == 
         // ---- the warps that bring the operands: W, the queries, the keys and G, a plane a lane, and the values' rows
         const int bringer = threadIdx.x - L::kThreads, p = min(lane, 2);
         auto bring = [&](int chunk) {
+            if (a.skip_loads) return;
             unsigned char* dst = mem + (chunk % STAGES) * L::kStage;
             uint64_t* bar = full + chunk % STAGES;
             const int first = chunk * kTokens, n_here = min(kTokens, n_tokens - first);
@@ -396,7 +398,10 @@ __global__ void __launch_bounds__(32 * CG * KS + (BROUGHT ? 128 : 0), STAGES == 
         bring(0);
         if (n_chunks > 1) bring(1);
         for (int chunk = 0; chunk < n_chunks; ++chunk) {
-            if (!all_agree(true)) return;
+            if (!all_agree(true)) {
+                let_copies_land();
+                return;
+            }
             if (chunk > 0 && chunk + 1 < n_chunks) bring(chunk + 1);      // (the chunk ahead of this one is through: its buffer is free)
         }
         return;
@@ -474,6 +479,7 @@ __global__ void __launch_bounds__(32 * CG * KS + (BROUGHT ? 128 : 0), STAGES == 
         if constexpr (BROUGHT) {
             if (!all_agree(mbar_wait(full + chunk % STAGES, chunk / STAGES & 1))) {
                 if (threadIdx.x == 0 && a.err) atomicOr(a.err, THN_ERR_WAIT_TIMEOUT);
+                let_copies_land();
                 return;
             }
         } else {

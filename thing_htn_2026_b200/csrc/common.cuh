@@ -218,6 +218,12 @@ struct WaitClock {
         return waited > limit_ns;
     }
 };
+// What a block does ahead of its end where one of its waits has run out: copies and products that it has started are given a
+// millisecond to land, for what lands later lands in the shared memory of the multiprocessor's next block.
+__device__ __forceinline__ void let_copies_land() {
+    WaitClock clock;
+    while (!clock.ran_out(1000 * 1000)) __nanosleep(1000);
+}
 
 // How attention scores are shaped between q . k and the softmax, beyond the plain scale:
 //   temperature  the scores of the query at position p are multiplied by

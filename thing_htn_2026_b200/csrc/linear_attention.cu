@@ -606,7 +606,8 @@ THN_API long long thn_linear_attention_chunks_scratch_bytes(int n_rows, int n_se
 
 // The recurrence of a step with gated decays chunk by chunk: bfloat16 rows as thn_linear_attention takes them (no silu), keys of
 // 128, values of whole groups of 16; v's columns start on 16-byte boundaries, q's and k's on 8-byte ones, gate and its bias on
-// 16-byte ones; max_tokens: the most rows of a sequence.  shape: 0, or which blocks walk (tests and measurement).
+// 16-byte ones; max_tokens: the most rows of a sequence.  shape: 0, or which blocks walk (tests and measurement); with 16 added a brought
+// walk brings nothing, so that its wait runs out (for the test of the wait only).
 THN_API int thn_linear_attention_chunks(float* o, float* state, void* scratch, long long scratch_bytes, const void* proj, int proj_width, int q_offset, int k_offset,
                                         int v_offset, const float* gate, int gate_width, const float* gate_bias, float tau,
                                         const int* cu_seqlens, const int* slots, int n_rows, int max_tokens, int n_seqs, int n_heads,
@@ -637,6 +638,8 @@ THN_API int thn_linear_attention_chunks(float* o, float* state, void* scratch, l
                proj_width, q_offset, k_offset, gate, gate_width, gate_bias, 1.0f / tau, cu_seqlens, n_rows, n_heads);
     chunk::WalkArgs a{};
     a.err = err;
+    a.skip_loads = shape & 16;
+    shape &= 15;
     a.o = o; a.state = state;
     a.q = queries; a.k = keys;
     a.key_plane = plane; a.key_unit = 3 * plane; a.key_row = chunk::kKeyRow;

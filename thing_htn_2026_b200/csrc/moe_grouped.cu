@@ -74,6 +74,7 @@ struct PairArgs {
     const int* place;            // [rows, top]: the sorted position of a row's choices
     int top;
     int* err;
+    int skip_loads;              // the test of the bounded waits: nothing is loaded
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -295,7 +296,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) pair_ge
                 if (MODE == kPartial) k0 = t.group * a.k;
                 if (MODE == kCombine) k0 = a.up_row;        // (where the shared expert's columns begin)
             }
-            for (int kb = 0; kb < n_k; ++kb, ++it) {
+            for (int kb = 0; kb < n_k && !a.skip_loads; ++kb, ++it) {
                 const int s = it % kStages;
                 if (!mbar_wait(empty + s, ((it / kStages) & 1) ^ 1)) {
                     if (a.err) atomicOr(a.err, THN_ERR_WAIT_TIMEOUT);
@@ -466,10 +467,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) pair_ge
                 asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(leader_addr(acc_empty + buf)) : "memory");
         }
     }
-    if (*give_up) {                            // copies and products on their way are given a millisecond to land
-        WaitClock clock;
-        while (!clock.ran_out(1000 * 1000)) __nanosleep(1000);
-    }
+    if (*give_up) let_copies_land();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     pair_barrier();                            // neither block leaves while the other may reach into it
@@ -651,12 +649,13 @@ THN_API int thn_moe_grouped_supported(int hidden, int n_experts, int ff, int sha
 //   shared_logit the rows' gate logits of the shared expert, logit_stride apart (null: no gate)
 //   sorted_x, act, shared_act bfloat16 [rows * top, hidden], [rows * top, ff], [rows, shared_ff]; partial float32
 //                [rows * top, hidden]; ints int32 [2 * rows * top + experts + 1]; floats float32 [rows * top]: scratch
-// All matrices 16-byte aligned.  err: device error word (THN_ERR_WAIT_TIMEOUT if a pipeline wait gave up).
+// All matrices 16-byte aligned.  err: device error word (THN_ERR_WAIT_TIMEOUT if a pipeline wait gave up).  skip_loads: 0; otherwise no
+// operand is loaded, so that the products' waits run out (for the test of the waits only).
 THN_API int thn_moe_grouped_bf16(void* out, const void* x, const int* chosen, const float* dense, const void* w_up, const void* w_down,
                                  const float* shared_logit, long long logit_stride, void* sorted_x, void* act, void* shared_act,
                                  float* partial, int* ints, float* floats, int n_rows, int hidden, int n_experts, int top, int ff,
                                  int shared_ff, int glu, float limit, float shared_limit, float alpha, float up_shift, int weight_output,
-                                 int* err, cudaStream_t stream) {
+                                 int skip_loads, int* err, cudaStream_t stream) {
     THN_UNSUPPORTED_IF(!thn_moe_grouped_supported(hidden, n_experts, ff, shared_ff), "moe_grouped: %d experts of %d (and %d) over rows of %d not supported",
                        n_experts, ff, shared_ff, hidden);
     THN_CHECK_ARG(n_rows >= 0 && top > 0 && top <= n_experts, "moe_grouped: %d rows, top %d of %d experts", n_rows, top, n_experts);
@@ -699,6 +698,7 @@ THN_API int thn_moe_grouped_bf16(void* out, const void* x, const int* chosen, co
     up.shared_logit = shared_logit;
     up.logit_stride = logit_stride;
     up.err = err;
+    up.skip_loads = skip_loads;
     const int up_tile = glu ? kFeatures / 2 : kFeatures;
     const long long up_tiles = tiles_of(n, n_experts, ff, up_tile, kGlu) + (shared_ff ? tiles_of(n_rows, 1, shared_ff, up_tile, kGlu) : 0);
     int status = glu ? launch_pairs<kGlu>(map_up, map_sorted, map_x, up, up_tiles, stream)
@@ -711,6 +711,7 @@ THN_API int thn_moe_grouped_bf16(void* out, const void* x, const int* chosen, co
     down.k = ff;
     down.out = partial;
     down.err = err;
+    down.skip_loads = skip_loads;
     status = launch_pairs<kPartial>(map_down, map_act, map_act, down, tiles_of(n, n_experts, hidden, kFeatures, kPartial), stream);
     if (status != THN_OK) return status;
     if (shared_ff == 0) {
@@ -727,5 +728,6 @@ THN_API int thn_moe_grouped_bf16(void* out, const void* x, const int* chosen, co
     sum.place = place;
     sum.top = top;
     sum.err = err;
+    sum.skip_loads = skip_loads;
     return launch_pairs<kCombine>(map_down, map_shared, map_shared, sum, tiles_of(n_rows, 1, hidden, kFeatures, kCombine), stream);
 }

@@ -129,7 +129,7 @@ _SIGNATURES = {
     "thn_moe_grouped_supported": [c_int, c_int, c_int, c_int],
     "thn_moe_grouped_bf16": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p,
                              c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_float,
-                             c_float, c_int, c_void_p, c_void_p],
+                             c_float, c_int, c_int, c_void_p, c_void_p],
     "thn_clamped_glu": [c_void_p, c_void_p, c_longlong, c_int, c_int, c_float, c_float, c_int, c_void_p],
     "thn_qk_prepare": [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_float, c_float, c_void_p, c_void_p,
                        c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
@@ -1735,6 +1735,7 @@ def routed_gelu(u: torch.Tensor, routing: Routing, ff: int, shared_ff: int,
 # rows 131 / 134, 2,048 313 / 585; gelu: 512 129 / 124, 1,024 154 / 204.  64 of 512 over 2,048, top 6: 256 rows 127 / 140, 2,048 180 / 587.  16 of 1,024,
 # top 4, none shared: 256 rows 74 / 81, 2,048 148 / 280.  4 of 512 over 1,024, top 2: 4,096 rows 64 / 60.)
 GROUPED_MIN_ROWS = 256
+GROUPED_SKIP_LOADS = 0       # the test of the products' bounded waits sets it: nothing is loaded
 GROUPED_MIN_SAVED = {True: 60e9, False: 100e9}       # gated, gelu
 
 
@@ -1781,7 +1782,7 @@ def grouped_experts(x: torch.Tensor, routing: Routing, w_up: torch.Tensor, w_dow
     _call("thn_moe_grouped_bf16", _ptr(out), _ptr(x), _ptr(routing.chosen), _ptr(routing.dense), _ptr(w_up), _ptr(w_down), logit_ptr, stride,
           _ptr(sorted_x), _ptr(act), _ptr(shared_act), _ptr(partial), _ptr(ints), _ptr(weights), rows, hidden, n_experts, top, ff, shared_ff,
           int(glu is not None), float(limit), float(shared_limit or 1.0), float(alpha), float(up_shift), int(weight_at == "output"),
-          _ptr(err), _stream())
+          GROUPED_SKIP_LOADS, _ptr(err), _stream())
     return out
 
 
@@ -1850,7 +1851,7 @@ def set_recurrence_columns(columns: int = 0) -> None:
     lib().thn_set_recurrence_columns(int(columns))
 
 
-LINEAR_CHUNK_SHAPE = 0      # which blocks walk the chunks: 0 a rule of sizes, 1 to 4 one of them (tests and measurement)
+LINEAR_CHUNK_SHAPE = 0      # which blocks walk the chunks: 0 a rule of sizes, 1 to 4 one of them (tests and measurement); + 16: see thn_linear_attention_chunks
 
 
 def _linear_in_chunks(proj: torch.Tensor, offsets: Tuple[int, int, int], state: torch.Tensor, rows: StepRows, n_heads: int, key_dim: int,
