@@ -512,6 +512,7 @@ __global__ void __launch_bounds__(kThreads, 2) attention_tcgen05_kernel(
             *give_up = 1;
         }
     }
+    if (*give_up) let_copies_land();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 1) {

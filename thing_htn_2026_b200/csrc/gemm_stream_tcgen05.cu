@@ -394,6 +394,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_stream_kernel(
             }
         }
     }
+    if (*give_up) let_copies_land();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 1) {
@@ -576,6 +577,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_stream_cluster_kernel(
             if (n < N) out[(size_t)j * N + n] = from_f32<OutT>(sum);
         }
     }
+    if (*give_up) let_copies_land();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 1) {
