@@ -654,7 +654,7 @@ def kernel_table(torch, lan, peak, batch, context):
         tokens = n * len(who)
         state_bytes = len(who) * Hd * dk * dv * 4 * 2
         row(f"{tag}: delta_rule (conv, norms, recurrence)",
-            lambda: ops.delta_rule(proj, conv_w, a_log, dt_bias, state, ring, rows_, cache.seq_lens, shape, 1e-6),
+            lambda: ops.delta_rule(proj, conv_w, a_log, dt_bias, state, ring, rows_, cache.seq_lens, shape, 1e-6, err),
             nbytes=state_bytes + tokens * (shape.proj_width * 2 + Hd * dv * 4), flops=6.0 * tokens * Hd * dk * dv,
             flop_peak=FP32_CORE_TFLOPS * 1e12, like=f"{tag}: attention (all keys)" if len(tag) < 8 else None)
         if len(tag) >= 8:
@@ -880,7 +880,7 @@ def bunudra_kernel_table(torch, bun, peak, batch, context):
         state_bytes = len(who) * Hm * dk * dv * 4 * 2
         row(f"{tag}: delta_rule (conv, norms, recurrence)",
             lambda: ops.delta_rule(dproj, conv_w, a_log, dt_bias, dcache.state_view(0, 0), dcache.state_view(0, 1), drows,
-                                   dcache.seq_lens, shape, 1e-6),
+                                   dcache.seq_lens, shape, 1e-6, err),
             nbytes=state_bytes + tokens * (shape.proj_width * 2 + Hm * dv * 4), flops=6.0 * tokens * Hm * dk * dv,
             flop_peak=FP32_CORE_TFLOPS * 1e12)
         row(f"{tag}: mlstm (gates, recurrence)",
@@ -1270,7 +1270,7 @@ def dubazen_kernel_table(torch, dub, peak, batch, context):
             nbytes=state_bytes + io_bytes, flops=6.0 * tokens * Hg * dk * dv, flop_peak=cores, like=like)
         row(f"{tag}: linear_attention (a gated decay per key channel)",
             lambda: ops.linear_attention(proj, (0, Hg * dk, 2 * Hg * dk), cache.state_view(1), rows_, Hg, dk, dv, gate=zgate,
-                                         gate_bias=gate_bias, tau=16.0, q_scale=dk ** -0.5),
+                                         gate_bias=gate_bias, tau=16.0, q_scale=dk ** -0.5, err=err),
             nbytes=state_bytes + io_bytes + tokens * Hg * dk * 4, flops=6.0 * tokens * Hg * dk * dv, flop_peak=cores, like=like)
         xz = rnd(tokens, 2 * inner).to(bf)
         row(f"{tag}: causal_conv (taps, bias, silu) and its ring",
@@ -1448,7 +1448,7 @@ def futepel_kernel_table(torch, fut, peak, batch, context):
         state_bytes, like_state = len(who) * h * d * d * 8, len(who) * Hg * dg * dg * 8
         like_la = f"{tag}: linear_attention (gated decays)"
         la = lambda: ops.linear_attention(lin, (0, Hg * dg, 2 * Hg * dg), cache.state_view(2), rows_, Hg, dg, dg, gate=zg,
-                                          gate_bias=gate_bias, tau=16.0, q_scale=dg ** -0.5)
+                                          gate_bias=gate_bias, tau=16.0, q_scale=dg ** -0.5, err=err)
         row(like_la, la, nbytes=like_state + m * Hg * dg * (3 * 2 + 4 + 4), flops=6.0 * m * Hg * dg * dg, flop_peak=cores)
         o_like = rnd(m, Hg, dg)
         row(f"{tag}: gated_head_norm (one gain)", lambda: ops.gated_head_norm(o_like, lin, 3 * Hg * dg, gain_g, 1e-6, Hg, dg, bf),
@@ -1475,7 +1475,8 @@ def futepel_kernel_table(torch, fut, peak, batch, context):
         # ---- state-space duality
         proj, dt = rnd(m, H2 * e2 + channels).to(bf), rnd(m, H2)
         row(f"{tag}: state_space (convolution, decays, recurrence, ring)",
-            lambda: ops.state_space(proj, H2 * e2, dt, shape, cache.state_view(1, 0), cache.state_view(1, 1), rows_, cache.seq_lens),
+            lambda: ops.state_space(proj, H2 * e2, dt, shape, cache.state_view(1, 0), cache.state_view(1, 1), rows_, cache.seq_lens,
+                                    err),
             nbytes=len(who) * H2 * e2 * N * 8 + m * (channels * 2 + H2 * e2 * 4), flops=6.0 * m * H2 * e2 * N, flop_peak=cores,
             like=like_la)
         y32 = rnd(m, H2, e2)

@@ -39,15 +39,21 @@ def test_delta_rule(heads, vdim):
     state = draw(len(LENS) + 1, heads, vdim, 128) * 0.2
     err = ops.new_error_word(torch.device("cuda"))
 
-    def run(part, s, r, n):
+    def run(part, s, r, n, word=err):
         ring = torch.zeros(s.shape[0], 4, shape.conv_channels, dtype=BF16, device="cuda")
-        return ops.delta_rule(proj[part].contiguous(), w, a_log, dt, s, ring, r, n, shape, 1e-6, err)
+        return ops.delta_rule(proj[part].contiguous(), w, a_log, dt, s, ring, r, n, shape, 1e-6, word)
     together = state.clone()
     o = run(slice(0, cu[-1]), together, rows, lens)
     want, states = alone(run, state, slots, cu)
     close(o, want)
     close(together[1:], states[1:])
     assert int(err.item()) == 0
+    # without an error word the warps copy themselves: the same to the bit, in wide blocks and in narrow ones
+    copied = state.clone()
+    assert torch.equal(run(slice(0, cu[-1]), copied, rows, lens, None), o) and torch.equal(copied, together)
+    narrow, copied = state[:2].clone(), state[:2].clone()
+    r, n, _, _ = step([cu[1]])
+    assert torch.equal(run(slice(0, cu[1]), narrow, r, n), run(slice(0, cu[1]), copied, r, n, None)) and torch.equal(narrow, copied)
 
 
 @pytest.mark.parametrize("heads,vdim", [(16, 64), (8, 128)])
@@ -61,15 +67,21 @@ def test_state_space(heads, vdim):
     state = draw(len(LENS) + 1, heads, vdim, 128) * 0.1
     err = ops.new_error_word(torch.device("cuda"))
 
-    def run(part, s, r, n):
+    def run(part, s, r, n, word=err):
         ring = torch.zeros(s.shape[0], 4, channels, dtype=BF16, device="cuda")
-        return ops.state_space(proj[part].contiguous(), inner, dt[part].contiguous(), shape, s, ring, r, n, err)
+        return ops.state_space(proj[part].contiguous(), inner, dt[part].contiguous(), shape, s, ring, r, n, word)
     together = state.clone()
     o = run(slice(0, cu[-1]), together, rows, lens)
     want, states = alone(run, state, slots, cu)
     close(o, want)
     close(together[1:], states[1:])
     assert int(err.item()) == 0
+    # without an error word the warps copy themselves: the same to the bit, in wide blocks and in narrow ones
+    copied = state.clone()
+    assert torch.equal(run(slice(0, cu[-1]), copied, rows, lens, None), o) and torch.equal(copied, together)
+    narrow, copied = state[:2].clone(), state[:2].clone()
+    r, n, _, _ = step([cu[1]])
+    assert torch.equal(run(slice(0, cu[1]), narrow, r, n), run(slice(0, cu[1]), copied, r, n, None)) and torch.equal(narrow, copied)
 
 
 # the blocks' shapes of the matrix memory, by how many heads are walked at once: 32 columns and four warps over the keys, 64 and two,

@@ -98,3 +98,15 @@ def test_a_wait_that_runs_out_sets_its_bit_and_the_kernel_returns(monkeypatch, s
     monkeypatch.setattr(ops, "LINEAR_CHUNK_SHAPE", shape)
     again = run(proj, gate, bias, state, rows, 2, 128, 16.0)
     assert torch.equal(again[0], want[0]) and torch.equal(again[1], want[1])
+
+
+@pytest.mark.parametrize("shape", [1, 2, 3, 4])
+def test_without_an_error_word_no_warp_waits_for_another(monkeypatch, shape):
+    """A walk that has no word to say so cannot run out of a wait: with nothing brought its results are the same to the bit."""
+    rows, _, _, _ = step([70, 33, 1])
+    proj, gate, bias, state = operands([70, 33, 1], 2, 128, 6)
+    monkeypatch.setattr(ops, "LINEAR_CHUNK_SHAPE", shape)
+    want, want_state = run(proj, gate, bias, state, rows, 2, 128, 16.0)
+    monkeypatch.setattr(ops, "LINEAR_CHUNK_SHAPE", shape + 16)
+    o = ops.linear_attention(proj, (8, 8 + 2 * KEY, 16 + 4 * KEY), state, rows, 2, KEY, 128, gate=gate, gate_bias=bias, tau=16.0, q_scale=KEY ** -0.5)
+    assert torch.equal(o, want) and torch.equal(state, want_state)

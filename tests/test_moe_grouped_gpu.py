@@ -132,3 +132,12 @@ def test_a_wait_that_runs_out_sets_its_bit_and_the_kernels_return(form, shared_f
     torch.cuda.synchronize()
     assert int(err.item()) == ops.ERR_WAIT_TIMEOUT
     check(300, 256, 8, 2, 128, shared_ff, glu, False)
+
+
+def test_without_an_error_word_a_wait_that_runs_out_raises(monkeypatch):
+    from thing_htn_2026_b200 import ops
+    x, w_up, w_down = rand((300, 256), 1).bfloat16(), rand((2048, 256), 2).bfloat16(), rand((256, 1024), 3).bfloat16()
+    routing = ops.moe_route(rand((300, 8), 4), 8, 1, 1, 2, 1.0, scoring="softmax_chosen")
+    monkeypatch.setattr(ops, "GROUPED_SKIP_LOADS", 1)
+    with pytest.raises(ops.KernelError, match="bounded wait"):
+        ops.grouped_experts(x, routing, w_up, w_down, 128, 0, SILU)

@@ -46,7 +46,9 @@ def test_a_part_gives_the_same_on_both_sides(kind, monkeypatch):
         inner = ops.grouped_experts
         monkeypatch.setattr(ops, "grouped_experts", lambda *a, **k: calls.append(1) or inner(*a, **k))
         grouped = part.forward(x, ctx)
-    assert calls and int(ctx.err.item()) == 0
+        assert len(calls) == 1
+        part.forward(x, SimpleNamespace(err=None))          # no word for the kernels' waits: the dense form
+    assert len(calls) == 1 and int(ctx.err.item()) == 0
     # each side rounds the activations and the result (1.6e-3 from 64 bits), the dense one gates and ups too (1.6e-3 more)
     assert float((dense.double() - grouped.double()).norm() / dense.double().norm()) < 8e-3
 

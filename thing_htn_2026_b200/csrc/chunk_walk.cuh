@@ -70,7 +70,7 @@ struct WalkArgs {
     float* normaliser;         // [slots, heads, value_dim / 16, kKeys + 1]: copies of n, then m
     const float* key_sums;     // [chunk_place, heads, kKeys]: sum_j w_j k_j of every chunk; a decay per key: the chunk's decay of S
     float floor_;
-    int* err;                  // the caller's error word, or null
+    int* err;                  // the caller's error word, or null: walks that are brought need one
     int skip_loads;            // the test of the bounded wait: nothing is brought
 };
 
@@ -478,7 +478,7 @@ __global__ void __launch_bounds__(32 * CG * KS + (BROUGHT ? 128 : 0), STAGES == 
         // this chunk is in place; the other buffer, and the shares, are free again
         if constexpr (BROUGHT) {
             if (!all_agree(mbar_wait(full + chunk % STAGES, chunk / STAGES & 1))) {
-                if (threadIdx.x == 0 && a.err) atomicOr(a.err, THN_ERR_WAIT_TIMEOUT);
+                if (threadIdx.x == 0) atomicOr(a.err, THN_ERR_WAIT_TIMEOUT);
                 let_copies_land();
                 return;
             }
@@ -787,6 +787,14 @@ void launch_walk(const WalkArgs& a, int n_seqs, cudaStream_t stream) {
     auto kernel = walk_kernel<T, CG, KS, KIND, STAGES, BROUGHT>;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes);
     thn_launch_ordered(kernel, dim3(a.value_dim / L::kColumns, a.n_heads, n_seqs), L::kThreads + L::kBringers, L::kBytes, stream, a);
+}
+
+// The walk whose operands are brought, where the caller has an error word in which its wait can say that it ran out; otherwise the warps copy
+// themselves, with the same results to the bit.
+template <typename T, int CG, int KS, Kind KIND>
+void launch_brought_walk(const WalkArgs& a, int n_seqs, cudaStream_t stream) {
+    if (a.err) launch_walk<T, CG, KS, KIND, 2, true>(a, n_seqs, stream);
+    else launch_walk<T, CG, KS, KIND, 2, false>(a, n_seqs, stream);
 }
 
 // Whether a step's sequences are so short that the blocks' starts weigh more than their chunks: the warps then copy themselves.  us of the whole

@@ -977,11 +977,11 @@ THN_API int thn_delta_chunks(float* o, float* state, void* scratch, long long sc
     using namespace chunk;
     if (dv % 64 == 0 && pairs * (dv / 64) >= 128) {
         if (many_short(n_rows, n_seqs, max_tokens)) launch_walk<float, 4, 2, kDelta, 2, false>(a, n_seqs, stream);
-        else launch_walk<float, 4, 2, kDelta, 2, true>(a, n_seqs, stream);
+        else launch_brought_walk<float, 4, 2, kDelta>(a, n_seqs, stream);
     } else if (dv % 32 == 0 && pairs * (dv / 32) >= 128) {
-        launch_walk<float, 2, 4, kDelta, 2, true>(a, n_seqs, stream);
+        launch_brought_walk<float, 2, 4, kDelta>(a, n_seqs, stream);
     } else {
-        launch_walk<float, 1, 4, kDelta, 2, true>(a, n_seqs, stream);
+        launch_brought_walk<float, 1, 4, kDelta>(a, n_seqs, stream);
     }
     return thn_launch_status("delta_chunks");
 }

@@ -659,8 +659,8 @@ THN_API int thn_linear_attention_chunks(float* o, float* state, void* scratch, l
     if (value_dim % 64 != 0) shape = std::min(shape, 2);
     if (value_dim % 32 != 0) shape = 1;
     if (shape == 4) launch_walk<T, 4, 2, kPerKey, 1, false>(a, n_seqs, stream);
-    else if (shape == 3) launch_walk<T, 4, 2, kPerKey, 2, true>(a, n_seqs, stream);
-    else if (shape == 2) launch_walk<T, 2, 4, kPerKey, 2, true>(a, n_seqs, stream);
-    else launch_walk<T, 1, 4, kPerKey, 2, true>(a, n_seqs, stream);
+    else if (shape == 3) launch_brought_walk<T, 4, 2, kPerKey>(a, n_seqs, stream);
+    else if (shape == 2) launch_brought_walk<T, 2, 4, kPerKey>(a, n_seqs, stream);
+    else launch_brought_walk<T, 1, 4, kPerKey>(a, n_seqs, stream);
     return thn_launch_status("linear_attention_chunks");
 }

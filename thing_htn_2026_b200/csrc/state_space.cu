@@ -542,11 +542,11 @@ THN_API int thn_state_space_chunks(float* y, float* state, void* scratch, long l
     using namespace chunk;
     if (vdim % 64 == 0 && pairs * (vdim / 64) >= 128) {
         if (pairs * (vdim / 64) >= 384 && many_short(n_rows, n_seqs, max_tokens)) launch_walk<float, 4, 2, kPlain, 1, false>(a, n_seqs, stream);
-        else launch_walk<float, 4, 2, kPlain, 2, true>(a, n_seqs, stream);
+        else launch_brought_walk<float, 4, 2, kPlain>(a, n_seqs, stream);
     } else if (vdim % 32 == 0) {
-        launch_walk<float, 2, 4, kPlain, 2, true>(a, n_seqs, stream);
+        launch_brought_walk<float, 2, 4, kPlain>(a, n_seqs, stream);
     } else {
-        launch_walk<float, 1, 4, kPlain, 2, true>(a, n_seqs, stream);
+        launch_brought_walk<float, 1, 4, kPlain>(a, n_seqs, stream);
     }
     return thn_launch_status("state_space_chunks");
 }

@@ -1473,7 +1473,8 @@ def delta_rule(proj: torch.Tensor, conv_w: torch.Tensor, a_log: torch.Tensor, dt
     read-out, float32 [rows, heads, value_dim].  Steps of one token per sequence run as one
     kernel; others as three (prepare, recurrence, ring update), or with bfloat16 rows and keys of 128 as
     four (prepare, what a chunk of 32 tokens needs beside the state, the walk over the chunks, ring
-    update), equal up to rounding.  With float32 activations the recurrence carries the state in double between a step's first and last token."""
+    update), equal up to rounding.  With float32 activations the recurrence carries the state in double between a step's first and last token.  ``err``: the step's device error word; with one,
+    the walk over chunks may have its operands brought by warps of their own, for which the others wait a bounded time."""
     _delta_check(proj, conv_w, a_log, dt_bias, state, ring, shape, "delta_rule")
     if proj.shape[0] != rows.n_rows:
         raise KernelError(f"delta_rule: {proj.shape[0]} projected rows for a step of {rows.n_rows}")
@@ -1754,7 +1755,7 @@ def grouped_experts(x: torch.Tensor, routing: Routing, w_up: torch.Tensor, w_dow
     the chosen experts alone (tcgen05; csrc/moe_grouped.cu).  ``glu`` (limit, shared limit, alpha, up shift, weight at): experts of the form
     of ``routed_clamped_glu``, ``w_up`` [2 * (experts * ff + shared_ff), hidden]; without it those of ``routed_gelu``,
     ``w_up`` [experts * ff + shared_ff, hidden].  ``w_down`` [hidden, experts * ff + shared_ff].  ``err``: the step's device error
-    word for the kernels' bounded waits."""
+    word for the kernels' bounded waits; without one the call waits for the device and raises if a wait ran out."""
     _need(x, "grouped_experts x", torch.bfloat16)
     _need(w_up, "grouped_experts w_up", torch.bfloat16)
     _need(w_down, "grouped_experts w_down", torch.bfloat16)
@@ -1774,6 +1775,7 @@ def grouped_experts(x: torch.Tensor, routing: Routing, w_up: torch.Tensor, w_dow
     if shared_logit is not None:
         _need(shared_logit, "grouped_experts gate logits", torch.float32)
         logit_ptr, stride = shared_logit.data_ptr() + 4 * logit_column, shared_logit.shape[1]
+    word = new_error_word(x.device) if err is None else err
     n, new = rows * top, functools.partial(torch.empty, device=x.device)
     sorted_x, act, shared_act = (new(shape, dtype=x.dtype) for shape in ((n, hidden), (n, ff), (rows, shared_ff)))
     partial, weights = new((n, hidden), dtype=torch.float32), new(n, dtype=torch.float32)
@@ -1782,7 +1784,9 @@ def grouped_experts(x: torch.Tensor, routing: Routing, w_up: torch.Tensor, w_dow
     _call("thn_moe_grouped_bf16", _ptr(out), _ptr(x), _ptr(routing.chosen), _ptr(routing.dense), _ptr(w_up), _ptr(w_down), logit_ptr, stride,
           _ptr(sorted_x), _ptr(act), _ptr(shared_act), _ptr(partial), _ptr(ints), _ptr(weights), rows, hidden, n_experts, top, ff, shared_ff,
           int(glu is not None), float(limit), float(shared_limit or 1.0), float(alpha), float(up_shift), int(weight_at == "output"),
-          GROUPED_SKIP_LOADS, _ptr(err), _stream())
+          GROUPED_SKIP_LOADS, _ptr(word), _stream())
+    if err is None:
+        raise_on_device_error(word, "grouped_experts")
     return out
 
 
@@ -1878,7 +1882,8 @@ def linear_attention(proj: torch.Tensor, offsets: Tuple[int, int, int], state: t
     ``state`` float32 [slots, heads, value_dim, key_dim] is read and updated.  Returns the read-out,
     float32 [rows, heads, value_dim].  Two kernels: the inputs' activations and the decays once per
     entry into float32 scratch rows, then the recurrence; or, prompts with gated decays, bfloat16 rows and keys of 128, what a
-    chunk of 32 tokens needs beside the state, then the walk over the chunks, equal up to rounding."""
+    chunk of 32 tokens needs beside the state, then the walk over the chunks, equal up to rounding.  ``err``: the step's device error word; with one,
+    the walk over chunks may have its operands brought by warps of their own, for which the others wait a bounded time."""
     _need(proj, "linear_attention proj")
     _need(state, "linear_attention state", torch.float32)
     if (decay is None) == (gate is None):
@@ -2101,7 +2106,8 @@ def state_space(proj: torch.Tensor, offset: int, dt_pre: torch.Tensor, shape: St
     [slots, taps, channels] (position p at ``p mod taps``) are read and updated; ``seq_lens`` holds the
     tokens each slot held before the step.  Returns y float32 [rows, heads, vdim].  Steps of one token
     per sequence run as one kernel, others as three (prepare, recurrence, ring update); long bfloat16 ones
-    over a state of 128 in chunks of 32 tokens, equal up to rounding."""
+    over a state of 128 in chunks of 32 tokens, equal up to rounding.  ``err``: the step's device error word; with one,
+    the walk over chunks may have its operands brought by warps of their own, for which the others wait a bounded time."""
     _need(proj, "state_space proj")
     _need(dt_pre, "state_space dt", torch.float32)
     _need(state, "state_space state", torch.float32)

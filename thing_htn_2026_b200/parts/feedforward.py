@@ -16,7 +16,7 @@ number per token; ``shared_gated`` False: added as it is).  The up-projections o
 one product, the activation carries the routing weights (zero for an expert that was not chosen),
 and one down-projection over all experts' columns sums the chosen ones: the result does not
 depend on the other rows of the step.  With many rows the chosen experts are multiplied alone, over the rows sorted by
-expert (``ops.experts_in_groups``).  Kernels: csrc/moe.cu, csrc/moe_grouped.cu.
+expert (``ops.experts_in_groups``; in a step that has an error word for those kernels' bounded waits).  Kernels: csrc/moe.cu, csrc/moe_grouped.cu.
 
 ``polynorm``: ``down(act(up(x)))`` with ``act(z) = a N(z) + b N(z^2) + c N(z^3) + e``, powers
 taken entry by entry and ``N`` the division of a token's vector by its root mean square (``eps``
@@ -147,7 +147,7 @@ class RoutedExperts:
         err = getattr(ctx, "err", None)
         z = ops.linear(x, self.w_route, out_dtype=torch.float32, err=err)
         routing = ops.moe_route(z, self.n_experts, self.groups, self.keep, self.top, self.scale)
-        if ops.experts_in_groups(x, self.n_experts, self.top, self.ff, self.shared_ff, False):
+        if err is not None and ops.experts_in_groups(x, self.n_experts, self.top, self.ff, self.shared_ff, False):
             return ops.grouped_experts(x, routing, self.w_up, self.w_down, self.ff, self.shared_ff, None,
                                        z if self.shared_gated else None, self.n_experts, err)
         u = ops.linear(x, self.w_up, err=err)
@@ -252,7 +252,7 @@ class RoutedClampedExperts:
         err = getattr(ctx, "err", None)
         z = ops.linear(x, self.w_route, out_dtype=torch.float32, err=err)
         routing = ops.moe_route(z, self.n_experts, 1, 1, self.top, 1.0, scoring=self.scoring, renormalise=self.renormalise)
-        if ops.experts_in_groups(x, self.n_experts, self.top, self.ff, self.shared_ff, True):
+        if err is not None and ops.experts_in_groups(x, self.n_experts, self.top, self.ff, self.shared_ff, True):
             glu = (self.limit, self.shared_limit, self.slope, self.up_shift, self.weight_at)
             return ops.grouped_experts(x, routing, self.w_gate_up, self.w_down, self.ff, self.shared_ff, glu,
                                        z if self.shared_gated else None, self.n_experts, err)
