@@ -84,10 +84,10 @@ def test_state_space(heads, vdim):
     assert torch.equal(run(slice(0, cu[1]), narrow, r, n), run(slice(0, cu[1]), copied, r, n, None)) and torch.equal(narrow, copied)
 
 
-# the blocks' shapes of the matrix memory, by how many heads are walked at once: 32 columns and four warps over the keys, 64 and two,
-# 32 and two, 64 and one
-@pytest.mark.parametrize("lens,heads,vdim", [([40, 33], 16, 128), ([40] * 4, 16, 128), ([64, 31, 64, 64], 24, 96), ([40] * 6, 16, 128),
-                                             ([33, 16], 32, 64), ([40] * 9, 16, 128)])
-def test_matrix_memory(monkeypatch, lens, heads, vdim):
+# the blocks' shapes of the matrix memory (thn_mlstm_walk_shape)
+@pytest.mark.parametrize("lens,heads,vdim,shape", [([70], 16, 128, 1), ([40, 33], 16, 128, 2), ([40] * 4, 16, 128, 3), ([64, 31, 64, 64], 24, 96, 4),
+                                                   ([40] * 6, 16, 128, 4), ([33, 16], 32, 64, 2), ([40] * 9, 16, 128, 5)])
+def test_matrix_memory(monkeypatch, lens, heads, vdim, shape):
     monkeypatch.setattr(ops, "_MLSTM_COST", ops._MLSTM_COST._replace(lead=1e9))
+    assert ops.lib().thn_mlstm_walk_shape(sum(lens), max(lens), len(lens), heads, vdim) == shape
     matrix_memory_matches_64_bits(lens, heads, vdim)
