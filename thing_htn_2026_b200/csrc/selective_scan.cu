@@ -500,7 +500,7 @@ __global__ void __launch_bounds__(kWalkThreads + HELPERS, HELPERS > 128 ? 2 : 3)
 }
 
 int launch_walk(void* y, float* state, const void* x, const float* dt_pre, const float* dt_bias, const void* bc, int bc_width,
-                const float* A, const float* D, const void* z, int z_stride, const int* cu_seqlens, const int* slots, int n_rows, int n_seqs,
+                const float* A, const float* D, const void* z, int z_stride, const int* cu_seqlens, const int* slots, int n_rows, int max_tokens, int n_seqs,
                 int channels, int n_state, cudaStream_t stream) {
     using T = __nv_bfloat16;
 #define THN_WALK_LAUNCH(L, P, H, G)                                                                                               \
@@ -511,14 +511,16 @@ int launch_walk(void* y, float* state, const void* x, const float* dt_pre, const
     // blocks of four lanes (32 channels) do not fill it once.  Eight warps beside the four that walk: with four, these were what the
     // walk waited for.  But two blocks of twelve warps share a multiprocessor where three of eight do, and a wave of two takes three
     // quarters of the time of one of three: few waves that come out worse so take four, and so do very short sequences, which
-    // have little to walk.  us, eight lanes and eight warps / four and eight / four and four, 16 entries: one prompt of 2,048 tokens, 4,096
+    // have little to walk.  So do blocks that are many for the time of the longest sequence: they fill the chip either way, and with eight
+    // issue more.  us, eight lanes and eight warps / four and eight / four and four, 16 entries: one prompt of 2,048 tokens, 4,096
     // channels 118 / 132 / 177, 8,192 channels 241 / 165 / 199; 2 x 700 tokens of 4,096 channels 89 / 62 / 75; 3 x 512 85 / 78 / 68;
-    // 8 x 512 185 / 153 / 164; 64 x 16 101 / 75 / 70.  32 entries, eight / four warps: 2 x 700 150 / 181, 3 x 512 163 / 161, 4 x 512
-    // 193 / 212, 64 x 16 171 / 133.
+    // 8 x 512 185 / 153 / 164; 64 x 16 101 / 75 / 70; 64 x 128 - / 300 / 287.  32 entries, eight / four warps: 2 x 700 150 / 181, 3 x 512 163 / 161,
+    // 4 x 512 193 / 212, 64 x 16 171 / 133, 64 x 128 742 / 716.  8 entries: 64 x 128 278 / 252.
     auto blocks = [&](int lanes) { return ((long long)channels * lanes + kWalkThreads - 1) / kWalkThreads * n_seqs; };
     auto four = [&](int lanes) {
         const long long n = blocks(lanes);
-        return n_rows < 64ll * n_seqs || (n <= 6 * 148 && (n + 295) / 296 * 3 > (n + 443) / 444 * 4);
+        return n_rows < 64ll * n_seqs || (n <= 6 * 148 && (n + 295) / 296 * 3 > (n + 443) / 444 * 4) ||
+               n * std::min(1.0, (double)n_rows / n_seqs / max_tokens) > (lanes == 4 ? 10 : 16) * 148;
     };
     if (n_state <= 8) {
         if (four(4)) THN_WALK_LAUNCH(4, 2, 128, 1);
@@ -638,8 +640,8 @@ THN_API int thn_selective_scan(void* y, float* state, const void* x, const float
         return launch_scan<float>(y, state, x, dt_pre, dt_bias, bc, bc_width, A, D, z, z_stride, cu_seqlens, slots, n_seqs,
                                   channels, n_state, stream);
     if (dtype == THN_BF16 && n_state <= 32 && walk_pays(n_rows, max_tokens, n_seqs, channels))
-        return launch_walk(y, state, x, dt_pre, dt_bias, bc, bc_width, A, D, z, z_stride, cu_seqlens, slots, n_rows, n_seqs, channels,
-                           n_state, stream);
+        return launch_walk(y, state, x, dt_pre, dt_bias, bc, bc_width, A, D, z, z_stride, cu_seqlens, slots, n_rows, max_tokens, n_seqs,
+                           channels, n_state, stream);
     if (dtype == THN_BF16)
         return launch_scan<__nv_bfloat16>(y, state, x, dt_pre, dt_bias, bc, bc_width, A, D, z, z_stride, cu_seqlens, slots,
                                           n_seqs, channels, n_state, stream);
