@@ -59,7 +59,7 @@ def test_a_scratch_that_is_too_small_is_refused():
     need = ops.lib().thn_mlstm_chunks_scratch_bytes(n, seqs, heads)
     with pytest.raises(ops.KernelError, match=f"{need - 1} bytes of scratch, {need} needed"):
         ops._call("thn_mlstm_chunks", at, at, at, at, need - 1, at, 3 * heads * 128, at, at, at, 15.0, at, at, n, 2048, seqs, heads, 128, 128, 1.0, 1e-6,
-                  None, None)
+                  None)
     need = ops.lib().thn_delta_chunks_scratch_bytes(n, heads, 16, 128)
     shape = ops.DeltaShape(heads, 16, 128, 128, 4)
     with pytest.raises(ops.KernelError, match=f"{need - 1} bytes of scratch, {need} needed"):

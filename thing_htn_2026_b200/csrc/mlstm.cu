@@ -541,7 +541,7 @@ THN_API int thn_mlstm_walk_shape(int n_rows, int max_tokens, int n_seqs, int n_h
 THN_API int thn_mlstm_chunks(float* o, float* S, float* nm, void* scratch, long long scratch_bytes, const void* proj, int proj_width, const float* gate_pre,
                              const float* bias_i, const float* bias_f, float cap, const int* cu_seqlens, const int* slots, int n_rows,
                              int max_tokens, int n_seqs, int n_heads, int key_dim, int value_dim, float q_scale, float floor_,
-                             int* err, cudaStream_t stream) {
+                             cudaStream_t stream) {
     THN_CHECK_ARG(n_seqs >= 0 && n_heads > 0 && cap > 0.f && proj_width >= n_heads * (2 * key_dim + value_dim), "mlstm_chunks: bad sizes");
     THN_UNSUPPORTED_IF(key_dim != chunk::kKeys || value_dim <= 0 || value_dim % 16 != 0 || proj_width % 8 != 0,
                        "mlstm_chunks: keys of %d, values of %d, rows of %d", key_dim, value_dim, proj_width);
@@ -558,7 +558,6 @@ THN_API int thn_mlstm_chunks(float* o, float* S, float* nm, void* scratch, long 
     thn_launch(mlstm_chunk_kernel, dim3(chunks, n_heads, n_seqs), kChunkThreads, 0, stream, scores, scalars, key_sums, rows, proj_width,
                gate_pre, bias_i, bias_f, cap, cu_seqlens, n_rows, n_heads);
     chunk::WalkArgs a{};
-    a.err = err;
     a.o = o; a.state = S;
     a.q = rows; a.k = rows + (size_t)n_heads * key_dim;
     a.key_plane = 0; a.key_unit = key_dim; a.key_row = proj_width;

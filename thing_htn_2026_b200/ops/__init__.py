@@ -123,7 +123,7 @@ _SIGNATURES = {
                              c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_float, c_int, c_void_p],
     "thn_mlstm_walk_shape": [c_int, c_int, c_int, c_int, c_int],
     "thn_mlstm_chunks": [c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_float, c_void_p,
-                         c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p, c_void_p],
+                         c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_float, c_void_p],
     "thn_moe_route": [c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_float,
                       c_int, c_int, c_float, c_void_p],
     "thn_routed_gelu": [c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_int, c_int, c_void_p],
@@ -1608,7 +1608,7 @@ def _mlstm_in_chunks(proj: torch.Tensor, state: torch.Tensor, rows: StepRows, n_
 
 def mlstm(proj: torch.Tensor, gate_pre: torch.Tensor, bias_i: torch.Tensor, bias_f: torch.Tensor, cap: float,
           state: torch.Tensor, normaliser: torch.Tensor, rows: StepRows, n_heads: int, key_dim: int, value_dim: int,
-          q_scale: float, floor: float = 1e-6, err: Optional[torch.Tensor] = None) -> torch.Tensor:
+          q_scale: float, floor: float = 1e-6) -> torch.Tensor:
     """The matrix-memory recurrence over a step's rows.  ``proj`` rows hold ``[q | k | v | ...]``
     (heads * key_dim, heads * key_dim, heads * value_dim); ``gate_pre`` float32 [rows, 2 * heads]
     the pre-activations of the input gates, then of the forget gates (biases are added here).
@@ -1635,7 +1635,7 @@ def mlstm(proj: torch.Tensor, gate_pre: torch.Tensor, bias_i: torch.Tensor, bias
                               device=proj.device)
         _call("thn_mlstm_chunks", _ptr(o), _ptr(state), _ptr(normaliser), _ptr(scratch), scratch.numel(), _ptr(proj), proj.shape[1], _ptr(gate_pre),
               _ptr(bias_i), _ptr(bias_f), float(cap), _ptr(rows.cu_seqlens), _ptr(rows.slots), n, rows.max_q_len, rows.n_seqs, n_heads,
-              key_dim, value_dim, float(q_scale), float(floor), _ptr(err), _stream())
+              key_dim, value_dim, float(q_scale), float(floor), _stream())
         return o
     raw = rows.max_q_len == 1
     gates = gate_pre

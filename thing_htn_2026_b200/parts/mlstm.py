@@ -76,7 +76,7 @@ class MatrixMemory:
         gate_pre = ops.linear(x, self.w_gates, out_dtype=torch.float32, err=ctx.err)
         o = ops.mlstm(proj, gate_pre, self.bias_i, self.bias_f, self.cap, ctx.cache.state_view(entry.cache, 0),
                       ctx.cache.state_view(entry.cache, 1), ctx.rows, self.n_heads, self.key_dim, self.value_dim,
-                      self.key_dim ** -0.5, self.floor, ctx.err)
+                      self.key_dim ** -0.5, self.floor)
         y = ops.gated_head_norm(o, proj, self.gate_offset, self.out_gain, self.norm_eps, self.n_heads, self.value_dim,
                                 self.dtype, gate_kind="logistic")
         return ops.linear(y, self.w_o, err=ctx.err)
