@@ -27,8 +27,14 @@ struct Source {
 
 __device__ __forceinline__ unsigned long long floats_of(uint32_t two) { return pack2(__uint_as_float(two << 16), __uint_as_float(two & 0xffff0000u)); }
 
+// Steps of few entries, for which the time of a launch counts: every row finds its place alone, all rows' places and the sequences' lengths
+// ahead of the first result.  (A first look that decides between two ways waits once more, and more instructions are fetched; us with / without, 16 to 512 rows
+// of 1,024 channels 5.2 / 4.4, 100 rows of 10,240 5.7 / 5.5, 2,048 of 1,024 6.6 / 7.1, 512 of 4,096 6.3 / 7.0.)
+constexpr long long kFewEntries = 1200000;
+inline bool few_entries(int n_rows, int channels) { return (long long)n_rows * channels <= kFewEntries; }
+
 // put(r, y): the four results of row r, for r in [0, n_here).  w[i][j]: tap j of channel i.  `first`: the run's first row's number.
-template <int ROWS, typename Put>
+template <int ROWS, bool FEW, typename Put>
 __device__ __forceinline__ void run(const Source& s, int first, int n_here, const float (&w)[4][kTaps], const float (&bias)[4], Put&& put) {
     uint2 raw[ROWS + kTaps - 1];       // raw[j]: the row j - 3 rows after `first`
 #pragma unroll
@@ -36,9 +42,22 @@ __device__ __forceinline__ void run(const Source& s, int first, int n_here, cons
         const int back = kTaps - 1 - j;
         raw[j] = back <= first && -back < n_here ? *reinterpret_cast<const uint2*>(s.rows - (long long)back * s.row_stride) : make_uint2(0, 0);
     }
-    const int slot0 = s.row_slot[first], pos0 = s.row_pos[first], last = first + n_here - 1;
-    const int slot1 = s.row_slot[last], pos1 = s.row_pos[last];
-    if (n_here == ROWS && slot0 == slot1 && pos1 - pos0 == ROWS - 1 && pos0 - s.seq_lens[slot0] >= kTaps - 1) {
+    int slot[ROWS], pos[ROWS], local[ROWS];       // (FEW) local: a row's index among its sequence's rows of this step
+    bool inside = false;
+    if constexpr (FEW) {
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            slot[r] = s.row_slot[first + min(r, n_here - 1)];
+            pos[r] = s.row_pos[first + min(r, n_here - 1)];
+        }
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) local[r] = pos[r] - s.seq_lens[slot[r]];
+    } else {
+        const int slot0 = s.row_slot[first], pos0 = s.row_pos[first], last = first + n_here - 1;
+        const int slot1 = s.row_slot[last], pos1 = s.row_pos[last];
+        inside = n_here == ROWS && slot0 == slot1 && pos1 - pos0 == ROWS - 1 && pos0 - s.seq_lens[slot0] >= kTaps - 1;
+    }
+    if (inside) {
         unsigned long long w01[kTaps], w23[kTaps], x01[kTaps], x23[kTaps];
         const unsigned long long b01 = pack2(bias[0], bias[1]), b23 = pack2(bias[2], bias[3]);
 #pragma unroll
@@ -70,16 +89,20 @@ __device__ __forceinline__ void run(const Source& s, int first, int n_here, cons
 #pragma unroll
     for (int r = 0; r < ROWS; ++r) {
         if (r >= n_here) break;
-        const int slot = s.row_slot[first + r], pos = s.row_pos[first + r], local = pos - s.seq_lens[slot];   // its index among its sequence's rows of this step
+        if constexpr (!FEW) {
+            slot[r] = s.row_slot[first + r];
+            pos[r] = s.row_pos[first + r];
+            local[r] = pos[r] - s.seq_lens[slot[r]];
+        }
         uint2 in[kTaps];
 #pragma unroll
         for (int j = 0; j < kTaps; ++j) in[j] = raw[r + j];
-        if (local < kTaps - 1) {
+        if (local[r] < kTaps - 1) {
 #pragma unroll
             for (int back = 1; back < kTaps; ++back) {
-                if (back <= local) continue;
-                in[kTaps - 1 - back] = back > pos ? make_uint2(0, 0)           // before the sequence's start
-                    : *reinterpret_cast<const uint2*>(s.ring + ((size_t)slot * kTaps + (pos - back) % kTaps) * s.channels);
+                if (back <= local[r]) continue;
+                in[kTaps - 1 - back] = back > pos[r] ? make_uint2(0, 0)           // before the sequence's start
+                    : *reinterpret_cast<const uint2*>(s.ring + ((size_t)slot[r] * kTaps + (pos[r] - back) % kTaps) * s.channels);
             }
         }
         float y[4];
@@ -88,7 +111,7 @@ __device__ __forceinline__ void run(const Source& s, int first, int n_here, cons
             float acc = bias[i];
 #pragma unroll
             for (int j = 0; j < kTaps; ++j) {
-                if (kTaps - 1 - j > pos) continue;
+                if (kTaps - 1 - j > pos[r]) continue;
                 const uint32_t two = i < 2 ? in[j].x : in[j].y;
                 acc = fmaf(w[i][j], __uint_as_float(i & 1 ? two & 0xffff0000u : two << 16), acc);
             }

@@ -331,6 +331,7 @@ constexpr size_t recurrence_smem() {
 constexpr int kRunRows = 8;
 constexpr int kRunTaps = 4;
 
+template <bool FEW>
 __global__ void __launch_bounds__(128) delta_prepare_chunks_kernel(
     __nv_bfloat16* __restrict__ planes, float* __restrict__ values, float* __restrict__ beta, float* __restrict__ decay,
     const __nv_bfloat16* __restrict__ proj, const float* __restrict__ conv_w, const float* __restrict__ a_log,
@@ -367,7 +368,7 @@ __global__ void __launch_bounds__(128) delta_prepare_chunks_kernel(
     float* value_dst = values + ((size_t)(is_value ? vc / s.dv : 0) * n_rows + first) * s.dv + (is_value ? vc % s.dv : 0);
     const float none[4] = {0.f, 0.f, 0.f, 0.f};
     const conv_run::Source source{proj + (size_t)first * s.proj_width + c, s.proj_width, ring + c, C, row_slot, row_pos, seq_lens};
-    conv_run::run<kRunRows>(source, first, n_here, w, none, [&](int r, const float (&y)[4]) {
+    conv_run::run<kRunRows, FEW>(source, first, n_here, w, none, [&](int r, const float (&y)[4]) {
         if (is_value) {
             *reinterpret_cast<float4*>(value_dst + (size_t)r * s.dv) = make_float4(y[0], y[1], y[2], y[3]);
         } else {
@@ -948,7 +949,7 @@ THN_API int thn_delta_chunks(float* o, float* state, void* scratch, long long sc
     float* beta = reinterpret_cast<float*>(scalars + (size_t)n_heads * n_rows);
     float* decay = beta + (size_t)n_heads * n_rows;
     const int items = s.conv_channels() / 4 + n_heads;
-    thn_launch(delta_prepare_chunks_kernel, dim3((items + 127) / 128, (n_rows + kRunRows - 1) / kRunRows), 128, 0, stream, planes,
+    thn_launch(conv_run::few_entries(n_rows, s.conv_channels()) ? delta_prepare_chunks_kernel<true> : delta_prepare_chunks_kernel<false>, dim3((items + 127) / 128, (n_rows + kRunRows - 1) / kRunRows), 128, 0, stream, planes,
                values, beta, decay, (const __nv_bfloat16*)proj, conv_w, a_log, dt_bias, (const __nv_bfloat16*)ring, row_slot, row_pos,
                seq_lens, n_rows, s, unit_eps);
     const dim3 chunks((max_tokens + chunk::kTokens - 1) / chunk::kTokens, n_heads, n_seqs);

@@ -69,6 +69,7 @@ __global__ void causal_conv_kernel(T* __restrict__ out, const T* __restrict__ pr
 constexpr int kConvTaps = 4;
 constexpr int kConvRows = 8;
 
+template <bool FEW>
 __global__ void __launch_bounds__(128) causal_conv_vec_kernel(
     __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ proj, int proj_width, int offset,
     const float* __restrict__ weight, const float* __restrict__ bias, const __nv_bfloat16* __restrict__ ring,
@@ -88,7 +89,7 @@ __global__ void __launch_bounds__(128) causal_conv_vec_kernel(
     pdl_wait();
     __nv_bfloat16* dst = out + (size_t)first * channels + c;
     const conv_run::Source source{proj + (size_t)first * proj_width + offset + c, proj_width, ring + c, channels, row_slot, row_pos, seq_lens};
-    conv_run::run<kConvRows>(source, first, n_here, w, b, [&](int t, const float (&y)[4]) {
+    conv_run::run<kConvRows, FEW>(source, first, n_here, w, b, [&](int t, const float (&y)[4]) {
         const __nv_bfloat162 lo = __floats2bfloat162_rn(y[0], y[1]), hi = __floats2bfloat162_rn(y[2], y[3]);
         *reinterpret_cast<uint2*>(dst + (size_t)t * channels) =
             make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
@@ -588,7 +589,8 @@ THN_API int thn_causal_conv(void* out, const void* proj, int proj_width, int off
     const bool pieces = channels % 4 == 0 && offset % 4 == 0 && proj_width % 4 == 0 &&
                         (((uintptr_t)out | (uintptr_t)proj | (uintptr_t)ring) & 7) == 0 && ((uintptr_t)weight & 15) == 0;
     if (dtype == THN_BF16 && taps == kConvTaps && pieces && (n_rows + kConvRows - 1) / kConvRows <= 65535)
-        thn_launch(causal_conv_vec_kernel, dim3((unsigned)((channels / 4 + 127) / 128), (unsigned)((n_rows + kConvRows - 1) / kConvRows)),
+        thn_launch(conv_run::few_entries(n_rows, channels) ? causal_conv_vec_kernel<true> : causal_conv_vec_kernel<false>,
+                   dim3((unsigned)((channels / 4 + 127) / 128), (unsigned)((n_rows + kConvRows - 1) / kConvRows)),
                    128, 0, stream, (__nv_bfloat16*)out, (const __nv_bfloat16*)proj, proj_width, offset, weight, bias,
                    (const __nv_bfloat16*)ring, row_slot, row_pos, seq_lens, n_rows, channels);
     else if (dtype == THN_F32)

@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(kPrepareThreads, 6) state_space_prepare_chunks
     __nv_bfloat16* key_dst = planes + ((in_part / chunk::kKeys) * 2 + which) * 3 * plane + (long long)first * chunk::kKeyRow + in_part % chunk::kKeys;
     float* value_dst = values + ((size_t)(is_value ? c / shape.vdim : 0) * n_rows + first) * shape.vdim + (is_value ? c % shape.vdim : 0);
     const conv_run::Source source{proj + (size_t)first * proj_width + offset + c, proj_width, ring + c, C, row_slot, row_pos, seq_lens};
-    conv_run::run<kRunRows>(source, first, n_here, w, b, [&](int r, const float (&y)[4]) {
+    conv_run::run<kRunRows, false>(source, first, n_here, w, b, [&](int r, const float (&y)[4]) {
         if (is_value) {
             *reinterpret_cast<float4*>(value_dst + (size_t)r * shape.vdim) = make_float4(y[0], y[1], y[2], y[3]);
         } else {
