@@ -670,14 +670,15 @@ THN_API int thn_moe_grouped_bf16(void* out, const void* x, const int* chosen, co
     int* place = sorted_row + n;
     thn_launch(moe_sort_kernel, n_experts, kSortThreads, 0, stream, offsets, sorted_row, floats, place, chosen, dense, n, top, n_experts);
     thn_launch(moe_gather_kernel, (n + 7) / 8, 256, 0, stream, (uint4*)sorted_x, (const uint4*)x, sorted_row, n, hidden / 8);
-    CUtensorMap map_up, map_down, map_sorted, map_x, map_act, map_shared;
-    if (!make_map(&map_up, w_up, (glu ? 2LL : 1LL) * width, hidden, 64) || !make_map(&map_down, w_down, hidden, width, 64) ||
-        !make_map(&map_sorted, sorted_x, n, hidden, kRows / 2) || !make_map(&map_x, x, n_rows, hidden, kRows / 2) ||
-        !make_map(&map_act, act, n, ff, kRows / 2) ||
-        !make_map(&map_shared, shared_ff ? shared_act : act, shared_ff ? n_rows : n, shared_ff ? shared_ff : ff, tile_rows(kCombine) / 2)) {
+    // (a launch's maps are made just ahead of it: the host works while the device sorts, gathers and multiplies)
+    auto no_map = [&] {
         thn_set_error("moe_grouped: cuTensorMapEncodeTiled failed for %d rows of %d, %d experts of %d", n_rows, hidden, n_experts, ff);
         return THN_BAD_ARGUMENT;
-    }
+    };
+    CUtensorMap map_up, map_down, map_sorted, map_x, map_act, map_shared;
+    if (!make_map(&map_up, w_up, (glu ? 2LL : 1LL) * width, hidden, 64) || !make_map(&map_sorted, sorted_x, n, hidden, kRows / 2) ||
+        !make_map(&map_x, x, n_rows, hidden, kRows / 2))
+        return no_map();
     PairArgs up = {};
     up.n_experts = n_experts;
     up.offsets = offsets;
@@ -704,6 +705,7 @@ THN_API int thn_moe_grouped_bf16(void* out, const void* x, const int* chosen, co
     int status = glu ? launch_pairs<kGlu>(map_up, map_sorted, map_x, up, up_tiles, stream)
                      : launch_pairs<kGelu>(map_up, map_sorted, map_x, up, up_tiles, stream);
     if (status != THN_OK) return status;
+    if (!make_map(&map_down, w_down, hidden, width, 64) || !make_map(&map_act, act, n, ff, kRows / 2)) return no_map();
     PairArgs down = {};
     down.n_experts = n_experts;
     down.offsets = offsets;
@@ -718,6 +720,7 @@ THN_API int thn_moe_grouped_bf16(void* out, const void* x, const int* chosen, co
         thn_launch(moe_combine_kernel, dim3(n_rows, (hidden / 4 + 255) / 256), 256, 0, stream, (__nv_bfloat16*)out, partial, place, hidden, top);
         return thn_launch_status("moe_combine");
     }
+    if (!make_map(&map_shared, shared_act, n_rows, shared_ff, tile_rows(kCombine) / 2)) return no_map();
     PairArgs sum = {};
     sum.n_rows = n_rows;
     sum.n_features = sum.shared_features = hidden;

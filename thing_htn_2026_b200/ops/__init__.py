@@ -7,7 +7,6 @@ else, and every product of the 32-bit path, is this library's own kernel.
 from __future__ import annotations
 
 import ctypes
-import functools
 import os
 from dataclasses import dataclass
 from typing import Dict, NamedTuple, Optional, Tuple
@@ -1777,13 +1776,15 @@ def grouped_experts(x: torch.Tensor, routing: Routing, w_up: torch.Tensor, w_dow
         _need(shared_logit, "grouped_experts gate logits", torch.float32)
         logit_ptr, stride = shared_logit.data_ptr() + 4 * logit_column, shared_logit.shape[1]
     word = new_error_word(x.device) if err is None else err
-    n, new = rows * top, functools.partial(torch.empty, device=x.device)
-    sorted_x, act, shared_act = (new(shape, dtype=x.dtype) for shape in ((n, hidden), (n, ff), (rows, shared_ff)))
-    partial, weights = new((n, hidden), dtype=torch.float32), new(n, dtype=torch.float32)
-    ints = new(2 * n + n_experts + 1, dtype=torch.int32)
+    # one piece of scratch: a call's host work is a good part of a short prompt's time
+    n, at = rows * top, [0]
+    for size in (2 * n * hidden, 2 * n * ff, 2 * rows * shared_ff, 4 * n * hidden, 4 * (2 * n + n_experts + 1), 4 * n):
+        at.append(at[-1] + (size + 255) // 256 * 256)
+    scratch = torch.empty(at[-1], dtype=torch.uint8, device=x.device)
+    sorted_x, act, shared_act, partial, ints, weights = (scratch.data_ptr() + a for a in at[:-1])
     out = torch.empty_like(x)
     _call("thn_moe_grouped_bf16", _ptr(out), _ptr(x), _ptr(routing.chosen), _ptr(routing.dense), _ptr(w_up), _ptr(w_down), logit_ptr, stride,
-          _ptr(sorted_x), _ptr(act), _ptr(shared_act), _ptr(partial), _ptr(ints), _ptr(weights), rows, hidden, n_experts, top, ff, shared_ff,
+          sorted_x, act, shared_act, partial, ints, weights, rows, hidden, n_experts, top, ff, shared_ff,
           int(glu is not None), float(limit), float(shared_limit or 1.0), float(alpha), float(up_shift), int(weight_at == "output"),
           GROUPED_SKIP_LOADS, _ptr(word), _stream())
     if err is None:
