@@ -20,6 +20,24 @@ def test_rule():
     assert not ops.experts_in_groups(x, 512, 2, 64, 0, True)
 
 
+# sizes, gated, rows: us in the dense form, in groups (B200, cold weights)
+MEASURED = [((2048, 8, 2, 1024, 1024), True, 640, 70, 77), ((2048, 8, 2, 1024, 1024), True, 896, 95, 76), ((2048, 8, 2, 1024, 1024), False, 1024, 73, 73),
+            ((2048, 8, 2, 1024, 1024), False, 2048, 126, 104), ((4096, 8, 2, 2048, 2048), True, 288, 126, 145), ((4096, 8, 2, 2048, 2048), True, 384, 149, 153),
+            ((4096, 8, 2, 2048, 2048), True, 448, 177, 150), ((4096, 8, 2, 2048, 2048), False, 512, 128, 131), ((4096, 8, 2, 2048, 2048), False, 768, 178, 159),
+            ((2048, 64, 6, 512, 512), True, 192, 115, 126), ((2048, 64, 6, 512, 512), True, 256, 135, 125), ((2048, 64, 6, 512, 512), False, 288, 109, 113),
+            ((2048, 16, 4, 1024, 0), True, 448, 98, 74), ((4096, 64, 8, 256, 0), True, 256, 119, 138), ((4096, 64, 8, 256, 0), True, 384, 140, 153),
+            ((4096, 64, 8, 256, 0), True, 640, 210, 180), ((4096, 16, 1, 2048, 0), True, 256, 209, 181), ((2048, 128, 8, 256, 256), True, 288, 130, 144),
+            ((2048, 128, 8, 256, 256), True, 448, 179, 153), ((7168, 32, 8, 512, 512), True, 352, 219, 267), ((7168, 32, 8, 512, 512), True, 576, 341, 273)]
+
+
+@pytest.mark.parametrize("sizes,gated,rows,dense,grouped", MEASURED)
+def test_the_faster_form_is_taken(sizes, gated, rows, dense, grouped):
+    from thing_htn_2026_b200 import ops
+    hidden, n_experts, top, ff, shared_ff = sizes
+    taken = grouped if ops.experts_in_groups(torch.empty(rows, hidden, dtype=torch.bfloat16), n_experts, top, ff, shared_ff, gated) else dense
+    assert taken <= 1.02 * min(dense, grouped)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind", ["routed_glu_experts", "routed_clamped_experts", "routed_experts"])
 def test_a_part_gives_the_same_on_both_sides(kind, monkeypatch):
