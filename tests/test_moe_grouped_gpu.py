@@ -87,6 +87,23 @@ def test_a_row_does_not_depend_on_the_others():
     assert torch.equal(alone, got[pick])
 
 
+@pytest.mark.parametrize("form", ["clamped", "gelu"])
+def test_a_step_in_pieces_gives_the_same(form, monkeypatch):
+    """Scratch that would be larger than the dense form's is taken for some of the rows at a time."""
+    from thing_htn_2026_b200 import ops
+    glu, hidden, experts, top, ff, shared_ff = {"clamped": CLAMPED, "gelu": None}[form], 512, 8, 4, 64, 64
+    x, z = rand((700, hidden), 1).bfloat16(), rand((700, experts + 1), 4)
+    width = experts * ff + shared_ff
+    w_up, w_down = rand(((2 if glu else 1) * width, hidden), 2, hidden ** -0.5).bfloat16(), rand((hidden, width), 3, ff ** -0.5).bfloat16()
+    routing = ops.moe_route(z, experts, 1, 1, top, 1.0, scoring="softmax_chosen")
+    whole = ops.grouped_experts(x, routing, w_up, w_down, ff, shared_ff, glu, z, experts)
+    calls, inner = [], ops._call
+    monkeypatch.setattr(ops, "GROUPED_SCRATCH", 0)
+    monkeypatch.setattr(ops, "_call", lambda name, *a: calls.append(name) or inner(name, *a))
+    pieces = ops.grouped_experts(x, routing, w_up, w_down, ff, shared_ff, glu, z, experts)
+    assert len(calls) == (4 if glu else 6) and torch.equal(whole, pieces)
+
+
 def test_a_row_that_is_not_a_number_stays_alone():
     from thing_htn_2026_b200 import ops
     x, routing, got, (w_up, w_down, z) = check(300, 256, 8, 2, 128, 0, SILU, False)

@@ -1741,6 +1741,7 @@ GROUPED_MIN_ROWS = 256
 GROUPED_ANY_ROWS = {True: 448, False: 640}           # gated, gelu
 GROUPED_MIN_SAVED = {True: 60e9, False: 100e9}
 GROUPED_FEW_ROWS_FF, GROUPED_FEW_ROWS_SHARE = 512, 8     # with fewer rows: columns of an expert; columns left out over columns multiplied
+GROUPED_SCRATCH = 1 << 30    # bytes of scratch that a call takes if the dense form would take less
 GROUPED_SKIP_LOADS = 0       # the test of the products' bounded waits sets it: nothing is loaded
 
 
@@ -1782,17 +1783,24 @@ def grouped_experts(x: torch.Tensor, routing: Routing, w_up: torch.Tensor, w_dow
         _need(shared_logit, "grouped_experts gate logits", torch.float32)
         logit_ptr, stride = shared_logit.data_ptr() + 4 * logit_column, shared_logit.shape[1]
     word = new_error_word(x.device) if err is None else err
-    # one piece of scratch: a call's host work is a good part of a short prompt's time
-    n, at = rows * top, [0]
-    for size in (2 * n * hidden, 2 * n * ff, 2 * rows * shared_ff, 4 * n * hidden, 4 * (2 * n + n_experts + 1), 4 * n):
+    # one piece of scratch: a call's host work is a good part of a short prompt's time.  No more of it than the dense form would take, or
+    # GROUPED_SCRATCH bytes: the rows of a longer step go piece by piece (a row's result does not depend on the others)
+    scratch_row = top * (6 * hidden + 2 * ff + 12) + 2 * shared_ff
+    most = max(GROUPED_SCRATCH, rows * width * (4 if glu is None else 6))
+    pieces = max(1, -(-rows * scratch_row // most))
+    at_once = -(-rows // pieces)
+    n, at = at_once * top, [0]
+    for size in (2 * n * hidden, 2 * n * ff, 2 * at_once * shared_ff, 4 * n * hidden, 4 * (2 * n + n_experts + 1), 4 * n):
         at.append(at[-1] + (size + 255) // 256 * 256)
     scratch = torch.empty(at[-1], dtype=torch.uint8, device=x.device)
     sorted_x, act, shared_act, partial, ints, weights = (scratch.data_ptr() + a for a in at[:-1])
     out = torch.empty_like(x)
-    _call("thn_moe_grouped_bf16", _ptr(out), _ptr(x), _ptr(routing.chosen), _ptr(routing.dense), _ptr(w_up), _ptr(w_down), logit_ptr, stride,
-          sorted_x, act, shared_act, partial, ints, weights, rows, hidden, n_experts, top, ff, shared_ff,
-          int(glu is not None), float(limit), float(shared_limit or 1.0), float(alpha), float(up_shift), int(weight_at == "output"),
-          GROUPED_SKIP_LOADS, _ptr(word), _stream())
+    for row in range(0, rows, max(1, at_once)):
+        _call("thn_moe_grouped_bf16", out.data_ptr() + 2 * row * hidden, x.data_ptr() + 2 * row * hidden, routing.chosen.data_ptr() + 4 * row * top,
+              routing.dense.data_ptr() + 4 * row * n_experts, _ptr(w_up), _ptr(w_down), None if logit_ptr is None else logit_ptr + 4 * row * stride, stride,
+              sorted_x, act, shared_act, partial, ints, weights, min(at_once, rows - row), hidden, n_experts, top, ff, shared_ff,
+              int(glu is not None), float(limit), float(shared_limit or 1.0), float(alpha), float(up_shift), int(weight_at == "output"),
+              GROUPED_SKIP_LOADS, _ptr(word), _stream())
     if err is None:
         raise_on_device_error(word, "grouped_experts")
     return out
