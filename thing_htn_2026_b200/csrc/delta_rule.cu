@@ -22,6 +22,8 @@
 // and from the ring otherwise; positions before the sequence's start read as zero.
 #include <math.h>
 
+#include <algorithm>
+
 #include "chunk_walk.cuh"
 #include "conv_run.cuh"
 #include "common.cuh"
@@ -953,7 +955,11 @@ THN_API int thn_delta_chunks(float* o, float* state, void* scratch, long long sc
                values, beta, decay, (const __nv_bfloat16*)proj, conv_w, a_log, dt_bias, (const __nv_bfloat16*)ring, row_slot, row_pos,
                seq_lens, n_rows, s, unit_eps);
     const dim3 chunks((max_tokens + chunk::kTokens - 1) / chunk::kTokens, n_heads, n_seqs);
-    if (n_heads / n_kv % 2 == 0) {
+    // Two heads a block share their products, but its longer program and its 98 KB pay only once blocks of one head would not all be on the chip
+    // together (three to a multiprocessor).  us of the whole call, two / one: 16 tokens of 32 heads 31.2 / 28.9, 16 x 128 of 4 heads 54.6 / 52.5, 512 tokens of 16 heads
+    // 59.6 / 58.8, of 32 heads 81.3 / 88.3, 2,048 tokens of 16 heads 176.6 / 183.3.
+    const long long longest = chunks.x, all = std::min(n_seqs * longest, n_rows / chunk::kTokens + (long long)n_seqs) * n_heads;      // at most
+    if (n_heads / n_kv % 2 == 0 && all > 3 * 148) {
         cudaFuncSetAttribute(delta_chunk_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, delta_chunk_bytes(2));
         thn_launch(delta_chunk_kernel<2>, dim3(chunks.x, n_heads / 2, n_seqs), 256, delta_chunk_bytes(2), stream, values, w, scores, scalars, planes,
                    beta, decay, cu_seqlens, n_rows, s);
