@@ -1435,20 +1435,20 @@ class _ChunkCost(NamedTuple):
         return max(self.chunk_chain * longest, self.chunk * chunks * heads) <= by_token + self.lead
 
 
-# Measured on B200, token by token / in chunks, us of the whole call; "a + b": one prompt of a tokens beside b single ones.
-#   delta rule, 16 heads of 128: 16 + 0 65 / 52, 16 + 60 91 / 187, 128 + 8 116 / 79, 128 + 60 142 / 192, 512 + 60 296 / 224,
-#     2,048 + 0 658 / 241, 2,048 + 60 1,054 / 542, 64 prompts of 33 tokens 294 / 319, 32 of 128 511 / 341
-_DELTA_COST = _ChunkCost(0.4, 0.007, 0.02, 3.0, 0.14, 12.0, 128)
-#   matrix memory, 16 heads of 128: 16 + 0 17 / 15, 16 + 60 52 / 69, 33 + 60 62 / 71, 128 + 60 116 / 73, 2,048 + 60 1,223 / 390,
-#     64 prompts of 16 tokens 173 / 77
+# Measured on B200, token by token / in chunks, us of the whole call in a graph; "a + b": a prompt of a tokens, or several, beside b single ones.
+#   delta rule, 16 heads of 128: 16 + 0 52 / 28, 16 + 8 57 / 37, 16 + 60 78 / 143, 128 + 8 100 / 50, 128 + 60 123 / 151, 512 + 60 294 / 186,
+#     2,048 + 0 658 / 177, 2,048 + 60 940 / 461, 33 + 0 (64 prompts) 284 / 292, 128 + 0 (32 prompts) 520 / 300
+_DELTA_COST = _ChunkCost(0.451, 0.0059, 0.0225, 3.0, 0.1152, 12.0, 128)
+#   matrix memory, 16 heads of 128: 16 + 0 10 / 8, 16 + 8 16 / 17, 16 + 60 41 / 60, 33 + 60 50 / 60, 128 + 60 108 / 62,
+#     2,048 + 60 1,320 / 210, 16 + 0 (64 prompts) 158 / 66
 _MLSTM_COST = _ChunkCost(0.5, 0.009, 0.03, 1.8, 0.055, 0.0, 128)
-#   state-space duality, 64 heads of 64: 96 + 0 38 / 43, 128 + 0 44 / 42, 128 + 60 108 / 171, 512 + 8 142 / 122, 512 + 60 151 / 198,
-#     2,048 + 60 517 / 460, 32 prompts of 128 tokens 568 / 349
+#   state-space duality, 64 heads of 64: 128 + 0 32 / 34, 128 + 8 41 / 51, 128 + 60 97 / 165, 512 + 8 128 / 112, 512 + 60 139 / 187,
+#     2,048 + 0 349 / 184, 2,048 + 60 494 / 322, 128 + 0 (32 prompts) 541 / 314
 _SPACE_COST = _ChunkCost(0.205, 0.0021, 0.016, 3.1, 0.035, -10.0, 64)
-#   linear attention with gated decays, 32 heads of 128: 16 + 0 15 / 24, 64 + 0 24 / 28, 128 + 0 36 / 32, 300 + 0 65 / 50, 2,048 + 0 368 / 222,
-#     16 + 60 103 / 155, 512 + 60 181 / 241, 2,048 + 60 419 / 439, 64 prompts of 16 tokens 247 / 183; 16 heads: 128 + 0 28 / 30, 300 + 0 50 / 42,
-#     2,048 + 0 263 / 155, 2,048 + 60 335 / 259
-_LINEAR_COST = _ChunkCost(0.128, 0.0055, 0.045, 2.6, 0.082, -12.0, 128)
+#   linear attention with gated decays, 32 heads of 128: 16 + 0 7 / 16, 64 + 0 15 / 23, 128 + 0 26 / 33, 300 + 0 55 / 44, 16 + 60 97 / 146, 512 + 60 174 / 212,
+#     2,048 + 0 358 / 184, 2,048 + 60 410 / 402, 16 + 0 (64 prompts) 238 / 176; 16 heads: 128 + 0 19 / 24, 300 + 0 40 / 38, 2,048 + 0 255 / 125,
+#     512 + 60 93 / 137, 2,048 + 60 328 / 236
+_LINEAR_COST = _ChunkCost(0.123, 0.0054, 0.045, 1.97, 0.0951, -15.7, 128)
 
 
 def _delta_in_chunks(proj: torch.Tensor, conv_w: torch.Tensor, state: torch.Tensor, ring: torch.Tensor, rows: StepRows,
