@@ -35,6 +35,9 @@
 // THN_ERR_WAIT_TIMEOUT, lets what is on its way land and returns; its results and state are then not written, those of other blocks may be.
 #pragma once
 
+#include <algorithm>
+#include <cmath>
+
 #include "common.cuh"
 
 namespace chunk {
@@ -795,6 +798,40 @@ template <typename T, int CG, int KS, Kind KIND>
 void launch_brought_walk(const WalkArgs& a, int n_seqs, cudaStream_t stream) {
     if (a.err) launch_walk<T, CG, KS, KIND, 2, true>(a, n_seqs, stream);
     else launch_walk<T, CG, KS, KIND, 2, false>(a, n_seqs, stream);
+}
+
+// What a step's walk takes in blocks of one shape, in us: a time to start; the longest sequence's chain of chunks, as often as its blocks must queue,
+// `per_sm` of them to a multiprocessor (0: any number), which is a whole number where all sequences are as long; what all chunks and sequences take
+// together, per hundred heads of 128 values; and how much of the shorter of both stays beside the longer.  The mixers' tables are fitted to measured
+// times of hundreds of steps: by pairs of sequence and head alone, single tokens beside a prompt count as much as the prompt, and blocks are too wide for its chain.
+struct WalkCost {
+    float start, chain, chunk, sequence, side;
+    int columns, per_sm;
+};
+constexpr int kMultiprocessors = 148;
+
+// The shape of the least such time, from 1 on; the first one's columns divide all values.
+template <int N>
+int cheapest_walk(const WalkCost (&costs)[N], int n_rows, int max_tokens, int n_seqs, int n_heads, int value_dim) {
+    const long long longest = (max_tokens + kTokens - 1) / kTokens;
+    const long long chunks = std::min(n_seqs * longest, n_rows / kTokens + (long long)n_seqs);      // at most
+    const double heads = (double)n_heads * value_dim / 128, together = heads * std::min((double)n_seqs, (double)n_rows / max_tokens);
+    const bool same = (long long)n_seqs * max_tokens == n_rows;
+    int best = 1;
+    double least = 0;
+    for (int i = 0; i < N; ++i) {
+        const WalkCost& c = costs[i];
+        if (value_dim % c.columns != 0) continue;
+        double waves = c.per_sm ? together * 128 / c.columns / (kMultiprocessors * c.per_sm) : 1.0;
+        waves = std::max(1.0, same ? std::ceil(waves) : waves);
+        const double chain = c.chain * longest * waves, all = (c.chunk * chunks + c.sequence * n_seqs) * heads / 100;
+        const double us = c.start + std::max(chain, all) + c.side * std::min(chain, all);
+        if (i == 0 || us < least) {
+            best = i + 1;
+            least = us;
+        }
+    }
+    return best;
 }
 
 // Whether a step's sequences are so short that the blocks' starts weigh more than their chunks: the warps then copy themselves.  us of the whole

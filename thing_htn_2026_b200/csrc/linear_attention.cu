@@ -604,6 +604,17 @@ THN_API long long thn_linear_attention_chunks_scratch_bytes(int n_rows, int n_se
     return (long long)n_heads * n_rows * 3 * (2 * chunk::kKeyRow + chunk::kScoreRow) * 2 + chunk::chunk_places(n_rows, n_seqs) * n_heads * chunk::kKeys * 4;
 }
 
+// Which blocks walk the chunks (WalkCost): 1 has 16 columns and four warps, which split the keys; 2: 32, four for a group of 16; 3: 64, two; 4: as 3, two
+// blocks on a multiprocessor with one buffer each, into which the warps copy themselves.  us of the whole call, 1 / 2 / 3 / 4, 16 heads of 128: one prompt of
+// 2,048 tokens 125 / 149 / 215 / 285, 33 tokens beside 60 single ones 153 / 109 / 90 / 78, 512 beside 60 187 / 137 / 112 / 114, 3 x 512 91 / 85 / 74 / 92, 8 x 512
+// 229 / 193 / 171 / 178; 32 heads, one prompt of 128 tokens 30 / 32 / 27 / 29.  Over 882 steps of 4 to 64 heads the chosen one takes 1.3 % longer than the best of four.
+constexpr chunk::WalkCost kWalkCosts[4] = {{2.89f, 1.30f, 7.64f, 6.67f, 0.22f, 16, 1}, {3.90f, 1.60f, 5.65f, 4.09f, 0.41f, 32, 1},
+                                           {4.55f, 2.51f, 4.77f, 2.96f, 0.50f, 64, 1}, {7.53f, 3.23f, 4.59f, 1.11f, 0.99f, 64, 2}};
+
+THN_API int thn_linear_attention_walk_shape(int n_rows, int max_tokens, int n_seqs, int n_heads, int value_dim) {
+    return chunk::cheapest_walk(kWalkCosts, n_rows, max_tokens, n_seqs, n_heads, value_dim);
+}
+
 // The recurrence of a step with gated decays chunk by chunk: bfloat16 rows as thn_linear_attention takes them (no silu), keys of
 // 128, values of whole groups of 16; v's columns start on 16-byte boundaries, q's and k's on 8-byte ones, gate and its bias on
 // 16-byte ones; max_tokens: the most rows of a sequence.  shape: 0, or which blocks walk (tests and measurement); with 16 added a brought
@@ -648,14 +659,8 @@ THN_API int thn_linear_attention_chunks(float* o, float* state, void* scratch, l
     a.cu_seqlens = cu_seqlens; a.slots = slots;
     a.n_rows = n_rows; a.n_heads = n_heads; a.heads_per_unit = 1; a.value_dim = value_dim; a.scale = q_scale;
     using T = __nv_bfloat16;
-    // Few sequences: narrow blocks, whose four warps split the keys; more: wide ones, which share a chunk's keys and queries; where blocks
-    // are many and short, two on a multiprocessor with one buffer each (4).  By the sequences that are walked at once for the longest one's time
-    // (or, with many short ones beside it, by all there are), us of the whole call with shapes 1 / 2 / 3 / 4 (the warps copying themselves): one prompt
-    // of 2,048 tokens of 16 heads 155 / 181 / 245 / 294, of 32 heads 290 / 218 / 279 / 335, 2 x 512 of 32 heads 157 / 122 / 103 / 120, 8 x 512 of 32 heads
-    // 542 / 411 / 376 / 368.
     using namespace chunk;
-    const double busy = (double)n_heads * value_dim / kKeys * std::max((double)n_rows / max_tokens, n_seqs / 30.0);
-    if (shape == 0) shape = busy <= 18 ? 1 : busy <= 48 ? 2 : busy > 100 && many_short(n_rows, n_seqs, max_tokens) ? 4 : 3;
+    if (shape == 0) shape = thn_linear_attention_walk_shape(n_rows, max_tokens, n_seqs, n_heads, value_dim);
     if (value_dim % 64 != 0) shape = std::min(shape, 2);
     if (value_dim % 32 != 0) shape = 1;
     if (shape == 4) launch_walk<T, 4, 2, kPerKey, 1, false>(a, n_seqs, stream);

@@ -25,7 +25,6 @@
 #include <math.h>
 
 #include <algorithm>
-#include <cmath>
 
 #include "chunk_walk.cuh"
 #include "common.cuh"
@@ -496,41 +495,17 @@ THN_API long long thn_mlstm_chunks_scratch_bytes(int n_rows, int n_seqs, int n_h
     return (long long)n_heads * n_rows * (3 * chunk::kScoreRow * 2 + 16) + chunk::chunk_places(n_rows, n_seqs) * n_heads * chunk::kKeys * 4;
 }
 
-// Which blocks walk the chunks: 1 has 16 columns and four warps for a group of them, which split the keys; 2: 32, four; 3: 64, two; 4: 32,
+// Which blocks walk the chunks (WalkCost): 1 has 16 columns and four warps for a group of them, which split the keys; 2: 32, four; 3: 64, two; 4: 32,
 // two; 5: 64, one.  Wide blocks share the loads of a chunk's keys and queries and its denominators, narrow ones give more blocks and shorter
-// chains.  Each is modelled as a time to start, the longest sequence's chain (as often as its blocks must queue, `per_sm` to a multiprocessor, where
-// all sequences are as long), what all chunks and sequences take together, and how much of the shorter of both stays beside the longer; fitted to 596
-// steps of 1 to 92 sequences of 1 to 2,048 tokens and 4 to 32 heads.  The chosen one takes 0.7 % longer than the best of five
+// chains.  Fitted to 596 steps of 1 to 92 sequences of 1 to 2,048 tokens and 4 to 32 heads; the chosen one takes 0.7 % longer than the best of five
 // on average (14 % at most).  us of the whole call, 1 / 2 / 3 / 4 / 5, 16 heads of 128: one prompt of 2,048 tokens 106 / 137 / 200 / 146 / 306, 128 tokens
 // beside 60 single ones 91 / 93 / 72 / 67 / 63, 4 x 1,024 152 / 146 / 113 / 116 / 167, 64 x 33 165 / 166 / 125 / 118 / 108.
-struct WalkCost {
-    float start, chain, chunk, sequence, side;       // us; chunk and sequence: a hundred heads'
-    int columns, per_sm;                             // per_sm 0: any number
-};
-constexpr WalkCost kWalkCosts[5] = {{6.34f, 1.64f, 6.92f, 2.03f, 0.42f, 16, 1}, {6.78f, 2.01f, 5.94f, 2.35f, 0.15f, 32, 0}, {6.88f, 2.81f, 4.73f, 1.46f, 0.16f, 64, 1},
-                                    {7.27f, 1.93f, 4.67f, 0.84f, 0.55f, 32, 3}, {8.80f, 5.43f, 4.04f, 0.74f, 0.22f, 64, 2}};
+constexpr chunk::WalkCost kWalkCosts[5] = {{6.34f, 1.64f, 6.92f, 2.03f, 0.42f, 16, 1}, {6.78f, 2.01f, 5.94f, 2.35f, 0.15f, 32, 0},
+                                           {6.88f, 2.81f, 4.73f, 1.46f, 0.16f, 64, 1}, {7.27f, 1.93f, 4.67f, 0.84f, 0.55f, 32, 3},
+                                           {8.80f, 5.43f, 4.04f, 0.74f, 0.22f, 64, 2}};
 
 THN_API int thn_mlstm_walk_shape(int n_rows, int max_tokens, int n_seqs, int n_heads, int value_dim) {
-    constexpr double kMultiprocessors = 148;
-    const long long longest = (max_tokens + chunk::kTokens - 1) / chunk::kTokens;
-    const long long chunks = std::min(n_seqs * longest, n_rows / chunk::kTokens + (long long)n_seqs);      // at most
-    const double heads = (double)n_heads * value_dim / chunk::kKeys, together = heads * std::min((double)n_seqs, (double)n_rows / max_tokens);
-    const bool same = (long long)n_seqs * max_tokens == n_rows;
-    int best = 1;
-    double least = 0;
-    for (int i = 0; i < 5; ++i) {
-        const WalkCost& c = kWalkCosts[i];
-        if (value_dim % c.columns != 0) continue;
-        double waves = c.per_sm ? together * chunk::kKeys / c.columns / (kMultiprocessors * c.per_sm) : 1.0;
-        waves = std::max(1.0, same ? std::ceil(waves) : waves);
-        const double chain = c.chain * longest * waves, all = (c.chunk * chunks + c.sequence * n_seqs) * heads / 100;
-        const double us = c.start + std::max(chain, all) + c.side * std::min(chain, all);
-        if (i == 0 || us < least) {
-            best = i + 1;
-            least = us;
-        }
-    }
-    return best;
+    return chunk::cheapest_walk(kWalkCosts, n_rows, max_tokens, n_seqs, n_heads, value_dim);
 }
 
 // The recurrence of a step chunk by chunk: bfloat16 rows whose q, k and v parts start on 16-byte boundaries, keys of

@@ -69,6 +69,7 @@ _SIGNATURES = {
                             c_int, c_longlong, c_float, c_int, c_void_p],
     "thn_hyper_norm": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_float,
                        c_int, c_int, c_int, c_int, c_void_p],
+    "thn_linear_attention_walk_shape": [c_int, c_int, c_int, c_int, c_int],
     "thn_linear_attention_chunks_scratch_bytes": [c_int, c_int, c_int],
     "thn_linear_attention_chunks": [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_float,
                                     c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p],
