@@ -919,6 +919,17 @@ THN_API long long thn_delta_chunks_scratch_bytes(int n_rows, int n_heads, int n_
     return 6 * n_kv * key_plane + n_heads * (3 * key_plane + 3 * score_plane + (long long)n_rows * (dv * 4 + 16 + 8));
 }
 
+// Which blocks walk the chunks (WalkCost): 1 has 16 columns and four warps, which split the keys; 2: 32, four for a group of 16; 3: 64, two; 4: as 3, the
+// warps copying themselves, which starts sooner.  us of the whole call, 1 / 2 / 3 / 4, 16 heads of 128: one prompt of 2,048 tokens 177 / 249 / 400 / 417,
+// beside 60 single ones 411 / 331 / 462 / 488, 512 tokens beside 8 81 / 79 / 117 / 121, 8 x 512 333 / 313 / 295 / 301, 64 x 33 419 / 335 / 305 / 293.  Over 882 steps of 4 to 48 heads
+// the chosen one takes 0.3 % longer than the best of four (15 % at most).
+constexpr chunk::WalkCost kWalkCosts[4] = {{9.38f, 1.94f, 13.14f, 8.99f, 0.10f, 16, 1}, {9.23f, 3.18f, 9.03f, 4.67f, 0.19f, 32, 1},
+                                           {10.35f, 5.60f, 9.37f, 3.54f, 0.15f, 64, 1}, {9.48f, 6.03f, 9.68f, 1.99f, 0.15f, 64, 1}};
+
+THN_API int thn_delta_walk_shape(int n_rows, int max_tokens, int n_seqs, int n_heads, int value_dim) {
+    return chunk::cheapest_walk(kWalkCosts, n_rows, max_tokens, n_seqs, n_heads, value_dim);
+}
+
 // prepare and recurrence of a step chunk by chunk, the state carried in float32: bfloat16 rows, four taps, keys of
 // 128, values of whole groups of 16 columns; max_tokens: the most rows of a sequence.  scratch:
 // thn_delta_chunks_scratch_bytes(...), 16-byte aligned, as the state and the taps must be; the rows and the
@@ -977,18 +988,12 @@ THN_API int thn_delta_chunks(float* o, float* state, void* scratch, long long sc
     a.w = w; a.scores = scores; a.scalars = scalars;
     a.cu_seqlens = cu_seqlens; a.slots = slots;
     a.n_rows = n_rows; a.n_heads = n_heads; a.heads_per_unit = n_heads / n_kv; a.value_dim = dv; a.scale = 1.f;
-    // More columns a block load the chunk's keys, queries and W less often, fewer give more blocks: wide blocks
-    // once they reach nearly every multiprocessor.  us of the whole call, 16 / 32 / 64 columns (the warps copying themselves): one prompt of
-    // 2,048 tokens, 16 heads 247 / 310 / 415, 32 heads 464 / 379 / 480; 8 x 512 tokens of 16 heads 427 / 375 / 316.
-    const long long pairs = (long long)n_seqs * n_heads;
     using namespace chunk;
-    if (dv % 64 == 0 && pairs * (dv / 64) >= 128) {
-        if (many_short(n_rows, n_seqs, max_tokens)) launch_walk<float, 4, 2, kDelta, 2, false>(a, n_seqs, stream);
-        else launch_brought_walk<float, 4, 2, kDelta>(a, n_seqs, stream);
-    } else if (dv % 32 == 0 && pairs * (dv / 32) >= 128) {
-        launch_brought_walk<float, 2, 4, kDelta>(a, n_seqs, stream);
-    } else {
-        launch_brought_walk<float, 1, 4, kDelta>(a, n_seqs, stream);
+    switch (thn_delta_walk_shape(n_rows, max_tokens, n_seqs, n_heads, dv)) {
+        case 4: launch_walk<float, 4, 2, kDelta, 2, false>(a, n_seqs, stream); break;
+        case 3: launch_brought_walk<float, 4, 2, kDelta>(a, n_seqs, stream); break;
+        case 2: launch_brought_walk<float, 2, 4, kDelta>(a, n_seqs, stream); break;
+        default: launch_brought_walk<float, 1, 4, kDelta>(a, n_seqs, stream);
     }
     return thn_launch_status("delta_chunks");
 }

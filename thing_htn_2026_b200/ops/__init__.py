@@ -140,6 +140,7 @@ _SIGNATURES = {
                           c_float, c_int, c_void_p],
     "thn_delta_recurrence": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                              c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p],
+    "thn_delta_walk_shape": [c_int, c_int, c_int, c_int, c_int],
     "thn_delta_chunks": [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                          c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_float,
                          c_void_p, c_void_p],
