@@ -493,6 +493,18 @@ THN_API long long thn_state_space_chunks_scratch_bytes(int n_rows, int n_heads, 
     return (long long)n_rows * (6ll * n_groups * chunk::kKeyRow * 2 + (long long)n_heads * (3 * chunk::kScoreRow * 2 + 16 + vdim * 4 + 4));
 }
 
+// Which blocks walk the chunks (WalkCost): 1 has 16 columns and four warps, which split the keys; 2: 32, four for a group of 16; 3: 64, two; 4: as 3, two
+// blocks on a multiprocessor with one buffer each, into which the warps copy themselves, where blocks are many and short.  us of the whole call, 1 / 2 / 3 / 4, 64 heads
+// of 64: one prompt of 2,048 tokens 236 / 184 / 286 / 356, beside 60 single ones 504 / 368 / 322 / 409, 512 tokens beside 8 112 / 90 / 94 / 112, 8 x 512
+// 415 / 326 / 327 / 330; 128 heads, one prompt of 2,048 tokens 449 / 347 / 319 / 393, 512 beside 60 700 / 496 / 420 / 339.  Over 588 steps of 16 to 128 heads the
+// chosen one takes 0.9 % longer than the best of four.
+constexpr chunk::WalkCost kWalkCosts[3] = {{6.63f, 1.28f, 6.59f, 0.00f, 0.17f, 16, 1}, {5.32f, 1.75f, 5.74f, 0.00f, 0.06f, 32, 1}, {5.30f, 2.86f, 4.42f, 0.31f, 0.07f, 64, 1}};
+
+THN_API int thn_state_space_walk_shape(int n_rows, int max_tokens, int n_seqs, int n_heads, int vdim) {
+    if (vdim % 64 == 0 && (long long)n_seqs * n_heads * (vdim / 64) >= 384 && chunk::many_short(n_rows, n_seqs, max_tokens)) return 4;
+    return chunk::cheapest_walk(kWalkCosts, n_rows, max_tokens, n_seqs, n_heads, vdim);
+}
+
 // thn_state_space chunk by chunk: bfloat16 rows in whole 8-byte pieces, four taps, a state of 128, vdim a multiple of 16;
 // max_tokens: the most rows of a sequence.  On B200, us against token by token: 8 x 512 tokens of 128 heads of 64 over a
 // state of 128 617 / 1,074, one prompt of 2,048 tokens of 64 heads 202 / 368, 128 tokens 42 / 44.  The error against 64 bits:
@@ -536,17 +548,12 @@ THN_API int thn_state_space_chunks(float* y, float* state, void* scratch, long l
     a.scores = scores; a.scalars = scalars;
     a.cu_seqlens = cu_seqlens; a.slots = slots;
     a.n_rows = n_rows; a.n_heads = n_heads; a.heads_per_unit = n_heads / n_groups; a.value_dim = vdim; a.scale = 1.f;
-    // us of the whole call with blocks of 64 columns and two to a multiprocessor, 64 with two buffers, 32 (the warps copying themselves): 8 x 512
-    // tokens of 128 heads 613 / 624 / 736, one prompt of 2,048 tokens of 128 heads 415 / 349 / 410, of 64 heads 372 / 306 / 220.
-    const long long pairs = (long long)n_seqs * n_heads;
     using namespace chunk;
-    if (vdim % 64 == 0 && pairs * (vdim / 64) >= 128) {
-        if (pairs * (vdim / 64) >= 384 && many_short(n_rows, n_seqs, max_tokens)) launch_walk<float, 4, 2, kPlain, 1, false>(a, n_seqs, stream);
-        else launch_brought_walk<float, 4, 2, kPlain>(a, n_seqs, stream);
-    } else if (vdim % 32 == 0) {
-        launch_brought_walk<float, 2, 4, kPlain>(a, n_seqs, stream);
-    } else {
-        launch_brought_walk<float, 1, 4, kPlain>(a, n_seqs, stream);
+    switch (thn_state_space_walk_shape(n_rows, max_tokens, n_seqs, n_heads, vdim)) {
+        case 4: launch_walk<float, 4, 2, kPlain, 1, false>(a, n_seqs, stream); break;
+        case 3: launch_brought_walk<float, 4, 2, kPlain>(a, n_seqs, stream); break;
+        case 2: launch_brought_walk<float, 2, 4, kPlain>(a, n_seqs, stream); break;
+        default: launch_brought_walk<float, 1, 4, kPlain>(a, n_seqs, stream);
     }
     return thn_launch_status("state_space_chunks");
 }
