@@ -493,6 +493,11 @@ THN_API long long thn_state_space_chunks_scratch_bytes(int n_rows, int n_heads, 
     return (long long)n_rows * (6ll * n_groups * chunk::kKeyRow * 2 + (long long)n_heads * (3 * chunk::kScoreRow * 2 + 16 + vdim * 4 + 4));
 }
 
+// Whether a step's blocks are so many and short that their starts weigh more than their chunks: they then copy themselves, two to a multiprocessor.  us of
+// the whole call, such blocks / the same columns brought, 64 heads of 64: 32 x 128 tokens 314 / 332, 128 beside 60 single ones 164 / 207, 512 beside 60 187 / 229,
+// 12 x 300 312 / 310, 2,048 beside 60 409 / 322.
+inline bool many_short(int n_rows, int n_seqs, int max_tokens) { return n_rows < 200ll * n_seqs && max_tokens < 1024; }
+
 // Which blocks walk the chunks (WalkCost): 1 has 16 columns and four warps, which split the keys; 2: 32, four for a group of 16; 3: 64, two; 4: as 3, two
 // blocks on a multiprocessor with one buffer each, into which the warps copy themselves, where blocks are many and short.  us of the whole call, 1 / 2 / 3 / 4, 64 heads
 // of 64: one prompt of 2,048 tokens 236 / 184 / 286 / 356, beside 60 single ones 504 / 368 / 322 / 409, 512 tokens beside 8 112 / 90 / 94 / 112, 8 x 512
@@ -501,7 +506,7 @@ THN_API long long thn_state_space_chunks_scratch_bytes(int n_rows, int n_heads, 
 constexpr chunk::WalkCost kWalkCosts[3] = {{6.63f, 1.28f, 6.59f, 0.00f, 0.17f, 16, 1}, {5.32f, 1.75f, 5.74f, 0.00f, 0.06f, 32, 1}, {5.30f, 2.86f, 4.42f, 0.31f, 0.07f, 64, 1}};
 
 THN_API int thn_state_space_walk_shape(int n_rows, int max_tokens, int n_seqs, int n_heads, int vdim) {
-    if (vdim % 64 == 0 && (long long)n_seqs * n_heads * (vdim / 64) >= 384 && chunk::many_short(n_rows, n_seqs, max_tokens)) return 4;
+    if (vdim % 64 == 0 && (long long)n_seqs * n_heads * (vdim / 64) >= 384 && many_short(n_rows, n_seqs, max_tokens)) return 4;
     return chunk::cheapest_walk(kWalkCosts, n_rows, max_tokens, n_seqs, n_heads, vdim);
 }
 
