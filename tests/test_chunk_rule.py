@@ -36,16 +36,17 @@ def test_long_prompts_alone_are_walked_in_chunks(name):
                 rows = SimpleNamespace(max_q_len=tokens, n_rows=tokens * prompts, n_seqs=prompts)
                 assert getattr(ops, name).chunks_pay(rows, heads, getattr(ops, name).size), (tokens, prompts, heads)
 
+
 # the same with the kernels of today, in a graph (launched one by one, the short ones are as long as the host's work)
-DELTA_IN_GRAPH = [((16, 0, 1), 52, 28), ((16, 8, 1), 57, 37), ((16, 60, 1), 78, 143), ((33, 8, 1), 64, 45), ((33, 60, 1), 88, 147),
-                  ((128, 0, 1), 84, 32), ((128, 8, 1), 100, 50), ((128, 60, 1), 123, 151), ((512, 8, 1), 252, 120), ((512, 60, 1), 294, 186),
-                  ((2048, 0, 1), 658, 177), ((2048, 60, 1), 940, 461), ((16, 0, 8), 66, 39), ((16, 0, 64), 175, 168), ((33, 0, 64), 284, 292),
+DELTA_IN_GRAPH = [((16, 0, 1), 52, 27), ((16, 8, 1), 57, 37), ((16, 60, 1), 78, 143), ((33, 8, 1), 64, 45), ((33, 60, 1), 88, 146),
+                  ((128, 0, 1), 84, 32), ((128, 8, 1), 100, 50), ((128, 60, 1), 123, 150), ((512, 8, 1), 255, 78), ((512, 60, 1), 290, 184),
+                  ((2048, 0, 1), 658, 177), ((2048, 60, 1), 971, 330), ((16, 0, 8), 66, 39), ((16, 0, 64), 174, 168), ((33, 0, 64), 284, 293),
                   ((128, 0, 32), 520, 300)]
-MLSTM_IN_GRAPH = [((16, 0, 1), 10, 8), ((16, 8, 1), 16, 17), ((16, 60, 1), 41, 60), ((33, 0, 1), 16, 10), ((33, 8, 1), 27, 20), ((33, 60, 1), 50, 60),
-                  ((128, 0, 1), 51, 14), ((128, 60, 1), 108, 62), ((512, 60, 1), 337, 91), ((2048, 60, 1), 1320, 210), ((16, 0, 8), 27, 16),
+MLSTM_IN_GRAPH = [((16, 0, 1), 10, 8), ((16, 8, 1), 16, 17), ((16, 60, 1), 40, 60), ((33, 0, 1), 16, 10), ((33, 8, 1), 26, 19), ((33, 60, 1), 50, 60),
+                  ((128, 0, 1), 51, 14), ((128, 60, 1), 103, 62), ((512, 60, 1), 345, 91), ((2048, 60, 1), 1292, 210), ((16, 0, 8), 27, 16),
                   ((16, 0, 64), 158, 66), ((33, 0, 64), 314, 108), ((128, 0, 32), 585, 113)]
-SPACE_IN_GRAPH = [((128, 0, 1), 32, 34), ((128, 8, 1), 41, 51), ((128, 60, 1), 97, 165), ((512, 0, 1), 93, 67), ((512, 8, 1), 128, 112),
-                  ((512, 60, 1), 139, 187), ((2048, 0, 1), 349, 184), ((2048, 8, 1), 493, 290), ((2048, 60, 1), 494, 322), ((128, 0, 32), 541, 314)]
+SPACE_IN_GRAPH = [((128, 0, 1), 32, 34), ((128, 8, 1), 41, 51), ((128, 60, 1), 97, 164), ((512, 0, 1), 93, 66), ((512, 8, 1), 129, 112),
+                  ((512, 60, 1), 139, 187), ((2048, 0, 1), 349, 184), ((2048, 8, 1), 493, 194), ((2048, 60, 1), 495, 321), ((128, 0, 32), 540, 313)]
 IN_GRAPH = [("_DELTA_COST", 16, 128, *m) for m in DELTA_IN_GRAPH] + [("_MLSTM_COST", 16, 128, *m) for m in MLSTM_IN_GRAPH] \
     + [("_SPACE_COST", 64, 64, *m) for m in SPACE_IN_GRAPH]
 

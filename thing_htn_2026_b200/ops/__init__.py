@@ -1439,18 +1439,18 @@ class _ChunkCost(NamedTuple):
 
 
 # Measured on B200, token by token / in chunks, us of the whole call in a graph; "a + b": a prompt of a tokens, or several, beside b single ones.
-#   delta rule, 16 heads of 128: 16 + 0 52 / 28, 16 + 8 57 / 37, 16 + 60 78 / 143, 128 + 8 100 / 50, 128 + 60 123 / 151, 512 + 60 294 / 186,
-#     2,048 + 0 658 / 177, 2,048 + 60 940 / 461, 33 + 0 (64 prompts) 284 / 292, 128 + 0 (32 prompts) 520 / 300
+#   delta rule, 16 heads of 128: 16 + 0 52 / 27, 16 + 8 57 / 37, 16 + 60 78 / 143, 128 + 8 100 / 50, 128 + 60 123 / 150, 512 + 60 290 / 184,
+#     2,048 + 0 658 / 177, 2,048 + 60 971 / 330, 33 + 0 (64 prompts) 284 / 293, 128 + 0 (32 prompts) 520 / 300
 _DELTA_COST = _ChunkCost(0.451, 0.0059, 0.0225, 3.0, 0.1152, 12.0, 128)
-#   matrix memory, 16 heads of 128: 16 + 0 10 / 8, 16 + 8 16 / 17, 16 + 60 41 / 60, 33 + 60 50 / 60, 128 + 60 108 / 62,
-#     2,048 + 60 1,320 / 210, 16 + 0 (64 prompts) 158 / 66
+#   matrix memory, 16 heads of 128: 16 + 0 10 / 8, 16 + 8 16 / 17, 16 + 60 40 / 60, 33 + 60 50 / 60, 128 + 60 103 / 62,
+#     2,048 + 60 1,292 / 210, 16 + 0 (64 prompts) 158 / 66
 _MLSTM_COST = _ChunkCost(0.5, 0.009, 0.03, 1.8, 0.055, 0.0, 128)
-#   state-space duality, 64 heads of 64: 128 + 0 32 / 34, 128 + 8 41 / 51, 128 + 60 97 / 165, 512 + 8 128 / 112, 512 + 60 139 / 187,
-#     2,048 + 0 349 / 184, 2,048 + 60 494 / 322, 128 + 0 (32 prompts) 541 / 314
+#   state-space duality, 64 heads of 64: 128 + 0 32 / 34, 128 + 8 41 / 51, 128 + 60 97 / 164, 512 + 8 129 / 112, 512 + 60 139 / 187,
+#     2,048 + 0 349 / 184, 2,048 + 60 495 / 321, 128 + 0 (32 prompts) 540 / 313
 _SPACE_COST = _ChunkCost(0.205, 0.0021, 0.016, 3.1, 0.035, -10.0, 64)
-#   linear attention with gated decays, 32 heads of 128: 16 + 0 7 / 16, 64 + 0 15 / 23, 128 + 0 26 / 33, 300 + 0 55 / 44, 16 + 60 97 / 146, 512 + 60 174 / 212,
-#     2,048 + 0 358 / 184, 2,048 + 60 410 / 402, 16 + 0 (64 prompts) 238 / 176; 16 heads: 128 + 0 19 / 24, 300 + 0 40 / 38, 2,048 + 0 255 / 125,
-#     512 + 60 93 / 137, 2,048 + 60 328 / 236
+#   linear attention with gated decays, 32 heads of 128: 16 + 0 7 / 16, 64 + 0 15 / 23, 128 + 0 26 / 33, 300 + 0 55 / 44, 16 + 60 97 / 146, 512 + 60 174 / 183,
+#     2,048 + 0 358 / 184, 2,048 + 60 409 / 400, 16 + 0 (64 prompts) 238 / 176; 16 heads: 128 + 0 19 / 24, 300 + 0 40 / 38, 2,048 + 0 255 / 125,
+#     512 + 60 93 / 111, 2,048 + 60 327 / 235
 _LINEAR_COST = _ChunkCost(0.123, 0.0054, 0.045, 1.97, 0.0951, -15.7, 128)
 
 
