@@ -66,7 +66,8 @@ def test_a_part_gives_the_same_on_both_sides(kind, monkeypatch):
         grouped = part.forward(x, ctx)
         assert len(calls) == 1
         part.forward(x, SimpleNamespace(err=None))          # no word for the kernels' waits: the dense form
+        short = part.forward(x[:300], ctx)                   # the same rows in a step of fewer: the dense form
     assert len(calls) == 1 and int(ctx.err.item()) == 0
     # each side rounds the activations and the result (1.6e-3 from 64 bits), the dense one gates and ups too (1.6e-3 more)
     assert float((dense.double() - grouped.double()).norm() / dense.double().norm()) < 8e-3
-
+    assert float((short.double() - grouped[:300].double()).norm() / short.double().norm()) < 8e-3

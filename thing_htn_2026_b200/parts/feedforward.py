@@ -14,9 +14,11 @@ output is weighted by ``s * scale`` (not renormalised).  With ``shared_ff`` a sh
 the same form runs for every token and is added, multiplied by ``logistic(shared_gate(x))`` (one
 number per token; ``shared_gated`` False: added as it is).  The up-projections of all experts are
 one product, the activation carries the routing weights (zero for an expert that was not chosen),
-and one down-projection over all experts' columns sums the chosen ones: the result does not
-depend on the other rows of the step.  With many rows the chosen experts are multiplied alone, over the rows sorted by
-expert (``ops.experts_in_groups``; in a step that has an error word for those kernels' bounded waits).  Kernels: csrc/moe.cu, csrc/moe_grouped.cu.
+and one down-projection over all experts' columns sums the chosen ones.  With many rows the chosen experts are
+multiplied alone, over the rows sorted by expert (``ops.experts_in_groups``; in a step that has an error word for those
+kernels' bounded waits).  In either form a row's result comes from that row alone; but which form it is depends on
+how many rows the step has, and the dense one rounds gates and ups to the activation type where the other
+keeps float32: the same row in a short and in a long step differs by these roundings.  Kernels: csrc/moe.cu, csrc/moe_grouped.cu.
 
 ``polynorm``: ``down(act(up(x)))`` with ``act(z) = a N(z) + b N(z^2) + c N(z^3) + e``, powers
 taken entry by entry and ``N`` the division of a token's vector by its root mean square (``eps``
