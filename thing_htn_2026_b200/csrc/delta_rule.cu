@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(128) delta_prepare_chunks_kernel(
 // its own entry of U is NaN.
 // Bound by the products (1,152 a head of m16n8k16 in its own block, 864 in one of two) and by what it writes: a fragment stored as it lies is
 // 16 bytes a row, so W goes out through shared memory, over the queries and keys, by bulk copies.  2,048 tokens of 16 heads on B200: 57 us with a
-// block per head and fragments stored one by one (of 30,000 clocks a block the products q k^T and k k^T took 5,500, W and U 9,000 each), 37 now.
+// block per head and fragments stored one by one, 37 now (issue slots 37 % busy, shared memory 24 %, tensor pipe 22 %).
 constexpr int kSquare = chunk::kTokens + 8;            // row of a 32 x 32 matrix of floats
 constexpr int kDotRow = chunk::kTokens + 4;
 constexpr int kValueRow = 128 + 4;
@@ -933,12 +933,12 @@ THN_API int thn_delta_walk_shape(int n_rows, int max_tokens, int n_seqs, int n_h
 // prepare and recurrence of a step chunk by chunk, the state carried in float32: bfloat16 rows, four taps, keys of
 // 128, values of whole groups of 16 columns; max_tokens: the most rows of a sequence.  scratch:
 // thn_delta_chunks_scratch_bytes(...), 16-byte aligned, as the state and the taps must be; the rows and the
-// ring are read in pieces of 8 bytes.  One prompt of 2,048 tokens, 16 heads of 128 x 128, on B200: 187 us
-// against 658 token by token; 32 heads 308 / 839; 8 x 512 tokens of 16 heads 298 / 571; steps of long and short sequences beside
+// ring are read in pieces of 8 bytes.  One prompt of 2,048 tokens, 16 heads of 128 x 128, on B200: 177 us
+// against 658 token by token; 32 heads 301 / 935; 8 x 512 tokens of 16 heads 296 / 587; steps of long and short sequences beside
 // the rule in ops (_DELTA_COST).  The read-out's error
 // against 64 bits is 1.37e-7 to 1.41e-7 (1.33e-7 to 1.36e-7 token by token), the state's 1.2e-7 to 1.4e-7 (1.1e-7 to 1.3e-7).
-THN_API int thn_delta_chunks(float* o, float* state, void* scratch, long long scratch_bytes, const void* proj, const float* conv_w, const float* a_log,
-                             const float* dt_bias, const void* ring, const int* row_slot, const int* row_pos, const int* seq_lens,
+THN_API int thn_delta_chunks(float* o, float* state, void* scratch, long long scratch_bytes, const void* proj, const float* conv_w,
+                             const float* a_log, const float* dt_bias, const void* ring, const int* row_slot, const int* row_pos, const int* seq_lens,
                              const int* cu_seqlens, const int* slots, int n_rows, int max_tokens, int n_seqs, int n_heads, int n_kv,
                              int dk, int dv, int taps, int proj_width, float unit_eps, int* err, cudaStream_t stream) {
     DeltaShape s{n_heads, n_kv, dk, dv, taps, proj_width};

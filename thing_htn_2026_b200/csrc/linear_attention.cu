@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(256) linear_attention_prepare_vec_kernel(
 // Bound by its 60 KB of planes a chunk and by issue: the decays' logarithms and exponentials, and the 528 pairs of tokens by 128
 // channels, which are taken two channels an instruction.  (A key a thread loaded its queries and decays from shared memory twice as often.)  The
 // sums over the channels of eight tokens are taken together, by halving (seven exchanges for eight sums).  Six blocks on a multiprocessor: 1,531
-// tokens of 32 heads on B200 56 us (five, in three waves: 63; a key a thread: 66).  The whole call 153 us, token by token 278.  The error against 64 bits is the
+// tokens of 32 heads on B200 56 us (five, in three waves: 63; a key a thread: 66).  The whole call for 1,024 tokens 97 us, token by token 181.  The error against 64 bits is the
 // same: read-out 7.4e-7 over 300 tokens, 1.63e-6 over 2,000 (token by token 7.4e-7, 1.66e-6), state 1.09e-6 and 1.75e-6 (1.08e-6, 1.78e-6).
 constexpr int kChunkThreads = 128, kChunkParts = 8;
 
@@ -619,8 +619,8 @@ THN_API int thn_linear_attention_walk_shape(int n_rows, int max_tokens, int n_se
 // 128, values of whole groups of 16; v's columns start on 16-byte boundaries, q's and k's on 8-byte ones, gate and its bias on
 // 16-byte ones; max_tokens: the most rows of a sequence.  shape: 0, or which blocks walk (tests and measurement); with 16 added a brought
 // walk brings nothing, so that its wait runs out (for the test of the wait only).
-THN_API int thn_linear_attention_chunks(float* o, float* state, void* scratch, long long scratch_bytes, const void* proj, int proj_width, int q_offset, int k_offset,
-                                        int v_offset, const float* gate, int gate_width, const float* gate_bias, float tau,
+THN_API int thn_linear_attention_chunks(float* o, float* state, void* scratch, long long scratch_bytes, const void* proj, int proj_width,
+                                        int q_offset, int k_offset, int v_offset, const float* gate, int gate_width, const float* gate_bias, float tau,
                                         const int* cu_seqlens, const int* slots, int n_rows, int max_tokens, int n_seqs, int n_heads,
                                         int key_dim, int value_dim, float q_scale, int shape, int* err, cudaStream_t stream) {
     THN_CHECK_ARG(n_seqs >= 0 && n_heads > 0 && gate != nullptr && tau > 0.f && gate_width >= n_heads * key_dim, "linear_attention_chunks: bad sizes");

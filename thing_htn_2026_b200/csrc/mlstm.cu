@@ -511,10 +511,10 @@ THN_API int thn_mlstm_walk_shape(int n_rows, int max_tokens, int n_seqs, int n_h
 // The recurrence of a step chunk by chunk: bfloat16 rows whose q, k and v parts start on 16-byte boundaries, keys of
 // 128, values of whole groups of 16 columns; max_tokens: the most rows of a sequence; gate_pre as the
 // pre-activations of thn_mlstm_gates.  16 heads of 128 x 128 on B200, us against token by token: one prompt of 2,048
-// tokens 118 / 767, four of up to 1,000 tokens 99 / 730, 8 x 512 tokens 122 / 652, 64 tokens 17 / 36.  The error
+// tokens 106 / 756, four of 256 to 2,048 tokens 144 / 1,471, 8 x 512 tokens 108 / 640, 64 tokens 10 / 28.  The error
 // against 64 bits is no larger: a median row's 1.7e-7 to 2.3e-7 (2.0e-7 to 2.9e-7), the state's 1.9e-7 to 3.0e-7 (2.8e-7 to 5.2e-7).
-THN_API int thn_mlstm_chunks(float* o, float* S, float* nm, void* scratch, long long scratch_bytes, const void* proj, int proj_width, const float* gate_pre,
-                             const float* bias_i, const float* bias_f, float cap, const int* cu_seqlens, const int* slots, int n_rows,
+THN_API int thn_mlstm_chunks(float* o, float* S, float* nm, void* scratch, long long scratch_bytes, const void* proj, int proj_width,
+                             const float* gate_pre, const float* bias_i, const float* bias_f, float cap, const int* cu_seqlens, const int* slots, int n_rows,
                              int max_tokens, int n_seqs, int n_heads, int key_dim, int value_dim, float q_scale, float floor_,
                              cudaStream_t stream) {
     THN_CHECK_ARG(n_seqs >= 0 && n_heads > 0 && cap > 0.f && proj_width >= n_heads * (2 * key_dim + value_dim), "mlstm_chunks: bad sizes");

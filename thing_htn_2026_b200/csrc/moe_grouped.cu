@@ -25,8 +25,8 @@
 // The rows of a pair's tile do not touch one another: a row's result depends on its own entries alone.
 //
 // B200, 2,048 rows of 2,048, eight experts of 1,024 of which two are chosen, a shared one, gated: sort 6 us, gather 5, up-projections 56 (51 GFLOP: 0.92
-// PFLOP/s; 196 tiles are 2.6 a pair, and the last one's epilogue stands alone), down-projections 27 and 20; the layer 122 to 127 us, 205 in the
-// dense form.  Sixteen epilogue warps: with eight the up-projections took 62 us.
+// PFLOP/s; 196 tiles are 2.6 a pair, and the last one's epilogue stands alone), down-projections 27 and 20; the layer 125 us, 207 in the
+// dense form.  The up-projections keep the tensor pipe 50 % busy, the L2 cache 32 % and the issue slots 34 %: what is left is the tail.  Sixteen epilogue warps: with eight the up-projections took 62 us.
 //
 // Every wait on an mbarrier is bounded: after kWaitLimitNs by the global timer the waiter sets
 // THN_ERR_WAIT_TIMEOUT in the caller's error word and goes on to the common exit, where

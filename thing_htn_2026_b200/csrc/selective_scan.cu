@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(kScanThreads) selective_scan_kernel(
 // memory for the other warps to add.  One barrier per stage, two buffers of everything.
 // Either side is a chain of latencies: with four helping warps and the walk a token at a time, one prompt of 2,048 tokens and 4,096 channels
 // took 141 us, the helpers alone 134, the walk alone 107.  The walk takes GROUP tokens' loads and exponentials ahead of their chain
-// through the state, the helpers are twice as many: 118.  What bounds it now is shared memory (three quarters of its cycles) and issue.  B200,
+// through the state, the helpers are twice as many: 118.  What bounds it now is shared memory (69 % of its cycles) and issue.  B200,
 // against the kernel above, us: one prompt of 2,048 tokens, 4,096 channels 118 / 763, 8,192 channels 165 / 770; 8 x 512
 // tokens of 4,096 153 / 447; 100 tokens 13 / 46.  (One set of warps for everything took 211 for the first; cutting
 // the tokens into segments that run side by side doubles the exponentials; step sizes once instead of twice in shared memory 124; loads

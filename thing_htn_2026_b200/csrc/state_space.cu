@@ -512,10 +512,10 @@ THN_API int thn_state_space_walk_shape(int n_rows, int max_tokens, int n_seqs, i
 
 // thn_state_space chunk by chunk: bfloat16 rows in whole 8-byte pieces, four taps, a state of 128, vdim a multiple of 16;
 // max_tokens: the most rows of a sequence.  On B200, us against token by token: 8 x 512 tokens of 128 heads of 64 over a
-// state of 128 617 / 1,074, one prompt of 2,048 tokens of 64 heads 202 / 368, 128 tokens 42 / 44.  The error against 64 bits:
+// state of 128 582 / 1,067, one prompt of 2,048 tokens of 64 heads 184 / 348, 128 tokens 34 / 32.  The error against 64 bits:
 // y 1.2e-7 (1.2e-7 to 1.3e-7), the state 1.1e-7 (1.2e-7).
-THN_API int thn_state_space_chunks(float* y, float* state, void* scratch, long long scratch_bytes, const void* proj, int proj_width, int offset,
-                                   const float* conv_w, const float* conv_b, const void* ring, const float* dt_pre,
+THN_API int thn_state_space_chunks(float* y, float* state, void* scratch, long long scratch_bytes, const void* proj, int proj_width,
+                                   int offset, const float* conv_w, const float* conv_b, const void* ring, const float* dt_pre,
                                    const float* dt_bias, const float* rate, const float* skip, const int* row_slot, const int* row_pos,
                                    const int* seq_lens, const int* cu_seqlens, const int* slots, int n_rows, int max_tokens, int n_seqs,
                                    int n_heads, int vdim, int n_state, int n_groups, int taps, int* err, cudaStream_t stream) {
