@@ -420,7 +420,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) pair_ge
                         const float before = scales_input ? w : 1.0f, after = scales_input ? 1.0f : w;
                         const float g = fminf(before * (ups ? other : v[j]), lim);
                         const float u = fminf(fmaxf(before * (ups ? v[16 + j] : other), -lim), lim);
-                        y[j] = g / (1.0f + expf(-a.alpha * g)) * (u + a.up_shift) * after;
+                        y[j] = __fdividef(g, 1.0f + expf(-a.alpha * g)) * (u + a.up_shift) * after;
                         if (w == 0.f && !t.shared) y[j] = 0.f;
                     }
                     __nv_bfloat16* out = (t.shared ? a.shared_out : static_cast<__nv_bfloat16*>(a.out)) + (long long)(t.row0 + from) * features + feature;
