@@ -420,6 +420,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1) pair_ge
                         const float before = scales_input ? w : 1.0f, after = scales_input ? 1.0f : w;
                         const float g = fminf(before * (ups ? other : v[j]), lim);
                         const float u = fminf(fmaxf(before * (ups ? v[16 + j] : other), -lim), lim);
+                        // (The fast division is off by up to two units in the last place of float32, 2^-15 of the rounding to bfloat16 that follows; the
+                        // layer's error against 64 bits is 2.3e-3 with either.  The exact one, whose slow path every lane may take, costs the layer 2 to 5 %: 16
+                        // experts of 1,024 over 2,048, 512 rows 75 / 78 us, 8 of 2,048 over 4,096, 2,048 rows 318 / 333.)
                         y[j] = __fdividef(g, 1.0f + expf(-a.alpha * g)) * (u + a.up_shift) * after;
                         if (w == 0.f && !t.shared) y[j] = 0.f;
                     }
