@@ -27,7 +27,9 @@ MEASURED = [((2048, 8, 2, 1024, 1024), True, 640, 70, 77), ((2048, 8, 2, 1024, 1
             ((2048, 64, 6, 512, 512), True, 192, 115, 126), ((2048, 64, 6, 512, 512), True, 256, 135, 125), ((2048, 64, 6, 512, 512), False, 288, 109, 113),
             ((2048, 16, 4, 1024, 0), True, 448, 98, 74), ((4096, 64, 8, 256, 0), True, 256, 119, 138), ((4096, 64, 8, 256, 0), True, 384, 140, 153),
             ((4096, 64, 8, 256, 0), True, 640, 210, 180), ((4096, 16, 1, 2048, 0), True, 256, 209, 181), ((2048, 128, 8, 256, 256), True, 288, 130, 144),
-            ((2048, 128, 8, 256, 256), True, 448, 179, 153), ((7168, 32, 8, 512, 512), True, 352, 219, 267), ((7168, 32, 8, 512, 512), True, 576, 341, 273)]
+            ((2048, 128, 8, 256, 256), True, 448, 179, 153), ((7168, 32, 8, 512, 512), True, 352, 219, 267), ((7168, 32, 8, 512, 512), True, 576, 341, 273),
+            ((4096, 8, 2, 2048, 0), True, 256, 112, 101), ((2048, 16, 4, 1024, 0), True, 416, 91, 71), ((7168, 32, 8, 512, 0), True, 320, 201, 222),
+            ((4096, 16, 2, 1024, 1024), True, 288, 116, 125), ((4096, 16, 2, 1024, 1024), True, 352, 137, 120), ((4096, 16, 2, 2048, 0), False, 256, 145, 129)]
 
 
 @pytest.mark.parametrize("sizes,gated,rows,dense,grouped", MEASURED)
