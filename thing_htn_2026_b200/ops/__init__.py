@@ -1753,7 +1753,7 @@ def experts_in_groups(x: torch.Tensor, n_experts: int, top: int, ff: int, shared
     """Whether ``grouped_experts`` takes these sizes and is the faster form."""
     rows, hidden = x.shape
     saved = (6.0 if gated else 4.0) * rows * (n_experts - top) * ff * hidden
-    left_out = (n_experts - top) * ff / (top + 6 * shared_ff / ff)
+    left_out = (n_experts - top) * ff / (top + 6 * shared_ff / max(1, ff))
     worth = rows >= GROUPED_ANY_ROWS[gated] or (rows >= GROUPED_MIN_ROWS and left_out >= GROUPED_MIN_LEFT_OUT) \
         or (rows >= GROUPED_SOME_ROWS and left_out >= GROUPED_SOME_LEFT_OUT and ff >= GROUPED_SOME_FF)
     return (x.dtype == torch.bfloat16 and worth and saved >= GROUPED_MIN_SAVED[gated] and rows * top <= 1 << 30
