@@ -37,7 +37,7 @@ def test_the_faster_form_is_taken(sizes, gated, rows, dense, grouped):
     from thing_htn_2026_b200 import ops
     hidden, n_experts, top, ff, shared_ff = sizes
     taken = grouped if ops.experts_in_groups(torch.empty(rows, hidden, dtype=torch.bfloat16), n_experts, top, ff, shared_ff, gated) else dense
-    assert taken <= 1.02 * min(dense, grouped)
+    assert taken <= 1.03 * min(dense, grouped)          # (nearer, the grouped form is taken: it rounds less)
 
 
 @pytest.mark.gpu

@@ -1735,16 +1735,15 @@ def routed_gelu(u: torch.Tensor, routing: Routing, ff: int, shared_ff: int,
 
 # Where the chosen experts are multiplied alone: where leaving the others out saves enough operations.  With few rows the library waits for the weights for most of
 # its time whatever it multiplies, the groups' tiles are half empty, and their partial sums (12 bytes a column of a row's every choice) weigh: there only where many columns
-# are left out for each choice, a shared expert counting as six of them.  (B200, grouped / dense in us, cold weights, gated unless said.  8 experts of 1,024 over 2,048, top 2, a
+# are left out for each choice (below 320 rows a shared expert counts as six of them).  (B200, grouped / dense in us, cold weights, gated unless said.  8 experts of 1,024 over 2,048, top 2, a
 # shared one: 768 rows 78 / 77, 1,024 82 / 95, 2,048 123 / 175, 3,072 168 / 257; gelu: 1,536 93 / 98, 2,048 104 / 126.  8 of 2,048 over 4,096, top 2, a shared one: 288
 # rows 145 / 126, 384 153 / 149, 448 150 / 177, 2,048 339 / 610; none shared: 256 101 / 112, 384 107 / 133; gelu: 512 131 / 128, 640 146 / 154.  64 of 512 over 2,048, top 6, a shared one:
 # 192 rows 126 / 115, 256 125 / 135, 2,048 222 / 621; gelu: 288 113 / 109, 448 119 / 145.  16 of 2,048 over 4,096, top 1: 256 rows 181 / 209.  64 of 256 over 4,096, top 8: 256
 # rows 138 / 119, 384 153 / 140, 448 160 / 165.  32 over 4,096, top 8, of 1,024: 256 rows 195 / 215.  32 of 512 over 7,168, top 8: 320 rows 222 / 201, 448 242 / 262.  16 of 1,024 over
 # 4,096, top 2, a shared one: 288 rows 125 / 116, 352 120 / 137.)
 GROUPED_MIN_SAVED = {True: 60e9, False: 100e9}       # operations; gated, gelu
-GROUPED_ANY_ROWS = {True: 400, False: 640}
-GROUPED_MIN_ROWS, GROUPED_MIN_LEFT_OUT = 256, 2300   # with fewer: rows, and columns left out for each choice
-GROUPED_SOME_ROWS, GROUPED_SOME_LEFT_OUT, GROUPED_SOME_FF = 320, 1700, 512      # or these, and columns of an expert
+GROUPED_ANY_ROWS = {True: 448, False: 640}
+GROUPED_MIN_ROWS, GROUPED_SOME_ROWS, GROUPED_LEFT_OUT, GROUPED_FF = 256, 320, 2300, 384      # with fewer: see below
 GROUPED_SCRATCH = 1 << 30    # bytes of scratch that a call takes if the dense form would take less
 GROUPED_SKIP_LOADS = 0       # the test of the products' bounded waits sets it: nothing is loaded
 
@@ -1753,9 +1752,10 @@ def experts_in_groups(x: torch.Tensor, n_experts: int, top: int, ff: int, shared
     """Whether ``grouped_experts`` takes these sizes and is the faster form."""
     rows, hidden = x.shape
     saved = (6.0 if gated else 4.0) * rows * (n_experts - top) * ff * hidden
-    left_out = (n_experts - top) * ff / (top + 6 * shared_ff / max(1, ff))
-    worth = rows >= GROUPED_ANY_ROWS[gated] or (rows >= GROUPED_MIN_ROWS and left_out >= GROUPED_MIN_LEFT_OUT) \
-        or (rows >= GROUPED_SOME_ROWS and left_out >= GROUPED_SOME_LEFT_OUT and ff >= GROUPED_SOME_FF)
+    left_out = (n_experts - top) * ff
+    worth = rows >= GROUPED_ANY_ROWS[gated] \
+        or (rows >= GROUPED_SOME_ROWS and left_out >= GROUPED_LEFT_OUT * top and ff >= GROUPED_FF) \
+        or (rows >= GROUPED_MIN_ROWS and left_out >= GROUPED_LEFT_OUT * (top + 6 * shared_ff / max(1, ff)))
     return (x.dtype == torch.bfloat16 and worth and saved >= GROUPED_MIN_SAVED[gated] and rows * top <= 1 << 30
             and x.data_ptr() % 16 == 0 and bool(lib().thn_moe_grouped_supported(hidden, n_experts, ff, shared_ff)))
 
